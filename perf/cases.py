@@ -225,6 +225,116 @@ def run(s):
 
 
 # ---------------------------------------------------------------------------------------------
+# the same in 64 bits
+# ---------------------------------------------------------------------------------------------
+def _exact_head(near, far, v, do, w, causal, aux):
+    """One head in float64: (o, lse, total, near gradients, far gradients, dv).  `near` and `far` are (q, k) pairs, `far`
+    None for plain attention; query rows are taken 2048 at a time, and `v` may carry no gradient (do None)."""
+    M, N, D = near[0].shape[0], near[1].shape[0], v.shape[1]
+    pairs = [near] if far is None else [near, far]
+    cols = torch.arange(N, device=v.device)
+    outs, lses, total = [], [], torch.zeros(N, dtype=torch.float64, device=v.device)
+    dqs, dks, dv = [[] for _ in pairs], [torch.zeros_like(k) for _, k in pairs], torch.zeros_like(v)
+    for a in range(0, M, 2048):
+        b = min(M, a + 2048)
+        at = torch.arange(a, b, device=v.device)[:, None] + (N - M)
+        n = min(N, b + N - M) if causal else N        # later keys are seen by none of these rows
+        s = near[0][a:b] @ near[1][:n].T
+        is_far = (at - cols[:n]) >= w
+        if far is not None:
+            s = torch.where(is_far, far[0][a:b] @ far[1][:n].T, s)
+        s *= D ** -0.5
+        if causal:
+            s.masked_fill_(cols[:n] > at, -math.inf)
+        lse = torch.logsumexp(s, 1, keepdim=True)
+        p = torch.exp_(s - lse)
+        del s
+        o = p @ v[:n]
+        outs.append(o)
+        lses.append(lse.squeeze(1))
+        if aux:
+            total[:n] += p.sum(0)
+        if do is None:
+            continue
+        dv[:n] += p.T @ do[a:b]
+        ds = do[a:b] @ v[:n].T
+        ds -= (do[a:b] * o).sum(1, keepdim=True)
+        ds *= p
+        ds *= D ** -0.5
+        del p
+        for i, (q, k) in enumerate(pairs):
+            d = ds if far is None else ds.masked_fill(is_far if i == 0 else ~is_far, 0.0)
+            dqs[i].append(d @ k[:n])
+            dks[i][:n] += d.T @ q[a:b]
+    grads = [(torch.cat(dq), dk) for dq, dk in zip(dqs, dks)] if do is not None else None
+    return torch.cat(outs), torch.cat(lses), total, grads, dv
+
+
+def _exact_heads(near, far, v, do, w, causal, aux=False):
+    """`_exact_head` over (batch, head), the gradients of keys and values summed over the heads of a group."""
+    q, k = near
+    B, H, Hk = q.shape[0], q.shape[1], k.shape[1]
+    new = lambda *shape: torch.zeros(shape, dtype=torch.float64, device=q.device)
+    o, lse, total = new(*q.shape), new(*q.shape[:3]), new(B, H, k.shape[2])
+    grads = [(new(*x.shape), new(*y.shape)) for x, y in ([near] if far is None else [near, far])] if do is not None else []
+    dv = new(*v.shape) if do is not None else None
+    for b in range(B):
+        for h in range(H):
+            g = h // (H // Hk)
+            at = lambda pair: None if pair is None else (pair[0][b, h].double(), pair[1][b, g].double())
+            o[b, h], lse[b, h], total[b, h], gs, gv = _exact_head(
+                at(near), at(far), v[b, g].double(), None if do is None else do[b, h].double(), w, causal, aux)
+            for (dq, dk), (x, y) in zip(grads, gs or ()):
+                dq[b, h] = x
+                dk[b, g] += y
+            if do is not None:
+                dv[b, g] += gv
+    return o, lse, total, grads, dv
+
+
+def _rotate(x, cos, sin, back=False):
+    lo, hi = x.double().chunk(2, -1)
+    c, s = cos.double(), -sin.double() if back else sin.double()
+    return torch.cat((lo * c - hi * s, hi * c + lo * s), -1)
+
+
+@torch.no_grad()
+def exact(case, seed):
+    """What `run` returns, in 64 bits.  None with dropout: its mask is a matter of the random stream, not of precision."""
+    c, kind = case, case["kind"]
+    if kind == "train" and c["dropout"]:
+        return None
+    s = prepare(case, seed)
+    if kind == "train":
+        o, lse, _, [(dq, dk)], dv = _exact_heads((s["q"], s["k"]), None, s["v"], s["do"], 0, c["causal"])
+        return (o, lse, dq, dk, dv) if c["lse"] else (o, dq, dk, dv)
+    if kind == "piecewise":
+        q1, k1, q2, k2, v = s["x"]
+        o, _, _, [(dq1, dk1), (dq2, dk2)], dv = _exact_heads((q1, k1), (q2, k2), v, s["do"], c["w"], c["causal"])
+        return o, dq1, dk1, dq2, dk2, dv
+    if kind == "nlpe":
+        cos1, sin1, cos2, sin2 = s["tables"]
+        near, far = ([_rotate(s[x], cos, sin) for x in "qk"] for cos, sin in ((cos1, sin1), (cos2, sin2)))
+        o, _, _, (g1, g2), dv = _exact_heads(near, far, s["v"], s["do"], c["w"], c["causal"])
+        dq, dk = (_rotate(x, cos1, sin1, True) + _rotate(y, cos2, sin2, True) for x, y in zip(g1, g2))
+        return o, dq, dk, dv
+    if kind in ("prefill", "score", "decode"):
+        o, lse, total, _, _ = _exact_heads((s["q"], s["k"]), None, s["v"], None, 0, c["causal"], kind == "score")
+        return (o, lse, total) if kind == "score" else o
+    kc, vc = s["cache"]
+    if c["append"]:
+        for cache, new in zip((kc, vc), s["new"]):
+            cache[s["slots"] // c["block"], :, s["slots"] % c["block"]] = new
+    out = torch.empty(s["q"].shape, dtype=torch.float64, device="cuda")
+    for i, n in enumerate(s["lens"].tolist()):
+        blocks = s["table"][i, :(n + c["block"] - 1) // c["block"]].long()
+        k, v = (x[blocks].double().transpose(0, 1).flatten(1, 2)[:, :n] for x in (kc, vc))
+        q = s["q"][i].double().unflatten(0, (c["Hk"], -1))
+        out[i] = (torch.softmax(q @ k.transpose(1, 2) * c["D"] ** -0.5, -1) @ v).flatten(0, 1)
+    return (out, kc, vc) if c["append"] else out
+
+
+# ---------------------------------------------------------------------------------------------
 # what a pass cannot do without
 # ---------------------------------------------------------------------------------------------
 def _pairs(M, N, causal):
