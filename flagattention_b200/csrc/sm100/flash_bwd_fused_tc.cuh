@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 
   if (warp == 0) {
     // ------------------------------ producer -----------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int sq = 0, phq = 1, sd = 0, phd = 1;   // ring slot and the "free" parity to wait for
       int inflight_q = 0, inflight_do = 0;    // loads requested (for the drain after an abort)
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = instr_desc_f16(BN, BM, TcElem<T>::kFormat, 0, 0);   // S^T, dP^T
       constexpr uint32_t idesc_acc = instr_desc_f16(BN, D, TcElem<T>::kFormat, 0, 1);  // dV, dK
       constexpr uint32_t idesc_dq = instr_desc_f16(BM, D / C::NH, TcElem<T>::kFormat, 1, 1);  // dQ

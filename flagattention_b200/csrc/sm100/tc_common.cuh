@@ -24,6 +24,23 @@ struct AbortCtx {
   int *status;              // device status word (may be null)
 };
 
+// One thread of a converged warp, chosen by the hardware (the same one every time).  Code that issues
+// tcgen05 / TMA work runs under this and not under `lane == 0`: their operands live in uniform
+// registers, and only behind elect.sync does the compiler know that a single thread is active.  The
+// issuing thread of the one-pass backward is on its critical path (40 MMAs, 10 waits and 8 commits a
+// tile): B=4 H=32 L=4096 D=128 causal bf16 1.573 -> 1.495 ms, B=2 H=16 L=8192 D=64 2.05 -> 1.88 ms.
+// In the forward, where two CTAs share an SM and hide each other's issuing, it is worth nothing to 2 %,
+// and a whole-warp form of the same loops (uniform waits by vote) measured no better than this.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 // ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------
@@ -69,7 +86,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const A
                                           int where) {
   return mbar_wait_limit(bar, parity, ctx, where, kWaitCycles);
 }
-
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 }
