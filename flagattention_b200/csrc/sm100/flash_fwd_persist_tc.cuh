@@ -248,7 +248,14 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
         mbar_arrive(bar(FP_ITEM_FREE + (ic & 3)));
         if (w >= total) break;
         const PersistItem it = decode(w);
-        if (it.E == 0) continue;
+        if (it.E == 0) {
+          // An item without keys brings no score product that would push out the P V closing the item
+          // before; the softmax warps wait for that one and free no further slot of the item ring, so
+          // four such items in a row would stop everything.
+          if (pend) ok = issue_pv(g - 1, pend_first, pend_item);
+          pend = false;
+          continue;
+        }
         // Q of this item: if it has not landed yet, the product that closes the item before goes first
         if (pend && !mbar_try_wait(bar(FP_Q_FULL), cnt & 1)) {
           ok = issue_pv(g - 1, pend_first, pend_item);

@@ -58,9 +58,9 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
 // Work-item counters of the persistent forward.  The forward entry points take no workspace, so
 // the counters live in the library: a table of 64 words per device, one word per launch, taken
 // round-robin, zeroed by a four-byte stream-ordered memset in front of the launch (a launch also
-// puts its word back to zero with its last fetch, but relying on that alone let one cut-short
-// launch spoil a later one: seen in the test suite).  A word is only touched while its kernel
-// runs, so two launches collide only if 64 later launches start while the first still runs.
+// puts its word back to zero with its last fetch, but one that gives up on a wait leaves it mid-way).
+// A word is only touched while its kernel runs, so two launches collide only if 64 later launches
+// start while the first still runs.
 static __device__ unsigned g_fwd_sched[64];
 static unsigned *fwd_sched_table() {
   static std::atomic<unsigned *> base[64];
