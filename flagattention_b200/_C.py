@@ -22,6 +22,7 @@ EXPORTED_SYMBOLS = (
     "fa_flash_bwd_dq", "fa_piecewise_fwd", "fa_piecewise_bwd_dkdv", "fa_piecewise_bwd_dq",
     "fa_paged_decode", "fa_paged_reduce", "fa_paged_workspace_bytes", "fa_paged_trace_blocks",
     "fa_paged_attention_noalloc", "fa_dropout_mask",
+    "fa_flash_bwd", "fa_flash_bwd_workspace_bytes",
     "fa_flash_bwd_fused", "fa_flash_bwd_fused_stages", "fa_flash_bwd_fused_workspace_bytes", "fa_piecewise_bwd_fused",
     "fa_piecewise_bwd_fused_workspace_bytes",
     "fa_paged_cache_append", "fa_rotary_pair_fwd", "fa_rotary_pair_bwd",
@@ -82,6 +83,7 @@ def load():
             lib.fa_version.restype = ctypes.c_char_p
             lib.fa_splitkv_workspace_bytes.restype = ctypes.c_int64
             lib.fa_paged_workspace_bytes.restype = ctypes.c_int64
+            lib.fa_flash_bwd_workspace_bytes.restype = ctypes.c_int64
             lib.fa_flash_bwd_fused_workspace_bytes.restype = ctypes.c_int64
             lib.fa_piecewise_bwd_fused_workspace_bytes.restype = ctypes.c_int64
             lib.fa_num_splits_heuristic.restype = ctypes.c_int32

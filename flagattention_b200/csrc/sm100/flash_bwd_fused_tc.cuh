@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 template <typename T, int D>
 __global__ void __launch_bounds__(256)
     dq_convert_kernel(const float *__restrict__ acc, void *dq, Strides sdq, int H, int M, int Mpad,
-                      float scale) {
+                      float scale, int d) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int m = blockIdx.x * 32 + lane;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -998,6 +998,7 @@ __global__ void __launch_bounds__(256)
   T *orow = row_ptr_mut<T>(dq, sdq, b, h, m);
 #pragma unroll
   for (int g = w; g < D / 16; g += 8) {
+    if (g * 16 >= d) return;   // padding up to D
     float4 f[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) f[i] = *reinterpret_cast<const float4 *>(src + (4 * g + i) * 512);
@@ -1019,11 +1020,11 @@ __global__ void __launch_bounds__(256)
 // the kernel above skips.
 template <typename T, int D>
 __global__ void __launch_bounds__(256)
-    zero_rows_kernel(void *out, Strides so, int r_begin, int r_end) {
+    zero_rows_kernel(void *out, Strides so, int r_begin, int r_end, int d) {
   const int m = r_begin + blockIdx.x * 16 + (threadIdx.x >> 4);
   if (m >= r_end) return;
   T *orow = row_ptr_mut<T>(out, so, blockIdx.z, blockIdx.y, m);
-  for (int c = (threadIdx.x & 15) * 8; c < D; c += 128)
+  for (int c = (threadIdx.x & 15) * 8; c < d; c += 128)
     *reinterpret_cast<uint4 *>(orow + c) = make_uint4(0u, 0u, 0u, 0u);
 }
 

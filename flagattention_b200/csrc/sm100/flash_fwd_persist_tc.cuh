@@ -437,7 +437,8 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
               v.y = TcElem<T>::pack(__uint_as_float(ov[hh][8 * i + 2]) * inv, __uint_as_float(ov[hh][8 * i + 3]) * inv);
               v.z = TcElem<T>::pack(__uint_as_float(ov[hh][8 * i + 4]) * inv, __uint_as_float(ov[hh][8 * i + 5]) * inv);
               v.w = TcElem<T>::pack(__uint_as_float(ov[hh][8 * i + 6]) * inv, __uint_as_float(ov[hh][8 * i + 7]) * inv);
-              *reinterpret_cast<uint4 *>(orow + c * 64 + hh * 32 + i * 8) = v;
+              if (c * 64 + hh * 32 + i * 8 < p.d)
+                *reinterpret_cast<uint4 *>(orow + c * 64 + hh * 32 + i * 8) = v;
             }
         }
       }

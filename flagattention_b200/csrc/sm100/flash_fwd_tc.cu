@@ -32,11 +32,11 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
                          const fa_tensor4 *o, float *lse, cudaStream_t stream) {
   using C = FwdTcCfg<D>;
   CUtensorMap mq, mk, mv, mq2, mk2;
-  if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, D, C::BM) ||
-      !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, D, C::BN) ||
-      !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, D, C::BN) ||
-      !make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, D, C::BM) ||
-      !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, D, C::BN))
+  if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
+      !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
+      !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
+      !make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
+      !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return 1;  // layout not expressible as a tensor map: caller falls back to the generic kernel
   auto kern = flash_fwd_tc_kernel<T, D, PW>;
   static unsigned long long done = 0;
@@ -46,6 +46,7 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   p.B = s->B, p.H = s->H, p.Hk = s->Hk, p.M = s->M, p.N = s->N;
   p.causal = s->causal, p.sm_scale = s->sm_scale, p.w = w;
   p.status = device_status_word();
+  p.d = s->D;
   // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise)
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = cta_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2), s->B * s->H);
@@ -104,9 +105,9 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
                               const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream) {
   using C = FwdPersistCfg<D>;
   CUtensorMap mq, mk, mv;
-  if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, D, C::BM) ||
-      !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, D, C::BN) ||
-      !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, D, C::BN))
+  if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
+      !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
+      !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return 1;
   auto kern = flash_fwd_persist_tc_kernel<T, D>;
   static unsigned long long done = 0;
@@ -117,6 +118,7 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
   p.B = s->B, p.H = s->H, p.Hk = s->Hk, p.M = s->M, p.N = s->N;
   p.causal = s->causal, p.sm_scale = s->sm_scale, p.w = 0;
   p.status = device_status_word();
+  p.d = s->D;
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = cta_group_size((int64_t)s->N * D * 2 * 2, s->B * s->H);
   const int64_t items = (int64_t)p.num_m_blocks * s->B * s->H;
@@ -132,8 +134,12 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
 }
 
 static bool covered(const fa_flash_shape *s) {
-  return !generic_forced() && s->sm_scale > 0.f && (s->D == 64 || s->D == 128) &&
-         s->dropout_p == 0.f;  // dropout runs on the shape-generic kernels
+  // head_dim 16 and 32 run as 64 with zero columns: the exponentials bound these kernels, not the padded
+  // products.  Forward, B=4 H=16 L=2048 causal bf16, shape-generic -> padded: 32: 137 -> 90 us, 16: 104 -> 91 us;
+  // B=1 H=8 L=8192: 414 -> 236 us, 288 -> 237 us.  Walks of a few tiles do not pay for it at 16 (B=16 H=16
+  // Hk=4 L=512: 54 -> 64 us; at 32 65 us either way).
+  if (s->D == 16 && s->N < 1024) return false;
+  return !generic_forced() && s->sm_scale > 0.f && s->dropout_p == 0.f;  // dropout runs on the shape-generic kernels
 }
 
 // Return FA_OK / a negative status, or 1 when this path does not cover the call.
@@ -145,7 +151,7 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
   // at 16384: its steady tile period is 1750-1840 clocks against 1534 of the one-CTA-per-tile
   // kernel (why is not known: starting the second CTA of every SM a fraction of a tile period late,
   // in case the two walked in step, changed nothing).
-  const bool short_walks = s->D == 64 || s->N <= 1536;
+  const bool short_walks = s->D <= 64 || s->N <= 1536;
   if (!one_cta_per_tile_forced() && short_walks &&
       (int64_t)((s->M + 127) / 128) * s->B * s->H > 2 * (int64_t)sm_count_fwd()) {
     int st;

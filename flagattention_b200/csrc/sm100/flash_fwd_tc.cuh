@@ -1,5 +1,6 @@
 // flash_attention forward on the 5th-generation tensor cores (tcgen05) for
-// head_dim 64 and 128.
+// head_dim 64 and 128; head_dim 16 and 32 run as 64 with columns that the copy
+// engine fills with zeros (past the tensor map's extent) and nobody stores.
 //
 // One CTA owns 128 query rows of one (batch, head) and walks the visible keys
 // in tiles of 64.  Warp roles:
@@ -30,6 +31,7 @@ struct FwdTcParams {
   int w;  // piecewise distance threshold (PW kernels only)
   int *status;
   int num_m_blocks, group_size;  // launch order, see grouped_cta()
+  int d;          // head_dim of the tensors: D, or less when the columns up to D are padding
 };
 
 template <int D>
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
             v.y = TcElem<T>::pack(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv);
             v.z = TcElem<T>::pack(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv);
             v.w = TcElem<T>::pack(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv);
-            *reinterpret_cast<uint4 *>(orow + c * 32 + i * 8) = v;
+            if (c * 32 + i * 8 < p.d) *reinterpret_cast<uint4 *>(orow + c * 32 + i * 8) = v;
           }
         }
       }

@@ -15,8 +15,8 @@ static int launch_total_tc(const fa_flash_shape *s, const fa_tensor4 *q, const f
                            const float *lse, float *total, cudaStream_t stream) {
   using C = TotalTcCfg<D>;
   CUtensorMap mq, mk;
-  if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, D, C::BM) ||
-      !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, D, C::BN))
+  if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
+      !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return 1;   // layout not expressible as a tensor map: the caller uses the generic kernel
   auto kern = total_attention_tc_kernel<T, D>;
   static unsigned long long done = 0;
@@ -35,7 +35,7 @@ static int launch_total_tc(const fa_flash_shape *s, const fa_tensor4 *q, const f
 // Returns FA_OK / a negative status, or 1 when this path does not cover the call.
 int total_attention_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                        const float *lse, float *total, cudaStream_t stream) {
-  if (generic_forced() || !(s->sm_scale > 0.f) || (s->D != 64 && s->D != 128)) return 1;
+  if (generic_forced() || !(s->sm_scale > 0.f)) return 1;   // (head_dim 16 and 32 padded to 64)
   if (s->dtype == FA_F16)
     return s->D == 128 ? launch_total_tc<__half, 128>(s, q, k, lse, total, stream)
                        : launch_total_tc<__half, 64>(s, q, k, lse, total, stream);

@@ -205,17 +205,30 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
     with torch.cuda.device(q.device):
         stream = _C.stream_ptr(q.device)
         shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
-        delta = torch.empty_like(L)
         # dk / dv come out with Hk heads: the group sum is done in the kernel
         dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=q.device)
         dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=q.device)
         dq = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
         tq, tk, tv, to, tdo = (_C.tensor4(x) for x in (q, k, v, o, do))
         tdk, tdv, tdq = _C.tensor4(dk), _C.tensor4(dv), _C.tensor4(dq)
+        if mark is None and use_one_pass_backward():
+            # everything in one call: one workspace, one trip through the binding
+            ws_bytes = lib.fa_flash_bwd_workspace_bytes(_C.byref(shape))
+            if ws_bytes > 0:
+                ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+                st = lib.fa_flash_bwd(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv), _C.byref(to),
+                                      _C.byref(tdo), _C.fptr(L), _C.byref(tdq), _C.byref(tdk), _C.byref(tdv),
+                                      _C.fptr(ws), ctypes.c_int64(ws_bytes), stream)
+                # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
+                if st != _C.FA_ERR_UNSUPPORTED:
+                    _C.check(st, "fa_flash_bwd")
+                    return dq, dk, dv
+        # the parts one by one
+        delta = torch.empty_like(L)
         if mark:
             mark("start")
         ws_bytes = (lib.fa_flash_bwd_fused_workspace_bytes(_C.byref(shape))
-                    if use_one_pass_backward() else 0)
+                    if mark and use_one_pass_backward() else 0)
         if ws_bytes > 0:
             # one pass over the score tiles; dq is accumulated in an fp32 workspace, which the
             # delta kernel fills with zeros on its way (two memory-bound passes in one launch)
@@ -233,16 +246,12 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
             args = (_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv), _C.byref(tdo),
                     _C.fptr(L), _C.fptr(delta), _C.byref(tdq), _C.byref(tdk), _C.byref(tdv),
                     _C.fptr(ws), ctypes.c_int64(ws_bytes))
-            if mark:
-                # the parts of the call one by one, so that each can be timed
-                st = 0
-                for stage, name in ((2, "dkdvdq"), (4, "dq_convert")):
-                    st = lib.fa_flash_bwd_fused_stages(*args, stage, stream)
-                    if st != 0:
-                        break
-                    mark(name)
-            else:
-                st = lib.fa_flash_bwd_fused_stages(*args, 6, stream)   # kernel + dq conversion
+            st = 0
+            for stage, name in ((2, "dkdvdq"), (4, "dq_convert")):
+                st = lib.fa_flash_bwd_fused_stages(*args, stage, stream)
+                if st != 0:
+                    break
+                mark(name)
             # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
             if st != _C.FA_ERR_UNSUPPORTED:
                 _C.check(st, "fa_flash_bwd_fused")

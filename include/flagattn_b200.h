@@ -156,6 +156,17 @@ int fa_flash_bwd_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_te
                        const fa_tensor4 *dv, void *workspace, int64_t workspace_bytes,
                        void *stream);
 
+/* The whole backward of flash_attention in one call: delta, the one-pass kernel above and the
+ * conversion of dq, head_dim 16 .. 128 (16 and 32 run padded to 64).  Replaces the three launches of
+ * src/flag_attn/flash.py:189-249.  `workspace` holds fa_flash_bwd_workspace_bytes bytes (16-byte aligned;
+ * 0: the shape is not covered, call fa_flash_bwd_delta, fa_flash_bwd_dkdv and fa_flash_bwd_dq).  Same
+ * reproducibility, and the same FA_ERR_UNSUPPORTED for broadcast strides, as fa_flash_bwd_fused. */
+int64_t fa_flash_bwd_workspace_bytes(const fa_flash_shape *s);
+int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
+                 const fa_tensor4 *v, const fa_tensor4 *o, const fa_tensor4 *d_o, const float *lse,
+                 const fa_tensor4 *dq, const fa_tensor4 *dk, const fa_tensor4 *dv, void *workspace,
+                 int64_t workspace_bytes, void *stream);
+
 /* Regenerates the dropout keep-mask of a flash_attention call: mask[b,h,m,n] (1 byte each,
  * contiguous) = 1 iff the element was kept.  Replaces `recompute_mask_kernel`
  * (src/flag_attn/testing/dropout.py:5-25). */
