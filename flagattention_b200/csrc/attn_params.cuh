@@ -74,6 +74,69 @@ __host__ __device__ __forceinline__ bool dropout_keep(uint64_t seed, uint64_t of
   return (float)x * 4.6566127342e-10f > dropout_p;
 }
 
+// ---- the same decision for the tcgen05 kernels ----
+// dropout_keep() as one unsigned range check: with x = u or ~u of the Philox word u (whichever is not
+// negative), (float)x * c > dropout_p holds from some smallest x = t on, hence for u in [t, 2^32 - t).
+// t by bisection with the very float operations of dropout_keep(); no x satisfies it: an empty range.
+struct DropoutRule {
+  uint64_t seed, offset;
+  uint32_t first, width;   // keep iff u - first < width
+  float rp;                // 1 / (1 - dropout_p)
+};
+inline DropoutRule make_dropout_rule(float dropout_p, uint64_t seed, uint64_t offset) {
+  uint64_t lo = 0, hi = 1ull << 31;   // smallest x in [lo, hi] that is kept (2^31: none)
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) / 2;
+    const volatile float u = (float)(int32_t)mid * 4.6566127342e-10f;
+    if (u > dropout_p) hi = mid;
+    else lo = mid + 1;
+  }
+  return DropoutRule{seed, offset, (uint32_t)lo, (uint32_t)(0u - 2u * (uint32_t)lo), 1.f / (1.f - dropout_p)};
+}
+
+// Keep bits of the elements whose counters are ctr, ctr + step, .. ctr + 31 step (bit i: the i-th).
+// What bounds a kernel with dropout is this: Philox costs 10 multiplications an element and only its
+// first output word is used.  While the counters share their upper 32 bits (all but one in 2^32 / (31
+// step) calls) one product of round 2 depends on nothing else and is taken out of the loop; words of
+// rounds 4 to 6 that do not reach the first output are not computed: 9 multiplications and 9 three-input
+// xors an element.
+__device__ __forceinline__ uint32_t dropout_keep_bits32(const DropoutRule &r, uint64_t ctr, uint32_t step) {
+  constexpr uint32_t A = 0xD2511F53u, B = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
+  const uint32_t k0 = (uint32_t)r.seed, k1 = (uint32_t)(r.seed >> 32);
+  const uint32_t lo = (uint32_t)ctr;
+  uint32_t bits = 0;
+  if ((uint64_t)lo + 31ull * step >> 32) {   // the upper half of the counter changes on the way
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i) {
+      const uint64_t c = ctr + (uint64_t)i * step;
+      const uint32_t u = philox4x32_6(k0, k1, (uint32_t)c, (uint32_t)(c >> 32));
+      if (u - r.first < r.width) bits |= 1u << i;
+    }
+    return bits;
+  }
+  const uint64_t fixed = (uint64_t)A * ((uint32_t)(ctr >> 32) ^ k0);   // round 2
+  const uint32_t fx = (uint32_t)(fixed >> 32) ^ (k1 + W1), fy = (uint32_t)fixed ^ (k1 + 2u * W1);
+#pragma unroll 8
+  for (int i = 0; i < 32; ++i) {
+    uint64_t pa = (uint64_t)A * (lo + (uint32_t)i * step);   // round 1
+    uint32_t c2 = (uint32_t)(pa >> 32) ^ k1;
+    uint64_t pb = (uint64_t)B * c2;   // round 2
+    uint32_t c0 = (uint32_t)(pb >> 32) ^ (k0 + W0), c1 = (uint32_t)pb;
+    c2 = (uint32_t)pa ^ fx;
+    pb = (uint64_t)B * c2, pa = (uint64_t)A * c0;   // round 3
+    c0 = (uint32_t)(pb >> 32) ^ c1 ^ (k0 + 2u * W0);
+    c2 = (uint32_t)(pa >> 32) ^ fy;
+    const uint32_t c3 = (uint32_t)pa;
+    pa = (uint64_t)A * c0;   // round 4
+    c0 = __umulhi(B, c2) ^ (uint32_t)pb ^ (k0 + 3u * W0);
+    c2 = (uint32_t)(pa >> 32) ^ c3 ^ (k1 + 3u * W1);
+    const uint32_t d2 = __umulhi(A, c0) ^ (uint32_t)pa ^ (k1 + 4u * W1);   // round 5
+    const uint32_t u = __umulhi(B, d2) ^ (B * c2) ^ (k0 + 5u * W0);        // round 6
+    if (u - r.first < r.width) bits |= 1u << i;
+  }
+  return bits;
+}
+
 template <typename T>
 __device__ __forceinline__ const T *row_ptr(const void *base, const Strides &s, int b, int h,
                                             int l) {

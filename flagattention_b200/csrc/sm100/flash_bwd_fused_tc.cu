@@ -16,11 +16,11 @@ namespace tc {
 bool generic_forced();
 
 static bool one_pass_covered(const fa_flash_shape *s) {
-  return !generic_forced() && s->sm_scale > 0.f && s->dropout_p == 0.f;
+  return !generic_forced() && s->sm_scale > 0.f;
 }
 // the entries that take the backward in parts
 static bool fused_covered(const fa_flash_shape *s) {
-  return one_pass_covered(s) && (s->D == 64 || s->D == 128);
+  return one_pass_covered(s) && (s->D == 64 || s->D == 128) && s->dropout_p == 0.f;
 }
 
 // Head_dim the kernel runs at: 16 and 32 are padded to 64 (zero columns in shared memory, from the copy
@@ -104,7 +104,7 @@ struct FarBranch {
 // key block is walked twice by the same CTA, near pairs with (q, k) -> (dq, dk), far pairs with
 // (q2, k2) -> (dq2, dk2); dV accumulates across the two walks and is rounded once).
 // Workspace: dq accumulator [| dq2 accumulator] | 16 bytes of work-item counter.
-template <typename T, int D>
+template <typename T, int D, bool DROP = false>
 static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                         const fa_tensor4 *v, const fa_tensor4 *d_o, const float *lse,
                         const float *delta, const fa_tensor4 *dq, const fa_tensor4 *dk,
@@ -123,7 +123,7 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
       !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
       !make_map_bhld(&mdk2, dk2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return FA_ERR_UNSUPPORTED;
-  auto kern = flash_bwd_fused_tc_kernel<T, D>;
+  auto kern = flash_bwd_fused_tc_kernel<T, D, DROP>;
   static unsigned long long done = 0;
   if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
   FusedBwdParams fp{};
@@ -135,6 +135,7 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
   p.mode = far ? 3 : 0, p.w = far ? far->w : 0, p.dv_accumulate = 0;
   p.dk = dk->ptr, p.dv = dv->ptr, p.sdk = strides_of(dk), p.sdv = strides_of(dv);
   p.dq = dq->ptr, p.sdq = strides_of(dq);
+  if (DROP) fp.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
   const int64_t acc_bytes = fused_dq_acc_bytes(s);
   const int n_acc = far ? 2 : 1;
   fp.dq_acc = workspace;
@@ -310,10 +311,16 @@ extern "C" int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const 
   float *delta = reinterpret_cast<float *>(static_cast<char *>(workspace) + acc);
   if (int rc = fa_flash_bwd_delta_zero(s, o, d_o, delta, workspace, acc, stream)) return rc;
 #define FA_BWD_ARGS s, q, k, v, d_o, lse, delta, dq, dk, dv, ws, st, nullptr, 6
-  if (s->dtype == FA_F16)
-    return s->D == 128 ? tc::launch_fused<__half, 128>(FA_BWD_ARGS)
-                       : tc::launch_fused<__half, 64>(FA_BWD_ARGS);
-  return s->D == 128 ? tc::launch_fused<__nv_bfloat16, 128>(FA_BWD_ARGS)
-                     : tc::launch_fused<__nv_bfloat16, 64>(FA_BWD_ARGS);
+#define FA_BWD_CASE(DROP)                                                        \
+  if (s->dtype == FA_F16)                                                        \
+    return s->D == 128 ? tc::launch_fused<__half, 128, DROP>(FA_BWD_ARGS)        \
+                       : tc::launch_fused<__half, 64, DROP>(FA_BWD_ARGS);        \
+  return s->D == 128 ? tc::launch_fused<__nv_bfloat16, 128, DROP>(FA_BWD_ARGS)   \
+                     : tc::launch_fused<__nv_bfloat16, 64, DROP>(FA_BWD_ARGS);
+  if (s->dropout_p > 0.f) {
+    FA_BWD_CASE(true)
+  }
+  FA_BWD_CASE(false)
+#undef FA_BWD_CASE
 #undef FA_BWD_ARGS
 }

@@ -26,7 +26,7 @@ int set_kernel_family(int family) {
   return g_kernel_family.exchange(family == 1 ? 1 : (family == 2 ? 2 : 0));
 }
 
-template <typename T, int D, bool PW>
+template <typename T, int D, bool PW, bool DROP = false>
 static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, const fa_tensor4 *k,
                          const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
                          const fa_tensor4 *o, float *lse, cudaStream_t stream) {
@@ -38,7 +38,7 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
       !make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
       !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return 1;  // layout not expressible as a tensor map: caller falls back to the generic kernel
-  auto kern = flash_fwd_tc_kernel<T, D, PW>;
+  auto kern = flash_fwd_tc_kernel<T, D, PW, DROP>;
   static unsigned long long done = 0;
   if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
   FwdTcParams p{};
@@ -47,6 +47,7 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   p.causal = s->causal, p.sm_scale = s->sm_scale, p.w = w;
   p.status = device_status_word();
   p.d = s->D;
+  if (DROP) p.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
   // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise)
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = cta_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2), s->B * s->H);
@@ -139,13 +140,23 @@ static bool covered(const fa_flash_shape *s) {
   // B=1 H=8 L=8192: 414 -> 236 us, 288 -> 237 us.  Walks of a few tiles do not pay for it at 16 (B=16 H=16
   // Hk=4 L=512: 54 -> 64 us; at 32 65 us either way).
   if (s->D == 16 && s->N < 1024) return false;
-  return !generic_forced() && s->sm_scale > 0.f && s->dropout_p == 0.f;  // dropout runs on the shape-generic kernels
+  return !generic_forced() && s->sm_scale > 0.f;
 }
 
 // Return FA_OK / a negative status, or 1 when this path does not cover the call.
 int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                  const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream) {
   if (!covered(s)) return 1;
+  // Dropout is bound by its random numbers (see dropout_keep_bits32()): one CTA per tile at every size.
+  // Forward at head_dim 64, p = 0.1, bf16, mma.sync kernel -> this: B=16 H=16 L=512 232 -> 174 us (57 us
+  // without dropout), B=4 H=16 L=2048 causal 565 -> 343 us.
+  if (s->dropout_p > 0.f) {
+    if (s->dtype == FA_F16)
+      return s->D == 128 ? launch_fwd_tc<__half, 128, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
+                         : launch_fwd_tc<__half, 64, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
+    return s->D == 128 ? launch_fwd_tc<__nv_bfloat16, 128, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
+                       : launch_fwd_tc<__nv_bfloat16, 64, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
+  }
   // More query tiles than CTA slots and short walks (or head_dim 64): the persistent kernel.  It
   // measured +3..5 % at N <= 1024 and at head_dim 64, but -10 % at head_dim 128 and N = 4096, -17 %
   // at 16384: its steady tile period is 1750-1840 clocks against 1534 of the one-CTA-per-tile
@@ -173,7 +184,7 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
 int piecewise_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q1, const fa_tensor4 *k1,
                      const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
                      const fa_tensor4 *o, float *lse, cudaStream_t stream) {
-  if (!covered(s) || w > (1 << 29) || w < -(1 << 29)) return 1;
+  if (!covered(s) || s->dropout_p > 0.f || w > (1 << 29) || w < -(1 << 29)) return 1;
   if (s->dtype == FA_F16)
     return s->D == 128 ? launch_fwd_tc<__half, 128, true>(s, w, q1, k1, q2, k2, v, o, lse, stream)
                        : launch_fwd_tc<__half, 64, true>(s, w, q1, k1, q2, k2, v, o, lse, stream);

@@ -32,6 +32,7 @@ struct FwdTcParams {
   int *status;
   int num_m_blocks, group_size;  // launch order, see grouped_cta()
   int d;          // head_dim of the tensors: D, or less when the columns up to D are padding
+  DropoutRule drop;   // DROP kernels only
 };
 
 template <int D>
@@ -60,7 +61,9 @@ enum FwdBar { Q_FULL = 0, K_FULL = 1, K_FREE = 3, V_FULL = 5, V_FREE = 7, S_FULL
 // tile that straddles the threshold appears twice, each time masked to its own branch, so each
 // entry is an ordinary flash tile and the online softmax simply sees a few more tiles.  Q is
 // re-loaded once, at the switch from the far to the near entries.
-template <typename T, int D, bool PW>
+// DROP = dropout on the probabilities that enter P V (the row sums stay undropped).  The keep bits of a
+// tile do not depend on its scores: they are computed before the wait for them.
+template <typename T, int D, bool PW, bool DROP>
 __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
     flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                         const __grid_constant__ CUtensorMap map_k,
@@ -248,6 +251,12 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       const bool far = PW && e < E2;
       const int j = (PW && e >= E2) ? jf + (e - E2) : e;
       const int st = e & 1, ph = (e >> 1) & 1, n0 = j * BN;
+      uint32_t keep[2] = {0u, 0u};
+      if (DROP) {
+        const uint64_t ctr = p.drop.offset + (((uint64_t)b * p.H + h) * p.M + row) * p.N + n0;
+        keep[0] = dropout_keep_bits32(p.drop, ctr, 1u);
+        keep[1] = dropout_keep_bits32(p.drop, ctr + 32, 1u);
+      }
       ok = mbar_wait(bar(S_FULL + st), ph, actx, 301);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -328,8 +337,12 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       for (int c = 0; c < BN; c += 2) {
         float x0, x1;
         f2_unpack(f2_fma(f2_pack(s[c], s[c + 1]), scale2, shift2), x0, x1);
-        const float p0 = ex2(x0), p1 = ex2(x1);
+        float p0 = ex2(x0), p1 = ex2(x1);
         rs2[(c >> 1) & 3] = f2_add(rs2[(c >> 1) & 3], f2_pack(p0, p1));
+        if (DROP) {
+          if (!(keep[c >> 5] >> (c & 31) & 1u)) p0 = 0.f;
+          if (!(keep[c >> 5] >> ((c + 1) & 31) & 1u)) p1 = 0.f;
+        }
         pk[c >> 1] = TcElem<T>::pack(p0, p1);
       }
       {
@@ -352,7 +365,8 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
     }
     if (ok) {
       tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if (DROP) inv *= p.drop.rp;
       T *orow = row_ptr_mut<T>(p.o, p.so, b, h, row);
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {

@@ -1,0 +1,41 @@
+"""The keep bits the tcgen05 kernels compute for themselves, element by element against the mask the library
+regenerates: counters that cross 2^32 inside a tile (and inside a thread's run of 32), ragged sizes, grouped heads.
+With q = k = 0 every weight is 1 / N, so the outputs of one-hot values are the mask itself."""
+import pytest
+import torch
+
+import flagattention_b200 as fa
+from flagattention_b200 import flash
+
+pytestmark = pytest.mark.gpu
+
+STREAMS = [(0, 0), (2 ** 63 + 12345, 2 ** 32 - 4000), (2 ** 40 + 17, 2 ** 34 - 100), (7, 2 ** 33 + 3)]
+
+
+@pytest.mark.parametrize("seed,offset", STREAMS)
+@pytest.mark.parametrize("p", [0.1, 0.5, 0.9999])
+@pytest.mark.parametrize("H,M,N,D", [(3, 300, 64, 64), (2, 129, 128, 128), (5, 70, 31, 32), (2, 500, 16, 16)])
+def test_forward_mask(H, M, N, D, p, seed, offset):
+    q, k = (torch.zeros(2, H, n, D, device="cuda", dtype=torch.float16) for n in (M, N))
+    v = torch.eye(N, D, device="cuda", dtype=torch.float16).expand(2, H, N, D).contiguous()
+    o, _ = flash._forward(q, k, v, False, 1.0, p, seed, offset)
+    mask = fa.testing.recompute_mask(2, H, M, N, p, seed, offset, "cuda")
+    assert torch.equal(o[..., :N] > 0.5 / (N * (1 - p)), mask)
+
+
+@pytest.mark.parametrize("seed,offset", STREAMS)
+@pytest.mark.parametrize("p", [0.1, 0.5])
+@pytest.mark.parametrize("M,N,D", [(64, 300, 64), (128, 257, 128), (31, 100, 32)])
+def test_backward_mask(M, N, D, p, seed, offset):
+    H, Hk = 4, 2
+    q = torch.zeros(2, H, M, D, device="cuda", dtype=torch.float16)
+    k, v = (torch.zeros(2, Hk, N, D, device="cuda", dtype=torch.float16) for _ in range(2))
+    # dV[n, m] = (keep of the group's first head + 2 * keep of its second) / (N (1 - p))
+    do = torch.eye(M, D, device="cuda", dtype=torch.float16) * torch.tensor([1., 2.] * 2, device="cuda").half()[:, None, None]
+    do = do.expand(2, H, M, D).contiguous()
+    o, lse = flash._forward(q, k, v, False, 1.0, p, seed, offset)
+    dq, dk, dv = flash._backward(q, k, v, o, lse, do, False, 1.0, None, p, seed, offset)
+    mask = fa.testing.recompute_mask(2, H, M, N, p, seed, offset, "cuda").to(torch.int64)
+    got = (dv.float() * (N * (1 - p))).round().to(torch.int64)[..., :M].transpose(2, 3)
+    assert torch.equal(got, mask[:, 0::2] + 2 * mask[:, 1::2])
+    assert not dq.any() and not dk.any()   # k = 0 and q = 0
