@@ -4,8 +4,10 @@ The library is loaded lazily on first use.  There is no fallback: when the
 shared library is missing or a call returns a non-zero status, a RuntimeError
 is raised.
 """
+import contextlib
 import ctypes
 import os
+import struct
 import threading
 
 import torch
@@ -132,9 +134,76 @@ def dtype_code(dtype):
     raise AssertionError("only float16 and bfloat16 are supported, got %s" % dtype)
 
 
+# ---- the operators' own calls -------------------------------------------------------------------
+# A small call is bound by the host: building ctypes structures field by field, converting every argument
+# and switching devices took most of its time.  Here the argument structs are packed in one go (the layouts
+# are checked against the ctypes declarations above by the CPU tests) and passed as byte strings to function
+# objects that know their argument types.
+_SHAPE = struct.Struct("@8i2f2Q")                                   # FlashShape
+_TENSOR4 = struct.Struct("@P3q")                                    # Tensor4
+PAGED_ARGS = struct.Struct("@9ifP2q2P3q2PqP2q3Pi4x")                # PagedArgs
+_SIGNATURES = {
+    "fa_flash_fwd": "ppppppp", "fa_flash_bwd": "ppppppppppplp", "fa_flash_bwd_workspace_bytes": "p",
+    "fa_piecewise_fwd": "pipppppppp", "fa_paged_decode": "pp", "fa_paged_reduce": "pp",
+    "fa_paged_cache_append": "iiiiippllpplllpp", "fa_splitkv_fwd": "ppppiippp", "fa_splitkv_combine": "pippppp",
+    "fa_total_attention": "pppppp", "fa_flash_bwd_delta": "ppppp", "fa_piecewise_bwd_fused_workspace_bytes": "p",
+    "fa_piecewise_bwd_fused": "pi" + "p" * 14 + "lp", "fa_rotary_pair_fwd": "iiiiii" + "p" * 5 + "liplppp",
+    "fa_rotary_pair_bwd": "iiiiii" + "p" * 6 + "liplpp",
+}
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int32, "l": ctypes.c_int64}
+_calls = {}
+
+
+def call(name):
+    """The library function `name` with typed arguments: pointers as integers or as packed structs."""
+    f = _calls.get(name)
+    if f is None:
+        f = load()[name]   # (subscripting gives a function object of its own, without touching lib.<name>)
+        f.argtypes = [_CTYPES[c] for c in _SIGNATURES[name]]
+        f.restype = ctypes.c_int64 if name.endswith("_bytes") else ctypes.c_int
+        _calls[name] = f
+    return f
+
+
+def pack_shape(dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p=0.0, seed=0, offset=0):
+    return _SHAPE.pack(dtype_code(dtype), B, H, Hk, M, N, D, 1 if causal else 0, sm_scale, dropout_p,
+                       int(seed) & (2 ** 64 - 1), int(offset) & (2 ** 64 - 1))
+
+
+def pack4(x):
+    """tensor4() as a packed struct."""
+    b, h, l, _ = x.shape
+    sb, sh, sl, _ = x.stride()
+    return _TENSOR4.pack(x.data_ptr(), sb if b > 1 else 0, sh if h > 1 else 0, sl if l > 1 else 0)
+
+
+_sm_counts = {}
+
+
+def sm_count(device):
+    n = _sm_counts.get(device)
+    if n is None:
+        n = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return n
+
+
+_NO_SWITCH = contextlib.nullcontext()
+
+
+def device_guard(device):
+    """torch.cuda.device(device), or nothing when that is the current device already."""
+    return _NO_SWITCH if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def raw_stream(device):
+    return torch.cuda.current_stream(device).cuda_stream
+
+
 def kernel_ready(x):
     """Returns x, or a contiguous copy when x breaks the kernels' layout rule
     (unit inner stride, 16-byte aligned rows)."""
+    if x.is_contiguous() and x.shape[-1] % 8 == 0 and x.data_ptr() % 16 == 0:
+        return x      # every outer stride is a multiple of the inner size
     if x.stride(-1) != 1:
         return x.contiguous()
     if x.data_ptr() % 16 != 0:

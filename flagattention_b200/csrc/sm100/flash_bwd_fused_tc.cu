@@ -118,10 +118,12 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
       !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
       !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
       !make_map_bhld(&mdk, dk, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
-      !make_map_bhld(&mdv, dv, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
-      !make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
-      !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
-      !make_map_bhld(&mdk2, dk2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
+      !make_map_bhld(&mdv, dv, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
+    return FA_ERR_UNSUPPORTED;
+  mq2 = mq, mk2 = mk, mdk2 = mdk;
+  if (far && (!make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
+              !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
+              !make_map_bhld(&mdk2, dk2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN)))
     return FA_ERR_UNSUPPORTED;
   auto kern = flash_bwd_fused_tc_kernel<T, D, DROP>;
   static unsigned long long done = 0;

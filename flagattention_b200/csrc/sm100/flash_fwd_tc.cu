@@ -34,10 +34,12 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   CUtensorMap mq, mk, mv, mq2, mk2;
   if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
       !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
-      !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
-      !make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
-      !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
+      !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return 1;  // layout not expressible as a tensor map: caller falls back to the generic kernel
+  mq2 = mq, mk2 = mk;
+  if (PW && (!make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
+             !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN)))
+    return 1;
   auto kern = flash_fwd_tc_kernel<T, D, PW, DROP>;
   static unsigned long long done = 0;
   if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;

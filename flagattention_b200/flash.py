@@ -13,6 +13,7 @@ import torch
 
 from . import _C
 from .dropout import philox_cuda_seed_offset
+from .paged import partition_workspace
 from .split_kv import get_fwd_config as get_fwd_config_kv_split
 from .split_kv import num_splits_herustic, _splitkv_forward
 
@@ -80,13 +81,11 @@ def get_bwd_config(B, H, M, N, D, causal):
 def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0):
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
-    lib = _C.load()
-    o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    o = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
     L = torch.empty((B, H, M), device=q.device, dtype=torch.float32)
-    shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
-    tq, tk, tv, to = _C.tensor4(q), _C.tensor4(k), _C.tensor4(v), _C.tensor4(o)
-    st = lib.fa_flash_fwd(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv), _C.byref(to),
-                          _C.fptr(L), _C.stream_ptr(q.device))
+    st = _C.call("fa_flash_fwd")(
+        _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset), _C.pack4(q), _C.pack4(k),
+        _C.pack4(v), _C.pack4(o), L.data_ptr(), _C.raw_stream(q.device))
     _C.check(st, "fa_flash_fwd")
     return o, L
 
@@ -139,8 +138,7 @@ def _decode_forward(q, k, v, sm_scale, causal=False):
     Hk, N = k.shape[1], k.shape[2]
     BS = 16
     sb, sh, sl, _ = k.stride()
-    lib = _C.load()
-    num_sms = torch.cuda.get_device_properties(q.device).multi_processor_count
+    num_sms = _C.sm_count(q.device)
     # partitions of the key axis: enough (batch, kv head, partition) CTAs for about eight waves,
     # each long enough (>= 256 keys) to amortise its pipeline fill
     partition_size = 256
@@ -153,44 +151,29 @@ def _decode_forward(q, k, v, sm_scale, causal=False):
     if q2.stride(-1) != 1 or q2.data_ptr() % 16 or q2.stride(0) % 8 or q2.stride(1) % 8:
         q2 = q2.contiguous()
     o = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
-    args = _C.PagedArgs()
-    args.dtype = _C.dtype_code(q.dtype)
-    args.num_seqs, args.num_q_heads, args.num_kv_heads = B, H * M, Hk
-    args.causal_rows = M if (causal and M > 1) else 0
-    args.head_size, args.block_size = D, BS
-    args.max_context_len = N
-    args.block_table_is_i64 = 0
-    args.partition_size = partition_size
-    args.attn_scale = float(sm_scale)
-    args.query, args.q_stride_s, args.q_stride_h = q2.data_ptr(), q2.stride(0), q2.stride(1)
-    args.key_cache, args.value_cache = k.data_ptr(), v.data_ptr()
-    args.kv_stride_b, args.kv_stride_h, args.kv_stride_t = BS * sl, sh if Hk > 1 else 0, sl
-    args.context_lens = ctx_lens.data_ptr()
-    args.block_tables, args.bt_stride_s = table.data_ptr(), table.stride(0)
-    args.out, args.o_stride_s, args.o_stride_h = o.data_ptr(), H * M * D, D
-    stream = _C.stream_ptr(q.device)
+    part_out = part_max = part_sum = 0
     if partition_size:
         P = (N + partition_size - 1) // partition_size
-        part_out = torch.empty((B, H * M, P, D), dtype=torch.float32, device=q.device)
-        part_max = torch.empty((B, H * M, P), dtype=torch.float32, device=q.device)
-        part_sum = torch.empty_like(part_max)
-        args.part_out, args.part_max, args.part_sum = (part_out.data_ptr(), part_max.data_ptr(),
-                                                       part_sum.data_ptr())
-    _C.check(lib.fa_paged_decode(_C.byref(args), stream), "fa_paged_decode")
+        ws, part_out, part_max, part_sum = partition_workspace(B * H * M, P, D, q.device)
+    args = _C.PAGED_ARGS.pack(
+        _C.dtype_code(q.dtype), B, H * M, Hk, D, BS, N, 0, partition_size, sm_scale,
+        q2.data_ptr(), q2.stride(0), q2.stride(1), k.data_ptr(), v.data_ptr(),
+        BS * sl, sh if Hk > 1 else 0, sl, ctx_lens.data_ptr(), table.data_ptr(), table.stride(0),
+        o.data_ptr(), H * M * D, D, part_out, part_max, part_sum, M if (causal and M > 1) else 0)
+    stream = _C.raw_stream(q.device)
+    _C.check(_C.call("fa_paged_decode")(args, stream), "fa_paged_decode")
     if partition_size:
-        _C.check(lib.fa_paged_reduce(_C.byref(args), stream), "fa_paged_reduce")
+        _C.check(_C.call("fa_paged_reduce")(args, stream), "fa_paged_reduce")
     return o
 
 
 def _total_attention(q, k, L, causal, sm_scale):
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
-    lib = _C.load()
     tot = torch.empty((B, H, N), device=q.device, dtype=torch.float32)
-    shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale)
-    tq, tk = _C.tensor4(q), _C.tensor4(k)
-    st = lib.fa_total_attention(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.fptr(L),
-                                _C.fptr(tot), _C.stream_ptr(q.device))
+    st = _C.call("fa_total_attention")(
+        _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale), _C.pack4(q), _C.pack4(k), L.data_ptr(),
+        tot.data_ptr(), _C.raw_stream(q.device))
     _C.check(st, "fa_total_attention")
     return tot
 
@@ -202,28 +185,29 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
     N, Hk = k.shape[2], k.shape[1]
     lib = _C.load()
     do = _C.kernel_ready(do)
-    with torch.cuda.device(q.device):
-        stream = _C.stream_ptr(q.device)
-        shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
+    with _C.device_guard(q.device):
         # dk / dv come out with Hk heads: the group sum is done in the kernel
         dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=q.device)
         dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=q.device)
         dq = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
-        tq, tk, tv, to, tdo = (_C.tensor4(x) for x in (q, k, v, o, do))
-        tdk, tdv, tdq = _C.tensor4(dk), _C.tensor4(dv), _C.tensor4(dq)
         if mark is None and use_one_pass_backward():
             # everything in one call: one workspace, one trip through the binding
-            ws_bytes = lib.fa_flash_bwd_workspace_bytes(_C.byref(shape))
+            packed = _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
+            ws_bytes = _C.call("fa_flash_bwd_workspace_bytes")(packed)
             if ws_bytes > 0:
                 ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-                st = lib.fa_flash_bwd(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv), _C.byref(to),
-                                      _C.byref(tdo), _C.fptr(L), _C.byref(tdq), _C.byref(tdk), _C.byref(tdv),
-                                      _C.fptr(ws), ctypes.c_int64(ws_bytes), stream)
+                st = _C.call("fa_flash_bwd")(
+                    packed, _C.pack4(q), _C.pack4(k), _C.pack4(v), _C.pack4(o), _C.pack4(do), L.data_ptr(),
+                    _C.pack4(dq), _C.pack4(dk), _C.pack4(dv), ws.data_ptr(), ws_bytes, _C.raw_stream(q.device))
                 # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
                 if st != _C.FA_ERR_UNSUPPORTED:
                     _C.check(st, "fa_flash_bwd")
                     return dq, dk, dv
         # the parts one by one
+        stream = _C.stream_ptr(q.device)
+        shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
+        tq, tk, tv, to, tdo = (_C.tensor4(x) for x in (q, k, v, o, do))
+        tdk, tdv, tdq = _C.tensor4(dk), _C.tensor4(dv), _C.tensor4(dq)
         delta = torch.empty_like(L)
         if mark:
             mark("start")
@@ -299,16 +283,15 @@ class FlashAttention(torch.autograd.Function):
             # gather kernel, which streams K and V once; a few queries go there when the reference
             # would split the keys (src/flag_attn/flash.py:59-61), i.e. when the tile grid alone
             # would leave most of the GPU idle.
-            with torch.cuda.device(q.device):
+            with _C.device_guard(q.device):
                 take = M == 1
                 if not take:
-                    num_sms = torch.cuda.get_device_properties(q.device).multi_processor_count
                     cfg = get_fwd_config_kv_split(B, H, M, N, D, causal)
-                    take = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], num_sms, 128) > 1
+                    take = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], _C.sm_count(q.device), 128) > 1
                 if take:
                     return _decode_forward(q, k, v, sm_scale, causal)
 
-        with torch.cuda.device(q.device):
+        with _C.device_guard(q.device):
             # dropout: one Philox counter per element of the (B, H, M, N) attention matrix
             is_dropout = dropout_p > 0
             if is_dropout:
@@ -316,9 +299,8 @@ class FlashAttention(torch.autograd.Function):
             else:
                 seed, offset = 0, 0
 
-            num_sms = torch.cuda.get_device_properties(q.device).multi_processor_count
             cfg = get_fwd_config_kv_split(B, H, M, N, D, causal)
-            S = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], num_sms, 128)
+            S = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], _C.sm_count(q.device), 128)
             if S > 1:
                 assert not is_dropout, "Cannot apply dropout with splitkv."
                 o, L = _splitkv_forward(q, k, v, causal, sm_scale, S)
@@ -335,7 +317,6 @@ class FlashAttention(torch.autograd.Function):
         ctx.seed = seed
         ctx.offset = offset
 
-        has_extra_return = True in (return_log_normalizer, return_total_attention, return_seed_offset)
         if has_extra_return:
             return (o, L if return_log_normalizer else None, tot_attn,
                     seed if is_dropout and return_seed_offset else None,

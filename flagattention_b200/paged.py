@@ -41,6 +41,16 @@ def plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_
     return num_splits, partition_size
 
 
+def partition_workspace(rows, P, D, device):
+    """One allocation for the partial results of `rows` (sequence, query head) rows over P partitions:
+    (tensor, address of the outputs (rows, P, D), of the maxima (rows, P), of the sums (rows, P)), all fp32."""
+    stats = (rows * P + 63) // 64 * 64
+    ws = torch.empty(rows * P * D + 2 * stats, dtype=torch.float32, device=device)
+    base = ws.data_ptr()
+    part_max = base + rows * P * D * 4
+    return ws, base, part_max, part_max + stats * 4
+
+
 def attention(query, key_cache, value_cache, context_lens, block_tables, attn_scale,
               max_context_len, num_splits=0):
     """query [num_seqs, kv_heads * group, head]; caches [num_blocks, kv_heads, block, head]
@@ -71,45 +81,29 @@ def attention(query, key_cache, value_cache, context_lens, block_tables, attn_sc
     if key_cache.stride(-1) != 1 or any(s % 8 for s in key_cache.stride()[:-1]):
         key_cache, value_cache = key_cache.contiguous(), value_cache.contiguous()
 
-    lib = _C.load()
-    with torch.cuda.device(query.device):
-        num_sms = torch.cuda.get_device_properties(query.device).multi_processor_count
-        num_splits, partition_size = plan_partitions(num_seqs, num_kv_heads, kv_block_size,
-                                                     max_context_len, num_splits, num_sms)
+    with _C.device_guard(query.device):
+        num_splits, partition_size = plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_splits,
+                                                     _C.sm_count(query.device))
+        part_out = part_max = part_sum = 0
         if partition_size:
             assert partition_size >= kv_block_size and partition_size % kv_block_size == 0, \
                 f"partition_size={partition_size}, kv_block_size={kv_block_size}"
             assert partition_size % 16 == 0, f"partition_size={partition_size}"
+            ws, part_out, part_max, part_sum = partition_workspace(
+                num_seqs * num_q_heads, _cdiv(int(max_context_len), partition_size), head_size, query.device)
 
         out = torch.empty(query.shape, dtype=query.dtype, device=query.device)
-        args = _C.PagedArgs()
-        args.dtype = _C.dtype_code(query.dtype)
-        args.num_seqs, args.num_q_heads, args.num_kv_heads = num_seqs, num_q_heads, num_kv_heads
-        args.head_size, args.block_size = head_size, kv_block_size
-        args.max_context_len = int(max_context_len)
-        args.block_table_is_i64 = 1 if block_tables.dtype == torch.int64 else 0
-        args.partition_size = partition_size
-        args.attn_scale = float(attn_scale)
-        args.query, args.q_stride_s, args.q_stride_h = query.data_ptr(), query.stride(0), query.stride(1)
-        args.key_cache, args.value_cache = key_cache.data_ptr(), value_cache.data_ptr()
-        args.kv_stride_b, args.kv_stride_h, args.kv_stride_t = key_cache.stride()[:3]
-        args.context_lens = context_lens.data_ptr()
-        args.block_tables, args.bt_stride_s = block_tables.data_ptr(), block_tables.stride(0)
-        args.out, args.o_stride_s, args.o_stride_h = out.data_ptr(), out.stride(0), out.stride(1)
-        stream = _C.stream_ptr(query.device)
-
+        kb, kh, kt = key_cache.stride()[:3]
+        args = _C.PAGED_ARGS.pack(
+            _C.dtype_code(query.dtype), num_seqs, num_q_heads, num_kv_heads, head_size, kv_block_size,
+            int(max_context_len), 1 if block_tables.dtype == torch.int64 else 0, partition_size, attn_scale,
+            query.data_ptr(), query.stride(0), query.stride(1), key_cache.data_ptr(), value_cache.data_ptr(), kb, kh, kt,
+            context_lens.data_ptr(), block_tables.data_ptr(), block_tables.stride(0),
+            out.data_ptr(), out.stride(0), out.stride(1), part_out, part_max, part_sum, 0)
+        stream = _C.raw_stream(query.device)
+        _C.check(_C.call("fa_paged_decode")(args, stream), "fa_paged_decode")
         if partition_size:
-            P = _cdiv(int(max_context_len), partition_size)
-            part_out = torch.empty((num_seqs, num_q_heads, P, head_size), dtype=torch.float32,
-                                   device=query.device)
-            part_max = torch.empty((num_seqs, num_q_heads, P), dtype=torch.float32,
-                                   device=query.device)
-            part_sum = torch.empty_like(part_max)
-            args.part_out, args.part_max, args.part_sum = (part_out.data_ptr(), part_max.data_ptr(),
-                                                           part_sum.data_ptr())
-        _C.check(lib.fa_paged_decode(_C.byref(args), stream), "fa_paged_decode")
-        if partition_size:
-            _C.check(lib.fa_paged_reduce(_C.byref(args), stream), "fa_paged_reduce")
+            _C.check(_C.call("fa_paged_reduce")(args, stream), "fa_paged_reduce")
     return out
 
 
@@ -120,7 +114,6 @@ def reshape_and_cache(key, value, key_cache, value_cache, slot_mapping):
     slot_mapping [num_tokens] integer: token i goes to block slot // block, position slot % block;
     negative slots are skipped.  The reference has no writer (its tests fill the caches with random
     numbers); a serving loop runs this step right before the decode kernel."""
-    import ctypes
     num_tokens, num_kv_heads, head_size = key.shape
     assert value.shape == key.shape and key_cache.shape == value_cache.shape
     assert key_cache.shape[1] == num_kv_heads and key_cache.shape[3] == head_size
@@ -137,12 +130,10 @@ def reshape_and_cache(key, value, key_cache, value_cache, slot_mapping):
             or key.data_ptr() % 16 or value.data_ptr() % 16:
         key, value = key.contiguous(), value.contiguous()
     slots = slot_mapping.to(torch.int64).contiguous()
-    lib = _C.load()
-    with torch.cuda.device(key.device):
-        st = lib.fa_paged_cache_append(
-            _C.dtype_code(key.dtype), num_tokens, num_kv_heads, head_size, key_cache.shape[2],
-            _C.fptr(key), _C.fptr(value), ctypes.c_int64(key.stride(0)), ctypes.c_int64(key.stride(1)),
-            _C.fptr(key_cache), _C.fptr(value_cache), ctypes.c_int64(key_cache.stride(0)),
-            ctypes.c_int64(key_cache.stride(1)), ctypes.c_int64(key_cache.stride(2)),
-            _C.fptr(slots), _C.stream_ptr(key.device))
+    kb, kh, kt = key_cache.stride()[:3]
+    with _C.device_guard(key.device):
+        st = _C.call("fa_paged_cache_append")(
+            _C.dtype_code(key.dtype), num_tokens, num_kv_heads, head_size, key_cache.shape[2], key.data_ptr(),
+            value.data_ptr(), key.stride(0), key.stride(1), key_cache.data_ptr(), value_cache.data_ptr(), kb, kh, kt,
+            slots.data_ptr(), _C.raw_stream(key.device))
     _C.check(st, "fa_paged_cache_append")

@@ -4,7 +4,6 @@ Mirrors src/flag_attn/piecewise.py:25-191: score(m, n) = q2.k2 when the
 bottom-right-aligned distance (m + N - M) - n is at least `dist_threshold`,
 else q1.k1; returns the output only; gradients for the five tensors.
 """
-import ctypes
 import math
 
 import torch
@@ -32,15 +31,12 @@ class PiecewiseAttention(torch.autograd.Function):
         if sm_scale is None:
             sm_scale = 1. / math.sqrt(D)
         q1, k1, q2, k2, v = (_C.kernel_ready(x) for x in (q1, k1, q2, k2, v))
-        lib = _C.load()
-
-        with torch.cuda.device(q1.device):
+        with _C.device_guard(q1.device):
             o = torch.empty(q1.shape, dtype=q1.dtype, device=q1.device)
             L = torch.empty((B, H, M), device=q1.device, dtype=torch.float32)
-            shape = _C.flash_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale)
-            ts = [_C.tensor4(x) for x in (q1, k1, q2, k2, v, o)]
-            st = lib.fa_piecewise_fwd(_C.byref(shape), int(w), *[_C.byref(t) for t in ts],
-                                      _C.fptr(L), _C.stream_ptr(q1.device))
+            st = _C.call("fa_piecewise_fwd")(
+                _C.pack_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale), int(w),
+                *[_C.pack4(x) for x in (q1, k1, q2, k2, v, o)], L.data_ptr(), _C.raw_stream(q1.device))
             _C.check(st, "fa_piecewise_fwd")
 
         ctx.save_for_backward(q1, k1, q2, k2, v, o, L)
@@ -55,23 +51,20 @@ class PiecewiseAttention(torch.autograd.Function):
         w, causal, sm_scale = ctx.w, ctx.causal, ctx.sm_scale
         B, H, M, D = q1.shape
         N = k1.shape[2]
-        lib = _C.load()
         do = _C.kernel_ready(do)
 
-        with torch.cuda.device(q1.device):
-            stream = _C.stream_ptr(q1.device)
-            shape = _C.flash_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale)
+        with _C.device_guard(q1.device):
+            raw = _C.raw_stream(q1.device)
+            packed = _C.pack_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale)
+            packed_do = _C.pack4(do)
             delta = torch.empty_like(L)
-            to, tdo = _C.tensor4(o), _C.tensor4(do)
-            st = lib.fa_flash_bwd_delta(_C.byref(shape), _C.byref(to), _C.byref(tdo),
-                                        _C.fptr(delta), stream)
+            st = _C.call("fa_flash_bwd_delta")(packed, _C.pack4(o), packed_do, delta.data_ptr(), raw)
             _C.check(st, "fa_flash_bwd_delta")
 
-            ins = [_C.tensor4(x) for x in (q1, k1, q2, k2, v)]
             dk1 = torch.empty(k1.shape, dtype=k1.dtype, device=k1.device)
             dk2 = torch.empty(k2.shape, dtype=k2.dtype, device=k2.device)
             dv = torch.empty(v.shape, dtype=v.dtype, device=v.device)
-            ws_bytes = (lib.fa_piecewise_bwd_fused_workspace_bytes(_C.byref(shape))
+            ws_bytes = (_C.call("fa_piecewise_bwd_fused_workspace_bytes")(packed)
                         if use_one_pass_backward() else 0)
             if ws_bytes > 0:
                 # one launch: every key block walks its near tiles, then its far tiles; dq1 / dq2
@@ -79,15 +72,18 @@ class PiecewiseAttention(torch.autograd.Function):
                 dq1 = torch.empty(q1.shape, dtype=q1.dtype, device=q1.device)
                 dq2 = torch.empty(q2.shape, dtype=q2.dtype, device=q2.device)
                 ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q1.device)
-                outs = [_C.tensor4(x) for x in (dq1, dq2, dk1, dk2, dv)]
-                st = lib.fa_piecewise_bwd_fused(_C.byref(shape), w, *[_C.byref(t) for t in ins],
-                                                _C.byref(tdo), _C.fptr(L), _C.fptr(delta),
-                                                *[_C.byref(t) for t in outs], _C.fptr(ws),
-                                                ctypes.c_int64(ws_bytes), stream)
+                st = _C.call("fa_piecewise_bwd_fused")(
+                    packed, w, *[_C.pack4(x) for x in (q1, k1, q2, k2, v)], packed_do, L.data_ptr(), delta.data_ptr(),
+                    *[_C.pack4(x) for x in (dq1, dq2, dk1, dk2, dv)], ws.data_ptr(), ws_bytes, raw)
                 # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
                 if st != _C.FA_ERR_UNSUPPORTED:
                     _C.check(st, "fa_piecewise_bwd_fused")
                     return dq1, dk1, dq2, dk2, dv, None, None, None
+            lib = _C.load()
+            stream = _C.stream_ptr(q1.device)
+            shape = _C.flash_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale)
+            tdo = _C.tensor4(do)
+            ins = [_C.tensor4(x) for x in (q1, k1, q2, k2, v)]
             outs = [_C.tensor4(x) for x in (dk1, dk2, dv)]
             st = lib.fa_piecewise_bwd_dkdv(_C.byref(shape), w, *[_C.byref(t) for t in ins],
                                            _C.byref(tdo), _C.fptr(L), _C.fptr(delta),

@@ -65,13 +65,11 @@ class RotaryPair(torch.autograd.Function):
         tables, rows, stride = _tables_ready([cos1, sin1, cos2, sin2], D // 2, x.device)
         pos, pos_ptr, pos_stride = _positions_ready(positions, B, L, x.device)
         out1, out2 = torch.empty_like(x), torch.empty_like(x)
-        lib = _C.load()
-        with torch.cuda.device(x.device):
-            st = lib.fa_rotary_pair_fwd(
-                _C.dtype_code(x.dtype), B, H, L, D, 1 if interleaved else 0,
-                _C.byref(_C.tensor4(x)), *[_C.fptr(t) for t in tables], ctypes.c_int64(stride), rows,
-                pos_ptr, ctypes.c_int64(pos_stride), _C.byref(_C.tensor4(out1)),
-                _C.byref(_C.tensor4(out2)), _C.stream_ptr(x.device))
+        with _C.device_guard(x.device):
+            st = _C.call("fa_rotary_pair_fwd")(
+                _C.dtype_code(x.dtype), B, H, L, D, 1 if interleaved else 0, _C.pack4(x),
+                *[t.data_ptr() for t in tables], stride, rows, pos_ptr, pos_stride, _C.pack4(out1), _C.pack4(out2),
+                _C.raw_stream(x.device))
         _C.check(st, "fa_rotary_pair_fwd")
         ctx.save_for_backward(*tables, *([pos] if pos is not None else []))
         ctx.args = (stride, rows, pos_stride, bool(interleaved), pos is not None)
@@ -87,13 +85,11 @@ class RotaryPair(torch.autograd.Function):
         g1, g2 = _C.kernel_ready(g1), _C.kernel_ready(g2)
         B, H, L, D = g1.shape
         dx = torch.empty_like(g1)
-        lib = _C.load()
-        with torch.cuda.device(g1.device):
-            st = lib.fa_rotary_pair_bwd(
-                _C.dtype_code(g1.dtype), B, H, L, D, 1 if interleaved else 0,
-                _C.byref(_C.tensor4(g1)), _C.byref(_C.tensor4(g2)), *[_C.fptr(t) for t in tables],
-                ctypes.c_int64(stride), rows, pos_ptr, ctypes.c_int64(pos_stride),
-                _C.byref(_C.tensor4(dx)), _C.stream_ptr(g1.device))
+        with _C.device_guard(g1.device):
+            st = _C.call("fa_rotary_pair_bwd")(
+                _C.dtype_code(g1.dtype), B, H, L, D, 1 if interleaved else 0, _C.pack4(g1), _C.pack4(g2),
+                *[t.data_ptr() for t in tables], stride, rows, pos_ptr, pos_stride, _C.pack4(dx),
+                _C.raw_stream(g1.device))
         _C.check(st, "fa_rotary_pair_bwd")
         return dx, None, None, None, None, None, None
 

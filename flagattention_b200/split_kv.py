@@ -24,28 +24,26 @@ def get_fwd_config(B, H, M, N, D, causal):
 def num_splits_herustic(B, H, M, N, BLOCK_M, BLOCK_N, num_sms, max_splits):
     """Split count, computed by the library's restatement of
     src/flag_attn/split_kv.py:234-262 (name kept as spelled there)."""
+    if B * H * ((M + BLOCK_M - 1) // BLOCK_M) >= 0.8 * num_sms:
+        return 1      # the library's first rule: the unsplit grid fills the GPU
     return int(_C.load().fa_num_splits_heuristic(B, H, M, N, BLOCK_M, BLOCK_N, num_sms, max_splits))
 
 
 def _splitkv_forward(q, k, v, causal, sm_scale, S):
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
-    lib = _C.load()
     n_blocks = (N + _SPLIT_BLOCK_N - 1) // _SPLIT_BLOCK_N
     n_split_size = ((n_blocks + S - 1) // S) * _SPLIT_BLOCK_N
     S = (N + n_split_size - 1) // n_split_size  # drop splits that would be empty
     o_part = torch.empty((B, H, S, M, D), dtype=torch.float32, device=q.device)
     l_part = torch.empty((B, H, S, M), dtype=torch.float32, device=q.device)
-    o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    o = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
     L = torch.empty((B, H, M), dtype=torch.float32, device=q.device)
-    shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale)
-    tq, tk, tv, to = _C.tensor4(q), _C.tensor4(k), _C.tensor4(v), _C.tensor4(o)
-    stream = _C.stream_ptr(q.device)
-    st = lib.fa_splitkv_fwd(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv), S,
-                            n_split_size, _C.fptr(o_part), _C.fptr(l_part), stream)
+    shape, stream = _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale), _C.raw_stream(q.device)
+    st = _C.call("fa_splitkv_fwd")(shape, _C.pack4(q), _C.pack4(k), _C.pack4(v), S, n_split_size, o_part.data_ptr(),
+                                   l_part.data_ptr(), stream)
     _C.check(st, "fa_splitkv_fwd")
-    st = lib.fa_splitkv_combine(_C.byref(shape), S, _C.fptr(o_part), _C.fptr(l_part),
-                                _C.byref(to), _C.fptr(L), stream)
+    st = _C.call("fa_splitkv_combine")(shape, S, o_part.data_ptr(), l_part.data_ptr(), _C.pack4(o), L.data_ptr(), stream)
     _C.check(st, "fa_splitkv_combine")
     return o, L
 
