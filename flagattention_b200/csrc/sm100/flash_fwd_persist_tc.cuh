@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = instr_desc_f16(BM, BN, TcElem<T>::kFormat, 0, 0);
       constexpr uint32_t idesc_pv = instr_desc_f16(BM, D, TcElem<T>::kFormat, 0, 1);
       const uint32_t q_lo = smem_desc_lo(smem + C::kQ, 0);

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0 && E > 0) {
+    if (elect_one() && E > 0) {
       constexpr uint32_t idesc_s = instr_desc_f16(BM, BN, TcElem<T>::kFormat, 0, 0);
       constexpr uint32_t idesc_pv = instr_desc_f16(BM, D, TcElem<T>::kFormat, 0, 1);
       // descriptor low words: the issuing thread only adds a constant per MMA

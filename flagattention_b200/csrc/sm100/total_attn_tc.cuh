@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(TotalTcCfg<D>::kThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ---------------------------------
-    if (lane == 0 && T_tiles > 0) {
+    if (elect_one() && T_tiles > 0) {
       constexpr uint32_t idesc_s = instr_desc_f16(BN, BM, TcElem<T>::kFormat, 0, 0);
       constexpr uint32_t kTile16 = C::kTile >> 4;
       const uint32_t k_lo = smem_desc_lo(smem + C::kK, 0);
