@@ -13,7 +13,7 @@ import torch
 
 from . import _C
 from .dropout import philox_cuda_seed_offset
-from .paged import partition_workspace
+from .paged import coarsen_partition, partition_workspace
 from .split_kv import get_fwd_config as get_fwd_config_kv_split
 from .split_kv import num_splits_herustic, _splitkv_forward
 
@@ -139,11 +139,14 @@ def _decode_forward(q, k, v, sm_scale, causal=False):
     BS = 16
     sb, sh, sl, _ = k.stride()
     num_sms = _C.sm_count(q.device)
-    # partitions of the key axis: enough (batch, kv head, partition) CTAs for about eight waves,
-    # each long enough (>= 256 keys) to amortise its pipeline fill
-    partition_size = 256
-    while partition_size < 8192 and B * Hk * (N // (2 * partition_size)) >= 8 * num_sms:
-        partition_size *= 2
+    # Partitions of the key axis, long enough to amortise a CTA's pipeline fill and the reduction (one block a
+    # row goes through the row's partitions): about one wave of CTAs, up to 8192 keys where that leaves three.
+    # fp16, eight waves of at least 256 keys -> this: B=1 H=32 Hk=8 N=131072 D=128 218 -> 99 us (2048 keys: 117,
+    # 8192: 112), B=4 H=16 N=16384 D=64 67 -> 56 us (8192: 79), B=1 H=8 N=32768 73 -> 40 us, B=2 H=16 N=131072
+    # 339 -> 325 us (4096: 339).
+    partition_size = coarsen_partition(256, B * Hk, N, num_sms, 4096)
+    if partition_size == 4096 and B * Hk * ((N + 8191) // 8192) >= 3 * num_sms:
+        partition_size = 8192
     if N <= partition_size:
         partition_size = 0   # one pass, no reduction kernel
     table, ctx_lens = _identity_block_table(B, N // BS, sb // (BS * sl), q.device)
