@@ -184,7 +184,7 @@ extern "C" int fa_total_attention(const fa_flash_shape *s, const fa_tensor4 *q,
   if (int st = validate_shape(s)) return st;
   if (int st = validate_tensors({q, k})) return st;
   if (!lse || !total) return FA_ERR_BAD_ARG;
-  // head_dim 64 / 128 run on tcgen05; everything else on the shape-generic kernel
+  // what a tensor map can express runs on tcgen05; everything else on the shape-generic kernel
   const int tc_status = tc::total_attention_tc(s, q, k, lse, total, static_cast<cudaStream_t>(stream));
   if (tc_status <= 0) return tc_status;
   return dispatch_dtype_d(s->dtype, s->D,

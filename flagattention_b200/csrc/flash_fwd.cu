@@ -77,7 +77,7 @@ extern "C" int fa_flash_fwd(const fa_flash_shape *s, const fa_tensor4 *q, const 
   if (int st = validate_shape(s)) return st;
   if (int st = validate_tensors({q, k, v, o})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
-  // head_dim 64 / 128 run on tcgen05; everything else on the shape-generic kernel
+  // what a tensor map can express runs on tcgen05; everything else on the shape-generic kernel
   const int tc_status = tc::flash_fwd_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream));
   if (tc_status <= 0) return tc_status;
   FwdParams p = make_fwd_params(s, q, k, v);

@@ -39,7 +39,7 @@ extern "C" int fa_piecewise_fwd(const fa_flash_shape *s, int32_t dist_threshold,
   if (s->H != s->Hk) return FA_ERR_BAD_ARG;
   if (int st = validate_tensors({q1, k1, q2, k2, v, o})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
-  // head_dim 64 / 128 run on tcgen05; everything else on the shape-generic kernel
+  // what a tensor map can express runs on tcgen05; everything else on the shape-generic kernel
   const int tc_status = tc::piecewise_fwd_tc(s, dist_threshold, q1, k1, q2, k2, v, o, lse,
                                              static_cast<cudaStream_t>(stream));
   if (tc_status <= 0) return tc_status;

@@ -1,4 +1,4 @@
-// total_attention on tcgen05 (head_dim 64 and 128): tot[b, h, n] = sum over queries m of
+// total_attention on tcgen05 (head_dim 64 and 128; 16 and 32 as 64): tot[b, h, n] = sum over queries m of
 // P[m, n] = exp(sm_scale * q_m . k_n - lse_m), the column sums of the attention matrix recomputed
 // from the saved log-normaliser.
 //

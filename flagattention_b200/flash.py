@@ -19,7 +19,7 @@ from .split_kv import num_splits_herustic, _splitkv_forward
 
 __all__ = ["attention", "set_backward_mode", "get_backward_mode", "backward_mode"]
 
-# Which kernels compute the gradients at head_dim 64 / 128:
+# Which kernels compute the gradients:
 #   "one_pass"   one kernel for dq, dk, dv (five matrix products per tile); dq is summed with fp32
 #                reductions in global memory, so it is reproducible to fp32 rounding only;
 #   "two_kernel" a dK/dV kernel and a dQ kernel without any global reduction or atomic (seven

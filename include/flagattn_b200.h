@@ -157,7 +157,7 @@ int fa_flash_bwd_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_te
                        void *stream);
 
 /* The whole backward of flash_attention in one call: delta, the one-pass kernel above and the
- * conversion of dq, head_dim 16 .. 128 (16 and 32 run padded to 64).  Replaces the three launches of
+ * conversion of dq, head_dim 16 .. 128 (16 and 32 run padded to 64), with or without dropout.  Replaces the three launches of
  * src/flag_attn/flash.py:189-249.  `workspace` holds fa_flash_bwd_workspace_bytes bytes (16-byte aligned;
  * 0: the shape is not covered, call fa_flash_bwd_delta, fa_flash_bwd_dkdv and fa_flash_bwd_dq).  Same
  * reproducibility, and the same FA_ERR_UNSUPPORTED for broadcast strides, as fa_flash_bwd_fused. */
@@ -378,7 +378,8 @@ int fa_device_status(int32_t *out, int32_t clear);
 int fa_debug_wait_probe(int64_t limit_cycles, int32_t *left_flag, void *stream);
 
 /* Kernel family used by the flash / piecewise entry points: 0 (default) = tcgen05 kernels where
- * they cover the call (head_dim 64 / 128, no dropout, layouts a tensor map can express), the
+ * they cover the call (layouts a tensor map can express; head_dim 16 / 32 as 64, but the pair
+ * fa_flash_bwd_dkdv / fa_flash_bwd_dq at 64 / 128 without dropout only), the
  * shape-generic mma.sync kernels elsewhere; 1 = shape-generic kernels only (what the tests use to
  * cross-check the two families); 2 = as 0, but fa_flash_fwd launches one CTA per query tile even
  * where it would run its persistent kernel (calls with more query tiles than two per SM; that
