@@ -17,6 +17,7 @@ _lib = None
 _lock = threading.Lock()
 
 FA_F16, FA_BF16 = 0, 1
+FA_BLOCK_TABLE_IN_PLACE = 2
 
 EXPORTED_SYMBOLS = (
     "fa_flash_fwd", "fa_splitkv_fwd", "fa_splitkv_combine", "fa_splitkv_workspace_bytes",

@@ -6,15 +6,23 @@
 // gathers, swizzled shared memory), so nothing in the main loop needs a
 // CTA-wide barrier.  The tiny GEMMs (query group padded to 16 rows) run on
 // m16n8k16 tensor-core MMAs so that arithmetic never limits the stream.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace fa {
 
+// IdxT: the table's entry type, or InPlace where there is no table (FA_BLOCK_TABLE_IN_PLACE)
+struct InPlace {};
 template <typename IdxT>
 __device__ __forceinline__ int64_t phys_block(const void *block_tables, int64_t bt_stride_s,
                                               int seq, int logical_block) {
-  return (int64_t) reinterpret_cast<const IdxT *>(block_tables)[(int64_t)seq * bt_stride_s +
-                                                                logical_block];
+  const int64_t i = (int64_t)seq * bt_stride_s + logical_block;
+  if constexpr (std::is_same<IdxT, InPlace>::value) return i;
+  else return (int64_t) reinterpret_cast<const IdxT *>(block_tables)[i];
+}
+__device__ __forceinline__ int context_len(const fa_paged_args &a, int seq) {
+  return a.context_lens ? a.context_lens[seq] : a.max_context_len;
 }
 
 template <int D>
@@ -50,7 +58,7 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
   const int rows = min(16, G - qt * 16);          // valid query rows of this CTA
   const int qh0 = hk * G + qt * 16;               // first query head
 
-  const int ctx = a.context_lens[seq];
+  const int ctx = context_len(a, seq);
   const int t_begin = a.partition_size > 0 ? part * a.partition_size : 0;
   if (a.partition_size > 0 && t_begin >= ctx) return;
   const int t_end = a.partition_size > 0 ? min(ctx, t_begin + a.partition_size) : ctx;
@@ -332,7 +340,7 @@ __global__ void paged_reduce_kernel(const fa_paged_args a) {
   const int seq = blockIdx.x, qh = blockIdx.y;
   const int D = a.head_size;
   const int P = (a.max_context_len + a.partition_size - 1) / a.partition_size;
-  const int ctx = a.context_lens[seq];
+  const int ctx = context_len(a, seq);
   const int np = min(P, (ctx + a.partition_size - 1) / a.partition_size);
   const int64_t base = ((int64_t)seq * a.num_q_heads + qh) * P;
   float mm = -INFINITY;
@@ -369,10 +377,14 @@ __global__ void paged_trace_kernel(const fa_paged_args a, int64_t *visited, int 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+// no table and no lengths: the blocks of a sequence follow one another in memory
+static bool in_place(const fa_paged_args *a) {
+  return a->block_table_is_i64 == FA_BLOCK_TABLE_IN_PLACE && !a->block_tables && !a->context_lens;
+}
+
 static int validate_paged(const fa_paged_args *a, bool need_ws) {
-  if (!a || !a->query || !a->key_cache || !a->value_cache || !a->context_lens ||
-      !a->block_tables || !a->out)
-    return FA_ERR_BAD_ARG;
+  if (!a || !a->query || !a->key_cache || !a->value_cache || !a->out) return FA_ERR_BAD_ARG;
+  if ((!a->context_lens || !a->block_tables) && !in_place(a)) return FA_ERR_BAD_ARG;
   if (a->dtype != FA_F16 && a->dtype != FA_BF16) return FA_ERR_BAD_ARG;
   if (a->num_seqs <= 0 || a->num_q_heads <= 0 || a->num_kv_heads <= 0 || a->block_size <= 0 ||
       a->max_context_len <= 0 || a->partition_size < 0)
@@ -431,6 +443,9 @@ extern "C" int fa_paged_decode(const fa_paged_args *a, void *stream) {
   int st = validate_paged(a, true);
   if (st != FA_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (in_place(a))
+    return a->dtype == FA_F16 ? dispatch_paged_d<__half, InPlace>(a, s)
+                              : dispatch_paged_d<__nv_bfloat16, InPlace>(a, s);
   if (a->dtype == FA_F16)
     return a->block_table_is_i64 ? dispatch_paged_d<__half, int64_t>(a, s)
                                  : dispatch_paged_d<__half, int32_t>(a, s);
@@ -464,7 +479,7 @@ extern "C" int fa_paged_trace_blocks(const fa_paged_args *a, int64_t *visited, i
                                      void *stream) {
   int st = validate_paged(a, false);
   if (st != FA_OK) return st;
-  if (!visited || max_blocks <= 0) return FA_ERR_BAD_ARG;
+  if (!visited || max_blocks <= 0 || in_place(a)) return FA_ERR_BAD_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->block_table_is_i64)
     paged_trace_kernel<int64_t><<<a->num_seqs, 256, 0, s>>>(*a, visited, max_blocks);

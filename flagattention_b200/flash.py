@@ -90,23 +90,13 @@ def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0):
     return o, L
 
 
-_identity_tables = {}
-
-
 def _identity_block_table(B, blocks_per_batch, id_stride, device):
-    """(block_tables, context_lens) with block_tables[b, c] = b * id_stride + c, cached: the block
-    table under which a (B, Hk, N, D) key tensor is, in place, a paged cache of 16-token blocks."""
-    key = (B, blocks_per_batch, id_stride, str(device))
-    tab = _identity_tables.get(key)
-    if tab is None:
-        if len(_identity_tables) >= 8:
-            _identity_tables.clear()
-        tab = (torch.arange(B, device=device, dtype=torch.int32)[:, None] * id_stride +
-               torch.arange(blocks_per_batch, device=device, dtype=torch.int32)[None, :]).contiguous()
-        lens = torch.full((B,), blocks_per_batch * 16, dtype=torch.int32, device=device)
-        tab = (tab, lens)
-        _identity_tables[key] = tab
-    return tab
+    """(block_tables, context_lens) with block_tables[b, c] = b * id_stride + c: what FA_BLOCK_TABLE_IN_PLACE
+    stands for, under which a (B, Hk, N, D) key tensor is a paged cache of 16-token blocks.  The kernel works
+    the entries out itself; the tests hold it to this table."""
+    tab = (torch.arange(B, device=device, dtype=torch.int32)[:, None] * id_stride +
+           torch.arange(blocks_per_batch, device=device, dtype=torch.int32)[None, :]).contiguous()
+    return tab, torch.full((B,), blocks_per_batch * 16, dtype=torch.int32, device=device)
 
 
 _DECODE_MAX_ROWS = 64   # query rows (group x queries) per kv head the gather kernel is given
@@ -115,7 +105,7 @@ _DECODE_MAX_ROWS = 64   # query rows (group x queries) per kv head the gather ke
 def _decode_covered(q, k, v, causal=False):
     """Decode-shaped forward (a few queries per head, at most _DECODE_MAX_ROWS rows per kv head)
     that the paged-decode kernels can run directly on k and v: the keys of a batch element are then
-    a block table of 16-token blocks in place."""
+    16-token blocks that follow one another in memory."""
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
     if M < 1 or N % 16 != 0 or N == 0 or (H // Hk) * M > _DECODE_MAX_ROWS:
@@ -149,7 +139,6 @@ def _decode_forward(q, k, v, sm_scale, causal=False):
         partition_size = 8192
     if N <= partition_size:
         partition_size = 0   # one pass, no reduction kernel
-    table, ctx_lens = _identity_block_table(B, N // BS, sb // (BS * sl), q.device)
     q2 = q.reshape(B, H * M, D)
     if q2.stride(-1) != 1 or q2.data_ptr() % 16 or q2.stride(0) % 8 or q2.stride(1) % 8:
         q2 = q2.contiguous()
@@ -159,9 +148,9 @@ def _decode_forward(q, k, v, sm_scale, causal=False):
         P = (N + partition_size - 1) // partition_size
         ws, part_out, part_max, part_sum = partition_workspace(B * H * M, P, D, q.device)
     args = _C.PAGED_ARGS.pack(
-        _C.dtype_code(q.dtype), B, H * M, Hk, D, BS, N, 0, partition_size, sm_scale,
+        _C.dtype_code(q.dtype), B, H * M, Hk, D, BS, N, _C.FA_BLOCK_TABLE_IN_PLACE, partition_size, sm_scale,
         q2.data_ptr(), q2.stride(0), q2.stride(1), k.data_ptr(), v.data_ptr(),
-        BS * sl, sh if Hk > 1 else 0, sl, ctx_lens.data_ptr(), table.data_ptr(), table.stride(0),
+        BS * sl, sh if Hk > 1 else 0, sl, 0, 0, sb // (BS * sl),
         o.data_ptr(), H * M * D, D, part_out, part_max, part_sum, M if (causal and M > 1) else 0)
     stream = _C.raw_stream(q.device)
     _C.check(_C.call("fa_paged_decode")(args, stream), "fa_paged_decode")

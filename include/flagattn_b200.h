@@ -231,11 +231,17 @@ int fa_piecewise_bwd_fused(const fa_flash_shape *s, int32_t dist_threshold, cons
 /* paged_attention (single-token decode over a block-table KV cache)       */
 /* ---------------------------------------------------------------------- */
 
+/* fa_paged_args.block_table_is_i64 where there is no table: block_tables and context_lens are NULL,
+ * block c of sequence i is block i * bt_stride_s + c of the cache, and every context is
+ * max_context_len long.  That is a (batch, kv_heads, length, head) tensor read in place. */
+#define FA_BLOCK_TABLE_IN_PLACE 2
+
 typedef struct fa_paged_args {
   int32_t dtype;                 /* fa_dtype of query, caches and out              */
   int32_t num_seqs, num_q_heads, num_kv_heads, head_size, block_size;
   int32_t max_context_len;       /* host upper bound of context_lens               */
-  int32_t block_table_is_i64;    /* 0: int32 entries, 1: int64 entries             */
+  int32_t block_table_is_i64;    /* 0: int32 entries, 1: int64 entries, or         */
+                                 /* FA_BLOCK_TABLE_IN_PLACE                        */
   int32_t partition_size;        /* 0: one pass per (seq, kv head); else tokens    */
                                  /* per split-KV partition, a multiple of 16       */
   float attn_scale;
