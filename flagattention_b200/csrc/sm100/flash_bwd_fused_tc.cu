@@ -307,6 +307,11 @@ extern "C" int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const 
   if (!workspace || workspace_bytes < fa_flash_bwd_workspace_bytes(s) ||
       (reinterpret_cast<uintptr_t>(workspace) & 15))
     return FA_ERR_WORKSPACE;
+  // before the first launch: the caller's other path starts with delta again
+  for (const fa_tensor4 *t : {q, d_o, dq})
+    if (tc::is_broadcast(t, s->B, s->H, s->M)) return FA_ERR_UNSUPPORTED;
+  for (const fa_tensor4 *t : {k, v, dk, dv})
+    if (tc::is_broadcast(t, s->B, s->Hk, s->N)) return FA_ERR_UNSUPPORTED;
   float *ws = static_cast<float *>(workspace);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t acc = tc::fused_workspace_bytes(s);

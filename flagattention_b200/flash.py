@@ -195,6 +195,7 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
                 if st != _C.FA_ERR_UNSUPPORTED:
                     _C.check(st, "fa_flash_bwd")
                     return dq, dk, dv
+                del ws
         # the parts one by one
         stream = _C.stream_ptr(q.device)
         shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)

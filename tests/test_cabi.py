@@ -117,3 +117,21 @@ def test_rotary_pair_validation_needs_no_gpu(built_lib):
                                   i64(0), None, None) == 0    # empty batch: nothing to do
     assert lib.fa_rotary_pair_bwd(_C.FA_F16, 1, 2, 128, 64, 1, None, ctypes.byref(t), f, f, f, f, i64(32),
                                   10, None, i64(0), ctypes.byref(t), None) == -1
+
+
+def test_whole_backward_refuses_broadcast_views_before_any_launch(built_lib):
+    """A stride of 0 on a dimension longer than one goes to the pair of kernels, which starts with delta: fa_flash_bwd
+    must not have spent a launch and the zero-fill of its workspace by then (without a GPU a launch would be -4)."""
+    lib = _C.load()
+    shape = _C.FlashShape(_C.FA_BF16, 2, 4, 2, 300, 500, 32, 1, 0.1, 0.5, 1, 0)
+    dense = lambda heads, length: _C.Tensor4(0x1000, heads * length * 32, length * 32, 32)
+    q, kv = dense(4, 300), dense(2, 500)
+    n = _C.call("fa_flash_bwd_workspace_bytes")(bytes(shape))
+    call = lambda *ts: _C.call("fa_flash_bwd")(bytes(shape), *[bytes(t) for t in ts[:5]], 0x1000, *[bytes(t) for t in ts[5:]],
+                                               0x1000, n, 0)
+    shared_heads, shared_batch, one_row = (_C.Tensor4(0x1000, *s) for s in ((500 * 32, 0, 32), (0, 500 * 32, 32),
+                                                                           (2 * 32, 32, 0)))
+    for bad in (shared_heads, shared_batch, one_row):
+        assert call(q, bad, kv, q, q, q, kv, kv) == -2
+        assert call(q, kv, bad, q, q, q, kv, kv) == -2
+    assert call(_C.Tensor4(0x1000, 0, 32, 4 * 32), kv, kv, q, q, q, kv, kv) == -2
