@@ -149,7 +149,7 @@ _SIGNATURES = {
     "fa_paged_cache_append": "iiiiippllpplllpp", "fa_splitkv_fwd": "ppppiippp", "fa_splitkv_combine": "pippppp",
     "fa_total_attention": "pppppp", "fa_flash_bwd_delta": "ppppp", "fa_piecewise_bwd_fused_workspace_bytes": "p",
     "fa_piecewise_bwd_fused": "pi" + "p" * 14 + "lp", "fa_rotary_pair_fwd": "iiiiii" + "p" * 5 + "liplppp",
-    "fa_rotary_pair_bwd": "iiiiii" + "p" * 6 + "liplpp",
+    "fa_rotary_pair_bwd": "iiiiii" + "p" * 6 + "liplpp", "fa_num_splits_heuristic": "iiiiiiii",
 }
 _CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int32, "l": ctypes.c_int64}
 _calls = {}

@@ -24,9 +24,7 @@ def get_fwd_config(B, H, M, N, D, causal):
 def num_splits_herustic(B, H, M, N, BLOCK_M, BLOCK_N, num_sms, max_splits):
     """Split count, computed by the library's restatement of
     src/flag_attn/split_kv.py:234-262 (name kept as spelled there)."""
-    if B * H * ((M + BLOCK_M - 1) // BLOCK_M) >= 0.8 * num_sms:
-        return 1      # the library's first rule: the unsplit grid fills the GPU
-    return int(_C.load().fa_num_splits_heuristic(B, H, M, N, BLOCK_M, BLOCK_N, num_sms, max_splits))
+    return _C.call("fa_num_splits_heuristic")(B, H, M, N, BLOCK_M, BLOCK_N, num_sms, max_splits)
 
 
 def _splitkv_forward(q, k, v, causal, sm_scale, S):
