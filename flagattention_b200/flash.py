@@ -115,9 +115,8 @@ def _decode_covered(q, k, v, causal=False):
     if k.stride() != v.stride() or k.stride(3) != 1 or k.data_ptr() % 16 or v.data_ptr() % 16:
         return False
     sb, sh, sl, _ = k.stride()
-    if sl % 8 or sh % 8 or sb % (16 * sl) or (B * (sb // (16 * sl))) >= 2 ** 31:
-        return False
-    return True
+    # (one row broadcast over the length has stride 0: no block of it follows another)
+    return sl > 0 and not (sl % 8 or sh % 8 or sb % (16 * sl))
 
 
 def _decode_forward(q, k, v, sm_scale, causal=False):

@@ -144,6 +144,8 @@ def test_single_query_dispatch_rule():
     kt = torch.zeros(2, 1024, 2, 64, dtype=torch.float16).transpose(1, 2)                   # BTHD view
     assert fl._decode_covered(q, kt, kt.clone(memory_format=torch.preserve_format))
     assert not fl._decode_covered(q, kt, v)                                                 # strides differ
+    one = torch.zeros(2, 2, 1, 64, dtype=torch.float16).expand(2, 2, 1024, 64)              # one key, broadcast
+    assert not fl._decode_covered(q, one, one)
     tab, lens = fl._identity_block_table(2, 4, 16, "cpu")
     assert tab.tolist() == [[0, 1, 2, 3], [16, 17, 18, 19]] and lens.tolist() == [64, 64]
 
