@@ -69,7 +69,8 @@ static __device__ __noinline__ PersistItem persist_decode(const FwdTcParams &p, 
   return it;
 }
 
-template <typename T, int D>
+// PAD as in flash_fwd_tc_kernel.
+template <typename T, int D, bool PAD>
 __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
     flash_fwd_persist_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                 const __grid_constant__ CUtensorMap map_k,
@@ -235,6 +236,11 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
         for (int kk = 0; kk < BN / 16; ++kk)
           mma_ts_lo(tmem + C::kColO, a_col + kk * 8, b_lo + ((kk * 16 * 128) >> 4), idesc_pv,
                     (kk > 0 || !first) ? 1u : 0u);
+        if (PAD) {   // the remainder of P
+#pragma unroll
+          for (int kk = 0; kk < BN / 16; ++kk)
+            mma_ts_lo(tmem + C::kColO, a_col + BN / 2 + kk * 8, b_lo + ((kk * 16 * 128) >> 4), idesc_pv, 1u);
+        }
         mma_commit(bar(FP_PV_DONE + st));
         mma_commit(bar(FP_V_FREE + st));
         return true;
@@ -375,7 +381,7 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
         }
         const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
         const float neg_ms = -m_eff * qk_scale;
-        uint32_t pk[BN / 2];
+        uint32_t pk[BN / 2], pr[PAD ? BN / 2 : 1];
         // packed fp32 pairs: one FMA and one add per two elements
         const uint64_t scale2 = f2_pack(qk_scale, qk_scale), shift2 = f2_pack(neg_ms, neg_ms);
         uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};
@@ -386,6 +392,10 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
           const float p0 = ex2(x0), p1 = ex2(x1);
           rs2[(c >> 1) & 3] = f2_add(rs2[(c >> 1) & 3], f2_pack(p0, p1));
           pk[c >> 1] = TcElem<T>::pack(p0, p1);
+          if (PAD) {
+            const float2 f = TcElem<T>::unpack(pk[c >> 1]);
+            pr[c >> 1] = TcElem<T>::pack(p0 - f.x, p1 - f.y);
+          }
         }
         {
           float a0, a1;
@@ -393,6 +403,7 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
           l += a0 + a1;
         }
         tmem_st32(scol, reinterpret_cast<const uint32_t(&)[32]>(pk));
+        if constexpr (PAD) tmem_st32(scol + BN / 2, pr);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -437,7 +448,7 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
               v.y = TcElem<T>::pack(__uint_as_float(ov[hh][8 * i + 2]) * inv, __uint_as_float(ov[hh][8 * i + 3]) * inv);
               v.z = TcElem<T>::pack(__uint_as_float(ov[hh][8 * i + 4]) * inv, __uint_as_float(ov[hh][8 * i + 5]) * inv);
               v.w = TcElem<T>::pack(__uint_as_float(ov[hh][8 * i + 6]) * inv, __uint_as_float(ov[hh][8 * i + 7]) * inv);
-              if (c * 64 + hh * 32 + i * 8 < p.d)
+              if (!PAD || c * 64 + hh * 32 + i * 8 < p.d)
                 *reinterpret_cast<uint4 *>(orow + c * 64 + hh * 32 + i * 8) = v;
             }
         }
@@ -445,7 +456,7 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
       if (row < p.M) {
         const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
         p.lse[((int64_t)it.b * p.H + it.h) * p.M + row] =
-            l > 0.f ? m_eff * p.sm_scale + logf(l) : -INFINITY;
+            l > 0.f ? (PAD ? m_eff * qk_scale * kLn2 : m_eff * p.sm_scale) + logf(l) : -INFINITY;
       }
     }
   }

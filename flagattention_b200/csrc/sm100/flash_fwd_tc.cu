@@ -26,7 +26,7 @@ int set_kernel_family(int family) {
   return g_kernel_family.exchange(family == 1 ? 1 : (family == 2 ? 2 : 0));
 }
 
-template <typename T, int D, bool PW, bool DROP = false>
+template <typename T, int D, bool PW, bool DROP = false, bool PAD = false>
 static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, const fa_tensor4 *k,
                          const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
                          const fa_tensor4 *o, float *lse, cudaStream_t stream) {
@@ -40,7 +40,7 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   if (PW && (!make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
              !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN)))
     return 1;
-  auto kern = flash_fwd_tc_kernel<T, D, PW, DROP>;
+  auto kern = flash_fwd_tc_kernel<T, D, PW, DROP, PAD>;
   static unsigned long long done = 0;
   if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
   FwdTcParams p{};
@@ -103,7 +103,7 @@ static int sm_count_fwd() {
 }
 
 // The persistent form (flash_fwd_persist_tc.cuh): two CTAs per SM that work through the query tiles.
-template <typename T, int D>
+template <typename T, int D, bool PAD = false>
 static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                               const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream) {
   using C = FwdPersistCfg<D>;
@@ -112,7 +112,7 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
       !make_map_bhld(&mk, k, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
       !make_map_bhld(&mv, v, s->dtype, s->B, s->Hk, s->N, s->D, C::BN))
     return 1;
-  auto kern = flash_fwd_persist_tc_kernel<T, D>;
+  auto kern = flash_fwd_persist_tc_kernel<T, D, PAD>;
   static unsigned long long done = 0;
   if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
   FwdPersistParams fp{};
@@ -168,7 +168,10 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
   if (!one_cta_per_tile_forced() && short_walks &&
       (int64_t)((s->M + 127) / 128) * s->B * s->H > 2 * (int64_t)sm_count_fwd()) {
     int st;
-    if (s->dtype == FA_F16)
+    if (s->D < 64)
+      st = s->dtype == FA_F16 ? launch_fwd_persist<__half, 64, true>(s, q, k, v, o, lse, stream)
+                              : launch_fwd_persist<__nv_bfloat16, 64, true>(s, q, k, v, o, lse, stream);
+    else if (s->dtype == FA_F16)
       st = s->D == 128 ? launch_fwd_persist<__half, 128>(s, q, k, v, o, lse, stream)
                        : launch_fwd_persist<__half, 64>(s, q, k, v, o, lse, stream);
     else
@@ -176,6 +179,10 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
                        : launch_fwd_persist<__nv_bfloat16, 64>(s, q, k, v, o, lse, stream);
     if (st != 1) return st;
   }
+  if (s->D < 64)
+    return s->dtype == FA_F16
+               ? launch_fwd_tc<__half, 64, false, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
+               : launch_fwd_tc<__nv_bfloat16, 64, false, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
   if (s->dtype == FA_F16)
     return s->D == 128 ? launch_fwd_tc<__half, 128, false>(s, 0, q, k, q, k, v, o, lse, stream)
                        : launch_fwd_tc<__half, 64, false>(s, 0, q, k, q, k, v, o, lse, stream);
@@ -187,6 +194,10 @@ int piecewise_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q1, const
                      const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
                      const fa_tensor4 *o, float *lse, cudaStream_t stream) {
   if (!covered(s) || s->dropout_p > 0.f || w > (1 << 29) || w < -(1 << 29)) return 1;
+  if (s->D < 64)
+    return s->dtype == FA_F16
+               ? launch_fwd_tc<__half, 64, true, false, true>(s, w, q1, k1, q2, k2, v, o, lse, stream)
+               : launch_fwd_tc<__nv_bfloat16, 64, true, false, true>(s, w, q1, k1, q2, k2, v, o, lse, stream);
   if (s->dtype == FA_F16)
     return s->D == 128 ? launch_fwd_tc<__half, 128, true>(s, w, q1, k1, q2, k2, v, o, lse, stream)
                        : launch_fwd_tc<__half, 64, true>(s, w, q1, k1, q2, k2, v, o, lse, stream);

@@ -31,7 +31,7 @@ struct FwdTcParams {
   int w;  // piecewise distance threshold (PW kernels only)
   int *status;
   int num_m_blocks, group_size;  // launch order, see grouped_cta()
-  int d;          // head_dim of the tensors: D, or less when the columns up to D are padding
+  int d;          // head_dim of the tensors: D, or less when the columns up to D are padding (DROP and PAD kernels)
   DropoutRule drop;   // DROP kernels only
 };
 
@@ -63,7 +63,13 @@ enum FwdBar { Q_FULL = 0, K_FULL = 1, K_FREE = 3, V_FULL = 5, V_FREE = 7, S_FULL
 // re-loaded once, at the switch from the far to the near entries.
 // DROP = dropout on the probabilities that enter P V (the row sums stay undropped).  The keep bits of a
 // tile do not depend on its scores: they are computed before the wait for them.
-template <typename T, int D, bool PW, bool DROP>
+// PAD = the head_dim of the tensors is below D.
+// Both also give P to P V as a 16-bit value and a 16-bit remainder, in the two halves of the S columns: these
+// calls once ran on kernels that follow the row maximum exactly, so that a row's largest weight is 1 and has no
+// rounding error; here the reference may lag it by 2^8.  B=2 H=8 L=777 D=32 causal, bf16, scores of deviation 4,
+// error of o against 64 bits: exact maximum 1.73e-3, P rounded once 2.06e-3, with the remainder 1.66e-3 (the rounding
+// of o).  It costs 4 to 20 % of the kernel: D=32 B=4 H=16 L=2048 causal 74 -> 84 us, dropout at D=64 317 -> 336 us.
+template <typename T, int D, bool PW, bool DROP, bool PAD>
 __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
     flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                         const __grid_constant__ CUtensorMap map_k,
@@ -72,6 +78,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
                         const __grid_constant__ CUtensorMap map_k2, const FwdTcParams p) {
   using C = FwdTcCfg<D>;
   constexpr int BM = C::BM, BN = C::BN, KSUB = C::KSUB;
+  constexpr bool FINE = DROP || PAD;
   extern __shared__ uint8_t smem_unaligned[];
   const uint32_t smem = (smem_u32(smem_unaligned) + 1023u) & ~1023u;
   uint8_t *smem_gen = smem_unaligned + (smem - smem_u32(smem_unaligned));
@@ -212,6 +219,11 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
         for (int kk = 0; kk < BN / 16; ++kk)
           mma_ts_lo(tmem + C::kColO, a_col + kk * 8, b_lo + ((kk * 16 * 128) >> 4), idesc_pv,
                     kk > 0 ? 1u : acc);
+        if (FINE) {
+#pragma unroll
+          for (int kk = 0; kk < BN / 16; ++kk)
+            mma_ts_lo(tmem + C::kColO, a_col + BN / 2 + kk * 8, b_lo + ((kk * 16 * 128) >> 4), idesc_pv, 1u);
+        }
         mma_commit(bar(PV_DONE + st));
         mma_commit(bar(V_FREE + st));
         return true;
@@ -329,7 +341,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       }
       const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
       const float neg_ms = -m_eff * qk_scale;
-      uint32_t pk[BN / 2];
+      uint32_t pk[BN / 2], pr[FINE ? BN / 2 : 1];
       // packed fp32 pairs: one FMA and one add per two elements
       const uint64_t scale2 = f2_pack(qk_scale, qk_scale), shift2 = f2_pack(neg_ms, neg_ms);
       uint64_t rs2[4] = {0ull, 0ull, 0ull, 0ull};
@@ -344,6 +356,10 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
           if (!(keep[c >> 5] >> ((c + 1) & 31) & 1u)) p1 = 0.f;
         }
         pk[c >> 1] = TcElem<T>::pack(p0, p1);
+        if (FINE) {
+          const float2 f = TcElem<T>::unpack(pk[c >> 1]);
+          pr[c >> 1] = TcElem<T>::pack(p0 - f.x, p1 - f.y);
+        }
       }
       {
         float a0, a1;
@@ -351,6 +367,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
         l += a0 + a1;
       }
       tmem_st32(scol, reinterpret_cast<const uint32_t(&)[32]>(pk));
+      if constexpr (FINE) tmem_st32(scol + BN / 2, pr);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -386,14 +403,15 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
             v.y = TcElem<T>::pack(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv);
             v.z = TcElem<T>::pack(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv);
             v.w = TcElem<T>::pack(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv);
-            if (c * 32 + i * 8 < p.d) *reinterpret_cast<uint4 *>(orow + c * 32 + i * 8) = v;
+            if (!FINE || c * 32 + i * 8 < p.d) *reinterpret_cast<uint4 *>(orow + c * 32 + i * 8) = v;
           }
         }
       }
       if (row < p.M) {
         const float m_eff = (m_used == -INFINITY) ? 0.f : m_used;
+        // FINE: from the shift that the exponents were rounded with
         p.lse[((int64_t)b * p.H + h) * p.M + row] =
-            l > 0.f ? m_eff * p.sm_scale + logf(l) : -INFINITY;
+            l > 0.f ? (FINE ? m_eff * qk_scale * kLn2 : m_eff * p.sm_scale) + logf(l) : -INFINITY;
       }
     }
   }
