@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "flagattn_b200.h"
 
 namespace fa {
@@ -58,6 +60,24 @@ struct Elem<__nv_bfloat16> {
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
 };
+
+// Two weights x, y >= 0 as packed 16-bit values and packed 16-bit remainders.  The values are rounded down and the
+// remainders kept above 0 wherever the weight is, so that both have its sign: times an infinite V they give that
+// infinity and not NaN (a weight of 0 gives NaN, as it always did).
+template <typename T>
+__device__ __forceinline__ void split_weights(float x, float y, uint32_t &value, uint32_t &rest) {
+  if constexpr (std::is_same<T, __half>::value) {
+    constexpr float tiny = 5.9604645e-8f;   // 2^-24, the smallest fp16 number
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;\n" : "=r"(value) : "f"(y), "f"(x));
+    const float2 f = Elem<T>::unpack(value);
+    rest = Elem<T>::pack(fminf(fmaxf(x - f.x, tiny), x), fminf(fmaxf(y - f.y, tiny), y));
+  } else {
+    constexpr float up = 1.f + 9.5367431640625e-7f;   // 1 + 2^-20, the same factor for every weight
+    asm("cvt.rz.bf16x2.f32 %0, %1, %2;\n" : "=r"(value) : "f"(y), "f"(x));
+    const float2 f = Elem<T>::unpack(value);
+    rest = Elem<T>::pack(fmaf(x, up, -f.x), fmaf(y, up, -f.y));
+  }
+}
 
 // ---------------------------------------------------------------------------
 // shared memory tiles: ROWS x D 16-bit elements, 16-byte chunks XOR-swizzled

@@ -6,8 +6,6 @@
 // gathers, swizzled shared memory), so nothing in the main loop needs a
 // CTA-wide barrier.  The tiny GEMMs (query group padded to 16 rows) run on
 // m16n8k16 tensor-core MMAs so that arithmetic never limits the stream.
-#include <type_traits>
-
 #include "common.cuh"
 
 namespace fa {
@@ -40,11 +38,13 @@ struct PagedCfg {
   static constexpr int kTotal = kRing + (kRingBytes > kMergeBytes ? kRingBytes : kMergeBytes);
 };
 
-template <typename T, int D, typename IdxT>
+// HALF: at most 8 query rows, the upper half of the 16-row tile; the lower half serves the remainder of P.
+template <typename T, int D, typename IdxT, bool HALF>
 __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
     const fa_paged_args a) {
   using C = PagedCfg<D>;
   constexpr int NW = C::kWarps, NS = C::kStages, CPR = D / 8;
+  constexpr int R = HALF ? 1 : 2;   // accumulator rows of a thread: g and, in a full tile, g + 8
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const uint32_t smem = smem_u32(smem_raw);
 
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
   int row_end[2] = {t_end, t_end};
   if (a.causal_rows > 0) {
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < R; ++r) {
       const int m = (qt * 16 + g + 8 * r) % a.causal_rows;
       row_end[r] = min(t_end, ctx - (a.causal_rows - 1 - m));
     }
@@ -191,11 +191,11 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
         Elem<T>::mma(s[1], qa, bb[2], bb[3]);
       }
     }
-    const bool tail = tok0 + 16 > min(row_end[0], row_end[1]);
+    const bool tail = tok0 + 16 > min(row_end[0], row_end[R - 1]);
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 2 * R; ++e) {
         const int tok = tok0 + j * 8 + 2 * t4 + (e & 1);
         s[j][e] = (tail && tok >= row_end[e >> 1]) ? -INFINITY : s[j][e] * qk_scale;
       }
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
     float m_new[2];
     bool need = false;
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < R; ++r) {
       float mx = fmaxf(fmaxf(s[0][2 * r], s[0][2 * r + 1]), fmaxf(s[1][2 * r], s[1][2 * r + 1]));
       mx = quad_max(mx);
       m_new[r] = fmaxf(m_i[r], mx);  // -inf only while a row has not seen a token it may see
@@ -213,19 +213,18 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
     }
     if (__any_sync(0xffffffffu, need)) {
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
+      for (int r = 0; r < R; ++r) {
         const float alpha = (m_new[r] == -INFINITY) ? 1.f : fast_exp2(m_i[r] - m_new[r]);
         l_i[r] *= alpha;
         m_i[r] = m_new[r];
 #pragma unroll
-        for (int j = 0; j < D / 8; ++j) {
-          acc[j][2 * r] *= alpha;
-          acc[j][2 * r + 1] *= alpha;
-        }
+        for (int j = 0; j < D / 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4 / R; ++e) acc[j][2 * r + e] *= alpha;
       }
     }
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < R; ++r) {
       float rs = 0.f;
       const float m_ref = (m_i[r] == -INFINITY) ? 0.f : m_i[r];   // all scores -inf: P = 0
 #pragma unroll
@@ -238,15 +237,15 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
     }
     // P goes in as a 16-bit value and a 16-bit remainder.  Rounded once, its error depends on the run of tokens a
     // warp takes: the one that sets the run's reference maximum has weight 1 and no error, so shorter runs have
-    // less of it (fp16, 2048 tokens, the rounding restated on the host: 2.83e-4 with runs of 64, 2.93e-4 of 512;
-    // with the remainder 2.04e-4 for both, the rounding of the output alone).
+    // less of it (fp16, 64 sequences to 32768: 2.79e-4 with partitions of 256, 2.90e-4 of 2048; with the remainder
+    // 2.07e-4, the rounding of the output alone).
     uint32_t pa[4], pr[4];
+    if (HALF) {
+      split_weights<T>(s[0][0], s[0][1], pa[0], pa[1]);
+      split_weights<T>(s[1][0], s[1][1], pa[2], pa[3]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float x = s[i >> 1][2 * (i & 1)], y = s[i >> 1][2 * (i & 1) + 1];
-      pa[i] = Elem<T>::pack(x, y);
-      const float2 f = Elem<T>::unpack(pa[i]);
-      pr[i] = Elem<T>::pack(x - f.x, y - f.y);
+      for (int i = 0; i < 4; ++i) split_weights<T>(s[i >> 1][2 * (i & 1)], s[i >> 1][2 * (i & 1) + 1], pa[i], pr[i]);
     }
 #pragma unroll
     for (int dj = 0; dj < D / 16; ++dj) {
@@ -254,19 +253,26 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
       load_B_kn<D>(bb, st + C::kGroupBytes, 0, dj * 2, lane);
       Elem<T>::mma(acc[2 * dj], pa, bb[0], bb[1]);
       Elem<T>::mma(acc[2 * dj + 1], pa, bb[2], bb[3]);
-      Elem<T>::mma(acc[2 * dj], pr, bb[0], bb[1]);
-      Elem<T>::mma(acc[2 * dj + 1], pr, bb[2], bb[3]);
+      if (!HALF) {
+        Elem<T>::mma(acc[2 * dj], pr, bb[0], bb[1]);
+        Elem<T>::mma(acc[2 * dj + 1], pr, bb[2], bb[3]);
+      }
     }
     __syncwarp();  // stage may be refilled by the next iteration's issue
   }
   cp_async_wait<0>();
+
+  if (HALF) {
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) acc[j][0] += acc[j][2], acc[j][1] += acc[j][3];
+  }
 
   // ---- merge the warps' partial states --------------------------------------
   float *stat_m = reinterpret_cast<float *>(smem_raw + C::kQBytes);
   float *stat_l = stat_m + NW * 16;
   float *merge = reinterpret_cast<float *>(smem_raw + C::kRing);
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
+  for (int r = 0; r < R; ++r) {
     const float l = quad_sum(l_i[r]);
     if (t4 == 0) {
       stat_m[warp * 16 + g + 8 * r] = m_i[r];
@@ -274,18 +280,17 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
     }
   }
   __syncthreads();  // stats visible; every warp has drained its ring
-  float m_all[2], scale_w[2];
+  float scale_w[2];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
+  for (int r = 0; r < R; ++r) {
     const int row = g + 8 * r;
     float mm = -INFINITY;
 #pragma unroll
     for (int w2 = 0; w2 < NW; ++w2) mm = fmaxf(mm, stat_m[w2 * 16 + row]);
-    m_all[r] = mm;
     scale_w[r] = (m_i[r] == -INFINITY) ? 0.f : fast_exp2(m_i[r] - mm);
   }
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
+  for (int r = 0; r < R; ++r) {
     const int row = g + 8 * r;
     if (row < rows) {
       float *dst = merge + ((int64_t)warp * 16 + row) * D;
@@ -331,7 +336,6 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
       *reinterpret_cast<uint2 *>(dst) = pk;
     }
   }
-  (void)m_all;
 }
 
 // One CTA per (seq, query head); thread d4 owns 4 output columns.
@@ -406,10 +410,10 @@ static int validate_paged(const fa_paged_args *a, bool need_ws) {
   return FA_OK;
 }
 
-template <typename T, int D, typename IdxT>
+template <typename T, int D, typename IdxT, bool HALF>
 static int launch_paged(const fa_paged_args *a, cudaStream_t stream) {
   using C = PagedCfg<D>;
-  auto kern = paged_decode_kernel<T, D, IdxT>;
+  auto kern = paged_decode_kernel<T, D, IdxT, HALF>;
   static unsigned long long attr_done = 0;  // per instantiation, one bit per device
   if (int st = ensure_dyn_smem(kern, C::kTotal, &attr_done)) return st;
   const int G = a->num_q_heads / a->num_kv_heads;
@@ -425,12 +429,18 @@ static int launch_paged(const fa_paged_args *a, cudaStream_t stream) {
 
 template <typename T, typename IdxT>
 static int dispatch_paged_d(const fa_paged_args *a, cudaStream_t stream) {
+  const bool half = a->num_q_heads / a->num_kv_heads <= 8;
   switch (a->head_size) {
-    case 16: return launch_paged<T, 16, IdxT>(a, stream);
-    case 32: return launch_paged<T, 32, IdxT>(a, stream);
-    case 64: return launch_paged<T, 64, IdxT>(a, stream);
-    case 128: return launch_paged<T, 128, IdxT>(a, stream);
-    case 256: return launch_paged<T, 256, IdxT>(a, stream);
+    case 16:
+      return half ? launch_paged<T, 16, IdxT, true>(a, stream) : launch_paged<T, 16, IdxT, false>(a, stream);
+    case 32:
+      return half ? launch_paged<T, 32, IdxT, true>(a, stream) : launch_paged<T, 32, IdxT, false>(a, stream);
+    case 64:
+      return half ? launch_paged<T, 64, IdxT, true>(a, stream) : launch_paged<T, 64, IdxT, false>(a, stream);
+    case 128:
+      return half ? launch_paged<T, 128, IdxT, true>(a, stream) : launch_paged<T, 128, IdxT, false>(a, stream);
+    case 256:
+      return half ? launch_paged<T, 256, IdxT, true>(a, stream) : launch_paged<T, 256, IdxT, false>(a, stream);
   }
   return FA_ERR_UNSUPPORTED;
 }

@@ -391,11 +391,8 @@ __global__ void __launch_bounds__(FwdPersistCfg<D>::kThreads, 2)
           f2_unpack(f2_fma(f2_pack(s[c], s[c + 1]), scale2, shift2), x0, x1);
           const float p0 = ex2(x0), p1 = ex2(x1);
           rs2[(c >> 1) & 3] = f2_add(rs2[(c >> 1) & 3], f2_pack(p0, p1));
-          pk[c >> 1] = TcElem<T>::pack(p0, p1);
-          if (PAD) {
-            const float2 f = TcElem<T>::unpack(pk[c >> 1]);
-            pr[c >> 1] = TcElem<T>::pack(p0 - f.x, p1 - f.y);
-          }
+          if constexpr (PAD) split_weights<T>(p0, p1, pk[c >> 1], pr[c >> 1]);
+          else pk[c >> 1] = TcElem<T>::pack(p0, p1);
         }
         {
           float a0, a1;

@@ -355,11 +355,8 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
           if (!(keep[c >> 5] >> (c & 31) & 1u)) p0 = 0.f;
           if (!(keep[c >> 5] >> ((c + 1) & 31) & 1u)) p1 = 0.f;
         }
-        pk[c >> 1] = TcElem<T>::pack(p0, p1);
-        if (FINE) {
-          const float2 f = TcElem<T>::unpack(pk[c >> 1]);
-          pr[c >> 1] = TcElem<T>::pack(p0 - f.x, p1 - f.y);
-        }
+        if constexpr (FINE) split_weights<T>(p0, p1, pk[c >> 1], pr[c >> 1]);
+        else pk[c >> 1] = TcElem<T>::pack(p0, p1);
       }
       {
         float a0, a1;

@@ -46,3 +46,15 @@ def test_dense(B, H, Hk, M, N, D, dtype):
     kk, vv = (x.double().repeat_interleave(H // Hk, 1) for x in (k, v))
     want = torch.softmax(q.double() @ kk.transpose(2, 3) * D ** -0.5, -1) @ vv
     assert _relative(fa.flash_attention(q, k, v), want) <= _limit(want, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("group", [1, 8, 16])
+def test_infinite_values(group, dtype):
+    """An infinite value gives its column that infinity, with the remainder in rows of its own (up to 8) and without."""
+    gen = torch.Generator(device="cuda").manual_seed(group)
+    q, k, v = (torch.randn((2, h, n, 64), generator=gen, device="cuda", dtype=dtype) for h, n in ((2 * group, 1), (2, 1040), (2, 1040)))
+    v[:, :, 700, 3], v[:, :, 5, 60] = float("inf"), -float("inf")
+    o = fa.flash_attention(q, k, v)
+    assert (o[..., 3] == float("inf")).all() and (o[..., 60] == -float("inf")).all()
+    assert o.isfinite().sum() == o.numel() // 64 * 62

@@ -70,3 +70,14 @@ def test_dropout(B, H, Hk, M, N, D, causal, dtype, scale):
     o, _, _, seed, offset = fa.flash_attention(q, k, v, causal, dropout_p=p, return_seed_offset=True)
     keep = fa.testing.recompute_mask(B, H, M, N, p, seed, offset, "cuda").double() / (1 - p)
     _check(o, _exact(q, k, v, causal, keep)[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,M,N,D", [(2, 300, 2100, 16), (2, 300, 1100, 32), (40, 300, 1100, 32)])
+def test_infinite_values(B, M, N, D, dtype):
+    """An infinite value that every query sees gives its column that infinity."""
+    q, k, v = _inputs(dtype, 1.0, (B, 4, M, D), (B, 4, N, D), (B, 4, N, D))
+    v[:, :, 100, 3], v[:, :, 5, 9] = float("inf"), -float("inf")
+    o = fa.flash_attention(q, k, v)
+    assert (o[..., 3] == float("inf")).all() and (o[..., 9] == -float("inf")).all()
+    assert o.isfinite().sum() == o.numel() // D * (D - 2)
