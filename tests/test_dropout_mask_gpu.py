@@ -1,6 +1,6 @@
 """The keep bits the tcgen05 kernels compute for themselves, element by element against the mask the library
-regenerates: counters that cross 2^32 inside a tile (and inside a thread's run of 32), ragged sizes, grouped heads.
-With q = k = 0 every weight is 1 / N, so the outputs of one-hot values are the mask itself."""
+regenerates: counters that cross 2^32 inside a tile (and inside a thread's run of 32), ragged sizes, grouped heads,
+both memory layouts.  With q = k = 0 every weight is 1 / N, so the outputs of one-hot values are the mask itself."""
 import pytest
 import torch
 
@@ -39,3 +39,36 @@ def test_backward_mask(M, N, D, p, seed, offset):
     got = (dv.float() * (N * (1 - p))).round().to(torch.int64)[..., :M].transpose(2, 3)
     assert torch.equal(got, mask[:, 0::2] + 2 * mask[:, 1::2])
     assert not dq.any() and not dk.any()   # k = 0 and q = 0
+
+
+@pytest.mark.parametrize("seed,offset", STREAMS)
+@pytest.mark.parametrize("D", [16, 32])
+def test_forward_mask_of_long_rows(D, seed, offset):
+    """head_dim 16 and 32 padded (from 1024 keys on): the values are one-hot over a window of D keys."""
+    H, M, N, p = 3, 130, 1100, 0.1
+    q, k = (torch.zeros(2, H, n, D, device="cuda", dtype=torch.float16) for n in (M, N))
+    mask = fa.testing.recompute_mask(2, H, M, N, p, seed, offset, "cuda")
+    for first in (0, 56, 1024, N - D):
+        v = torch.zeros(2, H, N, D, device="cuda", dtype=torch.float16)
+        v[:, :, first:first + D] = torch.eye(D, device="cuda", dtype=torch.float16)
+        o, _ = flash._forward(q, k, v, False, 1.0, p, seed, offset)
+        assert torch.equal(o > 0.5 / (N * (1 - p)), mask[..., first:first + D])
+
+
+@pytest.mark.parametrize("H,Hk,M,N,D,causal", [(4, 2, 300, 300, 64, True), (4, 4, 129, 200, 128, False), (8, 2, 150, 1030, 32, True)])
+def test_layouts(H, Hk, M, N, D, causal):
+    """(batch, length, heads, head_dim) in memory gives the bits of the contiguous call; dq is a sum of fp32 reductions
+    in any order, rounded once: a unit of bf16 at most."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    make = lambda h, n: torch.randn(2, n, h, D, generator=gen, device="cuda", dtype=torch.bfloat16).transpose(1, 2)
+    q, k, v, do = make(H, M), make(Hk, N), make(Hk, N), make(H, M)
+    got = []
+    for ready in (lambda x: x, lambda x: x.contiguous()):
+        a, b, c, d = map(ready, (q, k, v, do))
+        o, lse = flash._forward(a, b, c, causal, D ** -0.5, 0.2, 11, 2 ** 32 - 999)
+        got.append((o, lse) + flash._backward(a, b, c, o, lse, d, causal, D ** -0.5, None, 0.2, 11, 2 ** 32 - 999))
+    for name, x, y in zip(("o", "lse", "dq", "dk", "dv"), *got):
+        if name == "dq":
+            torch.testing.assert_close(x, y, atol=2 ** -8 * y.abs().max().item() * 2 ** -6, rtol=2 ** -7)
+        else:
+            assert torch.equal(x, y), name
