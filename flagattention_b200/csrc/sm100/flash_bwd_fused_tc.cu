@@ -15,7 +15,12 @@ namespace tc {
 
 bool generic_forced();
 
+// head_dim 16 and 32, padded to 64 (see fused_padded_dim()), from some size on: backward, bf16 causal, pair of kernels
+// -> this, us: 32: B=2 H=8 L=64 9.2 -> 12.2, B=16 H=16 L=160 36 -> 38, B=2 H=8 L=256 19.7 -> 15.3; 16: B=2 H=8 L=160
+// 13.3 -> 15.0, L=256 15.8 -> 14.8, B=4 H=16 M=32 N=512 16.6 -> 17.9; with dropout 32: B=16 H=16 L=64 23 -> 28, B=1 H=8
+// L=200 43 -> 23.
 static bool one_pass_covered(const fa_flash_shape *s) {
+  if (s->D < 64 && (int64_t)s->M * s->N < (s->dropout_p > 0.f ? 96 * 96 : 192 * 192)) return false;
   return !generic_forced() && s->sm_scale > 0.f;
 }
 // the entries that take the backward in parts

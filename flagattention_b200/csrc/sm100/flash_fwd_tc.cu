@@ -136,13 +136,23 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
   return FA_OK;
 }
 
-static bool covered(const fa_flash_shape *s) {
-  // head_dim 16 and 32 run as 64 with zero columns: the exponentials bound these kernels, not the padded
-  // products.  Forward, B=4 H=16 L=2048 causal bf16, shape-generic -> padded: 32: 137 -> 90 us, 16: 104 -> 91 us;
-  // B=1 H=8 L=8192: 414 -> 236 us, 288 -> 237 us.  Walks of a few tiles do not pay for it at 16 (B=16 H=16
-  // Hk=4 L=512: 54 -> 64 us; at 32 65 us either way).
-  if (s->D == 16 && s->N < 1024) return false;
-  return !generic_forced() && s->sm_scale > 0.f;
+// head_dim 16 and 32 run as 64 with zero columns: the exponentials bound these kernels, not the padded products.
+// Short walks do not pay for it.  bf16 causal, shape-generic -> padded, us:
+//   32            B=16 H=16 L=160 13.8 -> 16.9, B=2 H=8 L=256 7.1 -> 7.4, B=16 H=16 Hk=4 L=512 43 -> 38, B=4 H=16 L=2048
+//                 122 -> 84, B=4 H=16 M=2048 N=64 12.8 -> 17.4
+//   32 piecewise  B=2 H=8 L=512 13.8 -> 14.8, B=4 H=16 L=1024 50 -> 42, L=2048 140 -> 95
+//   32 dropout    B=2 H=8 L=128 10.5 -> 11.1, B=16 H=16 L=512 140 -> 119
+//   16            B=1 H=4 L=1536 20.9 -> 21.6, B=4 H=16 L=1024 31 -> 33, L=2048 86 -> 84, B=1 H=8 L=4096 65 -> 54
+//   16 piecewise  B=4 H=16 L=1024 40 -> 42, L=2048 109 -> 95
+//   16 dropout    B=4 H=16 L=1024 139 -> 114
+static int fewest_keys(const fa_flash_shape *s, bool piecewise) {
+  if (s->D > 32) return 0;
+  if (s->dropout_p > 0.f) return s->D == 32 ? 160 : 1024;
+  if (piecewise) return s->D == 32 ? 640 : 1280;
+  return s->D == 32 ? 384 : 2048;
+}
+static bool covered(const fa_flash_shape *s, bool piecewise = false) {
+  return !generic_forced() && s->sm_scale > 0.f && s->N >= fewest_keys(s, piecewise);
 }
 
 // Return FA_OK / a negative status, or 1 when this path does not cover the call.
@@ -193,7 +203,7 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
 int piecewise_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q1, const fa_tensor4 *k1,
                      const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
                      const fa_tensor4 *o, float *lse, cudaStream_t stream) {
-  if (!covered(s) || s->dropout_p > 0.f || w > (1 << 29) || w < -(1 << 29)) return 1;
+  if (!covered(s, true) || s->dropout_p > 0.f || w > (1 << 29) || w < -(1 << 29)) return 1;
   if (s->D < 64)
     return s->dtype == FA_F16
                ? launch_fwd_tc<__half, 64, true, false, true>(s, w, q1, k1, q2, k2, v, o, lse, stream)

@@ -1,6 +1,7 @@
 """The keep bits the tcgen05 kernels compute for themselves, element by element against the mask the library
 regenerates: counters that cross 2^32 inside a tile (and inside a thread's run of 32), ragged sizes, grouped heads,
-both memory layouts.  With q = k = 0 every weight is 1 / N, so the outputs of one-hot values are the mask itself."""
+both memory layouts; the shortest cases at head_dim 16 and 32 run on the shape-generic kernels.  With q = k = 0 every
+weight is 1 / N, so the outputs of one-hot values are the mask itself."""
 import pytest
 import torch
 
@@ -25,7 +26,7 @@ def test_forward_mask(H, M, N, D, p, seed, offset):
 
 @pytest.mark.parametrize("seed,offset", STREAMS)
 @pytest.mark.parametrize("p", [0.1, 0.5])
-@pytest.mark.parametrize("M,N,D", [(64, 300, 64), (128, 257, 128), (31, 100, 32)])
+@pytest.mark.parametrize("M,N,D", [(64, 300, 64), (128, 257, 128), (31, 100, 32), (32, 320, 32)])
 def test_backward_mask(M, N, D, p, seed, offset):
     H, Hk = 4, 2
     q = torch.zeros(2, H, M, D, device="cuda", dtype=torch.float16)
@@ -44,7 +45,7 @@ def test_backward_mask(M, N, D, p, seed, offset):
 @pytest.mark.parametrize("seed,offset", STREAMS)
 @pytest.mark.parametrize("D", [16, 32])
 def test_forward_mask_of_long_rows(D, seed, offset):
-    """head_dim 16 and 32 padded (from 1024 keys on): the values are one-hot over a window of D keys."""
+    """head_dim 16 and 32 padded: the values are one-hot over a window of D keys."""
     H, M, N, p = 3, 130, 1100, 0.1
     q, k = (torch.zeros(2, H, n, D, device="cuda", dtype=torch.float16) for n in (M, N))
     mask = fa.testing.recompute_mask(2, H, M, N, p, seed, offset, "cuda")

@@ -1,8 +1,9 @@
 """head_dim 16 and 32 on the tcgen05 kernels, which run them as 64 with zero columns: sizes around a tile,
 grouped heads, keys and queries of different length, views of a fused projection whose neighbouring columns
 hold NaN (they lie past the tensor map's extent and must never enter a product).  Short calls run on the
-shape-generic kernels in part; from 1024 keys on every kernel is a padded one, with few query tiles (one CTA a
-tile) and with more than two an SM (the persistent forward)."""
+shape-generic kernels in part; the last three run on the padded ones at both head_dims: the forward with few query
+tiles (one CTA a tile) and with more than two an SM (the persistent form), the backward, and total_attention where
+there are 1024 queries or more."""
 import pytest
 import torch
 
@@ -16,7 +17,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("D", [16, 32])
 @pytest.mark.parametrize("B,H,Hk,M,N,causal", [
     (32, 8, 8, 64, 64, True), (16, 16, 4, 127, 129, True), (8, 16, 16, 385, 385, False), (4, 16, 2, 1000, 700, True),
-    (2, 8, 4, 200, 1100, True), (4, 16, 8, 640, 1056, True)])
+    (2, 8, 4, 200, 1100, True), (2, 8, 4, 200, 2100, True), (4, 16, 8, 640, 2056, True), (1, 4, 2, 1100, 2050, True)])
 def test_forward_backward_against_oracle(B, H, Hk, M, N, D, causal):
     gen = torch.Generator().manual_seed(M + N + D)
 
