@@ -129,13 +129,11 @@ def _decode_forward(q, k, v, sm_scale, causal=False):
     sb, sh, sl, _ = k.stride()
     num_sms = _C.sm_count(q.device)
     # Partitions of the key axis, long enough to amortise a CTA's pipeline fill and the reduction (one block a
-    # row goes through the row's partitions): about one wave of CTAs, up to 8192 keys where that leaves three.
-    # fp16, eight waves of at least 256 keys -> this: B=1 H=32 Hk=8 N=131072 D=128 218 -> 99 us (2048 keys: 117,
-    # 8192: 112), B=4 H=16 N=16384 D=64 67 -> 56 us (8192: 79), B=1 H=8 N=32768 73 -> 40 us, B=2 H=16 N=131072
-    # 339 -> 325 us (4096: 339).
+    # row goes through the row's partitions): about one wave of CTAs, up to 4096 keys.  Every context is N long
+    # here, so that the rule may count CTAs at the bound.  fp16, 2048 / 4096 / 8192 keys: B=32 H=32 N=8192 D=128
+    # 619 / 625 / 654 us, B=8 H=32 N=32768 633 / 630 / 645, B=2 H=32 N=131072 D=64 336 / 333 / 345, B=2 H=16
+    # N=131072 340 / 326 / 311; by the rule 1024 of N=8192 B=4 H=32 Hk=4 M=6 D=64 22.9 (2048: 28.4, 512: 27.2).
     partition_size = coarsen_partition(256, B * Hk, N, num_sms, 4096)
-    if partition_size == 4096 and B * Hk * ((N + 8191) // 8192) >= 3 * num_sms:
-        partition_size = 8192
     if N <= partition_size:
         partition_size = 0   # one pass, no reduction kernel
     q2 = q.reshape(B, H * M, D)

@@ -27,6 +27,18 @@ def test_no_device_state_behind_the_call(monkeypatch):
     assert not held
 
 
+@pytest.mark.parametrize("B,Hk,N,size", [(32, 32, 8192, 4096), (8, 32, 32768, 4096), (2, 16, 131072, 4096), (32, 32, 4096, 0)])
+def test_partitions_of_long_contexts(monkeypatch, B, Hk, N, size):
+    """At most 4096 keys: longer ones are slower for most shapes that would have three waves of them."""
+    seen = []
+    monkeypatch.setattr(_C, "sm_count", lambda device: 148)
+    monkeypatch.setattr(_C, "raw_stream", lambda device: 0)
+    monkeypatch.setattr(_C, "call", lambda name: lambda args, stream: seen.append(args) or 0)
+    k = torch.empty(B, Hk, N, 128, dtype=torch.float16, device="meta")
+    flash._decode_forward(torch.empty(B, Hk, 1, 128, dtype=torch.float16, device="meta"), k, k, 1.0)
+    assert _C.PagedArgs.from_buffer_copy(seen[0]).partition_size == size
+
+
 def test_a_missing_table_is_refused(built_lib):
     """Before any CUDA call: null tables stay an error unless the caller says that there are none."""
     args = _C.PagedArgs()
