@@ -38,10 +38,45 @@ struct PagedCfg {
   static constexpr int kTotal = kRing + (kRingBytes > kMergeBytes ? kRingBytes : kMergeBytes);
 };
 
+// How the kernels size the partitions of fa_paged_attention from the lengths themselves; finest == 0: every sequence
+// takes a.partition_size.  Sizes are finest * 2^k.
+struct Sizing {
+  int finest, coarsest;
+  int ctas;    // > 0: the largest size, up to `coarsest`, that leaves the whole call this many CTAs
+  int parts;   // ctas == 0: the smallest size that cuts a sequence into this many at most
+};
+// The lengths of the first 64 sequences, two a lane, requested ahead of their use.
+struct LaneLens {
+  int first, second;
+};
+__device__ __forceinline__ LaneLens lane_lens(const fa_paged_args &a, const Sizing &z) {
+  const int lane = threadIdx.x & 31;
+  return LaneLens{z.ctas > 0 && lane < a.num_seqs ? context_len(a, lane) : 0,
+                  z.ctas > 0 && lane + 32 < a.num_seqs ? context_len(a, lane + 32) : 0};
+}
+// Tokens per partition of a sequence of `ctx` tokens, called by whole warps; never more partitions than the P of the
+// workspace.
+__device__ __forceinline__ int partition_tokens(const fa_paged_args &a, const Sizing &z, LaneLens lens, int ctx, int P) {
+  if (z.finest == 0) return a.partition_size;
+  int k = 0;
+  if (z.ctas > 0) {
+    auto count = [&](int len) { return min(((unsigned)max(len, 0) + z.finest - 1) / z.finest, 1u << 20); };
+    unsigned lane_n = count(lens.first) + count(lens.second);
+    for (int i = (threadIdx.x & 31) + 64; i < a.num_seqs; i += 32) lane_n += count(context_len(a, i));
+    // (a sum below 2^32: at most 2048 sequences)
+    const unsigned long long n = (unsigned long long)__reduce_add_sync(0xffffffffu, lane_n) *
+                                 (a.num_kv_heads * ((a.num_q_heads / a.num_kv_heads + 15) / 16));
+    while ((z.finest << k) < z.coarsest && (n >> (k + 1)) >= (unsigned)z.ctas) ++k;
+  }
+  const int parts = z.ctas > 0 ? P : min(P, z.parts);
+  while ((z.finest << k) < a.partition_size && (long long)parts * (z.finest << k) < ctx) ++k;
+  return z.finest << k;
+}
+
 // HALF: at most 8 query rows, the upper half of the 16-row tile; the lower half serves the remainder of P.
 template <typename T, int D, typename IdxT, bool HALF>
 __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
-    const fa_paged_args a) {
+    const fa_paged_args a, const Sizing z) {
   using C = PagedCfg<D>;
   constexpr int NW = C::kWarps, NS = C::kStages, CPR = D / 8;
   constexpr int R = HALF ? 1 : 2;   // accumulator rows of a thread: g and, in a full tile, g + 8
@@ -59,9 +94,15 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
   const int qh0 = hk * G + qt * 16;               // first query head
 
   const int ctx = context_len(a, seq);
-  const int t_begin = a.partition_size > 0 ? part * a.partition_size : 0;
-  if (a.partition_size > 0 && t_begin >= ctx) return;
-  const int t_end = a.partition_size > 0 ? min(ctx, t_begin + a.partition_size) : ctx;
+  int t_begin = 0, t_end = ctx;
+  if (a.partition_size > 0) {
+    const LaneLens lens = lane_lens(a, z);   // in flight together with ctx
+    if ((long long)part * (z.finest ? z.finest : a.partition_size) >= ctx) return;
+    const int size = partition_tokens(a, z, lens, ctx, gridDim.z);
+    if ((long long)part * size >= ctx) return;
+    t_begin = part * size;
+    t_end = (int)min((long long)ctx, (long long)t_begin + size);
+  }
   const int BS = a.block_size;
   const bool group_in_block = (BS % 16 == 0) && (t_begin % 16 == 0);
   // Several queries per head (a.causal_rows = Mq > 0): query head index = head * Mq + m, and query
@@ -247,15 +288,22 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
 #pragma unroll
       for (int i = 0; i < 4; ++i) split_weights<T>(s[i >> 1][2 * (i & 1)], s[i >> 1][2 * (i & 1) + 1], pa[i], pr[i]);
     }
+    constexpr int U = HALF ? 1 : D / 16 < 4 ? D / 16 : 4;   // chunks whose two products are kept apart
 #pragma unroll
-    for (int dj = 0; dj < D / 16; ++dj) {
-      uint32_t bb[4];
-      load_B_kn<D>(bb, st + C::kGroupBytes, 0, dj * 2, lane);
-      Elem<T>::mma(acc[2 * dj], pa, bb[0], bb[1]);
-      Elem<T>::mma(acc[2 * dj + 1], pa, bb[2], bb[3]);
+    for (int d0 = 0; d0 < D / 16; d0 += U) {
+      uint32_t bb[U][4];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        load_B_kn<D>(bb[u], st + C::kGroupBytes, 0, (d0 + u) * 2, lane);
+        Elem<T>::mma(acc[2 * (d0 + u)], pa, bb[u][0], bb[u][1]);
+        Elem<T>::mma(acc[2 * (d0 + u) + 1], pa, bb[u][2], bb[u][3]);
+      }
       if (!HALF) {
-        Elem<T>::mma(acc[2 * dj], pr, bb[0], bb[1]);
-        Elem<T>::mma(acc[2 * dj + 1], pr, bb[2], bb[3]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          Elem<T>::mma(acc[2 * (d0 + u)], pr, bb[u][0], bb[u][1]);
+          Elem<T>::mma(acc[2 * (d0 + u) + 1], pr, bb[u][2], bb[u][3]);
+        }
       }
     }
     __syncwarp();  // stage may be refilled by the next iteration's issue
@@ -340,12 +388,13 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
 
 // One CTA per (seq, query head); thread d4 owns 4 output columns.
 template <typename T>
-__global__ void paged_reduce_kernel(const fa_paged_args a) {
+__global__ void paged_reduce_kernel(const fa_paged_args a, const Sizing z) {
   const int seq = blockIdx.x, qh = blockIdx.y;
   const int D = a.head_size;
   const int P = (a.max_context_len + a.partition_size - 1) / a.partition_size;
   const int ctx = context_len(a, seq);
-  const int np = min(P, (ctx + a.partition_size - 1) / a.partition_size);
+  const int size = partition_tokens(a, z, lane_lens(a, z), ctx, P);
+  const int np = min(P, (ctx + size - 1) / size);
   const int64_t base = ((int64_t)seq * a.num_q_heads + qh) * P;
   float mm = -INFINITY;
   for (int p = 0; p < np; ++p) mm = fmaxf(mm, a.part_max[base + p]);
@@ -411,7 +460,7 @@ static int validate_paged(const fa_paged_args *a, bool need_ws) {
 }
 
 template <typename T, int D, typename IdxT, bool HALF>
-static int launch_paged(const fa_paged_args *a, cudaStream_t stream) {
+static int launch_paged(const fa_paged_args *a, const Sizing &z, cudaStream_t stream) {
   using C = PagedCfg<D>;
   auto kern = paged_decode_kernel<T, D, IdxT, HALF>;
   static unsigned long long attr_done = 0;  // per instantiation, one bit per device
@@ -422,27 +471,54 @@ static int launch_paged(const fa_paged_args *a, cudaStream_t stream) {
                     ? (a->max_context_len + a->partition_size - 1) / a->partition_size
                     : 1;
   dim3 grid(a->num_seqs, a->num_kv_heads * q_tiles, P);
-  kern<<<grid, C::kWarps * 32, C::kTotal, stream>>>(*a);
+  kern<<<grid, C::kWarps * 32, C::kTotal, stream>>>(*a, z);
   FA_CHECK_LAUNCH();
   return FA_OK;
 }
 
 template <typename T, typename IdxT>
-static int dispatch_paged_d(const fa_paged_args *a, cudaStream_t stream) {
+static int dispatch_paged_d(const fa_paged_args *a, const Sizing &z, cudaStream_t stream) {
   const bool half = a->num_q_heads / a->num_kv_heads <= 8;
   switch (a->head_size) {
     case 16:
-      return half ? launch_paged<T, 16, IdxT, true>(a, stream) : launch_paged<T, 16, IdxT, false>(a, stream);
+      return half ? launch_paged<T, 16, IdxT, true>(a, z, stream) : launch_paged<T, 16, IdxT, false>(a, z, stream);
     case 32:
-      return half ? launch_paged<T, 32, IdxT, true>(a, stream) : launch_paged<T, 32, IdxT, false>(a, stream);
+      return half ? launch_paged<T, 32, IdxT, true>(a, z, stream) : launch_paged<T, 32, IdxT, false>(a, z, stream);
     case 64:
-      return half ? launch_paged<T, 64, IdxT, true>(a, stream) : launch_paged<T, 64, IdxT, false>(a, stream);
+      return half ? launch_paged<T, 64, IdxT, true>(a, z, stream) : launch_paged<T, 64, IdxT, false>(a, z, stream);
     case 128:
-      return half ? launch_paged<T, 128, IdxT, true>(a, stream) : launch_paged<T, 128, IdxT, false>(a, stream);
+      return half ? launch_paged<T, 128, IdxT, true>(a, z, stream) : launch_paged<T, 128, IdxT, false>(a, z, stream);
     case 256:
-      return half ? launch_paged<T, 256, IdxT, true>(a, stream) : launch_paged<T, 256, IdxT, false>(a, stream);
+      return half ? launch_paged<T, 256, IdxT, true>(a, z, stream) : launch_paged<T, 256, IdxT, false>(a, z, stream);
   }
   return FA_ERR_UNSUPPORTED;
+}
+
+static int decode(const fa_paged_args *a, const Sizing &z, cudaStream_t s) {
+  if (in_place(a))
+    return a->dtype == FA_F16 ? dispatch_paged_d<__half, InPlace>(a, z, s)
+                              : dispatch_paged_d<__nv_bfloat16, InPlace>(a, z, s);
+  if (a->dtype == FA_F16)
+    return a->block_table_is_i64 ? dispatch_paged_d<__half, int64_t>(a, z, s)
+                                 : dispatch_paged_d<__half, int32_t>(a, z, s);
+  return a->block_table_is_i64 ? dispatch_paged_d<__nv_bfloat16, int64_t>(a, z, s)
+                               : dispatch_paged_d<__nv_bfloat16, int32_t>(a, z, s);
+}
+
+static int reduce(const fa_paged_args *a, const Sizing &z, cudaStream_t s) {
+  dim3 grid(a->num_seqs, a->num_q_heads);
+  const int threads = a->head_size / 4 < 32 ? 32 : a->head_size / 4;
+  if (a->dtype == FA_F16)
+    paged_reduce_kernel<__half><<<grid, threads, 0, s>>>(*a, z);
+  else
+    paged_reduce_kernel<__nv_bfloat16><<<grid, threads, 0, s>>>(*a, z);
+  FA_CHECK_LAUNCH();
+  return FA_OK;
+}
+
+// size / finest is a power of two
+static bool nests(int size, int finest) {
+  return size % finest == 0 && ((size / finest) & (size / finest - 1)) == 0;
 }
 
 }  // namespace fa
@@ -450,32 +526,26 @@ static int dispatch_paged_d(const fa_paged_args *a, cudaStream_t stream) {
 using namespace fa;
 
 extern "C" int fa_paged_decode(const fa_paged_args *a, void *stream) {
-  int st = validate_paged(a, true);
-  if (st != FA_OK) return st;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (in_place(a))
-    return a->dtype == FA_F16 ? dispatch_paged_d<__half, InPlace>(a, s)
-                              : dispatch_paged_d<__nv_bfloat16, InPlace>(a, s);
-  if (a->dtype == FA_F16)
-    return a->block_table_is_i64 ? dispatch_paged_d<__half, int64_t>(a, s)
-                                 : dispatch_paged_d<__half, int32_t>(a, s);
-  return a->block_table_is_i64 ? dispatch_paged_d<__nv_bfloat16, int64_t>(a, s)
-                               : dispatch_paged_d<__nv_bfloat16, int32_t>(a, s);
+  if (int st = validate_paged(a, true)) return st;
+  return decode(a, Sizing{}, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int fa_paged_reduce(const fa_paged_args *a, void *stream) {
-  int st = validate_paged(a, true);
-  if (st != FA_OK) return st;
+  if (int st = validate_paged(a, true)) return st;
   if (a->partition_size <= 0) return FA_ERR_BAD_ARG;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  dim3 grid(a->num_seqs, a->num_q_heads);
-  const int threads = a->head_size / 4 < 32 ? 32 : a->head_size / 4;
-  if (a->dtype == FA_F16)
-    paged_reduce_kernel<__half><<<grid, threads, 0, s>>>(*a);
-  else
-    paged_reduce_kernel<__nv_bfloat16><<<grid, threads, 0, s>>>(*a);
-  FA_CHECK_LAUNCH();
-  return FA_OK;
+  return reduce(a, Sizing{}, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int fa_paged_attention(const fa_paged_args *a, int32_t finest, int32_t coarsest, int32_t ctas,
+                                  int32_t parts, void *stream) {
+  if (int st = validate_paged(a, true)) return st;
+  if (a->partition_size <= 0 || a->partition_size > (1 << 24) || finest <= 0 || finest % 16 || finest > a->partition_size ||
+      coarsest < finest || coarsest > (1 << 24) || !nests(a->partition_size, finest) || !nests(coarsest, finest))
+    return FA_ERR_BAD_ARG;
+  if (ctas < 0 || (ctas == 0 && parts <= 0) || (ctas > 0 && a->num_seqs > 2048)) return FA_ERR_BAD_ARG;
+  const Sizing z{finest, coarsest, ctas, parts};
+  if (int st = decode(a, z, static_cast<cudaStream_t>(stream))) return st;
+  return reduce(a, z, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int64_t fa_paged_workspace_bytes(const fa_paged_args *a) {

@@ -4,6 +4,8 @@ Mirrors src/flag_attn/paged.py:6-163: same arguments, same split rule
 (num_splits == 0 picks it automatically, 1 disables it, > 1 fixes the count),
 returns a new tensor shaped like `query`.
 """
+import functools
+
 import torch
 
 from . import _C
@@ -42,16 +44,48 @@ def plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_
 
 
 def coarsen_partition(partition_size, pairs, context_len, num_sms, most=2048):
-    """Partitions of `partition_size` tokens, doubled up to `most` while the GPU stays busy with them.
+    """Partitions of `partition_size` tokens, doubled up to `most` while `pairs` contexts of `context_len` tokens, one
+    CTA a partition, keep the GPU busy with them.
 
-    A CTA's four warps fill a ring of loads and merge their results once per partition, and every partition
-    writes and re-reads a row of fp32 partial output, so short ones cost bandwidth; fewer CTAs than SMs cost more.
-    fp16, contexts uniform in [max / 8, max], 256 -> what this picks: 64 sequences x 8 kv heads x 128, 32768 tokens:
-    833 -> 677 us (4096: 678); 16 x 8, 32768: 266 -> 186; 64 x 8, 8192: 237 -> 203; 4 x 8, 32768: 115 -> 70;
-    1 x 4, 32768: 54 -> 33 (512: 37, 2048: 40)."""
+    A CTA's four warps fill a ring of loads and merge their results once per partition, and every partition writes and
+    re-reads a row of fp32 partial output, so short ones cost bandwidth; fewer CTAs than SMs cost more (fp16, one
+    context of 32768 over 4 kv heads: 256: 54 us, 512: 37, 1024: 33, 2048: 40)."""
     while partition_size < most and pairs * _cdiv(int(context_len), 2 * partition_size) >= 0.8 * num_sms:
         partition_size *= 2
     return partition_size
+
+
+@functools.lru_cache(maxsize=1024)
+def size_partitions(base, num_seqs, ctas, max_context_len, num_sms):
+    """(workspace partition, finest, coarsest, ctas, parts) of a fa_paged_attention call: how far partitions of `base`
+    tokens may grow when max_context_len is an upper bound and lengths differ.  `ctas`: CTAs that a partition of one
+    sequence takes; workspace partition 0: one pass does it.
+
+    The workspace partition is the largest at which one sequence still has CTAs enough for the GPU, or until the grid is
+    down to 35 CTAs an SM: doubling lengthens the longest partition (1 us per 100 tokens of a CTA by itself) and spares
+    half the launches (1 ns each).  Shorter sequences are cut finer on the GPU: into two waves' worth each where there
+    are fewer sequences than that; or, where the workspace partition had to stay small but many sequences might fill
+    larger ones, by the sum of all lengths (both kernels then read every length: below 1 us).  fp16, head_size 128, us;
+    256 tokens each / sized by the bound as if every context had it / this:
+      8 kv heads   4 x 1500 under 32768 15 / 20 / 10, 16 x 2048 at most 22 / 27 / 20, 4096 and 63 x 200 35 / 36 / 31,
+                   64 x 32768 at most 852 / 642 / 647, 64 x 8192 at most 233 / 189 / 192, 4 x 32768 at most 103 / 74 / 75
+      2 kv heads   4 x 1500 under 32768 9.5 / 21 / 10.3, 4096 and 63 x 200 16.5 / 26 / 17.5, 16 x 32768 at most
+                   96 / 52 / 55, 32768 and 15 x 1000 44 / 33 / 32, 64 x 32768 at most 253 / 159 / 174"""
+    coarsest = base
+    while coarsest < 2048:
+        coarsest *= 2
+    size = base
+    while size < coarsest and (ctas * _cdiv(max_context_len, 2 * size) >= 0.8 * num_sms
+                               or num_seqs * ctas * _cdiv(max_context_len, size) > 35 * num_sms):
+        size *= 2
+    if max_context_len <= size:
+        return 0, base, coarsest, 0, 1
+    pairs = num_seqs * ctas
+    by_length = (size < min(coarsest, 4 * base) and num_seqs <= 2048
+                 and pairs * _cdiv(max_context_len, 2 * size) >= 0.8 * num_sms)
+    if by_length:
+        return size, base, coarsest, int(0.8 * num_sms), 0
+    return size, base if pairs < 2 * num_sms else size, coarsest, 0, max(1, _cdiv(2 * num_sms, pairs))
 
 
 def partition_workspace(rows, P, D, device):
@@ -98,8 +132,10 @@ def attention(query, key_cache, value_cache, context_lens, block_tables, attn_sc
         sms, free_choice = _C.sm_count(query.device), num_splits == 0
         num_splits, partition_size = plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_splits,
                                                      sms)
+        sizing = None
         if free_choice and partition_size:
-            partition_size = coarsen_partition(partition_size, num_seqs * num_kv_heads, max_context_len, sms)
+            partition_size, *sizing = size_partitions(
+                partition_size, num_seqs, num_kv_heads * _cdiv(query_group_size, 16), int(max_context_len), sms)
         part_out = part_max = part_sum = 0
         if partition_size:
             assert partition_size >= kv_block_size and partition_size % kv_block_size == 0, \
@@ -117,6 +153,9 @@ def attention(query, key_cache, value_cache, context_lens, block_tables, attn_sc
             context_lens.data_ptr(), block_tables.data_ptr(), block_tables.stride(0),
             out.data_ptr(), out.stride(0), out.stride(1), part_out, part_max, part_sum, 0)
         stream = _C.raw_stream(query.device)
+        if sizing and partition_size:
+            _C.check(_C.call("fa_paged_attention")(args, *sizing, stream), "fa_paged_attention")
+            return out
         _C.check(_C.call("fa_paged_decode")(args, stream), "fa_paged_decode")
         if partition_size:
             _C.check(_C.call("fa_paged_reduce")(args, stream), "fa_paged_reduce")

@@ -284,6 +284,15 @@ int fa_paged_decode(const fa_paged_args *a, void *stream);
  * kernel :352-435). */
 int fa_paged_reduce(const fa_paged_args *a, void *stream);
 
+/* fa_paged_decode and fa_paged_reduce with partitions sized on the GPU, from the lengths that the kernels find in
+ * context_lens: a->partition_size and max_context_len only set the workspace, P partitions a sequence.  Sizes are
+ * `finest` * 2^k tokens.  ctas > 0: the largest one, up to `coarsest`, that leaves the whole call about `ctas` CTAs.
+ * ctas == 0: for each sequence the smallest one that cuts it into at most `parts`.  Either way no sequence gets more
+ * than its P partitions.  `finest` is a multiple of 16; a->partition_size and `coarsest` are `finest` times a power of
+ * two, at most 2^24; with ctas > 0 num_seqs is at most 2048; else FA_ERR_BAD_ARG. */
+int fa_paged_attention(const fa_paged_args *a, int32_t finest, int32_t coarsest, int32_t ctas, int32_t parts,
+                       void *stream);
+
 /* Bytes needed for part_out + part_max + part_sum (host-only helper). */
 int64_t fa_paged_workspace_bytes(const fa_paged_args *a);
 
