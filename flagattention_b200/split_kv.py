@@ -4,6 +4,7 @@ Mirrors src/flag_attn/split_kv.py:229-330: `attention` is the standalone
 forward-only operator, `num_splits_herustic` the split-count rule that
 flash_attention's forward also consults.
 """
+import functools
 import math
 
 import torch
@@ -21,6 +22,7 @@ def get_fwd_config(B, H, M, N, D, causal):
     return (16, 128, 1, 4)
 
 
+@functools.lru_cache(maxsize=1024)
 def num_splits_herustic(B, H, M, N, BLOCK_M, BLOCK_N, num_sms, max_splits):
     """Split count, computed by the library's restatement of
     src/flag_attn/split_kv.py:234-262 (name kept as spelled there)."""
