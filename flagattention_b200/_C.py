@@ -150,6 +150,9 @@ _SIGNATURES = {
     "fa_total_attention": "pppppp", "fa_flash_bwd_delta": "ppppp", "fa_piecewise_bwd_fused_workspace_bytes": "p",
     "fa_piecewise_bwd_fused": "pi" + "p" * 14 + "lp", "fa_rotary_pair_fwd": "iiiiii" + "p" * 5 + "liplppp",
     "fa_rotary_pair_bwd": "iiiiii" + "p" * 6 + "liplpp", "fa_num_splits_heuristic": "iiiiiiii",
+    "fa_flash_bwd_fused_workspace_bytes": "p", "fa_flash_bwd_delta_zero": "pppppl" + "p",
+    "fa_flash_bwd_fused_stages": "p" * 11 + "lip", "fa_flash_bwd_dkdv": "p" * 10, "fa_flash_bwd_dq": "p" * 9,
+    "fa_piecewise_bwd_dkdv": "pi" + "p" * 12, "fa_piecewise_bwd_dq": "pi" + "p" * 11,
 }
 _CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int32, "l": ctypes.c_int64}
 _calls = {}

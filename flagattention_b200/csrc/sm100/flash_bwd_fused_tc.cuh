@@ -160,7 +160,9 @@ struct FusedItem {
 // DROP = dropout (flash_attention): dV takes the kept probabilities, dS = P (keep / (1 - p) dP - delta).
 // The 32 keep bits of a thread do not depend on the scores and are computed before the wait for them.
 // Backward at head_dim 64, p = 0.1, bf16, pair of mma.sync kernels (bits computed in both) -> this:
-// B=16 H=16 L=512 662 -> 246 us (120 us without dropout), B=4 H=16 L=2048 causal 1521 -> 451 us.
+// B=16 H=16 L=512 662 -> 246 us (120 us without dropout), B=4 H=16 L=2048 causal 1485 -> 421 us; at 128 1858 -> 481 us.
+// The drawing does not fit the 80 registers beside the rest: 80 bytes of spill stores and 140 of loads a thread at 64,
+// 64 and 152 at 128 (without dropout none, and 8 and 16).
 template <typename T, int D, bool DROP>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     flash_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap map_q,

@@ -30,8 +30,8 @@ struct AbortCtx {
 // issuing thread of the one-pass backward is on its critical path (40 MMAs, 10 waits and 8 commits a
 // tile): B=4 H=32 L=4096 D=128 causal bf16 1.573 -> 1.495 ms, B=2 H=16 L=8192 D=64 2.05 -> 1.88 ms.
 // In the forward, where two CTAs share an SM and hide each other's issuing, the MMA thread gains 0 to 5 %
-// (B=1 H=32 Hk=8 M=512 N=7300 D=128 101 -> 98 us, B=4 H=16 L=2048 D=64 93 -> 89 us, L=4096 D=128 as before)
-// and total_attention 2 % (306 -> 301 us with its forward at L=6144); their producers gain nothing.  A
+// (B=1 H=32 Hk=8 M=512 N=7300 D=128 93.7 -> 91.3 us, B=4 H=16 L=2048 D=64 93 -> 89 us, L=4096 D=128 as before)
+// and total_attention 1 % (321 -> 319 us with its forward at L=6144); their producers gain nothing.  A
 // whole-warp form of these loops (uniform waits by vote) measured no better than this.
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;

@@ -6,7 +6,6 @@ when any return_* flag is set), same AssertionErrors on bad shapes, autograd
 through q, k, v only.  The kernels run on the current CUDA stream of the
 inputs' device.
 """
-import ctypes
 import math
 
 import torch
@@ -172,57 +171,47 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
     and after each one (the benchmark records CUDA events there)."""
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
-    lib = _C.load()
     do = _C.kernel_ready(do)
     with _C.device_guard(q.device):
         # dk / dv come out with Hk heads: the group sum is done in the kernel
         dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=q.device)
         dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=q.device)
         dq = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
+        shape, stream = (_C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset),
+                         _C.raw_stream(q.device))
+        tq, tk, tv, to, tdo, tdq, tdk, tdv = (_C.pack4(x) for x in (q, k, v, o, do, dq, dk, dv))
         if mark is None and use_one_pass_backward():
             # everything in one call: one workspace, one trip through the binding
-            packed = _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
-            ws_bytes = _C.call("fa_flash_bwd_workspace_bytes")(packed)
+            ws_bytes = _C.call("fa_flash_bwd_workspace_bytes")(shape)
             if ws_bytes > 0:
                 ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-                st = _C.call("fa_flash_bwd")(
-                    packed, _C.pack4(q), _C.pack4(k), _C.pack4(v), _C.pack4(o), _C.pack4(do), L.data_ptr(),
-                    _C.pack4(dq), _C.pack4(dk), _C.pack4(dv), ws.data_ptr(), ws_bytes, _C.raw_stream(q.device))
+                st = _C.call("fa_flash_bwd")(shape, tq, tk, tv, to, tdo, L.data_ptr(), tdq, tdk, tdv, ws.data_ptr(),
+                                             ws_bytes, stream)
                 # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
                 if st != _C.FA_ERR_UNSUPPORTED:
                     _C.check(st, "fa_flash_bwd")
                     return dq, dk, dv
                 del ws
         # the parts one by one
-        stream = _C.stream_ptr(q.device)
-        shape = _C.flash_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
-        tq, tk, tv, to, tdo = (_C.tensor4(x) for x in (q, k, v, o, do))
-        tdk, tdv, tdq = _C.tensor4(dk), _C.tensor4(dv), _C.tensor4(dq)
         delta = torch.empty_like(L)
         if mark:
             mark("start")
-        ws_bytes = (lib.fa_flash_bwd_fused_workspace_bytes(_C.byref(shape))
-                    if mark and use_one_pass_backward() else 0)
+        ws_bytes = (_C.call("fa_flash_bwd_fused_workspace_bytes")(shape) if mark and use_one_pass_backward() else 0)
         if ws_bytes > 0:
             # one pass over the score tiles; dq is accumulated in an fp32 workspace, which the
             # delta kernel fills with zeros on its way (two memory-bound passes in one launch)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-            st = lib.fa_flash_bwd_delta_zero(_C.byref(shape), _C.byref(to), _C.byref(tdo), _C.fptr(delta),
-                                             _C.fptr(ws), ctypes.c_int64(ws_bytes), stream)
+            st = _C.call("fa_flash_bwd_delta_zero")(shape, to, tdo, delta.data_ptr(), ws.data_ptr(), ws_bytes, stream)
             _C.check(st, "fa_flash_bwd_delta_zero")
         else:
-            st = lib.fa_flash_bwd_delta(_C.byref(shape), _C.byref(to), _C.byref(tdo),
-                                        _C.fptr(delta), stream)
-            _C.check(st, "fa_flash_bwd_delta")
+            _C.check(_C.call("fa_flash_bwd_delta")(shape, to, tdo, delta.data_ptr(), stream), "fa_flash_bwd_delta")
         if mark:
             mark("delta")
+        ins = (shape, tq, tk, tv, tdo, L.data_ptr(), delta.data_ptr())
         if ws_bytes > 0:
-            args = (_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv), _C.byref(tdo),
-                    _C.fptr(L), _C.fptr(delta), _C.byref(tdq), _C.byref(tdk), _C.byref(tdv),
-                    _C.fptr(ws), ctypes.c_int64(ws_bytes))
             st = 0
             for stage, name in ((2, "dkdvdq"), (4, "dq_convert")):
-                st = lib.fa_flash_bwd_fused_stages(*args, stage, stream)
+                st = _C.call("fa_flash_bwd_fused_stages")(*ins, tdq, tdk, tdv, ws.data_ptr(), ws_bytes, stage, stream)
                 if st != 0:
                     break
                 mark(name)
@@ -230,15 +219,10 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
             if st != _C.FA_ERR_UNSUPPORTED:
                 _C.check(st, "fa_flash_bwd_fused")
                 return dq, dk, dv
-        st = lib.fa_flash_bwd_dkdv(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv),
-                                   _C.byref(tdo), _C.fptr(L), _C.fptr(delta), _C.byref(tdk),
-                                   _C.byref(tdv), stream)
-        _C.check(st, "fa_flash_bwd_dkdv")
+        _C.check(_C.call("fa_flash_bwd_dkdv")(*ins, tdk, tdv, stream), "fa_flash_bwd_dkdv")
         if mark:
             mark("dkdv")
-        st = lib.fa_flash_bwd_dq(_C.byref(shape), _C.byref(tq), _C.byref(tk), _C.byref(tv),
-                                 _C.byref(tdo), _C.fptr(L), _C.fptr(delta), _C.byref(tdq), stream)
-        _C.check(st, "fa_flash_bwd_dq")
+        _C.check(_C.call("fa_flash_bwd_dq")(*ins, tdq, stream), "fa_flash_bwd_dq")
         if mark:
             mark("dq")
     return dq, dk, dv

@@ -56,47 +56,30 @@ class PiecewiseAttention(torch.autograd.Function):
         with _C.device_guard(q1.device):
             raw = _C.raw_stream(q1.device)
             packed = _C.pack_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale)
-            packed_do = _C.pack4(do)
             delta = torch.empty_like(L)
-            st = _C.call("fa_flash_bwd_delta")(packed, _C.pack4(o), packed_do, delta.data_ptr(), raw)
-            _C.check(st, "fa_flash_bwd_delta")
+            tdo = _C.pack4(do)
+            _C.check(_C.call("fa_flash_bwd_delta")(packed, _C.pack4(o), tdo, delta.data_ptr(), raw), "fa_flash_bwd_delta")
 
             dk1 = torch.empty(k1.shape, dtype=k1.dtype, device=k1.device)
             dk2 = torch.empty(k2.shape, dtype=k2.dtype, device=k2.device)
             dv = torch.empty(v.shape, dtype=v.dtype, device=v.device)
+            dq1 = torch.empty(q1.shape, dtype=q1.dtype, device=q1.device)
+            dq2 = torch.empty(q2.shape, dtype=q2.dtype, device=q2.device)
+            ins = (packed, w, *[_C.pack4(x) for x in (q1, k1, q2, k2, v)], tdo, L.data_ptr(), delta.data_ptr())
+            tq1, tq2, tk1, tk2, tv = (_C.pack4(x) for x in (dq1, dq2, dk1, dk2, dv))
             ws_bytes = (_C.call("fa_piecewise_bwd_fused_workspace_bytes")(packed)
                         if use_one_pass_backward() else 0)
             if ws_bytes > 0:
                 # one launch: every key block walks its near tiles, then its far tiles; dq1 / dq2
                 # accumulate in two fp32 workspaces, dV in TMEM across both walks
-                dq1 = torch.empty(q1.shape, dtype=q1.dtype, device=q1.device)
-                dq2 = torch.empty(q2.shape, dtype=q2.dtype, device=q2.device)
                 ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q1.device)
-                st = _C.call("fa_piecewise_bwd_fused")(
-                    packed, w, *[_C.pack4(x) for x in (q1, k1, q2, k2, v)], packed_do, L.data_ptr(), delta.data_ptr(),
-                    *[_C.pack4(x) for x in (dq1, dq2, dk1, dk2, dv)], ws.data_ptr(), ws_bytes, raw)
+                st = _C.call("fa_piecewise_bwd_fused")(*ins, tq1, tq2, tk1, tk2, tv, ws.data_ptr(), ws_bytes, raw)
                 # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
                 if st != _C.FA_ERR_UNSUPPORTED:
                     _C.check(st, "fa_piecewise_bwd_fused")
                     return dq1, dk1, dq2, dk2, dv, None, None, None
-            lib = _C.load()
-            stream = _C.stream_ptr(q1.device)
-            shape = _C.flash_shape(q1.dtype, B, H, H, M, N, D, causal, sm_scale)
-            tdo = _C.tensor4(do)
-            ins = [_C.tensor4(x) for x in (q1, k1, q2, k2, v)]
-            outs = [_C.tensor4(x) for x in (dk1, dk2, dv)]
-            st = lib.fa_piecewise_bwd_dkdv(_C.byref(shape), w, *[_C.byref(t) for t in ins],
-                                           _C.byref(tdo), _C.fptr(L), _C.fptr(delta),
-                                           *[_C.byref(t) for t in outs], stream)
-            _C.check(st, "fa_piecewise_bwd_dkdv")
-
-            dq1 = torch.empty(q1.shape, dtype=q1.dtype, device=q1.device)
-            dq2 = torch.empty(q2.shape, dtype=q2.dtype, device=q2.device)
-            outs = [_C.tensor4(x) for x in (dq1, dq2)]
-            st = lib.fa_piecewise_bwd_dq(_C.byref(shape), w, *[_C.byref(t) for t in ins],
-                                         _C.byref(tdo), _C.fptr(L), _C.fptr(delta),
-                                         *[_C.byref(t) for t in outs], stream)
-            _C.check(st, "fa_piecewise_bwd_dq")
+            _C.check(_C.call("fa_piecewise_bwd_dkdv")(*ins, tk1, tk2, tv, raw), "fa_piecewise_bwd_dkdv")
+            _C.check(_C.call("fa_piecewise_bwd_dq")(*ins, tq1, tq2, raw), "fa_piecewise_bwd_dq")
         return dq1, dk1, dq2, dk2, dv, None, None, None
 
 
