@@ -393,7 +393,7 @@ int fa_device_status(int32_t *out, int32_t clear);
 int fa_debug_wait_probe(int64_t limit_cycles, int32_t *left_flag, void *stream);
 
 /* Kernel family used by the flash / piecewise entry points: 0 (default) = tcgen05 kernels where
- * they cover the call (layouts a tensor map can express; head_dim 16 / 32 as 64, but the pair
+ * they cover the call (layouts a tensor map can express; head_dim 16 / 32 as 64 unless the call is short, and the pair
  * fa_flash_bwd_dkdv / fa_flash_bwd_dq at 64 / 128 without dropout only), the
  * shape-generic mma.sync kernels elsewhere; 1 = shape-generic kernels only (what the tests use to
  * cross-check the two families); 2 = as 0, but fa_flash_fwd launches one CTA per query tile even
