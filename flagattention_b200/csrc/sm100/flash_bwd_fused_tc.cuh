@@ -22,14 +22,24 @@
 //   shared-memory store, no async-proxy fence, and P^T never competes with dS^T for a buffer.
 //   At head_dim 128 all 512 columns are taken, so P^T(t+1) borrows the first 64 columns of dQ:
 //   they are free between the read-out of dQ(t)'s first two quarters and the issue of dQ(t+1)
-//   (head_dim 64 has columns to spare and keeps P^T apart).
+//   At head_dim 64 S^T, dP^T, P^T and dQ all have columns of their own, so a score product is issued
+//   a tile ahead of the element-wise warps.
 // Shared memory:       K, V resident | Q ring | dO ring | one 16-bit 128 x 128 tile "PD" | dQ staging.
 //   PD holds dS^T of a tile: the K-major A operand of dK += dS^T Q and, under a second descriptor,
-//   the MN-major A operand of dQ = dS K.
+//   the MN-major A operand of dQ = dS K.  (Two of them at head_dim 64, where they fit.)
 //
 // Issue order (tensor pipe):  dP^T(t) | dV(t) | S^T(t+1) | dQ(t) | dK(t)
+//   at head_dim 64:           S^T(t+1) | dV(t) | dP^T(t+1) | dQ(t) | dK(t)
 // Element-wise order:         phase 1 (t) | phase 2 (t)
 //   phase 1: P^T = exp2(S^T * scale - L) -> TMEM     phase 2: dS^T = P^T * (dP^T - delta) -> PD
+//
+// What bounds it is the chain of an element-wise warp through a tile, not a unit (tensor pipe 35 % at
+// head_dim 64 and 56 % at 128, exponentials 28 and 23 %, issue 44 and 41 %): a wait costs such a warp 150 to
+// 300 clocks even where it is satisfied (cycle stamps), so it makes two a tile.  S_FULL is completed by
+// the product and by the statistics warp together, DP_FULL by the product, the statistics warp and (128) the
+// reduction warps, and since commits complete in issue order DP_FULL also says that dV(t-1) and dK have read
+// the P^T and dS^T that the tile is about to overwrite.  Seven waits -> two, with S^T and dP^T apart at 64,
+// backward call of B=2 H=16 L=4096 not causal, fp16: 478 -> 449 us at 64, 675 -> 655 us at 128.
 #pragma once
 
 #include "flash_bwd_tc.cuh"
@@ -48,28 +58,30 @@ struct FusedBwdCfg {
   static constexpr int kDO0 = kQ0 + NQ * kTile;        // dO ring
   static constexpr int kPD = kDO0 + NDO * kTile;       // P^T / dS^T: 128 key rows x 128 queries x 2 B
   static constexpr int kPdBytes = 128 * 128 * 2;
+  static constexpr int NPD = (D == 64 ? 2 : 1);        // P^T / dS^T buffers
   // dQ staging: two buffers of a quarter of a dQ tile, fp32, as D/16 runs of (128 queries x 4)
   static constexpr int kQuarter = (D / 16) * 2048;
-  static constexpr int kStage = kPD + kPdBytes;
+  static constexpr int kStage = kPD + NPD * kPdBytes;
   static constexpr int kBars = kStage + 2 * kQuarter;
   static constexpr int kMisc = kBars + 32 * 8;         // tmem base, abort flag, ring of work items
   static constexpr int kStats = kMisc + 32;            // -lse*log2e [128] | -delta [128] of a tile
   static constexpr int kTotal = kStats + 2 * 128 * 4 + 1024;
   static constexpr int kTmemCols = 512;
-  static constexpr int NH = 1;                         // parts dQ of a tile is produced in
-  // head_dim 128: dQ at 128..255 with P^T over 128..191; head_dim 64: P^T at 128..191, dQ at 192..255
+  // head_dim 128: S^T and dP^T share 0..127, dQ at 128..255 with P^T over 128..191.
+  // head_dim 64: S^T 0..127, dP^T 128..255, P^T 256..319, dQ 320..383.
+  static constexpr bool kApart = (D == 64);            // S^T and dP^T in columns of their own
   static constexpr bool kPAliasesDQ = (D == 128);
-  static constexpr int kColA = 0, kColP = 128, kColQ = (D == 128 ? 128 : 192), kColDK = 256, kColDV = 256 + D;
+  static constexpr int kColA = 0, kColB = kApart ? 128 : 0, kColP = kApart ? 256 : 128, kColQ = kApart ? 320 : 128,
+                       kColDK = 512 - 2 * D, kColDV = 512 - D;
   static_assert(kPdBytes >= kTile, "dK is staged in the P^T / dS^T tile");
   static_assert(kTotal <= 232448, "shared memory budget");
 };
 
 enum FusedBar { FB_KV_FULL = 0, FB_Q_FULL = 1, FB_Q_FREE = 3, FB_DO_FULL = 5, FB_DO_FREE = 7,
                 FB_S_FULL = 9, FB_S_LOADED = 10, FB_DP_FULL = 11, FB_DP_LOADED = 12,
-                FB_PT_FULL = 13, FB_PT_FREE = 14, FB_DS_FULL = 15, FB_DS_FREE = 16,
-                FB_DQ_FULL = 17, FB_DQ_FREE = 18, FB_DONE = 19, FB_LSE_FULL = 20, FB_DLT_FULL = 21,
-                FB_V_FULL = 22, FB_DV_STAGED = 23, FB_DK_STAGED = 24, FB_PD_STORED = 25,
-                FB_ITEM_FULL = 26 /* .. 29 */, FB_DQ_HALF = 30 };
+                FB_PT_FULL = 13, FB_DV_DONE = 14, FB_DS_FULL = 15, FB_DQ_FULL = 16, FB_DQ_FREE = 17, FB_DONE = 18,
+                FB_V_FULL = 19, FB_DV_STAGED = 20, FB_DK_STAGED = 21, FB_PD_STORED = 22,
+                FB_ITEM_FULL = 23 /* .. 26 */ };
 
 struct FusedBwdParams {
   BwdTcParams base;   // base.mode: 0 = flash_attention, 3 = piecewise_attention (both branches)
@@ -161,8 +173,8 @@ struct FusedItem {
 // The 32 keep bits of a thread do not depend on the scores and are computed before the wait for them.
 // Backward at head_dim 64, p = 0.1, bf16, pair of mma.sync kernels (bits computed in both) -> this:
 // B=16 H=16 L=512 662 -> 246 us (120 us without dropout), B=4 H=16 L=2048 causal 1485 -> 421 us; at 128 1858 -> 481 us.
-// The drawing does not fit the 80 registers beside the rest: 80 bytes of spill stores and 140 of loads a thread at 64,
-// 64 and 152 at 128 (without dropout none, and 8 and 16).
+// The drawing does not fit the registers beside the rest: 80 and 132 bytes of spill stores and loads a thread at 64, 80 and 172 at
+// 128 (without dropout 76 and 200, and none).
 template <typename T, int D, bool DROP>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     flash_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -266,20 +278,16 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       mbar_init(bar(FB_DO_FULL + s), 1);
       mbar_init(bar(FB_DO_FREE + s), 1);
     }
-    mbar_init(bar(FB_S_FULL), 1);
+    mbar_init(bar(FB_S_FULL), 2);                              // the product, the tile's lse
     mbar_init(bar(FB_S_LOADED), kEwWarps);
-    mbar_init(bar(FB_DP_FULL), 1);
+    mbar_init(bar(FB_DP_FULL), C::kPAliasesDQ ? 6 : 2);        // the product, the tile's delta, P^T's columns read
     mbar_init(bar(FB_DP_LOADED), kEwWarps);
     mbar_init(bar(FB_PT_FULL), kEwWarps);
-    mbar_init(bar(FB_PT_FREE), 1);
+    mbar_init(bar(FB_DV_DONE), 1);
     mbar_init(bar(FB_DS_FULL), kEwWarps);
-    mbar_init(bar(FB_DS_FREE), 1);
     mbar_init(bar(FB_DQ_FULL), 1);
     mbar_init(bar(FB_DQ_FREE), 4);
-    mbar_init(bar(FB_DQ_HALF), 4);
     mbar_init(bar(FB_DONE), 1);
-    mbar_init(bar(FB_LSE_FULL), 1);
-    mbar_init(bar(FB_DLT_FULL), 1);
     mbar_init(bar(FB_DV_STAGED), kEwWarps);
     mbar_init(bar(FB_DK_STAGED), kEwWarps);
     mbar_init(bar(FB_PD_STORED), 1);
@@ -487,7 +495,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     if (elect_one()) {
       constexpr uint32_t idesc_s = instr_desc_f16(BN, BM, TcElem<T>::kFormat, 0, 0);   // S^T, dP^T
       constexpr uint32_t idesc_acc = instr_desc_f16(BN, D, TcElem<T>::kFormat, 0, 1);  // dV, dK
-      constexpr uint32_t idesc_dq = instr_desc_f16(BM, D / C::NH, TcElem<T>::kFormat, 1, 1);  // dQ
+      constexpr uint32_t idesc_dq = instr_desc_f16(BM, D, TcElem<T>::kFormat, 1, 1);  // dQ
       constexpr uint32_t kTile16 = C::kTile >> 4;
       const uint32_t k_lo = smem_desc_lo(smem + C::kK, 0), v_lo = smem_desc_lo(smem + C::kV, 0);
       const uint32_t k_mn_lo = smem_desc_lo(smem + C::kK, BN * 128);     // K as MN-major B of dQ
@@ -515,20 +523,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       int real = 0;            // items with tiles so far
       int nv = 0;              // V tiles so far: the phase of V_FULL (a far walk after a near one loads none)
       uint32_t gt = 0;         // tiles so far, over all items: the phase of every per-tile barrier
-      uint32_t gh = 0;         // dQ parts so far: the phase of DQ_FULL / DQ_FREE
-      // part `hf` of dQ = dS K into the dQ columns, a fresh accumulator: the read-out of the part
-      // before must be over
-      auto issue_dq_part = [&](int hf) -> bool {
-        if (gh > 0 && !mbar_wait(bar(FB_DQ_FREE), (gh - 1) & 1, actx, 818)) return false;
+      // dP^T = V dO^T of the tile in slot sd
+      auto issue_dp = [&](int sd, int phd) -> bool {
+        if (!mbar_wait(bar(FB_DO_FULL + sd), phd, actx, 814)) return false;
         tc_fence_after();
-        const uint32_t b_lo = k_mn_lo + hf * ((BN * 128) >> 4);
+        const uint32_t b_lo = do_k_lo + sd * kTile16;
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t off16 = ((k / 4) * 128 * 128 + (k % 4) * 32) >> 4;
+          mma_ss_lo(tmem + C::kColB, v_lo + off16, b_lo + off16, idesc_s, k > 0 ? 1u : 0u);
+        }
+        mma_commit(bar(FB_DP_FULL));
+        return true;
+      };
+      // dQ = dS K into the dQ columns, a fresh accumulator: the read-out of the tile before must be over
+      auto issue_dq = [&](uint32_t pd16) -> bool {
+        if (gt > 0 && !mbar_wait(bar(FB_DQ_FREE), (gt - 1) & 1, actx, 818)) return false;
+        tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
           const uint32_t off16 = (kk * 16 * 128) >> 4;
-          mma_ss_lo(tmem + C::kColQ, pd_mn_lo + off16, b_lo + off16, idesc_dq, kk > 0 ? 1u : 0u);
+          mma_ss_lo(tmem + C::kColQ, pd_mn_lo + pd16 + off16, k_mn_lo + off16, idesc_dq, kk > 0 ? 1u : 0u);
         }
         mma_commit(bar(FB_DQ_FULL));
-        ++gh;
         return true;
       };
       for (int ic = 0; ok; ++ic) {
@@ -536,12 +553,16 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (w < 0 || w >= end_id) break;
         const FusedItem it = decode(w);
         ok = mbar_wait(bar(FB_KV_FULL), real & 1, actx, 811);
-        // the score columns still hold dP^T of the previous item's last tile until the
-        // element-wise warps have it in registers
-        if (ok && gt > 0) ok = mbar_wait(bar(FB_DP_LOADED), (gt - 1) & 1, actx, 821);
+        // shared score columns still hold dP^T of the previous item's last tile until the
+        // element-wise warps have it in registers (S^T of that tile was read before)
+        if (ok && gt > 0 && !C::kApart) ok = mbar_wait(bar(FB_DP_LOADED), (gt - 1) & 1, actx, 821);
         if (ok) {
           tc_fence_after();
           ok = issue_s(sq, phq);
+        }
+        if (C::kApart && ok) {   // dP^T of the first tile, too
+          if (it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
+          if (ok) ok = issue_dp(sd, phd);
         }
         for (int t = 0; t < it.T_tiles && ok; ++t, ++gt) {
           int nsq = sq + 1, nphq = phq;
@@ -549,28 +570,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           const uint32_t acc = t > 0 ? 1u : 0u;                  // dK: fresh per walk
           const uint32_t acc_dv = (t > 0 || !it.first) ? 1u : 0u;   // dV: fresh per key block
           const uint32_t par = gt & 1;
-          // dP^T(t) = V dO^T over S^T(t), once every element-wise warp holds S^T(t) in registers
+          int nsd = sd + 1, nphd = phd;
+          if (nsd == NDO) nsd = 0, nphd ^= 1;
           ok = mbar_wait(bar(FB_S_LOADED), par, actx, 813);
-          if (ok && t == 0 && it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
-          if (ok) ok = mbar_wait(bar(FB_DO_FULL + sd), phd, actx, 814);
           if (!ok) break;
-          tc_fence_after();
-          {
-            const uint32_t b_lo = do_k_lo + sd * kTile16;
-#pragma unroll
-            for (int k = 0; k < D / 16; ++k) {
-              const uint32_t off16 = ((k / 4) * 128 * 128 + (k % 4) * 32) >> 4;
-              mma_ss_lo(tmem + C::kColA, v_lo + off16, b_lo + off16, idesc_s, k > 0 ? 1u : 0u);
+          if (C::kApart) {
+            // S^T(t+1) over S^T(t), which every element-wise warp holds in registers
+            if (t + 1 < it.T_tiles) {
+              tc_fence_after();
+              ok = issue_s(nsq, nphq);
             }
-            mma_commit(bar(FB_DP_FULL));
+          } else {
+            // dP^T(t) over S^T(t)
+            if (t == 0 && it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
+            if (ok) ok = issue_dp(sd, phd);
           }
-          // the second part of dQ of the tile before (head_dim 128): its first part has been read
-          // out meanwhile; PD is free once it is through
-          if (C::NH == 2 && t > 0) {
-            ok = issue_dq_part(1);
-            if (!ok) break;
-            mma_commit(bar(FB_DS_FREE));
-          }
+          if (!ok) break;
           // dV += P^T(t) dO(t), P^T from TMEM
           ok = mbar_wait(bar(FB_PT_FULL), par, actx, 815);
           if (!ok) break;
@@ -582,19 +597,21 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
               mma_ts_lo(tmem + C::kColDV, tmem + C::kColP + kk * 8, b_lo + ((kk * 16 * 128) >> 4),
                         idesc_acc, kk > 0 ? 1u : acc_dv);
             mma_commit(bar(FB_DO_FREE + sd));
-            mma_commit(bar(FB_PT_FREE));
+            if (t + 1 == it.T_tiles) mma_commit(bar(FB_DV_DONE));
           }
-          // S^T(t+1), once every element-wise warp holds dP^T(t) in registers
+          // once every element-wise warp holds dP^T(t) in registers: the product that takes its columns,
+          // S^T(t+1) or, where S^T has its own, dP^T(t+1)
           if (t + 1 < it.T_tiles) {
             ok = mbar_wait(bar(FB_DP_LOADED), par, actx, 816);
             if (!ok) break;
             tc_fence_after();
-            ok = issue_s(nsq, nphq);
+            ok = C::kApart ? issue_dp(nsd, nphd) : issue_s(nsq, nphq);
             if (!ok) break;
           }
-          // the first part of dQ(t) = dS(t) K
+          // dQ(t) = dS(t) K
           ok = mbar_wait(bar(FB_DS_FULL), par, actx, 817);
-          if (ok) ok = issue_dq_part(0);
+          const uint32_t pd16 = C::NPD == 2 ? (gt & 1) * (C::kPdBytes >> 4) : 0;
+          if (ok) ok = issue_dq(pd16);
           if (!ok) break;
           // dK += dS^T(t) Q(t)
           {
@@ -602,21 +619,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 #pragma unroll
             for (int kk = 0; kk < BM / 16; ++kk) {
               const uint32_t a_off16 = ((kk / 4) * 128 * 128 + (kk % 4) * 32) >> 4;
-              mma_ss_lo(tmem + C::kColDK, pd_k_lo + a_off16, b_lo + ((kk * 16 * 128) >> 4), idesc_acc,
+              mma_ss_lo(tmem + C::kColDK, pd_k_lo + pd16 + a_off16, b_lo + ((kk * 16 * 128) >> 4), idesc_acc,
                         kk > 0 ? 1u : acc);
             }
             mma_commit(bar(FB_Q_FREE + sq));
-            if (C::NH == 1) mma_commit(bar(FB_DS_FREE));
           }
           sq = nsq, phq = nphq;
-          if (++sd == NDO) sd = 0, phd ^= 1;
+          sd = nsd, phd = nphd;
         }
         if (!ok) break;
-        if (C::NH == 2) {   // the second part of dQ of the item's last tile
-          ok = issue_dq_part(1);
-          if (!ok) break;
-          mma_commit(bar(FB_DS_FREE));
-        }
         mma_commit(bar(FB_DONE));
         ++real;
       }
@@ -655,13 +666,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (!ok) break;
         lse_s[lane] = make_float4(l[0], l[1], l[2], l[3]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(FB_LSE_FULL));
+        if (lane == 0) mbar_arrive(bar(FB_S_FULL));
         if (gt > 0) ok = mbar_wait(bar(FB_DS_FULL), (gt - 1) & 1, actx, 952);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         dlt_s[lane] = make_float4(d[0], d[1], d[2], d[3]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(FB_DLT_FULL));
+        if (lane == 0) mbar_arrive(bar(FB_DP_FULL));
       }
     }
   } else if (warp >= 2 + kEwWarps) {
@@ -681,8 +692,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     constexpr int QC = D / 4;                 // columns per quarter
     int buf = 0;
     bool ok = true;
-    uint32_t gt = 0, gh = 0;
-    constexpr int QPH = 4 / C::NH;            // quarters per part of dQ
+    uint32_t gt = 0;
+    if (C::kPAliasesDQ && lane == 0) mbar_arrive(bar(FB_DP_FULL));   // P^T of the first tile finds its columns free
     for (int ic = 0; ok; ++ic) {
       // every wait is bounded, so all four warps reach each vote; they leave together or not at all
       const int w = ring_item(ic, 920);
@@ -700,22 +711,21 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
 #pragma unroll
         for (int qd = 0; qd < 4; ++qd) {
-          if (qd % QPH == 0) {   // the next part of dQ
-            ok = red_warps_all(mbar_wait(bar(FB_DQ_FULL), gh & 1, actx, 921));
+          if (qd == 0) {
+            ok = red_warps_all(mbar_wait(bar(FB_DQ_FULL), gt & 1, actx, 921));
             if (!ok) break;
-            ++gh;
             tc_fence_after();
           }
           uint32_t qr[QC];
-          if (QC == 32) tmem_ld32(tlane + C::kColQ + (qd % QPH) * QC, *reinterpret_cast<uint32_t(*)[32]>(qr));
-          else tmem_ld16(tlane + C::kColQ + (qd % QPH) * QC, qr);
+          if (QC == 32) tmem_ld32(tlane + C::kColQ + qd * QC, *reinterpret_cast<uint32_t(*)[32]>(qr));
+          else tmem_ld16(tlane + C::kColQ + qd * QC, qr);
           tmem_wait_ld();
           if (C::kPAliasesDQ && qd == 1) {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(FB_DQ_HALF));   // the next P^T may take the first 64 columns
+            if (lane == 0) mbar_arrive(bar(FB_DP_FULL));   // the next P^T may take the first 64 columns
           }
-          if (qd % QPH == QPH - 1) {
+          if (qd == 3) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(FB_DQ_FREE));   // the next dQ may overwrite the columns
@@ -752,10 +762,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     // this thread's 64 bytes of a PD row: sub-tile cg / 2, 16-byte chunks (cg & 1) * 4 .. + 3
     uint8_t *pd_row = smem_gen + C::kPD + (cg >> 1) * (128 * 128) + row * 128;
     const int pd_chunk0 = (cg & 1) * 4, pd_xor = row & 7;
-    auto store_pd = [&](const uint32_t (&pk)[16]) {
+    auto store_pd = [&](const uint32_t (&pk)[16], uint32_t off) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<uint4 *>(pd_row + (((pd_chunk0 + j) ^ pd_xor) << 4)) =
+        *reinterpret_cast<uint4 *>(pd_row + off + (((pd_chunk0 + j) ^ pd_xor) << 4)) =
             make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
     };
     // -lse * log2(e) / -delta of this thread's 32 query columns, as staged by the statistics warp
@@ -825,10 +835,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
 
         // ---- phase 1: P^T = exp2(S^T * scale - lse) -> TMEM ----
-        ok = mbar_wait(bar(FB_LSE_FULL), gt & 1, actx, 910);
-        if (ok) ok = mbar_wait(bar(FB_S_FULL), gt & 1, actx, 911);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        ok = mbar_wait(bar(FB_S_FULL), gt & 1, actx, 911);
+        __syncwarp();
         tc_fence_after();
         float pv[32];
         uint32_t sr[32];
@@ -881,12 +889,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             pk[c >> 1] = DROP ? TcElem<T>::pack(keep >> c & 1u ? pv[c] : 0.f, keep >> (c + 1) & 1u ? pv[c + 1] : 0.f)
                               : TcElem<T>::pack(pv[c], pv[c + 1]);
           }
-          // the P^T columns still hold P^T of the tile before until its dV product has read them
-          if (gt > 0) ok = mbar_wait(bar(FB_PT_FREE), (gt - 1) & 1, actx, 912);
-          // ... and, where P^T borrows columns of dQ, dQ of the tile before until they are read out
-          if (C::kPAliasesDQ && ok && gt > 0) ok = mbar_wait(bar(FB_DQ_HALF), (gt - 1) & 1, actx, 918);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
+          // dP^T(t), by now usually there (issued as soon as S^T(t) had been read, or before).  Commits
+          // complete in issue order, so this barrier also says that the products which read what is
+          // overwritten below are through: dV(t-1) (P^T) and dK of the tile whose dS^T buffer this one
+          // takes.  At head_dim 128 the reduction warps have arrived on it, too: the columns of dQ(t-1)
+          // that P^T borrows are read out.
+          ok = mbar_wait(bar(FB_DP_FULL), gt & 1, actx, 913) && ok;
+          __syncwarp();
+          tc_fence_after();
           tmem_st16(tlane + C::kColP + cg * 16, pk);
           tmem_wait_st();
           tc_fence_before();
@@ -894,14 +904,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           if (lane == 0) mbar_arrive(bar(FB_PT_FULL));
         }
         // ---- phase 2: dS^T = P^T * (dP^T - delta) -> PD ----
-        // Its operands are there by now (dP^T(t) was issued as soon as S^T(t) had been read).
-        ok = mbar_wait(bar(FB_DLT_FULL), gt & 1, actx, 909);
-        if (ok) ok = mbar_wait(bar(FB_DP_FULL), gt & 1, actx, 913);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
         uint32_t sr0[16];
-        tmem_ld16(tlane + C::kColA + cg * 32, sr0);
+        tmem_ld16(tlane + C::kColB + cg * 32, sr0);
         {
           uint32_t pk[16];
           // P * (dP - delta) of 16 columns, two elements per instruction
@@ -937,24 +941,26 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           half_ds(0, sr0);
           {
             uint32_t sr1[16];
-            tmem_ld16(tlane + C::kColA + cg * 32 + 16, sr1);
+            tmem_ld16(tlane + C::kColB + cg * 32 + 16, sr1);
             tmem_wait_ld();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(FB_DP_LOADED));   // the next S^T may overwrite dP^T(t)
             half_ds(1, sr1);
           }
-          // PD still holds dS^T of the tile before until its dQ and dK products have read it, and,
-          // at the first tile of an item, the staged dK of the item before until it is stored
-          if (gt > 0) ok = mbar_wait(bar(FB_DS_FREE), (gt - 1) & 1, actx, 914);
-          if (ok && t == 0 && real > 0) ok = mbar_wait(bar(FB_PD_STORED), (real - 1) & 1, actx, 917);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          store_pd(pk);
+          // at the first tile of an item, PD may hold the staged dK of the item before until it is stored
+          if (t == 0 && real > 0) {
+            ok = mbar_wait(bar(FB_PD_STORED), (real - 1) & 1, actx, 917) && ok;
+            __syncwarp();
+          }
+          store_pd(pk, C::NPD == 2 ? (gt & 1) * C::kPdBytes : 0);
         }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(FB_DS_FULL));
+        // one vote a tile: after a wait that ran out the rest of the tile works on stale values, in bounds
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
       }
       if (!ok) break;
 
@@ -966,7 +972,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       // added to (the second launch of a piecewise backward) keeps per-thread global stores.
       {
         uint32_t ov[QC];
-        ok = mbar_wait(bar(FB_PT_FREE), (gt - 1) & 1, actx, 915);   // the last dV product
+        ok = mbar_wait(bar(FB_DV_DONE), real & 1, actx, 915);   // the last dV product
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
