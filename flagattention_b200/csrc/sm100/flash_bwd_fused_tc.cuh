@@ -11,9 +11,9 @@
 //
 //   warp 0       TMA producer
 //   warp 1       MMA issuer (one thread); every MMA is 128 x 128 x 16 (128 x 64 x 16 at D = 64)
-//   warps 2..17  element-wise stage, one thread per (accumulator row, 32 columns)
-//   warps 18..21 dQ reduction: TMEM -> shared-memory staging -> cp.reduce.async.bulk
-//   warp 22      stages lse / delta of every tile in shared memory
+//   warp 2       stages lse / delta of every tile in shared memory (warp 3 idles)
+//   warps 4..7   dQ reduction: TMEM -> shared-memory staging -> cp.reduce.async.bulk
+//   warps 8..23  element-wise stage, one thread per (accumulator row, 32 columns)
 //
 // TMEM (512 columns):  S^T, then dP^T (128) | dQ (D), P^T over its first 64 columns | dK | dV.
 //   The two score products of a tile share one 128-column region: dP^T is issued as soon as the
@@ -21,7 +21,7 @@
 //   P^T goes back to TMEM as packed 16-bit pairs and is the TMEM A operand of dV += P^T dO: no
 //   shared-memory store, no async-proxy fence, and P^T never competes with dS^T for a buffer.
 //   At head_dim 128 all 512 columns are taken, so P^T(t+1) borrows the first 64 columns of dQ:
-//   they are free between the read-out of dQ(t)'s first two quarters and the issue of dQ(t+1)
+//   they are free between the read-out of dQ(t)'s first half and the issue of dQ(t+1)
 //   At head_dim 64 S^T, dP^T, P^T and dQ all have columns of their own, so a score product is issued
 //   a tile ahead of the element-wise warps.
 // Shared memory:       K, V resident | Q ring | dO ring | one 16-bit 128 x 128 tile "PD" | dQ staging.
@@ -49,7 +49,7 @@ namespace tc {
 
 template <int D>
 struct FusedBwdCfg {
-  static constexpr int BM = 128, BN = 128, NQ = 2, NDO = (D == 128 ? 1 : 2);
+  static constexpr int BM = 128, BN = 128, NQ = (D == 128 ? 2 : 3), NDO = (D == 128 ? 1 : 3);
   static constexpr int KSUB = D / 64;
   static constexpr int kTile = 128 * D * 2;            // any 128-row operand tile
   static constexpr int kK = 0;
@@ -59,10 +59,10 @@ struct FusedBwdCfg {
   static constexpr int kPD = kDO0 + NDO * kTile;       // P^T / dS^T: 128 key rows x 128 queries x 2 B
   static constexpr int kPdBytes = 128 * 128 * 2;
   static constexpr int NPD = (D == 64 ? 2 : 1);        // P^T / dS^T buffers
-  // dQ staging: two buffers of a quarter of a dQ tile, fp32, as D/16 runs of (128 queries x 4)
-  static constexpr int kQuarter = (D / 16) * 2048;
+  // dQ staging: two buffers of 32 columns of a dQ tile, fp32, as 8 runs of (128 queries x 4)
+  static constexpr int kPart = 8 * 2048;
   static constexpr int kStage = kPD + NPD * kPdBytes;
-  static constexpr int kBars = kStage + 2 * kQuarter;
+  static constexpr int kBars = kStage + 2 * kPart;
   static constexpr int kMisc = kBars + 32 * 8;         // tmem base, abort flag, ring of work items
   static constexpr int kStats = kMisc + 32;            // -lse*log2e [128] | -delta [128] of a tile
   static constexpr int kTotal = kStats + 2 * 128 * 4 + 1024;
@@ -77,11 +77,11 @@ struct FusedBwdCfg {
   static_assert(kTotal <= 232448, "shared memory budget");
 };
 
-enum FusedBar { FB_KV_FULL = 0, FB_Q_FULL = 1, FB_Q_FREE = 3, FB_DO_FULL = 5, FB_DO_FREE = 7,
-                FB_S_FULL = 9, FB_S_LOADED = 10, FB_DP_FULL = 11, FB_DP_LOADED = 12,
-                FB_PT_FULL = 13, FB_DV_DONE = 14, FB_DS_FULL = 15, FB_DQ_FULL = 16, FB_DQ_FREE = 17, FB_DONE = 18,
-                FB_V_FULL = 19, FB_DV_STAGED = 20, FB_DK_STAGED = 21, FB_PD_STORED = 22,
-                FB_ITEM_FULL = 23 /* .. 26 */ };
+enum FusedBar { FB_KV_FULL = 0, FB_Q_FULL = 1 /* .. 3 */, FB_Q_FREE = 4, FB_DO_FULL = 7, FB_DO_FREE = 10,
+                FB_S_FULL = 13, FB_S_LOADED = 14, FB_DP_FULL = 15, FB_DP_LOADED = 16,
+                FB_PT_FULL = 17, FB_DV_DONE = 18, FB_DS_FULL = 19, FB_DQ_FULL = 20, FB_DQ_FREE = 21, FB_DONE = 22,
+                FB_V_FULL = 23, FB_DV_STAGED = 24, FB_DK_STAGED = 25, FB_PD_STORED = 26,
+                FB_ITEM_FULL = 27 /* .. 30 */ };
 
 struct FusedBwdParams {
   BwdTcParams base;   // base.mode: 0 = flash_attention, 3 = piecewise_attention (both branches)
@@ -142,9 +142,17 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, uint32_t sm
       : "memory");
 }
 
-// warps: 0 TMA producer, 1 MMA issuer, 2..17 element-wise, 18..21 dQ reduction (one per TMEM
-// lane slice), 22 statistics
-constexpr int kFusedThreads = kBwdThreads + 5 * 32;   // 736
+// warps: 0 TMA producer, 1 MMA issuer, 2 statistics, 4..7 dQ reduction (one per TMEM lane slice), 8..23 element-wise
+constexpr int kFusedRedWarp = 4, kFusedEwWarp = 8;
+constexpr int kFusedThreads = (kFusedEwWarp + kEwWarps) * 32;   // 768
+// Six warpgroups of 80 registers a thread, of which the element-wise four take 96 and the others keep 48
+// (2 x 128 x 48 + 512 x 96 = 768 x 80): a thread then holds the 32 dP values of a tile at once, beside its 32 P, and the
+// next product can be issued one load earlier.  With Q and dO three tiles deep at head_dim 64 (the wait for Q(t+1)
+// was 1400 of 3580 clocks there) and dQ read out 32 columns at a time, the call above took 389 us at 64 and 642 at 128.
+// 64 / 64 / 88 registers: 2 to 4 us more, 40 / 40 / 96: 30 us more.  Each role asks for its share inside
+// its own branch: asked for ahead of the branches, the compiler holds every role to the smallest.
+__device__ __forceinline__ void regs_keep_48() { asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n"); }
+__device__ __forceinline__ void regs_take_96() { asm volatile("setmaxnreg.inc.sync.aligned.u32 96;\n"); }
 
 // One work item = one block of 128 keys of one (batch, kv head) pair: its query-tile range.
 // Under piecewise_attention a block is walked twice, back to back by the same CTA: first the
@@ -173,8 +181,8 @@ struct FusedItem {
 // The 32 keep bits of a thread do not depend on the scores and are computed before the wait for them.
 // Backward at head_dim 64, p = 0.1, bf16, pair of mma.sync kernels (bits computed in both) -> this:
 // B=16 H=16 L=512 662 -> 246 us (120 us without dropout), B=4 H=16 L=2048 causal 1485 -> 421 us; at 128 1858 -> 481 us.
-// The drawing does not fit the registers beside the rest: 80 and 132 bytes of spill stores and loads a thread at 64, 80 and 172 at
-// 128 (without dropout 76 and 200, and none).
+// The drawing does not fit the registers beside the rest: 96 and 200 bytes of spill stores and loads a thread at 64, 64 and 144 at
+// 128 (without dropout 48 and 188, and 12 and 92).
 template <typename T, int D, bool DROP>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     flash_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -337,359 +345,363 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0) {
-    // ------------------------------ producer -----------------------------------
-    if (elect_one()) {
-      bool ok = true;
-      int sq = 0, phq = 1, sd = 0, phd = 1;   // ring slot and the "free" parity to wait for
-      int inflight_q = 0, inflight_do = 0;    // loads requested (for the drain after an abort)
-      int real = 0;                           // items with tiles handled so far
-      uint32_t gt = 0;                        // tiles of those items
-      bool pending = false;                   // dV / dK of the previous such item not stored yet
-      int pn0 = 0, phk = 0, pb = 0;           // its coordinates,
-      int pmode = 0;                          // its walk
-      bool plast = true;                      // and whether it closed its key block (dV final)
-      int nvl = 0;                            // V tiles requested so far: the phase of V_FULL
-      auto load_q = [&](const FusedItem &it, int h, int mt) {
-        mbar_expect_tx(bar(FB_Q_FULL + sq), C::kTile);
-        for (int s = 0; s < KSUB; ++s)
-          tma_load_4d(smem + C::kQ0 + sq * C::kTile + s * BM * 128, it.mode == 2 ? &map_q2 : &map_q,
-                      bar(FB_Q_FULL + sq), s * 64, mt * BM, h, it.b);
-        ++inflight_q;
-      };
-      auto load_do = [&](const FusedItem &it, int h, int mt) {
-        mbar_expect_tx(bar(FB_DO_FULL + sd), C::kTile);
-        for (int s = 0; s < KSUB; ++s)
-          tma_load_4d(smem + C::kDO0 + sd * C::kTile + s * BM * 128, &map_do, bar(FB_DO_FULL + sd),
-                      s * 64, mt * BM, h, it.b);
-        ++inflight_do;
-      };
-      // dV then dK of the previous item leave through the copy engine as soon as the element-wise
-      // warps have staged them; `between` runs after the dV store has been requested
-      auto store_dv = [&]() -> bool {
-        if (!mbar_wait(bar(FB_DV_STAGED), (real - 1) & 1, actx, 721)) return false;
-        if (plast && !p.dv_accumulate) {   // a near walk that a far walk follows stages nothing
+  if (warp < kFusedRedWarp) {
+    regs_keep_48();
+    if (warp == 0) {
+      // ------------------------------ producer -----------------------------------
+      if (elect_one()) {
+        bool ok = true;
+        int sq = 0, phq = 1, sd = 0, phd = 1;   // ring slot and the "free" parity to wait for
+        int inflight_q = 0, inflight_do = 0;    // loads requested (for the drain after an abort)
+        int real = 0;                           // items with tiles handled so far
+        uint32_t gt = 0;                        // tiles of those items
+        bool pending = false;                   // dV / dK of the previous such item not stored yet
+        int pn0 = 0, phk = 0, pb = 0;           // its coordinates,
+        int pmode = 0;                          // its walk
+        bool plast = true;                      // and whether it closed its key block (dV final)
+        int nvl = 0;                            // V tiles requested so far: the phase of V_FULL
+        auto load_q = [&](const FusedItem &it, int h, int mt) {
+          mbar_expect_tx(bar(FB_Q_FULL + sq), C::kTile);
+          for (int s = 0; s < KSUB; ++s)
+            tma_load_4d(smem + C::kQ0 + sq * C::kTile + s * BM * 128, it.mode == 2 ? &map_q2 : &map_q,
+                        bar(FB_Q_FULL + sq), s * 64, mt * BM, h, it.b);
+          ++inflight_q;
+        };
+        auto load_do = [&](const FusedItem &it, int h, int mt) {
+          mbar_expect_tx(bar(FB_DO_FULL + sd), C::kTile);
+          for (int s = 0; s < KSUB; ++s)
+            tma_load_4d(smem + C::kDO0 + sd * C::kTile + s * BM * 128, &map_do, bar(FB_DO_FULL + sd),
+                        s * 64, mt * BM, h, it.b);
+          ++inflight_do;
+        };
+        // dV then dK of the previous item leave through the copy engine as soon as the element-wise
+        // warps have staged them; `between` runs after the dV store has been requested
+        auto store_dv = [&]() -> bool {
+          if (!mbar_wait(bar(FB_DV_STAGED), (real - 1) & 1, actx, 721)) return false;
+          if (plast && !p.dv_accumulate) {   // a near walk that a far walk follows stages nothing
+#pragma unroll
+            for (int s = 0; s < KSUB; ++s)
+              tma_store_4d(&map_dv, smem + C::kV + s * BN * 128, s * 64, pn0, phk, pb);
+            bulk_commit();
+          }
+          return true;
+        };
+        auto store_dk = [&]() -> bool {
+          if (!mbar_wait(bar(FB_DK_STAGED), (real - 1) & 1, actx, 722)) return false;
 #pragma unroll
           for (int s = 0; s < KSUB; ++s)
-            tma_store_4d(&map_dv, smem + C::kV + s * BN * 128, s * 64, pn0, phk, pb);
+            tma_store_4d(pmode == 2 ? &map_dk2 : &map_dk, smem + C::kPD + s * BN * 128, s * 64, pn0, phk, pb);
           bulk_commit();
-        }
-        return true;
-      };
-      auto store_dk = [&]() -> bool {
-        if (!mbar_wait(bar(FB_DK_STAGED), (real - 1) & 1, actx, 722)) return false;
-#pragma unroll
-        for (int s = 0; s < KSUB; ++s)
-          tma_store_4d(pmode == 2 ? &map_dk2 : &map_dk, smem + C::kPD + s * BN * 128, s * 64, pn0, phk, pb);
-        bulk_commit();
-        return true;
-      };
-      int w = w_first, ic = 0;
-      if (w < end_id) nvl = 1;   // V of the first walk: see set-up
-      while (w < end_id && ok) {
-        const FusedItem it = decode(w);
-        // Unless the far walk of the same key block follows, ask for the next block now; the answer
-        // is looked at after this walk's first loads have gone out, so its latency hides behind them
-        const bool more = pw && !it.last;
-        const unsigned fetched = more ? 0u : atomicAdd(fp.sched, 1u);
-        int w_next = end_id;
-        {
-          int h = it.hk * G, mt = it.mt_lo;
-          const bool preissued = (ic == 0);   // tile 0, K and V of the first item: see set-up
-          if (preissued) {
-            inflight_q = inflight_do = 1;
-          } else {
-            ok = mbar_wait(bar(FB_Q_FREE + sq), phq, actx, 711);
-            if (!ok) break;
-            load_q(it, h, mt);
-            ok = mbar_wait(bar(FB_DO_FREE + sd), phd, actx, 712);
-            if (!ok) break;
-            load_do(it, h, mt);
-            if (pending) {
-              ok = store_dv();
-              // K is free once every product of the previous item has completed (the last one
-              // issued reads it).  This thread does not follow the per-tile barriers phase by
-              // phase, so it waits on the per-item one.
-              if (ok) ok = mbar_wait(bar(FB_DONE), (real - 1) & 1, actx, 723);
+          return true;
+        };
+        int w = w_first, ic = 0;
+        if (w < end_id) nvl = 1;   // V of the first walk: see set-up
+        while (w < end_id && ok) {
+          const FusedItem it = decode(w);
+          // Unless the far walk of the same key block follows, ask for the next block now; the answer
+          // is looked at after this walk's first loads have gone out, so its latency hides behind them
+          const bool more = pw && !it.last;
+          const unsigned fetched = more ? 0u : atomicAdd(fp.sched, 1u);
+          int w_next = end_id;
+          {
+            int h = it.hk * G, mt = it.mt_lo;
+            const bool preissued = (ic == 0);   // tile 0, K and V of the first item: see set-up
+            if (preissued) {
+              inflight_q = inflight_do = 1;
+            } else {
+              ok = mbar_wait(bar(FB_Q_FREE + sq), phq, actx, 711);
               if (!ok) break;
-            }
-            mbar_expect_tx(bar(FB_KV_FULL), C::kTile);
-            for (int s = 0; s < KSUB; ++s)
-              tma_load_4d(smem + C::kK + s * BN * 128, it.mode == 2 ? &map_k2 : &map_k, bar(FB_KV_FULL),
-                          s * 64, it.n0, it.hk, it.b);
-            if (pending) {
-              ok = store_dk();
+              load_q(it, h, mt);
+              ok = mbar_wait(bar(FB_DO_FREE + sd), phd, actx, 712);
               if (!ok) break;
-              bulk_wait_read_1();            // the dV store (if any) has read the shared memory of V
-            }
-            if (it.first) {                  // a far walk after a near one finds V in place
-              mbar_expect_tx(bar(FB_V_FULL), C::kTile);
+              load_do(it, h, mt);
+              if (pending) {
+                ok = store_dv();
+                // K is free once every product of the previous item has completed (the last one
+                // issued reads it).  This thread does not follow the per-tile barriers phase by
+                // phase, so it waits on the per-item one.
+                if (ok) ok = mbar_wait(bar(FB_DONE), (real - 1) & 1, actx, 723);
+                if (!ok) break;
+              }
+              mbar_expect_tx(bar(FB_KV_FULL), C::kTile);
               for (int s = 0; s < KSUB; ++s)
-                tma_load_4d(smem + C::kV + s * BN * 128, &map_v, bar(FB_V_FULL), s * 64, it.n0, it.hk, it.b);
-              ++nvl;
+                tma_load_4d(smem + C::kK + s * BN * 128, it.mode == 2 ? &map_k2 : &map_k, bar(FB_KV_FULL),
+                            s * 64, it.n0, it.hk, it.b);
+              if (pending) {
+                ok = store_dk();
+                if (!ok) break;
+                bulk_wait_read_1();            // the dV store (if any) has read the shared memory of V
+              }
+              if (it.first) {                  // a far walk after a near one finds V in place
+                mbar_expect_tx(bar(FB_V_FULL), C::kTile);
+                for (int s = 0; s < KSUB; ++s)
+                  tma_load_4d(smem + C::kV + s * BN * 128, &map_v, bar(FB_V_FULL), s * 64, it.n0, it.hk, it.b);
+                ++nvl;
+              }
+              if (pending) {
+                bulk_wait_read_all();          // the dK store has read the P^T / dS^T tile
+                mbar_arrive(bar(FB_PD_STORED));
+              }
             }
-            if (pending) {
-              bulk_wait_read_all();          // the dK store has read the P^T / dS^T tile
-              mbar_arrive(bar(FB_PD_STORED));
+            pending = true, pn0 = it.n0, phk = it.hk, pb = it.b, pmode = it.mode, plast = it.last;
+            ++real;
+            // hand the next walk's id to the other warps
+            if (more) {
+              w_next = w + 1;
+            } else {
+              if (fetched == (unsigned)total - 1u) atomicExch(fp.sched, 0u);
+              w_next = first_walk_of((int)gridDim.x + (int)fetched);
             }
-          }
-          pending = true, pn0 = it.n0, phk = it.hk, pb = it.b, pmode = it.mode, plast = it.last;
-          ++real;
-          // hand the next walk's id to the other warps
-          if (more) {
-            w_next = w + 1;
-          } else {
-            if (fetched == (unsigned)total - 1u) atomicExch(fp.sched, 0u);
-            w_next = first_walk_of((int)gridDim.x + (int)fetched);
-          }
-          item_ring[(ic + 1) & 3] = w_next;
-          mbar_arrive(bar(FB_ITEM_FULL + ((ic + 1) & 3)));
-          if (++sq == NQ) sq = 0, phq ^= 1;
-          if (++sd == NDO) sd = 0, phd ^= 1;
-          if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
-          for (int t = 1; t < it.T_tiles; ++t) {
-            ok = mbar_wait(bar(FB_Q_FREE + sq), phq, actx, 713);
-            if (!ok) break;
-            load_q(it, h, mt);
-            ok = mbar_wait(bar(FB_DO_FREE + sd), phd, actx, 714);
-            if (!ok) break;
-            load_do(it, h, mt);
+            item_ring[(ic + 1) & 3] = w_next;
+            mbar_arrive(bar(FB_ITEM_FULL + ((ic + 1) & 3)));
             if (++sq == NQ) sq = 0, phq ^= 1;
             if (++sd == NDO) sd = 0, phd ^= 1;
             if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
-          }
-          if (!ok) break;
-          gt += (uint32_t)it.T_tiles;
-          // K and V of the next item are read by nobody else: start them towards L2 now, a couple
-          // of tiles before this item ends (any earlier and they would be evicted again)
-          if (w_next < end_id) {
-            const FusedItem nx = decode(w_next);
-            for (int s = 0; s < KSUB; ++s) {
-              tma_prefetch_l2_4d(nx.mode == 2 ? &map_k2 : &map_k, s * 64, nx.n0, nx.hk, nx.b);
-              if (nx.first) tma_prefetch_l2_4d(&map_v, s * 64, nx.n0, nx.hk, nx.b);
+            for (int t = 1; t < it.T_tiles; ++t) {
+              ok = mbar_wait(bar(FB_Q_FREE + sq), phq, actx, 713);
+              if (!ok) break;
+              load_q(it, h, mt);
+              ok = mbar_wait(bar(FB_DO_FREE + sd), phd, actx, 714);
+              if (!ok) break;
+              load_do(it, h, mt);
+              if (++sq == NQ) sq = 0, phq ^= 1;
+              if (++sd == NDO) sd = 0, phd ^= 1;
+              if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
+            }
+            if (!ok) break;
+            gt += (uint32_t)it.T_tiles;
+            // K and V of the next item are read by nobody else: start them towards L2 now, a couple
+            // of tiles before this item ends (any earlier and they would be evicted again)
+            if (w_next < end_id) {
+              const FusedItem nx = decode(w_next);
+              for (int s = 0; s < KSUB; ++s) {
+                tma_prefetch_l2_4d(nx.mode == 2 ? &map_k2 : &map_k, s * 64, nx.n0, nx.hk, nx.b);
+                if (nx.first) tma_prefetch_l2_4d(&map_v, s * 64, nx.n0, nx.hk, nx.b);
+              }
             }
           }
+          w = w_next, ++ic;
         }
-        w = w_next, ++ic;
+        if (ok && pending) {
+          ok = store_dv();
+          if (ok) ok = store_dk();
+        }
+        bulk_wait_read_all();   // shared memory must outlive the copy engine's reads
+        if (!ok) {
+          // let copies already in flight land before the CTA gives its shared memory back
+          const long long t0 = clock64();
+          for (int i = max(0, inflight_q - NQ); i < inflight_q; ++i)
+            while (!mbar_try_wait(bar(FB_Q_FULL + i % NQ), (i / NQ) & 1) && clock64() - t0 < 2000000) {}
+          for (int i = max(0, inflight_do - NDO); i < inflight_do; ++i)
+            while (!mbar_try_wait(bar(FB_DO_FULL + i % NDO), (i / NDO) & 1) && clock64() - t0 < 2000000) {}
+          if (real > 0)
+            while (!mbar_try_wait(bar(FB_KV_FULL), (real - 1) & 1) && clock64() - t0 < 2000000) {}
+          if (nvl > 0)
+            while (!mbar_try_wait(bar(FB_V_FULL), (nvl - 1) & 1) && clock64() - t0 < 2000000) {}
+        }
       }
-      if (ok && pending) {
-        ok = store_dv();
-        if (ok) ok = store_dk();
-      }
-      bulk_wait_read_all();   // shared memory must outlive the copy engine's reads
-      if (!ok) {
-        // let copies already in flight land before the CTA gives its shared memory back
-        const long long t0 = clock64();
-        for (int i = max(0, inflight_q - NQ); i < inflight_q; ++i)
-          while (!mbar_try_wait(bar(FB_Q_FULL + i % NQ), (i / NQ) & 1) && clock64() - t0 < 2000000) {}
-        for (int i = max(0, inflight_do - NDO); i < inflight_do; ++i)
-          while (!mbar_try_wait(bar(FB_DO_FULL + i % NDO), (i / NDO) & 1) && clock64() - t0 < 2000000) {}
-        if (real > 0)
-          while (!mbar_try_wait(bar(FB_KV_FULL), (real - 1) & 1) && clock64() - t0 < 2000000) {}
-        if (nvl > 0)
-          while (!mbar_try_wait(bar(FB_V_FULL), (nvl - 1) & 1) && clock64() - t0 < 2000000) {}
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------ MMA issuer ---------------------------------
-    if (elect_one()) {
-      constexpr uint32_t idesc_s = instr_desc_f16(BN, BM, TcElem<T>::kFormat, 0, 0);   // S^T, dP^T
-      constexpr uint32_t idesc_acc = instr_desc_f16(BN, D, TcElem<T>::kFormat, 0, 1);  // dV, dK
-      constexpr uint32_t idesc_dq = instr_desc_f16(BM, D, TcElem<T>::kFormat, 1, 1);  // dQ
-      constexpr uint32_t kTile16 = C::kTile >> 4;
-      const uint32_t k_lo = smem_desc_lo(smem + C::kK, 0), v_lo = smem_desc_lo(smem + C::kV, 0);
-      const uint32_t k_mn_lo = smem_desc_lo(smem + C::kK, BN * 128);     // K as MN-major B of dQ
-      const uint32_t q_k_lo = smem_desc_lo(smem + C::kQ0, 0);            // Q as K-major B operand
-      const uint32_t q_mn_lo = smem_desc_lo(smem + C::kQ0, BM * 128);     // Q as MN-major B operand
-      const uint32_t do_k_lo = smem_desc_lo(smem + C::kDO0, 0);
-      const uint32_t do_mn_lo = smem_desc_lo(smem + C::kDO0, BM * 128);
-      const uint32_t pd_k_lo = smem_desc_lo(smem + C::kPD, 0);            // P^T / dS^T, K-major A
-      const uint32_t pd_mn_lo = smem_desc_lo(smem + C::kPD, BN * 128);    // dS, MN-major A of dQ
-      // S^T = K Q^T into the score columns
-      auto issue_s = [&](int sq, int phq) -> bool {
-        if (!mbar_wait(bar(FB_Q_FULL + sq), phq, actx, 812)) return false;
-        tc_fence_after();
-        const uint32_t b_lo = q_k_lo + sq * kTile16;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off16 = ((k / 4) * 128 * 128 + (k % 4) * 32) >> 4;
-          mma_ss_lo(tmem + C::kColA, k_lo + off16, b_lo + off16, idesc_s, k > 0 ? 1u : 0u);
-        }
-        mma_commit(bar(FB_S_FULL));
-        return true;
-      };
-      bool ok = true;
-      int sq = 0, phq = 0, sd = 0, phd = 0;
-      int real = 0;            // items with tiles so far
-      int nv = 0;              // V tiles so far: the phase of V_FULL (a far walk after a near one loads none)
-      uint32_t gt = 0;         // tiles so far, over all items: the phase of every per-tile barrier
-      // dP^T = V dO^T of the tile in slot sd
-      auto issue_dp = [&](int sd, int phd) -> bool {
-        if (!mbar_wait(bar(FB_DO_FULL + sd), phd, actx, 814)) return false;
-        tc_fence_after();
-        const uint32_t b_lo = do_k_lo + sd * kTile16;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off16 = ((k / 4) * 128 * 128 + (k % 4) * 32) >> 4;
-          mma_ss_lo(tmem + C::kColB, v_lo + off16, b_lo + off16, idesc_s, k > 0 ? 1u : 0u);
-        }
-        mma_commit(bar(FB_DP_FULL));
-        return true;
-      };
-      // dQ = dS K into the dQ columns, a fresh accumulator: the read-out of the tile before must be over
-      auto issue_dq = [&](uint32_t pd16) -> bool {
-        if (gt > 0 && !mbar_wait(bar(FB_DQ_FREE), (gt - 1) & 1, actx, 818)) return false;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk) {
-          const uint32_t off16 = (kk * 16 * 128) >> 4;
-          mma_ss_lo(tmem + C::kColQ, pd_mn_lo + pd16 + off16, k_mn_lo + off16, idesc_dq, kk > 0 ? 1u : 0u);
-        }
-        mma_commit(bar(FB_DQ_FULL));
-        return true;
-      };
-      for (int ic = 0; ok; ++ic) {
-        const int w = ring_item(ic, 801);
-        if (w < 0 || w >= end_id) break;
-        const FusedItem it = decode(w);
-        ok = mbar_wait(bar(FB_KV_FULL), real & 1, actx, 811);
-        // shared score columns still hold dP^T of the previous item's last tile until the
-        // element-wise warps have it in registers (S^T of that tile was read before)
-        if (ok && gt > 0 && !C::kApart) ok = mbar_wait(bar(FB_DP_LOADED), (gt - 1) & 1, actx, 821);
-        if (ok) {
+    } else if (warp == 1) {
+      // ------------------------------ MMA issuer ---------------------------------
+      if (elect_one()) {
+        constexpr uint32_t idesc_s = instr_desc_f16(BN, BM, TcElem<T>::kFormat, 0, 0);   // S^T, dP^T
+        constexpr uint32_t idesc_acc = instr_desc_f16(BN, D, TcElem<T>::kFormat, 0, 1);  // dV, dK
+        constexpr uint32_t idesc_dq = instr_desc_f16(BM, D, TcElem<T>::kFormat, 1, 1);  // dQ
+        constexpr uint32_t kTile16 = C::kTile >> 4;
+        const uint32_t k_lo = smem_desc_lo(smem + C::kK, 0), v_lo = smem_desc_lo(smem + C::kV, 0);
+        const uint32_t k_mn_lo = smem_desc_lo(smem + C::kK, BN * 128);     // K as MN-major B of dQ
+        const uint32_t q_k_lo = smem_desc_lo(smem + C::kQ0, 0);            // Q as K-major B operand
+        const uint32_t q_mn_lo = smem_desc_lo(smem + C::kQ0, BM * 128);     // Q as MN-major B operand
+        const uint32_t do_k_lo = smem_desc_lo(smem + C::kDO0, 0);
+        const uint32_t do_mn_lo = smem_desc_lo(smem + C::kDO0, BM * 128);
+        const uint32_t pd_k_lo = smem_desc_lo(smem + C::kPD, 0);            // P^T / dS^T, K-major A
+        const uint32_t pd_mn_lo = smem_desc_lo(smem + C::kPD, BN * 128);    // dS, MN-major A of dQ
+        // S^T = K Q^T into the score columns
+        auto issue_s = [&](int sq, int phq) -> bool {
+          if (!mbar_wait(bar(FB_Q_FULL + sq), phq, actx, 812)) return false;
           tc_fence_after();
-          ok = issue_s(sq, phq);
-        }
-        if (C::kApart && ok) {   // dP^T of the first tile, too
-          if (it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
-          if (ok) ok = issue_dp(sd, phd);
-        }
-        for (int t = 0; t < it.T_tiles && ok; ++t, ++gt) {
-          int nsq = sq + 1, nphq = phq;
-          if (nsq == NQ) nsq = 0, nphq ^= 1;
-          const uint32_t acc = t > 0 ? 1u : 0u;                  // dK: fresh per walk
-          const uint32_t acc_dv = (t > 0 || !it.first) ? 1u : 0u;   // dV: fresh per key block
-          const uint32_t par = gt & 1;
-          int nsd = sd + 1, nphd = phd;
-          if (nsd == NDO) nsd = 0, nphd ^= 1;
-          ok = mbar_wait(bar(FB_S_LOADED), par, actx, 813);
-          if (!ok) break;
-          if (C::kApart) {
-            // S^T(t+1) over S^T(t), which every element-wise warp holds in registers
-            if (t + 1 < it.T_tiles) {
-              tc_fence_after();
-              ok = issue_s(nsq, nphq);
-            }
-          } else {
-            // dP^T(t) over S^T(t)
-            if (t == 0 && it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
+          const uint32_t b_lo = q_k_lo + sq * kTile16;
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) {
+            const uint32_t off16 = ((k / 4) * 128 * 128 + (k % 4) * 32) >> 4;
+            mma_ss_lo(tmem + C::kColA, k_lo + off16, b_lo + off16, idesc_s, k > 0 ? 1u : 0u);
+          }
+          mma_commit(bar(FB_S_FULL));
+          return true;
+        };
+        bool ok = true;
+        int sq = 0, phq = 0, sd = 0, phd = 0;
+        int real = 0;            // items with tiles so far
+        int nv = 0;              // V tiles so far: the phase of V_FULL (a far walk after a near one loads none)
+        uint32_t gt = 0;         // tiles so far, over all items: the phase of every per-tile barrier
+        // dP^T = V dO^T of the tile in slot sd
+        auto issue_dp = [&](int sd, int phd) -> bool {
+          if (!mbar_wait(bar(FB_DO_FULL + sd), phd, actx, 814)) return false;
+          tc_fence_after();
+          const uint32_t b_lo = do_k_lo + sd * kTile16;
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) {
+            const uint32_t off16 = ((k / 4) * 128 * 128 + (k % 4) * 32) >> 4;
+            mma_ss_lo(tmem + C::kColB, v_lo + off16, b_lo + off16, idesc_s, k > 0 ? 1u : 0u);
+          }
+          mma_commit(bar(FB_DP_FULL));
+          return true;
+        };
+        // dQ = dS K into the dQ columns, a fresh accumulator: the read-out of the tile before must be over
+        auto issue_dq = [&](uint32_t pd16) -> bool {
+          if (gt > 0 && !mbar_wait(bar(FB_DQ_FREE), (gt - 1) & 1, actx, 818)) return false;
+          tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < BN / 16; ++kk) {
+            const uint32_t off16 = (kk * 16 * 128) >> 4;
+            mma_ss_lo(tmem + C::kColQ, pd_mn_lo + pd16 + off16, k_mn_lo + off16, idesc_dq, kk > 0 ? 1u : 0u);
+          }
+          mma_commit(bar(FB_DQ_FULL));
+          return true;
+        };
+        for (int ic = 0; ok; ++ic) {
+          const int w = ring_item(ic, 801);
+          if (w < 0 || w >= end_id) break;
+          const FusedItem it = decode(w);
+          ok = mbar_wait(bar(FB_KV_FULL), real & 1, actx, 811);
+          // shared score columns still hold dP^T of the previous item's last tile until the
+          // element-wise warps have it in registers (S^T of that tile was read before)
+          if (ok && gt > 0 && !C::kApart) ok = mbar_wait(bar(FB_DP_LOADED), (gt - 1) & 1, actx, 821);
+          if (ok) {
+            tc_fence_after();
+            ok = issue_s(sq, phq);
+          }
+          if (C::kApart && ok) {   // dP^T of the first tile, too
+            if (it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
             if (ok) ok = issue_dp(sd, phd);
           }
-          if (!ok) break;
-          // dV += P^T(t) dO(t), P^T from TMEM
-          ok = mbar_wait(bar(FB_PT_FULL), par, actx, 815);
-          if (!ok) break;
-          tc_fence_after();
-          {
-            const uint32_t b_lo = do_mn_lo + sd * kTile16;
-#pragma unroll
-            for (int kk = 0; kk < BM / 16; ++kk)
-              mma_ts_lo(tmem + C::kColDV, tmem + C::kColP + kk * 8, b_lo + ((kk * 16 * 128) >> 4),
-                        idesc_acc, kk > 0 ? 1u : acc_dv);
-            mma_commit(bar(FB_DO_FREE + sd));
-            if (t + 1 == it.T_tiles) mma_commit(bar(FB_DV_DONE));
-          }
-          // once every element-wise warp holds dP^T(t) in registers: the product that takes its columns,
-          // S^T(t+1) or, where S^T has its own, dP^T(t+1)
-          if (t + 1 < it.T_tiles) {
-            ok = mbar_wait(bar(FB_DP_LOADED), par, actx, 816);
+          for (int t = 0; t < it.T_tiles && ok; ++t, ++gt) {
+            int nsq = sq + 1, nphq = phq;
+            if (nsq == NQ) nsq = 0, nphq ^= 1;
+            const uint32_t acc = t > 0 ? 1u : 0u;                  // dK: fresh per walk
+            const uint32_t acc_dv = (t > 0 || !it.first) ? 1u : 0u;   // dV: fresh per key block
+            const uint32_t par = gt & 1;
+            int nsd = sd + 1, nphd = phd;
+            if (nsd == NDO) nsd = 0, nphd ^= 1;
+            ok = mbar_wait(bar(FB_S_LOADED), par, actx, 813);
+            if (!ok) break;
+            if (C::kApart) {
+              // S^T(t+1) over S^T(t), which every element-wise warp holds in registers
+              if (t + 1 < it.T_tiles) {
+                tc_fence_after();
+                ok = issue_s(nsq, nphq);
+              }
+            } else {
+              // dP^T(t) over S^T(t)
+              if (t == 0 && it.first) ok = mbar_wait(bar(FB_V_FULL), (nv++) & 1, actx, 820);
+              if (ok) ok = issue_dp(sd, phd);
+            }
+            if (!ok) break;
+            // dV += P^T(t) dO(t), P^T from TMEM
+            ok = mbar_wait(bar(FB_PT_FULL), par, actx, 815);
             if (!ok) break;
             tc_fence_after();
-            ok = C::kApart ? issue_dp(nsd, nphd) : issue_s(nsq, nphq);
-            if (!ok) break;
-          }
-          // dQ(t) = dS(t) K
-          ok = mbar_wait(bar(FB_DS_FULL), par, actx, 817);
-          const uint32_t pd16 = C::NPD == 2 ? (gt & 1) * (C::kPdBytes >> 4) : 0;
-          if (ok) ok = issue_dq(pd16);
-          if (!ok) break;
-          // dK += dS^T(t) Q(t)
-          {
-            const uint32_t b_lo = q_mn_lo + sq * kTile16;
+            {
+              const uint32_t b_lo = do_mn_lo + sd * kTile16;
 #pragma unroll
-            for (int kk = 0; kk < BM / 16; ++kk) {
-              const uint32_t a_off16 = ((kk / 4) * 128 * 128 + (kk % 4) * 32) >> 4;
-              mma_ss_lo(tmem + C::kColDK, pd_k_lo + pd16 + a_off16, b_lo + ((kk * 16 * 128) >> 4), idesc_acc,
-                        kk > 0 ? 1u : acc);
+              for (int kk = 0; kk < BM / 16; ++kk)
+                mma_ts_lo(tmem + C::kColDV, tmem + C::kColP + kk * 8, b_lo + ((kk * 16 * 128) >> 4),
+                          idesc_acc, kk > 0 ? 1u : acc_dv);
+              mma_commit(bar(FB_DO_FREE + sd));
+              if (t + 1 == it.T_tiles) mma_commit(bar(FB_DV_DONE));
             }
-            mma_commit(bar(FB_Q_FREE + sq));
-          }
-          sq = nsq, phq = nphq;
-          sd = nsd, phd = nphd;
-        }
-        if (!ok) break;
-        mma_commit(bar(FB_DONE));
-        ++real;
-      }
-      // the last commit's arrive must land before this CTA's shared memory is given back
-      if (ok && real > 0) mbar_wait(bar(FB_DONE), (real - 1) & 1, actx, 819);
-    }
-  } else if (warp == 2 + kEwWarps + 4) {
-    // ------------------------------ statistics warp ----------------------------
-    // -lse * log2(e) and -delta of the 128 queries of every tile go through shared memory, where
-    // the element-wise threads read them as broadcast vectors (every thread needs the values of
-    // all its 32 query columns; fetching them lane by lane and shuffling costs 64 shuffles per
-    // thread and tile in a load/store queue that is already the busiest unit).  Queries past M
-    // get lse = +inf, which makes their P exactly zero.  One buffer each: lse(t) may be written
-    // once phase 1 of the tile before is over, delta(t) once its phase 2 is.
-    float4 *lse_s = reinterpret_cast<float4 *>(smem_gen + C::kStats);
-    float4 *dlt_s = lse_s + 32;
-    bool ok = true;
-    uint32_t gt = 0;
-    for (int ic = 0; ok; ++ic) {
-      const int w = ring_item(ic, 950);
-      if (w < 0 || w >= end_id) break;
-      const FusedItem it = decode(w);
-      int h = it.hk * G, mt = it.mt_lo;
-      for (int t = 0; t < it.T_tiles; ++t, ++gt) {
-        const int m = mt * BM + lane * 4;
-        const int64_t li = ((int64_t)it.b * p.H + h) * p.M + m;
-        if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
-        float l[4], d[4];
+            // once every element-wise warp holds dP^T(t) in registers: the product that takes its columns,
+            // S^T(t+1) or, where S^T has its own, dP^T(t+1)
+            if (t + 1 < it.T_tiles) {
+              ok = mbar_wait(bar(FB_DP_LOADED), par, actx, 816);
+              if (!ok) break;
+              tc_fence_after();
+              ok = C::kApart ? issue_dp(nsd, nphd) : issue_s(nsq, nphq);
+              if (!ok) break;
+            }
+            // dQ(t) = dS(t) K
+            ok = mbar_wait(bar(FB_DS_FULL), par, actx, 817);
+            const uint32_t pd16 = C::NPD == 2 ? (gt & 1) * (C::kPdBytes >> 4) : 0;
+            if (ok) ok = issue_dq(pd16);
+            if (!ok) break;
+            // dK += dS^T(t) Q(t)
+            {
+              const uint32_t b_lo = q_mn_lo + sq * kTile16;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          l[j] = m + j < p.M ? -p.lse[li + j] * kLog2e : -INFINITY;
-          d[j] = m + j < p.M ? -p.delta[li + j] : 0.f;
+              for (int kk = 0; kk < BM / 16; ++kk) {
+                const uint32_t a_off16 = ((kk / 4) * 128 * 128 + (kk % 4) * 32) >> 4;
+                mma_ss_lo(tmem + C::kColDK, pd_k_lo + pd16 + a_off16, b_lo + ((kk * 16 * 128) >> 4), idesc_acc,
+                          kk > 0 ? 1u : acc);
+              }
+              mma_commit(bar(FB_Q_FREE + sq));
+            }
+            sq = nsq, phq = nphq;
+            sd = nsd, phd = nphd;
+          }
+          if (!ok) break;
+          mma_commit(bar(FB_DONE));
+          ++real;
         }
-        if (gt > 0) ok = mbar_wait(bar(FB_PT_FULL), (gt - 1) & 1, actx, 951);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        lse_s[lane] = make_float4(l[0], l[1], l[2], l[3]);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(FB_S_FULL));
-        if (gt > 0) ok = mbar_wait(bar(FB_DS_FULL), (gt - 1) & 1, actx, 952);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        dlt_s[lane] = make_float4(d[0], d[1], d[2], d[3]);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(FB_DP_FULL));
+        // the last commit's arrive must land before this CTA's shared memory is given back
+        if (ok && real > 0) mbar_wait(bar(FB_DONE), (real - 1) & 1, actx, 819);
+      }
+    } else if (warp == 2) {
+      // ------------------------------ statistics warp ----------------------------
+      // -lse * log2(e) and -delta of the 128 queries of every tile go through shared memory, where
+      // the element-wise threads read them as broadcast vectors (every thread needs the values of
+      // all its 32 query columns; fetching them lane by lane and shuffling costs 64 shuffles per
+      // thread and tile in a load/store queue that is already the busiest unit).  Queries past M
+      // get lse = +inf, which makes their P exactly zero.  One buffer each: lse(t) may be written
+      // once phase 1 of the tile before is over, delta(t) once its phase 2 is.
+      float4 *lse_s = reinterpret_cast<float4 *>(smem_gen + C::kStats);
+      float4 *dlt_s = lse_s + 32;
+      bool ok = true;
+      uint32_t gt = 0;
+      for (int ic = 0; ok; ++ic) {
+        const int w = ring_item(ic, 950);
+        if (w < 0 || w >= end_id) break;
+        const FusedItem it = decode(w);
+        int h = it.hk * G, mt = it.mt_lo;
+        for (int t = 0; t < it.T_tiles; ++t, ++gt) {
+          const int m = mt * BM + lane * 4;
+          const int64_t li = ((int64_t)it.b * p.H + h) * p.M + m;
+          if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
+          float l[4], d[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            l[j] = m + j < p.M ? -p.lse[li + j] * kLog2e : -INFINITY;
+            d[j] = m + j < p.M ? -p.delta[li + j] : 0.f;
+          }
+          if (gt > 0) ok = mbar_wait(bar(FB_PT_FULL), (gt - 1) & 1, actx, 951);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          lse_s[lane] = make_float4(l[0], l[1], l[2], l[3]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(FB_S_FULL));
+          if (gt > 0) ok = mbar_wait(bar(FB_DS_FULL), (gt - 1) & 1, actx, 952);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          dlt_s[lane] = make_float4(d[0], d[1], d[2], d[3]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(FB_DP_FULL));
+        }
       }
     }
-  } else if (warp >= 2 + kEwWarps) {
+  } else if (warp < kFusedEwWarp) {
+    regs_keep_48();
     // ------------------------------ dQ reduction warps --------------------------
     // dQ(t) = dS K is a complete 128 x D product per tile.  These four warps (one per TMEM lane
-    // slice = 32 query rows) move it out of TMEM a quarter of the columns at a time into a
+    // slice = 32 query rows) move it out of TMEM 32 columns at a time into a
     // shared-memory staging buffer, from where the copy engine adds it to the fp32 workspace
     // (`cp.reduce.async.bulk`, 2 KB runs).  An SM retires fp32 reductions at about 26 bytes per
     // clock whoever issues them, so the 64 KB of a tile take about as long as its GEMMs; issued
     // as `red` instructions they fill the load/store queue and stall every warp of the SM that
-    // shuffles or touches shared memory.  Two staging buffers: a quarter drains while the next
+    // shuffles or touches shared memory.  Two staging buffers: one part drains while the next
     // is staged.
     const int slice = warp & 3;
     const int row = slice * 32 + lane;
     const uint32_t tlane = tmem + ((uint32_t)(slice * 32) << 16);
-    const bool issuer = (warp == 2 + kEwWarps) && lane == 0;
-    constexpr int QC = D / 4;                 // columns per quarter
+    const bool issuer = warp == kFusedRedWarp && lane == 0;
+    constexpr int QC = 32, kParts = D / QC;   // columns of a part, parts of a tile
     int buf = 0;
     bool ok = true;
     uint32_t gt = 0;
@@ -710,30 +722,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                      (((int64_t)it.b * p.H + h) * (fp.Mpad / BM) + mt) * (int64_t)(BM * D);
         if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
 #pragma unroll
-        for (int qd = 0; qd < 4; ++qd) {
+        for (int qd = 0; qd < kParts; ++qd) {
           if (qd == 0) {
             ok = red_warps_all(mbar_wait(bar(FB_DQ_FULL), gt & 1, actx, 921));
             if (!ok) break;
             tc_fence_after();
           }
           uint32_t qr[QC];
-          if (QC == 32) tmem_ld32(tlane + C::kColQ + qd * QC, *reinterpret_cast<uint32_t(*)[32]>(qr));
-          else tmem_ld16(tlane + C::kColQ + qd * QC, qr);
+          tmem_ld32(tlane + C::kColQ + qd * QC, qr);
           tmem_wait_ld();
           if (C::kPAliasesDQ && qd == 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(FB_DP_FULL));   // the next P^T may take the first 64 columns
           }
-          if (qd == 3) {
+          if (qd == kParts - 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(FB_DQ_FREE));   // the next dQ may overwrite the columns
           }
-          // the copy engine must have read what this buffer held two quarters ago
+          // the copy engine must have read what this buffer held two parts ago
           if (issuer) bulk_wait_read_1();
           red_warps_sync();
-          uint8_t *stage = smem_gen + C::kStage + buf * C::kQuarter + row * 16;
+          uint8_t *stage = smem_gen + C::kStage + buf * C::kPart + row * 16;
 #pragma unroll
           for (int g = 0; g < QC / 4; ++g)
             *reinterpret_cast<uint4 *>(stage + g * 2048) =
@@ -741,9 +752,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           fence_proxy_async_smem();
           red_warps_sync();
           if (issuer) {
-            // one contiguous run per quarter; rows past M hold zeros and land in padding
-            bulk_reduce_add_f32(dst + qd * (C::kQuarter / 4), smem + C::kStage + buf * C::kQuarter,
-                                C::kQuarter);
+            // one contiguous run per part; rows past M hold zeros and land in padding
+            bulk_reduce_add_f32(dst + qd * (C::kPart / 4), smem + C::kStage + buf * C::kPart,
+                                C::kPart);
             bulk_commit();
           }
           buf ^= 1;
@@ -754,7 +765,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     if (issuer) bulk_wait_read_all();   // shared memory must outlive the copy engine's reads
   } else {
     // ------------------------------ element-wise warps --------------------------
-    const int ew = warp - 2;
+    regs_take_96();
+    const int ew = warp - kFusedEwWarp;
     const int slice = warp & 3, cg = ew >> 2;       // TMEM lane slice, 32-column group
     const int row = slice * 32 + lane;              // accumulator row of this thread
     const uint32_t tlane = tmem + ((uint32_t)(slice * 32) << 16);
@@ -839,9 +851,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         __syncwarp();
         tc_fence_after();
         float pv[32];
-        uint32_t sr[32];
+        uint32_t sr[32];     // S^T, then dP^T
         tmem_ld32(tlane + C::kColA + cg * 32, sr);
-        // while the load is in flight: the masks
+        tmem_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(FB_S_LOADED));   // the next product may overwrite S^T
         // Tiles away from every boundary (sequence end, causal diagonal, piecewise threshold) need no
         // masking at all; the others mask with one unsigned range check per element:
         // column c is visible iff cmin <= c < cmin + cwidth.
@@ -858,10 +873,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (!key_ok) cmin = 32;
         const unsigned cwidth = (unsigned)max(cmax - cmin, 0);
         {
-          tmem_wait_ld();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(FB_S_LOADED));   // dP^T(t) may overwrite S^T(t)
           // packed fp32 pairs: one FMA per two elements
           const uint64_t scale2 = f2_pack(qk_scale, qk_scale);
 #pragma unroll
@@ -898,55 +909,42 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           __syncwarp();
           tc_fence_after();
           tmem_st16(tlane + C::kColP + cg * 16, pk);
+          tmem_ld32(tlane + C::kColB + cg * 32, sr);   // dP^T comes while P^T goes
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(FB_PT_FULL));
         }
         // ---- phase 2: dS^T = P^T * (dP^T - delta) -> PD ----
-        uint32_t sr0[16];
-        tmem_ld16(tlane + C::kColB + cg * 32, sr0);
         {
           uint32_t pk[16];
-          // P * (dP - delta) of 16 columns, two elements per instruction
-          auto half_ds = [&](int hf, const uint32_t (&sr)[16]) {
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(FB_DP_LOADED));   // the next product may overwrite dP^T(t)
+          // P * (dP - delta), two elements per instruction
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 d4 = dlt_s[hf * 4 + i];
-              const int c = 4 * i;
-              float e0, e1, e2, e3;
-              if (DROP) {
-                const int k4 = keep >> (hf * 16 + c);
-                auto ds = [&](int i, float dlt) {
-                  return pv[hf * 16 + c + i] *
-                         fmaf(k4 >> i & 1 ? __uint_as_float(sr[c + i]) : 0.f, fp.drop.rp, dlt);
-                };
-                pk[hf * 8 + 2 * i] = TcElem<T>::pack(ds(0, d4.x), ds(1, d4.y));
-                pk[hf * 8 + 2 * i + 1] = TcElem<T>::pack(ds(2, d4.z), ds(3, d4.w));
-                continue;
-              }
-              f2_unpack(f2_mul(f2_pack(pv[hf * 16 + c], pv[hf * 16 + c + 1]),
-                               f2_add(f2_pack(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])),
-                                      f2_pack(d4.x, d4.y))),
-                        e0, e1);
-              f2_unpack(f2_mul(f2_pack(pv[hf * 16 + c + 2], pv[hf * 16 + c + 3]),
-                               f2_add(f2_pack(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])),
-                                      f2_pack(d4.z, d4.w))),
-                        e2, e3);
-              pk[hf * 8 + 2 * i] = TcElem<T>::pack(e0, e1);
-              pk[hf * 8 + 2 * i + 1] = TcElem<T>::pack(e2, e3);
+          for (int i = 0; i < 8; ++i) {
+            const float4 d4 = dlt_s[i];
+            const int c = 4 * i;
+            float e0, e1, e2, e3;
+            if (DROP) {
+              const int k4 = keep >> c;
+              auto ds = [&](int i, float dlt) {
+                return pv[c + i] * fmaf(k4 >> i & 1 ? __uint_as_float(sr[c + i]) : 0.f, fp.drop.rp, dlt);
+              };
+              pk[2 * i] = TcElem<T>::pack(ds(0, d4.x), ds(1, d4.y));
+              pk[2 * i + 1] = TcElem<T>::pack(ds(2, d4.z), ds(3, d4.w));
+              continue;
             }
-          };
-          tmem_wait_ld();            // first 16 columns (requested before the fence above)
-          half_ds(0, sr0);
-          {
-            uint32_t sr1[16];
-            tmem_ld16(tlane + C::kColB + cg * 32 + 16, sr1);
-            tmem_wait_ld();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(FB_DP_LOADED));   // the next S^T may overwrite dP^T(t)
-            half_ds(1, sr1);
+            f2_unpack(f2_mul(f2_pack(pv[c], pv[c + 1]),
+                             f2_add(f2_pack(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), f2_pack(d4.x, d4.y))),
+                      e0, e1);
+            f2_unpack(f2_mul(f2_pack(pv[c + 2], pv[c + 3]),
+                             f2_add(f2_pack(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), f2_pack(d4.z, d4.w))),
+                      e2, e3);
+            pk[2 * i] = TcElem<T>::pack(e0, e1);
+            pk[2 * i + 1] = TcElem<T>::pack(e2, e3);
           }
           // at the first tile of an item, PD may hold the staged dK of the item before until it is stored
           if (t == 0 && real > 0) {
