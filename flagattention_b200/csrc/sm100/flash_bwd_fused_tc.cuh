@@ -181,7 +181,7 @@ struct FusedItem {
 // The 32 keep bits of a thread do not depend on the scores and are computed before the wait for them.
 // Backward at head_dim 64, p = 0.1, bf16, pair of mma.sync kernels (bits computed in both) -> this:
 // B=16 H=16 L=512 662 -> 246 us (120 us without dropout), B=4 H=16 L=2048 causal 1485 -> 421 us; at 128 1858 -> 481 us.
-// The drawing does not fit the registers beside the rest: 96 and 200 bytes of spill stores and loads a thread at 64, 64 and 144 at
+// The drawing does not fit the registers beside the rest: 80 and 188 bytes of spill stores and loads a thread at 64, 48 and 136 at
 // 128 (without dropout 48 and 188, and 12 and 92).
 template <typename T, int D, bool DROP>
 __global__ void __launch_bounds__(kFusedThreads, 1)
@@ -652,8 +652,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       // thread and tile in a load/store queue that is already the busiest unit).  Queries past M
       // get lse = +inf, which makes their P exactly zero.  One buffer each: lse(t) may be written
       // once phase 1 of the tile before is over, delta(t) once its phase 2 is.
-      float4 *lse_s = reinterpret_cast<float4 *>(smem_gen + C::kStats);
-      float4 *dlt_s = lse_s + 32;
+      // Query 8 j + 2 q + e of a group of 32 lies at 8 q + 2 j + e: the eight a thread of the fragments needs are
+      // next to one another.
+      float2 *lse_s = reinterpret_cast<float2 *>(smem_gen + C::kStats) + (lane >> 3) * 16 + (lane & 1) * 8 + (lane >> 1 & 3);
+      float2 *dlt_s = lse_s + 64;
       bool ok = true;
       uint32_t gt = 0;
       for (int ic = 0; ok; ++ic) {
@@ -674,13 +676,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           if (gt > 0) ok = mbar_wait(bar(FB_PT_FULL), (gt - 1) & 1, actx, 951);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          lse_s[lane] = make_float4(l[0], l[1], l[2], l[3]);
+          lse_s[0] = make_float2(l[0], l[1]);
+          lse_s[4] = make_float2(l[2], l[3]);
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(FB_S_FULL));
           if (gt > 0) ok = mbar_wait(bar(FB_DS_FULL), (gt - 1) & 1, actx, 952);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          dlt_s[lane] = make_float4(d[0], d[1], d[2], d[3]);
+          dlt_s[0] = make_float2(d[0], d[1]);
+          dlt_s[4] = make_float2(d[2], d[3]);
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(FB_DP_FULL));
         }
@@ -771,17 +775,24 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     const int row = slice * 32 + lane;              // accumulator row of this thread
     const uint32_t tlane = tmem + ((uint32_t)(slice * 32) << 16);
     const float qk_scale = p.sm_scale * kLog2e;
-    // this thread's 64 bytes of a PD row: sub-tile cg / 2, 16-byte chunks (cg & 1) * 4 .. + 3
-    uint8_t *pd_row = smem_gen + C::kPD + (cg >> 1) * (128 * 128) + row * 128;
-    const int pd_chunk0 = (cg & 1) * 4, pd_xor = row & 7;
+    // S^T, dP^T, P^T and dS^T are held as fragments (tmem_ld_frag32()): 4 keys x 8 queries a thread.  Every
+    // thread needs lse and delta of its queries, and there the fragments take 4 16-byte loads from shared memory
+    // a tile where a row a thread takes 16 (two cycles each of the pipe that the stores and barriers need, too):
+    // backward call of B=2 H=16 L=4096 not causal, fp16, 389 -> 380 us at head_dim 64, 643 -> 640 us at 128.
+    const int frow = slice * 32 + (lane >> 2);      // its keys: frow + 8 i
+    const int fcol = cg * 32 + 2 * (lane & 3);      // its queries: fcol + 8 j + e
+    // PD: sub-tile cg / 2, 16-byte chunks (cg & 1) * 4 .. + 3 of 32 rows, one 8 x 8 matrix a chunk and 8 rows
+    const uint32_t pd_lane = smem + C::kPD + (cg >> 1) * (128 * 128) + (slice * 32 + (lane & 7)) * 128 +
+                             ((((cg & 1) * 4 + (lane >> 3)) ^ (lane & 7)) << 4);
     auto store_pd = [&](const uint32_t (&pk)[16], uint32_t off) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<uint4 *>(pd_row + off + (((pd_chunk0 + j) ^ pd_xor) << 4)) =
-            make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t *r = pk + (i >> 1) * 8 + (i & 1);
+        stmatrix4(pd_lane + off + i * (8 * 128), r[0], r[2], r[4], r[6]);
+      }
     };
-    // -lse * log2(e) / -delta of this thread's 32 query columns, as staged by the statistics warp
-    const float4 *lse_s = reinterpret_cast<const float4 *>(smem_gen + C::kStats) + cg * 8;
+    // -lse * log2(e) / -delta of this thread's 8 queries, as staged by the statistics warp
+    const float4 *lse_s = reinterpret_cast<const float4 *>(smem_gen + C::kStats) + cg * 8 + (lane & 3) * 2;
     const float4 *dlt_s = lse_s + 32;
     // write-out of dV and dK: warp (slice, cg) owns columns cg * D / 4 .. of its 32 rows
     constexpr int QC = D / 4;
@@ -841,9 +852,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       for (int t = 0; t < it.T_tiles; ++t, ++gt) {
         const int m0 = mt * BM;
         uint32_t keep = 0;
-        if (DROP)
+        if (DROP)   // (lane = key, bit = query)
           keep = dropout_keep_bits32(
               fp.drop, fp.drop.offset + (((uint64_t)it.b * p.H + h) * p.M + m0 + cg * 32) * p.N + key, (uint32_t)p.N);
+        auto kept = [&](uint32_t word, int j, int e) { return (word >> (8 * j + 2 * (lane & 3) + e) & 1u) != 0; };
+        uint32_t kw[4] = {0u, 0u, 0u, 0u};
+        if (DROP) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) kw[i] = __shfl_sync(0xffffffffu, keep, (lane >> 2) + 8 * i);
+        }
         if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
 
         // ---- phase 1: P^T = exp2(S^T * scale - lse) -> TMEM ----
@@ -852,7 +869,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         tc_fence_after();
         float pv[32];
         uint32_t sr[32];     // S^T, then dP^T
-        tmem_ld32(tlane + C::kColA + cg * 32, sr);
+        tmem_ld_frag32(tlane + C::kColA + cg * 32, sr);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
@@ -863,42 +880,50 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         bool interior = (n0 + BN <= p.N) && (!p.causal || m0 + p_seq >= n0 + BN - 1);
         if (it.mode == 1) interior = interior && (m0 + BM - 1 + p_seq - n0 < p.w);
         if (it.mode == 2) interior = interior && (m0 + p_seq - (n0 + BN - 1) >= p.w);
-        int cmin = 0, cmax = 32;
-        if (p.causal) cmin = max(cmin, key - p_seq - m0 - cg * 32);
-        if (it.mode) {
-          const int cnear = p.w + key - p_seq - m0 - cg * 32;  // columns below it are near pairs
-          if (it.mode == 1) cmax = min(cmax, cnear);
-          else cmin = max(cmin, cnear);
-        }
-        if (!key_ok) cmin = 32;
-        const unsigned cwidth = (unsigned)max(cmax - cmin, 0);
         {
           // packed fp32 pairs: one FMA per two elements
           const uint64_t scale2 = f2_pack(qk_scale, qk_scale);
+          const float4 la = lse_s[0], lb = lse_s[1];
+          const uint64_t l2[4] = {f2_pack(la.x, la.y), f2_pack(la.z, la.w), f2_pack(lb.x, lb.y), f2_pack(lb.z, lb.w)};
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 l4 = lse_s[i];
-            f2_unpack(f2_fma(f2_pack(__uint_as_float(sr[4 * i]), __uint_as_float(sr[4 * i + 1])), scale2,
-                             f2_pack(l4.x, l4.y)),
-                      pv[4 * i], pv[4 * i + 1]);
-            f2_unpack(f2_fma(f2_pack(__uint_as_float(sr[4 * i + 2]), __uint_as_float(sr[4 * i + 3])),
-                             scale2, f2_pack(l4.z, l4.w)),
-                      pv[4 * i + 2], pv[4 * i + 3]);
-          }
+          for (int k = 0; k < 16; ++k)
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(sr[2 * k]), __uint_as_float(sr[2 * k + 1])), scale2,
+                             l2[(k >> 1) & 3]),
+                      pv[2 * k], pv[2 * k + 1]);
         }
         if (!interior) {
 #pragma unroll
-          for (int c = 0; c < 32; ++c)
-            pv[c] = ((unsigned)(c - cmin) < cwidth) ? pv[c] : -INFINITY;  // exp2(-inf) = 0
+          for (int i = 0; i < 4; ++i) {
+            const int key = n0 + frow + 8 * i;
+            const int base = key - p_seq - m0 - fcol;   // column 8 j + e of this thread is at or past the key: c >= base
+            int cmin = 0, cmax = 32;
+            if (p.causal) cmin = max(cmin, base);
+            if (it.mode == 1) cmax = min(cmax, p.w + base);   // columns below p.w + base are near pairs
+            if (it.mode == 2) cmin = max(cmin, p.w + base);
+            if (key >= p.N) cmin = 32;
+            const unsigned cwidth = (unsigned)max(cmax - cmin, 0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                float &x = pv[(i >> 1) * 16 + 4 * j + (i & 1) * 2 + e];
+                x = ((unsigned)(8 * j + e - cmin) < cwidth) ? x : -INFINITY;   // exp2(-inf) = 0
+              }
+          }
         }
         {
           uint32_t pk[16];
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            pv[c] = ex2(pv[c]);
-            pv[c + 1] = ex2(pv[c + 1]);
-            pk[c >> 1] = DROP ? TcElem<T>::pack(keep >> c & 1u ? pv[c] : 0.f, keep >> (c + 1) & 1u ? pv[c + 1] : 0.f)
-                              : TcElem<T>::pack(pv[c], pv[c + 1]);
+          for (int k = 0; k < 16; ++k) {
+            pv[2 * k] = ex2(pv[2 * k]);
+            pv[2 * k + 1] = ex2(pv[2 * k + 1]);
+            if (DROP) {
+              const uint32_t word = kw[(k >> 3) * 2 + (k & 1)];
+              pk[k] = TcElem<T>::pack(kept(word, (k >> 1) & 3, 0) ? pv[2 * k] : 0.f,
+                                      kept(word, (k >> 1) & 3, 1) ? pv[2 * k + 1] : 0.f);
+            } else {
+              pk[k] = TcElem<T>::pack(pv[2 * k], pv[2 * k + 1]);
+            }
           }
           // dP^T(t), by now usually there (issued as soon as S^T(t) had been read, or before).  Commits
           // complete in issue order, so this barrier also says that the products which read what is
@@ -908,8 +933,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           ok = mbar_wait(bar(FB_DP_FULL), gt & 1, actx, 913) && ok;
           __syncwarp();
           tc_fence_after();
-          tmem_st16(tlane + C::kColP + cg * 16, pk);
-          tmem_ld32(tlane + C::kColB + cg * 32, sr);   // dP^T comes while P^T goes
+          tmem_st_frag16(tlane + C::kColP + cg * 16, pk);
+          tmem_ld_frag32(tlane + C::kColB + cg * 32, sr);   // dP^T comes while P^T goes
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
@@ -923,28 +948,23 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(FB_DP_LOADED));   // the next product may overwrite dP^T(t)
           // P * (dP - delta), two elements per instruction
+          const float4 da = dlt_s[0], db = dlt_s[1];
+          const float d8[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 d4 = dlt_s[i];
-            const int c = 4 * i;
-            float e0, e1, e2, e3;
+          for (int k = 0; k < 16; ++k) {
+            const int j = (k >> 1) & 3;
+            float e0, e1;
             if (DROP) {
-              const int k4 = keep >> c;
-              auto ds = [&](int i, float dlt) {
-                return pv[c + i] * fmaf(k4 >> i & 1 ? __uint_as_float(sr[c + i]) : 0.f, fp.drop.rp, dlt);
-              };
-              pk[2 * i] = TcElem<T>::pack(ds(0, d4.x), ds(1, d4.y));
-              pk[2 * i + 1] = TcElem<T>::pack(ds(2, d4.z), ds(3, d4.w));
-              continue;
+              const uint32_t word = kw[(k >> 3) * 2 + (k & 1)];
+              e0 = pv[2 * k] * fmaf(kept(word, j, 0) ? __uint_as_float(sr[2 * k]) : 0.f, fp.drop.rp, d8[2 * j]);
+              e1 = pv[2 * k + 1] * fmaf(kept(word, j, 1) ? __uint_as_float(sr[2 * k + 1]) : 0.f, fp.drop.rp, d8[2 * j + 1]);
+            } else {
+              f2_unpack(f2_mul(f2_pack(pv[2 * k], pv[2 * k + 1]),
+                               f2_add(f2_pack(__uint_as_float(sr[2 * k]), __uint_as_float(sr[2 * k + 1])),
+                                      f2_pack(d8[2 * j], d8[2 * j + 1]))),
+                        e0, e1);
             }
-            f2_unpack(f2_mul(f2_pack(pv[c], pv[c + 1]),
-                             f2_add(f2_pack(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), f2_pack(d4.x, d4.y))),
-                      e0, e1);
-            f2_unpack(f2_mul(f2_pack(pv[c + 2], pv[c + 3]),
-                             f2_add(f2_pack(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), f2_pack(d4.z, d4.w))),
-                      e2, e3);
-            pk[2 * i] = TcElem<T>::pack(e0, e1);
-            pk[2 * i + 1] = TcElem<T>::pack(e2, e3);
+            pk[k] = TcElem<T>::pack(e0, e1);
           }
           // at the first tile of an item, PD may hold the staged dK of the item before until it is stored
           if (t == 0 && real > 0) {

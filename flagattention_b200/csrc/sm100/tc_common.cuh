@@ -320,6 +320,42 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
       : "memory");
 }
 
+// The same 32 lanes x 32 columns in the fragments of an 8 x 8 matrix product (two 16-lane halves, 16x256b): thread l
+// holds rows l / 4 + 8 i (i = 0..3) and columns 8 j + 2 (l % 4) + e (j = 0..3, e = 0, 1) in
+// r[(i / 2) * 16 + 4 j + (i % 2) * 2 + e].
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&r)[32]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[16 * h]), "=r"(r[16 * h + 1]), "=r"(r[16 * h + 2]), "=r"(r[16 * h + 3]), "=r"(r[16 * h + 4]),
+          "=r"(r[16 * h + 5]), "=r"(r[16 * h + 6]), "=r"(r[16 * h + 7]), "=r"(r[16 * h + 8]), "=r"(r[16 * h + 9]),
+          "=r"(r[16 * h + 10]), "=r"(r[16 * h + 11]), "=r"(r[16 * h + 12]), "=r"(r[16 * h + 13]),
+          "=r"(r[16 * h + 14]), "=r"(r[16 * h + 15])
+        : "r"(taddr + ((uint32_t)(16 * h) << 16))
+        : "memory");
+}
+// 32 lanes x 16 columns of packed pairs: pair (row, columns 8 j + 2 (l % 4), + 1) of those fragments, r[k] = the pair
+// of elements 2 k, 2 k + 1 above
+__device__ __forceinline__ void tmem_st_frag16(uint32_t taddr, const uint32_t (&r)[16]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(
+            taddr + ((uint32_t)(16 * h) << 16)),
+        "r"(r[8 * h]), "r"(r[8 * h + 1]), "r"(r[8 * h + 2]), "r"(r[8 * h + 3]), "r"(r[8 * h + 4]),
+        "r"(r[8 * h + 5]), "r"(r[8 * h + 6]), "r"(r[8 * h + 7])
+        : "memory");
+}
+// four 8 x 8 matrices of 16-bit elements, fragments -> shared memory: lanes 8 m .. 8 m + 7 give the row addresses of
+// matrix m
+__device__ __forceinline__ void stmatrix4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(r0), "r"(r1),
+               "r"(r2), "r"(r3)
+               : "memory");
+}
+
 template <typename T>
 struct TcElem;
 template <>
