@@ -157,11 +157,12 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
   if (stages & 2) {
     // the CTAs of a (batch, kv head) pair share its Q and dO tiles and its slice of the dq workspace
     p.num_blocks = (s->N + C::BN - 1) / C::BN;
-    p.group_size = cta_group_size((int64_t)(s->H / s->Hk) * s->M * D * 8 * n_acc, s->B * s->Hk);
     const int64_t items = (int64_t)p.num_blocks * s->Hk * s->B;
     const int sms = sm_count();
     if (items > 0x3fffffff) return FA_ERR_TOO_LARGE;
     if (sms <= 0) return FA_ERR_LAUNCH;
+    p.group_size = backward_group_size((int64_t)(s->H / s->Hk) * s->M * D * 8 * n_acc, s->B * s->Hk, items, sms,
+                                       s->causal);
     fp.num_items = (int)items;
     // dk / dv rows of key blocks that walk no query tile (which the kernel skips) get their zeros
     // here: dk of a branch where the block holds no pair of that branch, dv where it holds none at all

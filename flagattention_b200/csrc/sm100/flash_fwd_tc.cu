@@ -50,9 +50,9 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   p.status = device_status_word();
   p.d = s->D;
   if (DROP) p.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
-  // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise)
+  // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise), with those of its group's heads
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
-  p.group_size = cta_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2), s->B * s->H);
+  p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal);
   dim3 grid((unsigned)((int64_t)p.num_m_blocks * s->B * s->H), 1, 1);
   kern<<<grid, C::kThreads, C::kTotal, stream>>>(mq, mk, mv, mq2, mk2, p);
   FA_CHECK_LAUNCH();
@@ -123,7 +123,7 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
   p.status = device_status_word();
   p.d = s->D;
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
-  p.group_size = cta_group_size((int64_t)s->N * D * 2 * 2, s->B * s->H);
+  p.group_size = forward_group_size((int64_t)s->N * D * 2 * 2 * s->Hk / s->H, s->B * s->H, s->causal);
   const int64_t items = (int64_t)p.num_m_blocks * s->B * s->H;
   const int sms = sm_count_fwd();
   fp.sched = fwd_sched_slot();

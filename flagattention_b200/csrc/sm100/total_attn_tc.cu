@@ -26,7 +26,9 @@ static int launch_total_tc(const fa_flash_shape *s, const fa_tensor4 *q, const f
   p.B = s->B, p.H = s->H, p.Hk = s->Hk, p.M = s->M, p.N = s->N;
   p.causal = s->causal, p.sm_scale = s->sm_scale;
   p.status = device_status_word();
-  dim3 grid((s->N + C::BN - 1) / C::BN, s->B * s->H, 1);
+  // the CTAs of a (batch, head) pair share its Q and lse
+  p.group_size = forward_group_size((int64_t)s->M * (D * 2 + 4), s->B * s->H, s->causal);
+  dim3 grid((unsigned)((int64_t)((s->N + C::BN - 1) / C::BN) * s->B * s->H), 1, 1);
   kern<<<grid, C::kThreads, C::kTotal, stream>>>(mq, mk, p);
   FA_CHECK_LAUNCH();
   return FA_OK;

@@ -24,7 +24,7 @@ struct TotalTcParams {
   const float *lse;
   float *total;
   int B, H, Hk, M, N;
-  int causal;
+  int causal, group_size;   // launch order, see grouped_cta()
   float sm_scale;
   int *status;
 };
@@ -64,8 +64,9 @@ __global__ void __launch_bounds__(TotalTcCfg<D>::kThreads, 1)
   const AbortCtx actx{abort_flag, p.status};
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * BN;
-  const int b = blockIdx.y / p.H, h = blockIdx.y % p.H;
+  const CtaCoord cta = grouped_cta(blockIdx.x, (p.N + BN - 1) / BN, p.B * p.H, p.group_size);   // heaviest first
+  const int n0 = cta.blk * BN;
+  const int b = cta.pair / p.H, h = cta.pair % p.H;
   const int hk = h / (p.H / p.Hk);
   const int p_seq = p.N - p.M;
   const int num_m_tiles = (p.M + BM - 1) / BM;
