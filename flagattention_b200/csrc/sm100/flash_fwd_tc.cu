@@ -1,4 +1,5 @@
 // Launcher of the tcgen05 flash_attention forward.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 
@@ -26,6 +27,48 @@ int set_kernel_family(int family) {
   return g_kernel_family.exchange(family == 1 ? 1 : (family == 2 ? 2 : 0));
 }
 
+static int sm_count_fwd() {
+  static std::atomic<int> n[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int v = n[dev].load(std::memory_order_relaxed);
+  if (!v) {
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n[dev].store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
+
+// CTAs that share the walk of a query tile (SPLIT): 1, 2, 4 or 8.  One CTA walks a 64-key tile in about 0.75 us and two
+// on an SM in 0.84 each, so an SM with a single CTA, or none, is idle for want of query tiles; combining costs about
+// five tiles.  Estimated in tiles, and taken where it saves a tenth; all CTAs have to be resident, except that two
+// may share a walk where the longest is about twice the mean load.  bf16, us at 1 / 2 / 4 / 8 CTAs a query tile:
+//   H=32 Hk=8 M=512 N=7300 D=128 (128 query tiles of 107..115 key tiles)   83.4 / 62.2 / 70.6 / 86.6
+//   H=32 Hk=8 M=64 N=7300 D=128 (32 of 115)    82.1 / 47.7 / 28.4 / 25.4
+//   H=8 M=1024 N=16384 D=128 (64 of 256)       185 / 99 / 69 / 79
+//   H=4 L=1024 D=128 causal (32 of 2..16)      16.1 / 13.7 / 11.2 / 14.4
+//   H=4 L=512 D=64 causal (16 of 2..8)          9.9 /  9.6 /  8.3 /  9.6
+//   B=2 H=4 L=256 D=64 causal (16 of 2..4)      7.1 /  8.2 /  7.5 /  9.6
+//   H=32 Hk=8 M=1024 N=4096 D=128 (256 of 50..64)  59.0 / 69.4 / 85.0 / 118
+//   H=4 L=8192 D=128 causal (256 of 2..128)    96.4 / 78.8 / 91.0 / 125
+//   H=12 L=4096 D=128 causal (384 of 2..64)    56.6 / 69.5 / 90.6 / 145
+static int key_split(const fa_flash_shape *s, int sms) {
+  const int64_t blocks = (s->M + 127) / 128, ctas = blocks * s->B * s->H;
+  if (sms <= 0 || ctas > 2ll * sms) return 1;
+  const int64_t longest = (s->N + 63) / 64;
+  // key tiles of the last query tile and, roughly, of the first
+  const int64_t shortest = s->causal ? std::max<int64_t>(0, (s->N - s->M + 128 + 63) / 64) : longest;
+  int best = 1;
+  double least = 0.9 * (double)longest * (ctas > sms ? 1.15 : 1.0);
+  for (int c = 2; c <= 8 && ctas * c <= 2ll * sms; c *= 2) {
+    const double tiles = (double)longest / c * (ctas * c > sms ? 1.15 : 1.0) + (c == 8 ? 7 : 5);
+    if (tiles < least) best = c, least = tiles;
+  }
+  const double load = (double)ctas * 0.5 * (double)(longest + std::min(shortest, longest)) / (2.0 * sms);
+  if (best == 1 && longest >= 64 && load <= 0.55 * (double)longest) best = 2;
+  return best;
+}
+
 template <typename T, int D, bool PW, bool DROP = false, bool PAD = false>
 static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, const fa_tensor4 *k,
                          const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
@@ -40,9 +83,6 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   if (PW && (!make_map_bhld(&mq2, q2, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
              !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN)))
     return 1;
-  auto kern = flash_fwd_tc_kernel<T, D, PW, DROP, PAD>;
-  static unsigned long long done = 0;
-  if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
   FwdTcParams p{};
   p.o = o->ptr, p.lse = lse, p.so = strides_of(o);
   p.B = s->B, p.H = s->H, p.Hk = s->Hk, p.M = s->M, p.N = s->N;
@@ -53,8 +93,28 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise), with those of its group's heads
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal);
-  dim3 grid((unsigned)((int64_t)p.num_m_blocks * s->B * s->H), 1, 1);
-  kern<<<grid, C::kThreads, C::kTotal, stream>>>(mq, mk, mv, mq2, mk2, p);
+  const int64_t tiles = (int64_t)p.num_m_blocks * s->B * s->H;
+  p.split = DROP || one_cta_per_tile_forced() ? 1 : key_split(s, sm_count_fwd());
+  if constexpr (!DROP) {
+    if (p.split > 1) {
+      auto kern = flash_fwd_tc_kernel<T, D, PW, DROP, PAD, true>;
+      static unsigned long long done = 0;
+      if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = (unsigned)p.split, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)(tiles * p.split), 1, 1), cfg.blockDim = dim3(C::kThreads, 1, 1);
+      cfg.dynamicSmemBytes = C::kTotal, cfg.stream = stream, cfg.attrs = &attr, cfg.numAttrs = 1;
+      if (cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mq2, mk2, p) != cudaSuccess) return FA_ERR_LAUNCH;
+      FA_CHECK_LAUNCH();
+      return FA_OK;
+    }
+  }
+  auto kern = flash_fwd_tc_kernel<T, D, PW, DROP, PAD>;
+  static unsigned long long done = 0;
+  if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
+  kern<<<dim3((unsigned)tiles, 1, 1), C::kThreads, C::kTotal, stream>>>(mq, mk, mv, mq2, mk2, p);
   FA_CHECK_LAUNCH();
   return FA_OK;
 }
@@ -90,17 +150,6 @@ int reset_fwd_sched() {
   return cudaMemset(b, 0, 64 * sizeof(unsigned)) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 
-static int sm_count_fwd() {
-  static std::atomic<int> n[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  int v = n[dev].load(std::memory_order_relaxed);
-  if (!v) {
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    n[dev].store(v, std::memory_order_relaxed);
-  }
-  return v;
-}
 
 // The persistent form (flash_fwd_persist_tc.cuh): two CTAs per SM that work through the query tiles.
 template <typename T, int D, bool PAD = false>

@@ -13,6 +13,8 @@
 // S(j+1) is issued before P(j) V(j), so the tensor pipe computes the next
 // scores while the softmax warps work on the current tile; two CTAs per SM
 // (256 of the 512 TMEM columns each) overlap each other's remaining gaps.
+// Where query tiles are too few to fill the SMs, or the longest walk outlasts the
+// mean load, a cluster of CTAs shares the walk of one query tile (SPLIT).
 #pragma once
 
 #include "../attn_params.cuh"
@@ -31,6 +33,7 @@ struct FwdTcParams {
   int w;  // piecewise distance threshold (PW kernels only)
   int *status;
   int num_m_blocks, group_size;  // launch order, see grouped_cta()
+  int split;      // CTAs (a cluster) that share the walk of a query tile (SPLIT kernels only)
   int d;          // head_dim of the tensors: D, or less when the columns up to D are padding (DROP and PAD kernels)
   DropoutRule drop;   // DROP kernels only
 };
@@ -50,7 +53,34 @@ struct FwdTcCfg {
   static constexpr int kTmemCols = 256;               // S0 | S1 | O, rounded to a power of two
   static constexpr int kColS0 = 0, kColS1 = 64, kColO = 128;
   static constexpr int kThreads = 192;
+  // SPLIT: the unnormalised O of a CTA (fp32, D / 4 runs of 128 rows x 4 columns) and its row statistics, over Q, K, V
+  static constexpr int kPartO = 0, kPartStats = BM * D * 4;
+  static_assert(kPartStats + BM * 8 <= kBars, "partial results fit the operands' shared memory");
 };
+
+// Barrier among all threads of the cluster (an exited thread counts as arrived), with release / acquire of shared memory.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+// the address of `smem` (this CTA's shared memory) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t peer_smem(uint32_t smem, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(smem), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 peer_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 peer_ld2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+  return v;
+}
 
 enum FwdBar { Q_FULL = 0, K_FULL = 1, K_FREE = 3, V_FULL = 5, V_FREE = 7, S_FULL = 9, P_READY = 11,
               PV_DONE = 13, Q_FREE = 15 };
@@ -69,7 +99,10 @@ enum FwdBar { Q_FULL = 0, K_FULL = 1, K_FREE = 3, V_FULL = 5, V_FREE = 7, S_FULL
 // rounding error; here the reference may lag it by 2^8.  B=2 H=8 L=777 D=32 causal, bf16, scores of deviation 4,
 // error of o against 64 bits: exact maximum 1.73e-3, P rounded once 2.06e-3, with the remainder 1.66e-3 (the rounding
 // of o).  It costs 4 to 20 % of the kernel: D=32 B=4 H=16 L=2048 causal 74 -> 84 us, dropout at D=64 317 -> 336 us.
-template <typename T, int D, bool PW, bool DROP, bool PAD>
+// SPLIT = a cluster of p.split CTAs per query tile, each with its share of the tile's list of key tiles and with
+// maximum, sum and O of its own.  They meet at the end through distributed shared memory: every CTA leaves its O (fp32)
+// and row statistics in its shared memory, and combines D / split columns of all of them, in the order of the ranks.
+template <typename T, int D, bool PW, bool DROP, bool PAD, bool SPLIT = false>
 __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
     flash_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                         const __grid_constant__ CUtensorMap map_k,
@@ -88,7 +121,9 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
   const AbortCtx actx{abort_flag, p.status};
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const CtaCoord cta = grouped_cta(blockIdx.x, p.num_m_blocks, p.B * p.H, p.group_size);
+  const int rank = SPLIT ? (int)(blockIdx.x % (unsigned)p.split) : 0;   // in the cluster
+  const CtaCoord cta = grouped_cta(SPLIT ? blockIdx.x / (unsigned)p.split : blockIdx.x, p.num_m_blocks, p.B * p.H,
+                                   p.group_size);
   const int mb = p.num_m_blocks - 1 - cta.blk;  // heaviest causal tiles first
   const int b = cta.pair / p.H, h = cta.pair % p.H;
   const int hk = h / (p.H / p.Hk);
@@ -104,16 +139,22 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
     jf = x < 0 ? 0 : min(T_tiles, x / BN + 1);
     jn = y < 0 ? 0 : min(T_tiles, y / BN + 1);
   }
-  const int E2 = jn;                    // entries of the far branch: tiles 0 .. jn-1
-  const int E = E2 + (T_tiles - jf);    // then the near branch: tiles jf .. T-1
+  const int far_all = jn;                              // entries of the far branch: tiles 0 .. jn-1
+  const int all = far_all + (T_tiles - jf);            // then the near branch: tiles jf .. T-1
+  // a wait that ran out earlier (this launch or a previous one) poisons the device status word:
+  // do no work until the host has read and cleared it (the CTAs of a cluster still meet, since they
+  // read one another's shared memory)
+  const bool dead = p.status && *reinterpret_cast<volatile int *>(p.status) != 0;
+  if (!SPLIT && dead) return;
+  // this CTA's entries: eb .. eb + E - 1 of the list, of which the first E2 belong to the far branch
+  const int eb = SPLIT ? (int)((int64_t)all * rank / p.split) : 0;
+  const int E = SPLIT ? (dead ? 0 : (int)((int64_t)all * (rank + 1) / p.split) - eb) : all;
+  const int E2 = min(max(far_all - eb, 0), E);
+  auto tile_of = [&](int e) { return PW && e >= E2 ? jf + (eb + e - far_all) : eb + e; };
   const bool reload_q = PW && E2 > 0 && E2 < E;
 
-  // a wait that ran out earlier (this launch or a previous one) poisons the device status word:
-  // do no work until the host has read and cleared it
-  if (p.status && *reinterpret_cast<volatile int *>(p.status) != 0) return;
-
   if (tid == 0) {
-    *abort_flag = 0;
+    *abort_flag = SPLIT && dead;
     mbar_init(bar(Q_FULL), 1);
     mbar_init(bar(Q_FREE), 1);
     for (int s = 0; s < 2; ++s) {
@@ -133,7 +174,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       tma_prefetch_desc(&map_k);
       tma_prefetch_desc(&map_v);
       const bool far0 = PW && E2 > 0;
-      const int n00 = ((PW && E2 == 0) ? jf : 0) * BN;
+      const int n00 = tile_of(0) * BN;
       mbar_expect_tx(bar(Q_FULL), C::kQBytes);
       for (int s = 0; s < KSUB; ++s)
         tma_load_4d(smem + C::kQ + s * BM * 128, far0 ? &map_q2 : &map_q, bar(Q_FULL), s * 64, m0, h, b);
@@ -162,8 +203,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       bool ok = true;
       for (int e = 1; e < E && ok; ++e) {
         const bool far = PW && e < E2;
-        const int j = (PW && e >= E2) ? jf + (e - E2) : e;
-        const int st = e & 1, ph = (e >> 1) & 1, n0 = j * BN;
+        const int st = e & 1, ph = (e >> 1) & 1, n0 = tile_of(e) * BN;
         if (reload_q && e == E2) {
           // every S of the far branch has been computed: swap q2 for q
           ok = mbar_wait(bar(Q_FREE), 0, actx, 103);
@@ -261,7 +301,7 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
 
     for (int e = 0; e < E; ++e) {
       const bool far = PW && e < E2;
-      const int j = (PW && e >= E2) ? jf + (e - E2) : e;
+      const int j = tile_of(e);
       const int st = e & 1, ph = (e >> 1) & 1, n0 = j * BN;
       uint32_t keep[2] = {0u, 0u};
       if (DROP) {
@@ -377,7 +417,25 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       ok = mbar_wait(bar(PV_DONE + (lj & 1)), (lj >> 1) & 1, actx, 303);
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (ok) {
+    if constexpr (SPLIT) {
+      tc_fence_after();
+      // every product has read its operands: O and the statistics take their place
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t ov[32];
+        if (E > 0) {
+          tmem_ld32(tlane + C::kColO + c * 32, ov);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) ov[i] = 0u;
+        }
+        uint4 *part = reinterpret_cast<uint4 *>(smem_gen + C::kPartO) + c * 8 * BM + row_in_tile;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i * BM] = make_uint4(ov[4 * i], ov[4 * i + 1], ov[4 * i + 2], ov[4 * i + 3]);
+      }
+      reinterpret_cast<float2 *>(smem_gen + C::kPartStats)[row_in_tile] = make_float2(m_used, l);
+    } else if (ok) {
       tc_fence_after();
       float inv = l > 0.f ? 1.f / l : 0.f;
       if (DROP) inv *= p.drop.rp;
@@ -411,6 +469,66 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
             l > 0.f ? (FINE ? m_eff * qk_scale * kLn2 : m_eff * p.sm_scale) + logf(l) : -INFINITY;
       }
     }
+  }
+
+  if constexpr (SPLIT) {
+    cluster_sync_all();
+    if (warp >= 2) {
+      const int row_in_tile = (warp & 3) * 32 + lane, row = m0 + row_in_tile;
+      const float qk_scale = p.sm_scale * kLog2e;
+      // a CTA whose waits ran out, or that found the status word set, leaves nothing to combine
+      bool whole = true;
+      float m = -INFINITY, l = 0.f, weight[8], sums[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        weight[c] = -INFINITY, sums[c] = 0.f;
+        if (c < p.split) {
+          int aborted;
+          asm volatile("ld.shared::cluster.u32 %0, [%1];\n"
+                       : "=r"(aborted)
+                       : "r"(peer_smem(smem + C::kMisc + 8, c))
+                       : "memory");
+          whole = whole && aborted == 0;
+          const float2 st = peer_ld2(peer_smem(smem + C::kPartStats + row_in_tile * 8, c));
+          weight[c] = st.x, sums[c] = st.y;
+          m = fmaxf(m, st.x);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        weight[c] = weight[c] == -INFINITY ? 0.f : ex2((weight[c] - m) * qk_scale);
+        if (c < p.split) l += sums[c] * weight[c];
+      }
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      if (whole && row < p.M) {
+        T *orow = row_ptr_mut<T>(p.o, p.so, b, h, row);
+        const int cols = D / p.split;   // 8 .. 64
+        for (int c0 = rank * cols; c0 < (rank + 1) * cols; c0 += 8) {
+          float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            if (c < p.split) {
+              const uint32_t at = peer_smem(smem + C::kPartO + ((c0 / 4) * BM + row_in_tile) * 16, c);
+              const float4 x = peer_ld4(at), y = peer_ld4(at + BM * 16);
+              acc[0] += x.x * weight[c], acc[1] += x.y * weight[c], acc[2] += x.z * weight[c], acc[3] += x.w * weight[c];
+              acc[4] += y.x * weight[c], acc[5] += y.y * weight[c], acc[6] += y.z * weight[c], acc[7] += y.w * weight[c];
+            }
+          }
+          uint4 v;
+          v.x = TcElem<T>::pack(acc[0] * inv, acc[1] * inv);
+          v.y = TcElem<T>::pack(acc[2] * inv, acc[3] * inv);
+          v.z = TcElem<T>::pack(acc[4] * inv, acc[5] * inv);
+          v.w = TcElem<T>::pack(acc[6] * inv, acc[7] * inv);
+          if (!FINE || c0 < p.d) *reinterpret_cast<uint4 *>(orow + c0) = v;
+        }
+        if (rank == 0) {
+          const float m_eff = (m == -INFINITY) ? 0.f : m;
+          p.lse[((int64_t)b * p.H + h) * p.M + row] =
+              l > 0.f ? (FINE ? m_eff * qk_scale * kLn2 : m_eff * p.sm_scale) + logf(l) : -INFINITY;
+        }
+      }
+    }
+    cluster_sync_all();   // nobody leaves while its shared memory is read
   }
 
   // ------------------------------ teardown -----------------------------------
