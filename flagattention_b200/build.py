@@ -18,6 +18,8 @@ INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libflagattn_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "ops.cpp")
+HOST_PATH = os.path.join(LIB_DIR, "flagattn_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -94,7 +96,34 @@ def build(force=False, verbose=False):
             raise RuntimeError("link failed:\n%s\n%s" % (res.stdout, res.stderr))
         if verbose:
             print("linked", LIB_PATH, flush=True)
+    _build_host(force, verbose)
     return LIB_PATH
+
+
+def _build_host(force, verbose):
+    """The operators' host side (csrc/host/ops.cpp), a Python extension on torch's C++ interface and the library."""
+    import sysconfig
+
+    import torch
+    header = os.path.join(INCLUDE, "flagattn_b200.h")
+    if not force and os.path.exists(HOST_PATH) and \
+            os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
+        return
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, "-I", INCLUDE,
+           "-isystem", os.path.join(root, "include"),
+           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-isystem", os.path.join(cuda, "include"), "-isystem", sysconfig.get_paths()["include"],
+           HOST_SRC, "-o", HOST_PATH, "-L", os.path.join(root, "lib"),
+           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
+           "-L", LIB_DIR, "-lflagattn_b200", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed for %s:\n%s\n%s" % (HOST_SRC, res.stdout, res.stderr))
+    if verbose:
+        print("linked", HOST_PATH, flush=True)
 
 
 if __name__ == "__main__":

@@ -10,7 +10,7 @@ import math
 
 import torch
 
-from . import _C
+from . import _C, _native
 from .dropout import philox_cuda_seed_offset
 from .paged import coarsen_partition, partition_workspace
 from .split_kv import get_fwd_config as get_fwd_config_kv_split
@@ -36,6 +36,7 @@ def set_backward_mode(mode):
     global _backward_mode
     assert mode in _BACKWARD_MODES, f"mode must be one of {_BACKWARD_MODES}"
     previous, _backward_mode = _backward_mode, mode
+    _native.set_backward_mode(_BACKWARD_MODES.index(mode))
     return previous
 
 
@@ -322,5 +323,10 @@ def attention(q, k, v, causal=False, sm_scale=None, dropout_p=0.0,
     Returns out, shape of q; log_normalizer (batch, heads_q, seqlen_q) fp32;
     total_attention (batch, heads_q, seqlen_k) fp32.
     """
+    if (dropout_p == 0 and not (return_log_normalizer or return_total_attention or return_seed_offset)
+            and _native.usable(q)):
+        o = _native.load().flash(q, k, v, causal, sm_scale)
+        if o is not None:
+            return o
     return FlashAttention.apply(q, k, v, causal, sm_scale, dropout_p, return_log_normalizer,
                                 return_total_attention, return_seed_offset)

@@ -8,7 +8,7 @@ import functools
 
 import torch
 
-from . import _C
+from . import _C, _native
 
 __all__ = ["attention", "reshape_and_cache"]
 
@@ -98,11 +98,30 @@ def partition_workspace(rows, P, D, device):
     return ws, base, part_max, part_max + stats * 4
 
 
+@functools.lru_cache(maxsize=1024)
+def _plan(num_seqs, num_q_heads, num_kv_heads, kv_block_size, max_context_len, num_splits, num_sms):
+    """(partition size, partitions of the workspace, sizing or None) of a call; partition size 0: one pass."""
+    free_choice = num_splits == 0
+    num_splits, partition_size = plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_splits,
+                                                 num_sms)
+    sizing = None
+    if free_choice and partition_size:
+        partition_size, *sizing = size_partitions(
+            partition_size, num_seqs, num_kv_heads * _cdiv(num_q_heads // num_kv_heads, 16), max_context_len, num_sms)
+    if not partition_size:
+        return 0, 0, None
+    return partition_size, _cdiv(max_context_len, partition_size), sizing
+
+
 def attention(query, key_cache, value_cache, context_lens, block_tables, attn_scale,
               max_context_len, num_splits=0):
     """query [num_seqs, kv_heads * group, head]; caches [num_blocks, kv_heads, block, head]
     with identical strides; context_lens [num_seqs] int32; block_tables
     [num_seqs, max_blocks] int32 or int64."""
+    if type(max_context_len) is int and max_context_len > 0 and num_splits == 0 and _native.usable(query):
+        out = _native_attention(query, key_cache, value_cache, context_lens, block_tables, attn_scale, max_context_len)
+        if out is not None:
+            return out
     num_seqs, num_q_heads, head_size = query.shape
     num_kv_heads, kv_block_size = key_cache.shape[1], key_cache.shape[2]
     assert key_cache.shape[3] == head_size
@@ -129,20 +148,15 @@ def attention(query, key_cache, value_cache, context_lens, block_tables, attn_sc
         key_cache, value_cache = key_cache.contiguous(), value_cache.contiguous()
 
     with _C.device_guard(query.device):
-        sms, free_choice = _C.sm_count(query.device), num_splits == 0
-        num_splits, partition_size = plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_splits,
-                                                     sms)
-        sizing = None
-        if free_choice and partition_size:
-            partition_size, *sizing = size_partitions(
-                partition_size, num_seqs, num_kv_heads * _cdiv(query_group_size, 16), int(max_context_len), sms)
+        partition_size, P, sizing = _plan(num_seqs, num_q_heads, num_kv_heads, kv_block_size, int(max_context_len),
+                                          num_splits, _C.sm_count(query.device))
         part_out = part_max = part_sum = 0
         if partition_size:
             assert partition_size >= kv_block_size and partition_size % kv_block_size == 0, \
                 f"partition_size={partition_size}, kv_block_size={kv_block_size}"
             assert partition_size % 16 == 0, f"partition_size={partition_size}"
             ws, part_out, part_max, part_sum = partition_workspace(
-                num_seqs * num_q_heads, _cdiv(int(max_context_len), partition_size), head_size, query.device)
+                num_seqs * num_q_heads, P, head_size, query.device)
 
         out = torch.empty(query.shape, dtype=query.dtype, device=query.device)
         kb, kh, kt = key_cache.stride()[:3]
@@ -162,6 +176,23 @@ def attention(query, key_cache, value_cache, context_lens, block_tables, attn_sc
     return out
 
 
+def _native_attention(query, key_cache, value_cache, context_lens, block_tables, attn_scale, max_context_len):
+    """The call through native code, or None: partitions and their workspace chosen here, the rest there."""
+    if query.dim() != 3 or key_cache.dim() != 4:
+        return None
+    num_seqs, num_q_heads, head_size = query.shape
+    num_kv_heads, kv_block_size = key_cache.shape[1:3]
+    if not num_seqs or not num_kv_heads or num_q_heads % num_kv_heads or not kv_block_size or head_size > 256:
+        return None
+    partition_size, P, sizing = _plan(num_seqs, num_q_heads, num_kv_heads, kv_block_size, max_context_len, 0,
+                                      _C.sm_count(query.device))
+    part_out = part_max = part_sum = 0
+    if partition_size:
+        ws, part_out, part_max, part_sum = partition_workspace(num_seqs * num_q_heads, P, head_size, query.device)
+    return _native.load().paged(query, key_cache, value_cache, context_lens, block_tables, attn_scale, max_context_len,
+                                partition_size, part_out, part_max, part_sum, *(sizing or (0, 0, 0, 0)))
+
+
 def reshape_and_cache(key, value, key_cache, value_cache, slot_mapping):
     """Writes new tokens into the paged caches `attention` reads.
 
@@ -169,6 +200,8 @@ def reshape_and_cache(key, value, key_cache, value_cache, slot_mapping):
     slot_mapping [num_tokens] integer: token i goes to block slot // block, position slot % block;
     negative slots are skipped.  The reference has no writer (its tests fill the caches with random
     numbers); a serving loop runs this step right before the decode kernel."""
+    if _native.usable(key) and _native.load().append(key, value, key_cache, value_cache, slot_mapping):
+        return
     num_tokens, num_kv_heads, head_size = key.shape
     assert value.shape == key.shape and key_cache.shape == value_cache.shape
     assert key_cache.shape[1] == num_kv_heads and key_cache.shape[3] == head_size

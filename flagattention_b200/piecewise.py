@@ -8,7 +8,7 @@ import math
 
 import torch
 
-from . import _C
+from . import _C, _native
 from .flash import use_one_pass_backward
 
 __all__ = ["attention"]
@@ -88,4 +88,8 @@ def attention(q1, k1, q2, k2, v, dist_threshold, causal=False, sm_scale=None):
     q1_i.k1_j when their distance is below `dist_threshold` and q2_i.k2_j
     otherwise.  All tensors are (batch, heads, seqlen, headdim); returns the
     output, shaped like q1."""
+    if _native.usable(q1):
+        o = _native.load().piecewise(q1, k1, q2, k2, v, dist_threshold, causal, sm_scale)
+        if o is not None:
+            return o
     return PiecewiseAttention.apply(q1, k1, q2, k2, v, dist_threshold, causal, sm_scale)

@@ -11,7 +11,7 @@ import ctypes
 
 import torch
 
-from . import _C
+from . import _C, _native
 
 __all__ = ["rotary_pair", "rotary_tables"]
 
@@ -102,4 +102,8 @@ def rotary_pair(x, cos1, sin1, cos2, sin2, positions=None, interleaved=False):
     positions: None (token l sits at position l) or integers of shape (length,) or (batch, length);
     values outside the tables are clamped.  interleaved: pairs are (2i, 2i + 1) instead of
     (i, i + head_dim / 2).  Differentiable with respect to x."""
+    if positions is None and _native.usable(x):
+        pair = _native.load().rotary_pair(x, cos1, sin1, cos2, sin2, interleaved)
+        if pair is not None:
+            return pair
     return RotaryPair.apply(x, cos1, sin1, cos2, sin2, positions, interleaved)

@@ -1,0 +1,188 @@
+"""The native form of the operators' usual calls against the Python form: the same bits, the same gradients, the same
+errors; and what it must leave to the Python form."""
+import pytest
+import torch
+
+import flagattention_b200 as fa
+from flagattention_b200 import _native, flash, paged, piecewise, rotary
+from helpers import make_qkv
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def python_form(monkeypatch):
+    """Calls `f` through the Python form."""
+    def run(f):
+        with monkeypatch.context() as m:
+            m.setattr(_native, "usable", lambda x: False)
+            return f()
+    return run
+
+
+def _same(a, b):
+    for x, y in zip(a, b):
+        assert x.shape == y.shape and x.stride() == y.stride() and x.dtype == y.dtype and x.device == y.device
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("B,H,Hk,M,N,D,causal,layout", [
+    (2, 8, 8, 256, 256, 64, True, "BHTD"), (2, 16, 4, 300, 333, 128, True, "BTHD"), (4, 8, 2, 160, 160, 32, False, "BHTD"),
+    (1, 8, 8, 1, 4096, 128, False, "BHTD"), (2, 8, 2, 1, 1024, 64, True, "BTHD"), (1, 4, 1, 4, 8192, 128, True, "BHTD"),
+    (3, 2, 2, 1, 1000, 64, False, "BHTD"), (1, 2, 2, 40, 40, 64, True, "BHTD")])
+def test_flash_calls(python_form, B, H, Hk, M, N, D, causal, layout):
+    q, k, v, do = make_qkv(B, H, Hk, M, N, D, torch.bfloat16, "cuda", layout=layout, seed=N)
+    call = lambda *a, **kw: fa.flash_attention(q, k, v, *a, **kw)
+    _same([call(causal)], [python_form(lambda: call(causal))])
+    _same([call(causal, 0.3)], [python_form(lambda: call(causal, 0.3))])
+    for x in (q, k, v):
+        x.requires_grad_()
+    grads = lambda: (lambda o: (o,) + torch.autograd.grad(o, (q, k, v), do))(call(causal))
+    with flash.backward_mode("two_kernel"):   # bitwise reproducible
+        _same(grads(), python_form(grads))
+    got, want = grads(), python_form(grads)
+    _same(got[2:], want[2:])   # dk, dv; dq is summed in any order: one rounding to 16 bits apart at most
+    _same(got[:1], want[:1])
+    assert (got[1].float() - want[1].float()).abs().max() <= 2 ** -7 * want[1].float().abs().max()
+    with torch.no_grad():
+        _same([call(causal)], [python_form(lambda: call(causal))])
+
+
+def test_piecewise_and_rotary_calls(python_form):
+    B, H, L, D = 2, 4, 300, 64
+    gen = torch.Generator().manual_seed(1)
+    x, y, v, do = (torch.randn((B, H, L, D), generator=gen).half().cuda().requires_grad_() for _ in range(4))
+    tables = rotary.rotary_tables(L, D, device="cuda") + rotary.rotary_tables(L, D, position_scale=0.25, device="cuda")
+
+    def run():
+        q1, q2 = rotary.rotary_pair(x, *tables)
+        k1, k2 = rotary.rotary_pair(y, *tables, interleaved=True)
+        o = fa.piecewise_attention(q1, k1, q2, k2, v, 100, True)
+        return (q1, q2, k1, k2, o) + torch.autograd.grad(o, (x, y, v), do.detach())
+
+    with flash.backward_mode("two_kernel"):
+        _same(run(), python_form(run))
+
+
+@pytest.mark.parametrize("index", [torch.int32, torch.int64])
+@pytest.mark.parametrize("most", [300, 5000])
+def test_paged_calls(python_form, index, most):
+    gen = torch.Generator(device="cuda").manual_seed(most)
+    rnd = lambda *s: torch.randn(s, generator=gen, device="cuda", dtype=torch.float16)
+    q, kc, vc, key, value = rnd(3, 8, 128), rnd(400, 2, 16, 128), rnd(400, 2, 16, 128), rnd(3, 2, 128), rnd(3, 2, 128)
+    lens = torch.tensor([most, 1, 250], dtype=torch.int32, device="cuda")
+    table = torch.randint(0, 400, (3, -(-most // 16)), generator=gen, device="cuda").to(index)
+    slots = torch.tensor([5, -1, 400 * 16 - 1], device="cuda")
+    call = lambda: fa.paged_attention(q, kc, vc, lens, table, 128 ** -0.5, most)
+    _same([call()], [python_form(call)])
+
+    def write():
+        caches = kc.clone(), vc.clone()
+        paged.reshape_and_cache(key, value, *caches, slots)
+        return caches
+    _same(write(), python_form(write))
+
+
+def test_the_usual_calls_are_taken():
+    """A check that went wrong would send every call to the Python form, unnoticed."""
+    n, x = _native.load(), torch.randn(2, 4, 256, 64, device="cuda", dtype=torch.float16)
+    t = rotary.rotary_tables(256, 64, device="cuda")
+    assert n.flash(x, x, x, True, None) is not None
+    assert n.flash(x[:, :, :1], x, x, False, 0.1) is not None
+    assert n.flash(x, x.requires_grad_(), torch.nn.Parameter(x.detach()), True, None).requires_grad
+    assert n.piecewise(x, x, x, x, x, 10, True, None) is not None
+    assert n.rotary_pair(x, *t, *t, False) is not None
+    q, cache, lens = x[0, :2, 0].detach()[:, None].contiguous(), x.detach()[..., :16, :].contiguous(), torch.ones(2, dtype=torch.int32, device="cuda")
+    assert n.paged(q.expand(2, 4, 64).contiguous(), cache, cache, lens, lens[:, None], 1.0, 16, 0, 0, 0, 0, 0, 0, 0, 0) is not None
+    assert n.append(x[:, :, 0].detach(), x[:, :, 0].detach(), cache, cache.clone(), torch.zeros(2, dtype=torch.int64, device="cuda"))
+
+
+def test_what_is_left_to_the_python_form():
+    """Transforms, modes, views that need a copy and errors."""
+    n, x = _native.load(), torch.randn(2, 4, 256, 64, device="cuda", dtype=torch.float16)
+    for q, k, v in ((x.cpu(), x, x), (x, x.float(), x), (x, x[:, :3], x[:, :3]), (x, x[:, :, :9], x), (x[..., ::2], x[..., ::2], x[..., ::2]),
+                    (x.transpose(2, 3), x, x), (x[0], x, x), (x[..., :48], x[..., :48], x[..., :48]), (x[:, :0], x, x),
+                    (x[:, :1, :40], x[:, :1], x[:, :1]), (None, x, x), (1, 2, 3)):
+        assert n.flash(q, k, v, True, None) is None
+    assert n.flash(x, x, x, 1, None) is None and n.flash(x, x, x, True, "no") is None and n.flash(x, x) is None
+
+    from torch.autograd import forward_ad
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    with Mode():
+        assert n.flash(x, x, x, True, None) is None
+    with forward_ad.dual_level():
+        dual = forward_ad.make_dual(x, torch.ones_like(x))
+        assert n.flash(dual, x, x, True, None) is None
+        with pytest.raises(Exception):
+            fa.flash_attention(dual, x, x, True)
+    with pytest.raises(Exception):   # no vmap rule, in either form
+        torch.func.vmap(lambda y: fa.flash_attention(y, x, x, True))(torch.stack([x, x]))
+    with pytest.raises(Exception):
+        torch.func.grad(lambda y: fa.flash_attention(y, x, x, True).float().sum())(x)
+    with pytest.raises(AssertionError, match="multiple"):
+        fa.flash_attention(x, x[:, :3], x[:, :3])
+    with pytest.raises(AssertionError):
+        fa.flash_attention(x.cpu(), x.cpu(), x.cpu())
+
+
+def test_saved_tensors_obey_hooks_and_versions():
+    q, k, v, do = make_qkv(1, 8, 8, 200, 200, 64, torch.float16, "cuda", seed=5)
+    for x in (q, k, v):
+        x.requires_grad_()
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or t.cpu(), lambda t: t.cuda()):
+        o = fa.flash_attention(q, k, v, True)
+    assert len(packed) == 5
+    with flash.backward_mode("two_kernel"):
+        got = torch.autograd.grad(o, (q, k, v), do)
+        _same(got, torch.autograd.grad(fa.flash_attention(q, k, v, True), (q, k, v), do))
+    o = fa.flash_attention(q, k, v, True)
+    with torch.no_grad():
+        k.mul_(2)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(o, (q, k, v), do)
+    o = fa.flash_attention(q, k, v, True)
+    torch.autograd.grad(o, q, do)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(o, q, do)
+
+
+def test_deterministic_switch_reaches_the_native_backward():
+    q, k, v, do = make_qkv(2, 8, 8, 700, 700, 64, torch.float16, "cuda", seed=6)
+    for x in (q, k, v):
+        x.requires_grad_()
+    run = lambda: torch.autograd.grad(fa.flash_attention(q, k, v, True), (q, k, v), do)
+    with flash.backward_mode("two_kernel"):
+        want = run()
+    torch.use_deterministic_algorithms(True)
+    try:
+        _same(run(), want)
+    finally:
+        torch.use_deterministic_algorithms(False)
+
+
+def test_several_threads_and_streams():
+    import threading
+    q, k, v, do = make_qkv(2, 8, 8, 300, 300, 64, torch.float16, "cuda", seed=7)
+    for x in (q, k, v):
+        x.requires_grad_()
+    want = fa.flash_attention(q, k, v, True)
+    torch.cuda.synchronize()
+    bad = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                o = fa.flash_attention(q, k, v, True)
+                torch.autograd.grad(o, (q, k, v), do)
+                if not torch.equal(o, want):
+                    bad.append(1)
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=work) for _ in range(3)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
