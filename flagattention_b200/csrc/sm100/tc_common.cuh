@@ -124,14 +124,14 @@ inline int cta_group_size(int64_t hot_bytes_per_pair, int npairs) {
 // The groups cost their own tail: the heavy blocks of the last group start when the grid is nearly through, which
 // with a few blocks an SM is up to 48 % of the mean load (list-scheduled).  So ALL pairs form one group, blocks in
 // strictly falling order, where L2 can bear it:
-//   forward, total attention: what all pairs share fits in L2 together (100 of 126 MB) and blocks differ (causal);
+//   forward, total attention: what all pairs share fits in L2 together (88 of 126 MB) and blocks differ (causal);
 //   one-pass backward: up to 8 blocks an SM and 64 pairs, so that several CTAs walk each pair at any time.
 // bf16 causal D=128, in groups -> in one, us: forward H=16 L=6144 175 -> 158 (50 MB), B=2 H=20 L=4096 237 -> 208 (84 MB),
-// H=48 L=4096 246 -> 240 (101 MB), B=2 H=32 L=4096 278 -> 311 (134 MB); backward B=3 H=32 Hk=8 L=1867 381 -> 321 (360
+// B=2 H=32 M=1627 N=2855 142 -> 148 (94 MB), B=2 H=32 L=4096 278 -> 311 (134 MB); backward B=3 H=32 Hk=8 L=1867 381 -> 321 (360
 // blocks), H=32 Hk=8 L=8192 1871 -> 1383 (512), H=16 L=6144 493 -> 409 (768), B=2 H=32 Hk=16 L=4096 840 -> 762 (1024),
 // B=4 H=32 L=1024 197 -> 203 (1024, 128 pairs), H=24 L=8192 1099 -> 1079 (1536), B=2 H=32 L=4096 760 -> 845 (2048).
 inline int forward_group_size(int64_t hot_bytes_per_pair, int npairs, bool causal) {
-  if (causal && hot_bytes_per_pair * npairs <= 100ll << 20) return npairs > 0 ? npairs : 1;
+  if (causal && hot_bytes_per_pair * npairs <= 88ll << 20) return npairs > 0 ? npairs : 1;
   return cta_group_size(hot_bytes_per_pair, npairs);
 }
 inline int backward_group_size(int64_t hot_bytes_per_pair, int npairs, int64_t blocks, int sms, bool causal) {

@@ -32,9 +32,9 @@ def test_every_block_is_visited_once(B, H, Hk, M, N, D, causal):
         assert_within_2x(x, r, t, name)
 
 
-@pytest.mark.parametrize("H,N", [(25, 8192), (26, 8192)])
+@pytest.mark.parametrize("H,N", [(22, 8192), (23, 8192)])
 def test_forward_at_the_l2_line(H, N):
-    """25 x 8192 keys at head_dim 128 are 100 MiB and one group, 26 heads go in groups of 8: the same bits as a call
+    """22 x 8192 keys at head_dim 128 are 88 MiB and one group, 23 heads go in groups of 8: the same bits as a call
     for some of the heads alone."""
     q, k, v, _ = make_qkv(1, H, H, N, N, 128, torch.float16, "cuda", seed=H)
     with _C.kernel_family("one_cta_per_tile"):   # (one head alone would be split over a cluster)
