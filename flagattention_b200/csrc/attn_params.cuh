@@ -82,6 +82,10 @@ struct DropoutRule {
   uint64_t seed, offset;
   uint32_t first, width;   // keep iff u - first < width
   float rp;                // 1 / (1 - dropout_p)
+  // Where the forward leaves the decisions for the backward (null: nowhere, the backward draws again): bit n % 32 of
+  // word ((b * H + h) * words + n / 32) * rows + m, 1 = keep.  rows: M rounded up to 128, words: N / 32 rounded up to 4.
+  uint32_t *bits;
+  int rows, words;
 };
 inline DropoutRule make_dropout_rule(float dropout_p, uint64_t seed, uint64_t offset) {
   uint64_t lo = 0, hi = 1ull << 31;   // smallest x in [lo, hi] that is kept (2^31: none)
@@ -91,24 +95,36 @@ inline DropoutRule make_dropout_rule(float dropout_p, uint64_t seed, uint64_t of
     if (u > dropout_p) hi = mid;
     else lo = mid + 1;
   }
-  return DropoutRule{seed, offset, (uint32_t)lo, (uint32_t)(0u - 2u * (uint32_t)lo), 1.f / (1.f - dropout_p)};
+  return DropoutRule{seed, offset, (uint32_t)lo, (uint32_t)(0u - 2u * (uint32_t)lo), 1.f / (1.f - dropout_p), nullptr, 0, 0};
 }
 
-// Keep bits of the elements whose counters are ctr, ctr + step, .. ctr + 31 step (bit i: the i-th).
+// The buffer of a call: B H words rows 4-byte words.  Kept while it takes no more memory than q and o together (N / 8
+// bytes a query row against 4 D): up to 32 D keys.
+inline int64_t keep_bits_bytes(const fa_flash_shape *s) {
+  if (!(s->dropout_p > 0.f) || s->N > 32 * s->D) return 0;
+  return (int64_t)s->B * s->H * ((s->N + 127) / 128 * 4) * (((int64_t)s->M + 127) / 128 * 128) * 4;
+}
+inline void keep_bits_in(DropoutRule &r, const fa_flash_shape *s, void *bits) {
+  r.bits = static_cast<uint32_t *>(bits);
+  r.rows = (s->M + 127) / 128 * 128, r.words = (s->N + 127) / 128 * 4;
+}
+
+// Keep bits of the elements whose counters are ctr + at(0), ctr + at(1), .. ctr + at(31) (bit i: the i-th), none
+// larger than `most`.
 // What bounds a kernel with dropout is this: Philox costs 10 multiplications an element and only its
-// first output word is used.  While the counters share their upper 32 bits (all but one in 2^32 / (31
-// step) calls) one product of round 2 depends on nothing else and is taken out of the loop; words of
+// first output word is used.  While the counters share their upper 32 bits (all but one in 2^32 / most calls) one product of round 2 depends on nothing else and is taken out of the loop; words of
 // rounds 4 to 6 that do not reach the first output are not computed: 9 multiplications and 9 three-input
 // xors an element.
-__device__ __forceinline__ uint32_t dropout_keep_bits32(const DropoutRule &r, uint64_t ctr, uint32_t step) {
+template <typename At>
+__device__ __forceinline__ uint32_t dropout_keep_bits32(const DropoutRule &r, uint64_t ctr, uint64_t most, At at) {
   constexpr uint32_t A = 0xD2511F53u, B = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
   const uint32_t k0 = (uint32_t)r.seed, k1 = (uint32_t)(r.seed >> 32);
   const uint32_t lo = (uint32_t)ctr;
   uint32_t bits = 0;
-  if ((uint64_t)lo + 31ull * step >> 32) {   // the upper half of the counter changes on the way
+  if ((uint64_t)lo + most >> 32) {   // the upper half of the counter changes on the way
 #pragma unroll 1
     for (int i = 0; i < 32; ++i) {
-      const uint64_t c = ctr + (uint64_t)i * step;
+      const uint64_t c = ctr + at(i);
       const uint32_t u = philox4x32_6(k0, k1, (uint32_t)c, (uint32_t)(c >> 32));
       if (u - r.first < r.width) bits |= 1u << i;
     }
@@ -118,7 +134,7 @@ __device__ __forceinline__ uint32_t dropout_keep_bits32(const DropoutRule &r, ui
   const uint32_t fx = (uint32_t)(fixed >> 32) ^ (k1 + W1), fy = (uint32_t)fixed ^ (k1 + 2u * W1);
 #pragma unroll 8
   for (int i = 0; i < 32; ++i) {
-    uint64_t pa = (uint64_t)A * (lo + (uint32_t)i * step);   // round 1
+    uint64_t pa = (uint64_t)A * (lo + (uint32_t)at(i));   // round 1
     uint32_t c2 = (uint32_t)(pa >> 32) ^ k1;
     uint64_t pb = (uint64_t)B * c2;   // round 2
     uint32_t c0 = (uint32_t)(pb >> 32) ^ (k0 + W0), c1 = (uint32_t)pb;

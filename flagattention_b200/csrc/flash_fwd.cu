@@ -65,7 +65,7 @@ static FwdParams make_fwd_params(const fa_flash_shape *s, const fa_tensor4 *q, c
 
 namespace tc {
 int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
-                 const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream);
+                 const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream, void *bits);
 }
 
 }  // namespace fa
@@ -78,11 +78,24 @@ extern "C" int fa_flash_fwd(const fa_flash_shape *s, const fa_tensor4 *q, const 
   if (int st = validate_tensors({q, k, v, o})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
   // what a tensor map can express runs on tcgen05; everything else on the shape-generic kernel
-  const int tc_status = tc::flash_fwd_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream));
+  const int tc_status = tc::flash_fwd_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream), nullptr);
   if (tc_status <= 0) return tc_status;
   FwdParams p = make_fwd_params(s, q, k, v);
   p.o = o->ptr, p.so = strides_of(o), p.lse = lse;
   return dispatch_dtype_d(s->dtype, s->D, FwdLaunch{p, static_cast<cudaStream_t>(stream)});
+}
+
+extern "C" int fa_flash_fwd_keep(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
+                                 const fa_tensor4 *v, const fa_tensor4 *o, float *lse, void *bits, int64_t bits_bytes,
+                                 void *stream) {
+  if (int st = validate_shape(s)) return st;
+  if (int st = validate_tensors({q, k, v, o})) return st;
+  if (!lse || !bits || (reinterpret_cast<uintptr_t>(bits) & 15)) return FA_ERR_BAD_ARG;
+  const int64_t need = fa_flash_keep_bits_bytes(s);
+  if (need == 0) return FA_ERR_UNSUPPORTED;
+  if (bits_bytes < need) return FA_ERR_WORKSPACE;
+  const int tc_status = tc::flash_fwd_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream), bits);
+  return tc_status == 1 ? FA_ERR_UNSUPPORTED : tc_status;   // 1: nothing launched
 }
 
 extern "C" int fa_splitkv_fwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,

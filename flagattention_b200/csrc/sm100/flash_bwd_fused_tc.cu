@@ -114,7 +114,7 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
                         const fa_tensor4 *v, const fa_tensor4 *d_o, const float *lse,
                         const float *delta, const fa_tensor4 *dq, const fa_tensor4 *dk,
                         const fa_tensor4 *dv, float *workspace, cudaStream_t stream,
-                        const FarBranch *far = nullptr, int stages = 7) {
+                        const FarBranch *far = nullptr, int stages = 7, const void *bits = nullptr) {
   using C = FusedBwdCfg<D>;
   const fa_tensor4 *q2 = far ? far->q2 : q, *k2 = far ? far->k2 : k, *dk2 = far ? far->dk2 : dk;
   CUtensorMap mq, mdo, mk, mv, mdk, mdv, mq2, mk2, mdk2;
@@ -142,7 +142,10 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
   p.mode = far ? 3 : 0, p.w = far ? far->w : 0, p.dv_accumulate = 0;
   p.dk = dk->ptr, p.dv = dv->ptr, p.sdk = strides_of(dk), p.sdv = strides_of(dv);
   p.dq = dq->ptr, p.sdq = strides_of(dq);
-  if (DROP) fp.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
+  if (DROP) {
+    fp.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
+    if (bits) keep_bits_in(fp.drop, s, const_cast<void *>(bits));
+  }
   const int64_t acc_bytes = fused_dq_acc_bytes(s);
   const int n_acc = far ? 2 : 1;
   fp.dq_acc = workspace;
@@ -301,11 +304,16 @@ extern "C" int64_t fa_flash_bwd_workspace_bytes(const fa_flash_shape *s) {
   return tc::fused_workspace_bytes(s) + (int64_t)s->B * s->H * s->M * 4;
 }
 
-extern "C" int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
-                            const fa_tensor4 *v, const fa_tensor4 *o, const fa_tensor4 *d_o,
-                            const float *lse, const fa_tensor4 *dq, const fa_tensor4 *dk,
-                            const fa_tensor4 *dv, void *workspace, int64_t workspace_bytes,
-                            void *stream) {
+// Both directions on the tcgen05 kernels, whatever the layout turns out to be
+extern "C" int64_t fa_flash_keep_bits_bytes(const fa_flash_shape *s) {
+  if (!s || validate_shape(s) != FA_OK || !tc::one_pass_covered(s)) return 0;
+  return keep_bits_bytes(s);
+}
+
+static int whole_backward(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
+                          const fa_tensor4 *o, const fa_tensor4 *d_o, const float *lse, const fa_tensor4 *dq,
+                          const fa_tensor4 *dk, const fa_tensor4 *dv, const void *bits, void *workspace,
+                          int64_t workspace_bytes, void *stream) {
   if (int st = validate_shape(s)) return st;
   if (int st = validate_tensors({q, k, v, o, d_o, dq, dk, dv})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
@@ -323,7 +331,7 @@ extern "C" int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const 
   const int64_t acc = tc::fused_workspace_bytes(s);
   float *delta = reinterpret_cast<float *>(static_cast<char *>(workspace) + acc);
   if (int rc = fa_flash_bwd_delta_zero(s, o, d_o, delta, workspace, acc, stream)) return rc;
-#define FA_BWD_ARGS s, q, k, v, d_o, lse, delta, dq, dk, dv, ws, st, nullptr, 6
+#define FA_BWD_ARGS s, q, k, v, d_o, lse, delta, dq, dk, dv, ws, st, nullptr, 6, bits
 #define FA_BWD_CASE(DROP)                                                        \
   if (s->dtype == FA_F16)                                                        \
     return s->D == 128 ? tc::launch_fused<__half, 128, DROP>(FA_BWD_ARGS)        \
@@ -336,4 +344,24 @@ extern "C" int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const 
   FA_BWD_CASE(false)
 #undef FA_BWD_CASE
 #undef FA_BWD_ARGS
+}
+
+extern "C" int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
+                            const fa_tensor4 *v, const fa_tensor4 *o, const fa_tensor4 *d_o,
+                            const float *lse, const fa_tensor4 *dq, const fa_tensor4 *dk,
+                            const fa_tensor4 *dv, void *workspace, int64_t workspace_bytes,
+                            void *stream) {
+  return whole_backward(s, q, k, v, o, d_o, lse, dq, dk, dv, nullptr, workspace, workspace_bytes, stream);
+}
+
+extern "C" int fa_flash_bwd_keep(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
+                                 const fa_tensor4 *v, const fa_tensor4 *o, const fa_tensor4 *d_o, const float *lse,
+                                 const fa_tensor4 *dq, const fa_tensor4 *dk, const fa_tensor4 *dv, const void *bits,
+                                 int64_t bits_bytes, void *workspace, int64_t workspace_bytes, void *stream) {
+  if (int st = validate_shape(s)) return st;
+  if (!bits || (reinterpret_cast<uintptr_t>(bits) & 15)) return FA_ERR_BAD_ARG;
+  const int64_t need = fa_flash_keep_bits_bytes(s);
+  if (need == 0) return FA_ERR_UNSUPPORTED;
+  if (bits_bytes < need) return FA_ERR_WORKSPACE;
+  return whole_backward(s, q, k, v, o, d_o, lse, dq, dk, dv, bits, workspace, workspace_bytes, stream);
 }

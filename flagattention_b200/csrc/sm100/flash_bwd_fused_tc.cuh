@@ -178,11 +178,12 @@ struct FusedItem {
 // tensor pipe computes its first score tile.
 //
 // DROP = dropout (flash_attention): dV takes the kept probabilities, dS = P (keep / (1 - p) dP - delta).
-// The 32 keep bits of a thread do not depend on the scores and are computed before the wait for them.
-// Backward at head_dim 64, p = 0.1, bf16, pair of mma.sync kernels (bits computed in both) -> this:
-// B=16 H=16 L=512 662 -> 246 us (120 us without dropout), B=4 H=16 L=2048 causal 1485 -> 421 us; at 128 1858 -> 481 us.
-// The drawing does not fit the registers beside the rest: 80 and 188 bytes of spill stores and loads a thread at 64, 48 and 136 at
-// 128 (without dropout 48 and 188, and 12 and 92).
+// The 32 keep bits of a thread do not depend on the scores and are there before the wait for them: read from where the
+// forward left them, or drawn again.  Backward at head_dim 64, p = 0.1, bf16, drawn by the pair of mma.sync kernels ->
+// drawn here: B=16 H=16 L=512 662 -> 246 us, B=4 H=16 L=2048 causal 1485 -> 421 us; at 128 1858 -> 481 us.  Drawing is
+// about 90 us of the 194 the first of them has come to since; read, the whole training call takes 363 -> 279 us.
+// The drawing does not fit the registers beside the rest: 76 and 180 bytes of spill stores and loads a thread at 64,
+// 32 and 32 at 128 (without dropout 48 and 188, and 12 and 92).
 template <typename T, int D, bool DROP>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     flash_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -851,16 +852,28 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 
       for (int t = 0; t < it.T_tiles; ++t, ++gt) {
         const int m0 = mt * BM;
+        // bit 8 i + 2 j + e: whether key frow + 8 i, query fcol + 8 j + e is kept
         uint32_t keep = 0;
-        if (DROP)   // (lane = key, bit = query)
-          keep = dropout_keep_bits32(
-              fp.drop, fp.drop.offset + (((uint64_t)it.b * p.H + h) * p.M + m0 + cg * 32) * p.N + key, (uint32_t)p.N);
-        auto kept = [&](uint32_t word, int j, int e) { return (word >> (8 * j + 2 * (lane & 3) + e) & 1u) != 0; };
-        uint32_t kw[4] = {0u, 0u, 0u, 0u};
         if (DROP) {
+          const int64_t bh = (int64_t)it.b * p.H + h;
+          if (fp.drop.bits) {
+            const uint32_t *word = fp.drop.bits + (bh * fp.drop.words + (n0 >> 5) + slice) * fp.drop.rows + m0 + fcol;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) kw[i] = __shfl_sync(0xffffffffu, keep, (lane >> 2) + 8 * i);
+            for (int j = 0; j < 4; ++j) {
+              const uint2 w = *reinterpret_cast<const uint2 *>(word + 8 * j);   // (32 keys of one query each)
+              keep |= (w.x >> (lane >> 2) & 0x01010101u) << (2 * j);
+              keep |= (w.y >> (lane >> 2) & 0x01010101u) << (2 * j + 1);
+            }
+          } else {
+            const uint64_t N = (uint32_t)p.N;
+            keep = dropout_keep_bits32(
+                fp.drop, fp.drop.offset + ((uint64_t)bh * p.M + m0 + fcol) * N + n0 + frow, 25 * N + 24,
+                [&](int i) { return (uint64_t)((i >> 1 & 3) * 8 + (i & 1)) * N + (uint64_t)(i >> 3) * 8; });
+          }
         }
+        auto kept = [&](int k, int e) {   // of pair k of the fragments
+          return (keep >> (8 * ((k >> 3) * 2 + (k & 1)) + 2 * (k >> 1 & 3) + e) & 1u) != 0;
+        };
         if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
 
         // ---- phase 1: P^T = exp2(S^T * scale - lse) -> TMEM ----
@@ -918,9 +931,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             pv[2 * k] = ex2(pv[2 * k]);
             pv[2 * k + 1] = ex2(pv[2 * k + 1]);
             if (DROP) {
-              const uint32_t word = kw[(k >> 3) * 2 + (k & 1)];
-              pk[k] = TcElem<T>::pack(kept(word, (k >> 1) & 3, 0) ? pv[2 * k] : 0.f,
-                                      kept(word, (k >> 1) & 3, 1) ? pv[2 * k + 1] : 0.f);
+              pk[k] = TcElem<T>::pack(kept(k, 0) ? pv[2 * k] : 0.f, kept(k, 1) ? pv[2 * k + 1] : 0.f);
             } else {
               pk[k] = TcElem<T>::pack(pv[2 * k], pv[2 * k + 1]);
             }
@@ -955,9 +966,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
             const int j = (k >> 1) & 3;
             float e0, e1;
             if (DROP) {
-              const uint32_t word = kw[(k >> 3) * 2 + (k & 1)];
-              e0 = pv[2 * k] * fmaf(kept(word, j, 0) ? __uint_as_float(sr[2 * k]) : 0.f, fp.drop.rp, d8[2 * j]);
-              e1 = pv[2 * k + 1] * fmaf(kept(word, j, 1) ? __uint_as_float(sr[2 * k + 1]) : 0.f, fp.drop.rp, d8[2 * j + 1]);
+              e0 = pv[2 * k] * fmaf(kept(k, 0) ? __uint_as_float(sr[2 * k]) : 0.f, fp.drop.rp, d8[2 * j]);
+              e1 = pv[2 * k + 1] * fmaf(kept(k, 1) ? __uint_as_float(sr[2 * k + 1]) : 0.f, fp.drop.rp, d8[2 * j + 1]);
             } else {
               f2_unpack(f2_mul(f2_pack(pv[2 * k], pv[2 * k + 1]),
                                f2_add(f2_pack(__uint_as_float(sr[2 * k]), __uint_as_float(sr[2 * k + 1])),

@@ -72,7 +72,7 @@ static int key_split(const fa_flash_shape *s, int sms) {
 template <typename T, int D, bool PW, bool DROP = false, bool PAD = false>
 static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, const fa_tensor4 *k,
                          const fa_tensor4 *q2, const fa_tensor4 *k2, const fa_tensor4 *v,
-                         const fa_tensor4 *o, float *lse, cudaStream_t stream) {
+                         const fa_tensor4 *o, float *lse, cudaStream_t stream, void *bits = nullptr) {
   using C = FwdTcCfg<D>;
   CUtensorMap mq, mk, mv, mq2, mk2;
   if (!make_map_bhld(&mq, q, s->dtype, s->B, s->H, s->M, s->D, C::BM) ||
@@ -89,7 +89,10 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   p.causal = s->causal, p.sm_scale = s->sm_scale, p.w = w;
   p.status = device_status_word();
   p.d = s->D;
-  if (DROP) p.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
+  if (DROP) {
+    p.drop = make_dropout_rule(s->dropout_p, s->philox_seed, s->philox_offset);
+    if (bits) keep_bits_in(p.drop, s, bits);
+  }
   // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise), with those of its group's heads
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal);
@@ -206,17 +209,17 @@ static bool covered(const fa_flash_shape *s, bool piecewise = false) {
 
 // Return FA_OK / a negative status, or 1 when this path does not cover the call.
 int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
-                 const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream) {
+                 const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream, void *bits) {
   if (!covered(s)) return 1;
   // Dropout is bound by its random numbers (see dropout_keep_bits32()): one CTA per tile at every size.
   // Forward, p = 0.1, bf16 causal, mma.sync kernel -> this: B=16 H=16 Hk=4 L=512 D=64 165 -> 119 us, B=4 H=16 L=2048
   // D=64 541 -> 336 us, D=128 731 -> 343 us.
   if (s->dropout_p > 0.f) {
     if (s->dtype == FA_F16)
-      return s->D == 128 ? launch_fwd_tc<__half, 128, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
-                         : launch_fwd_tc<__half, 64, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
-    return s->D == 128 ? launch_fwd_tc<__nv_bfloat16, 128, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
-                       : launch_fwd_tc<__nv_bfloat16, 64, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
+      return s->D == 128 ? launch_fwd_tc<__half, 128, false, true>(s, 0, q, k, q, k, v, o, lse, stream, bits)
+                         : launch_fwd_tc<__half, 64, false, true>(s, 0, q, k, q, k, v, o, lse, stream, bits);
+    return s->D == 128 ? launch_fwd_tc<__nv_bfloat16, 128, false, true>(s, 0, q, k, q, k, v, o, lse, stream, bits)
+                       : launch_fwd_tc<__nv_bfloat16, 64, false, true>(s, 0, q, k, q, k, v, o, lse, stream, bits);
   }
   // More query tiles than CTA slots and short walks (or head_dim 64): the persistent kernel.  It
   // measured +3..5 % at N <= 1024 and at head_dim 64, but -10 % at head_dim 128 and N = 4096, -17 %

@@ -306,8 +306,13 @@ __global__ void __launch_bounds__(FwdTcCfg<D>::kThreads, 2)
       uint32_t keep[2] = {0u, 0u};
       if (DROP) {
         const uint64_t ctr = p.drop.offset + (((uint64_t)b * p.H + h) * p.M + row) * p.N + n0;
-        keep[0] = dropout_keep_bits32(p.drop, ctr, 1u);
-        keep[1] = dropout_keep_bits32(p.drop, ctr + 32, 1u);
+        auto next = [](int i) { return (uint64_t)i; };
+        keep[0] = dropout_keep_bits32(p.drop, ctr, 31, next);
+        keep[1] = dropout_keep_bits32(p.drop, ctr + 32, 31, next);
+        if (p.drop.bits) {
+          uint32_t *word = p.drop.bits + (((int64_t)b * p.H + h) * p.drop.words + (n0 >> 5)) * p.drop.rows + row;
+          word[0] = keep[0], word[p.drop.rows] = keep[1];
+        }
       }
       ok = mbar_wait(bar(S_FULL + st), ph, actx, 301);
       ok = __all_sync(0xffffffffu, ok);

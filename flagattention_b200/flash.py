@@ -78,16 +78,27 @@ def get_bwd_config(B, H, M, N, D, causal):
     return (128, 128, 3, 18)
 
 
-def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0):
+def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0, keep=False):
+    """(o, log-normaliser), and with `keep` the buffer of dropout decisions for the backward, or None where the kernels
+    keep none."""
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
     o = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
     L = torch.empty((B, H, M), device=q.device, dtype=torch.float32)
-    st = _C.call("fa_flash_fwd")(
-        _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset), _C.pack4(q), _C.pack4(k),
-        _C.pack4(v), _C.pack4(o), L.data_ptr(), _C.raw_stream(q.device))
+    shape = _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale, dropout_p, seed, offset)
+    args = (shape, _C.pack4(q), _C.pack4(k), _C.pack4(v), _C.pack4(o), L.data_ptr())
+    stream = _C.raw_stream(q.device)
+    bits_bytes = _C.call("fa_flash_keep_bits_bytes")(shape) if keep else 0
+    if bits_bytes:
+        bits = torch.empty(bits_bytes, dtype=torch.uint8, device=q.device)
+        st = _C.call("fa_flash_fwd_keep")(*args, bits.data_ptr(), bits_bytes, stream)
+        if st != _C.FA_ERR_UNSUPPORTED:   # a layout for the kernels below
+            _C.check(st, "fa_flash_fwd_keep")
+            return o, L, bits
+        del bits
+    st = _C.call("fa_flash_fwd")(*args, stream)
     _C.check(st, "fa_flash_fwd")
-    return o, L
+    return (o, L, None) if keep else (o, L)
 
 
 def _identity_block_table(B, blocks_per_batch, id_stride, device):
@@ -167,7 +178,7 @@ def _total_attention(q, k, L, causal, sm_scale):
     return tot
 
 
-def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, seed=0, offset=0):
+def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, seed=0, offset=0, bits=None):
     """Launches delta, dK/dV and dQ. `mark(name)`, when given, is called before the first launch
     and after each one (the benchmark records CUDA events there)."""
     B, H, M, D = q.shape
@@ -186,8 +197,11 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
             ws_bytes = _C.call("fa_flash_bwd_workspace_bytes")(shape)
             if ws_bytes > 0:
                 ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-                st = _C.call("fa_flash_bwd")(shape, tq, tk, tv, to, tdo, L.data_ptr(), tdq, tdk, tdv, ws.data_ptr(),
-                                             ws_bytes, stream)
+                args = (shape, tq, tk, tv, to, tdo, L.data_ptr(), tdq, tdk, tdv)
+                if bits is None:
+                    st = _C.call("fa_flash_bwd")(*args, ws.data_ptr(), ws_bytes, stream)
+                else:   # the forward kept its dropout decisions
+                    st = _C.call("fa_flash_bwd_keep")(*args, bits.data_ptr(), bits.numel(), ws.data_ptr(), ws_bytes, stream)
                 # a layout the one-pass kernel cannot map (a broadcast stride) goes to the pair below
                 if st != _C.FA_ERR_UNSUPPORTED:
                     _C.check(st, "fa_flash_bwd")
@@ -274,18 +288,21 @@ class FlashAttention(torch.autograd.Function):
             else:
                 seed, offset = 0, 0
 
+            bits = None
             cfg = get_fwd_config_kv_split(B, H, M, N, D, causal)
             S = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], _C.sm_count(q.device), 128)
             if S > 1:
                 assert not is_dropout, "Cannot apply dropout with splitkv."
                 o, L = _splitkv_forward(q, k, v, causal, sm_scale, S)
+            elif is_dropout and any(ctx.needs_input_grad[:3]) and use_one_pass_backward():
+                o, L, bits = _forward(q, k, v, causal, sm_scale, dropout_p, seed, offset, True)
             else:
                 o, L = _forward(q, k, v, causal, sm_scale, dropout_p, seed, offset)
             tot_attn = None
             if return_total_attention:
                 tot_attn = _total_attention(q, k, L, causal, sm_scale)
 
-        ctx.save_for_backward(q, k, v, o, L)
+        ctx.save_for_backward(q, k, v, o, L, *([] if bits is None else [bits]))
         ctx.sm_scale = sm_scale
         ctx.causal = causal
         ctx.dropout_p = dropout_p
@@ -300,9 +317,9 @@ class FlashAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, do, *ignored):
-        q, k, v, o, L = ctx.saved_tensors
+        q, k, v, o, L, *bits = ctx.saved_tensors
         dq, dk, dv = _backward(q, k, v, o, L, do, ctx.causal, ctx.sm_scale, None, ctx.dropout_p,
-                               ctx.seed, ctx.offset)
+                               ctx.seed, ctx.offset, *bits)
         return dq, dk, dv, None, None, None, None, None, None
 
 

@@ -167,6 +167,19 @@ int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
                  const fa_tensor4 *dq, const fa_tensor4 *dk, const fa_tensor4 *dv, void *workspace,
                  int64_t workspace_bytes, void *stream);
 
+/* Dropout decisions kept from the forward for the backward, one bit an element, so that the backward need not
+ * draw them again.  fa_flash_keep_bits_bytes: the size of the buffer (16-byte aligned, no initial contents), 0 where
+ * none is kept (no dropout, more than 32 D keys, or not the tcgen05 kernels).  fa_flash_fwd_keep is fa_flash_fwd and
+ * writes it; FA_ERR_UNSUPPORTED, before anything is launched, for a layout that only the kernels without it take.
+ * fa_flash_bwd_keep is fa_flash_bwd and reads it: same shape, dropout_p, seed and offset as the forward. */
+int64_t fa_flash_keep_bits_bytes(const fa_flash_shape *s);
+int fa_flash_fwd_keep(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
+                      const fa_tensor4 *o, float *lse, void *bits, int64_t bits_bytes, void *stream);
+int fa_flash_bwd_keep(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
+                      const fa_tensor4 *o, const fa_tensor4 *d_o, const float *lse, const fa_tensor4 *dq,
+                      const fa_tensor4 *dk, const fa_tensor4 *dv, const void *bits, int64_t bits_bytes,
+                      void *workspace, int64_t workspace_bytes, void *stream);
+
 /* Regenerates the dropout keep-mask of a flash_attention call: mask[b,h,m,n] (1 byte each,
  * contiguous) = 1 iff the element was kept.  Replaces `recompute_mask_kernel`
  * (src/flag_attn/testing/dropout.py:5-25). */
