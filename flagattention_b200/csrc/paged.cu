@@ -77,6 +77,7 @@ __device__ __forceinline__ int partition_tokens(const fa_paged_args &a, const Si
 template <typename T, int D, typename IdxT, bool HALF>
 __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
     const fa_paged_args a, const Sizing z) {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // the reduction waits for all of this grid by itself
   using C = PagedCfg<D>;
   constexpr int NW = C::kWarps, NS = C::kStages, CPR = D / 8;
   constexpr int R = HALF ? 1 : 2;   // accumulator rows of a thread: g and, in a full tile, g + 8
@@ -386,35 +387,54 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
   }
 }
 
-// One CTA per (seq, query head); thread d4 owns 4 output columns.
+// One CTA per (seq, query head): its 256 threads are 1024 / D groups of D / 4, a thread owning 4 output columns of every
+// (1024 / D)-th partition.  What bounds it is latency, two round trips to L2 (statistics, then rows): a CTA that went
+// through the partitions one after another with the threads of one row took 13.4 us for 32 partitions of 32 rows (dense
+// decoding, B=2 H=16 N=131072, beside 299 us of decoding) and 8.9 us for 64 sequences of 32 heads up to 32768 tokens:
+// the first of these calls 317 -> 307 us.  It is launched while the decode kernel's last CTAs run (programmatic stream
+// serialization) and waits for that grid: 307 -> 305 us, H=16 N=512 7.9 -> 6.8 us, 4 sequences up to 1500 10.0 -> 8.4.
+constexpr int kReduceThreads = 256;
 template <typename T>
-__global__ void paged_reduce_kernel(const fa_paged_args a, const Sizing z) {
+__global__ void __launch_bounds__(kReduceThreads) paged_reduce_kernel(const fa_paged_args a, const Sizing z) {
+  __shared__ float4 part_o[kReduceThreads];
+  __shared__ float part_den[kReduceThreads];
   const int seq = blockIdx.x, qh = blockIdx.y;
-  const int D = a.head_size;
+  const int D = a.head_size, cols = D / 4, groups = kReduceThreads / cols;
+  const int g = threadIdx.x / cols, c4 = threadIdx.x % cols;
   const int P = (a.max_context_len + a.partition_size - 1) / a.partition_size;
   const int ctx = context_len(a, seq);
   const int size = partition_tokens(a, z, lane_lens(a, z), ctx, P);
   const int np = min(P, (ctx + size - 1) / size);
+  // launched beside the decode kernel's last CTAs (reduce()): its results are there from here on
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int64_t base = ((int64_t)seq * a.num_q_heads + qh) * P;
   float mm = -INFINITY;
-  for (int p = 0; p < np; ++p) mm = fmaxf(mm, a.part_max[base + p]);
-  for (int c4 = threadIdx.x; c4 < D / 4; c4 += blockDim.x) {
-    float den = 0.f;
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int p = 0; p < np; ++p) {
-      const float wgt = a.part_sum[base + p] * fast_exp2(a.part_max[base + p] - mm);
-      den += wgt;
-      const float4 v = *reinterpret_cast<const float4 *>(a.part_out + (base + p) * D + c4 * 4);
-      o.x += wgt * v.x, o.y += wgt * v.y, o.z += wgt * v.z, o.w += wgt * v.w;
-    }
-    const float inv = den > 0.f ? 1.f / den : 0.f;
-    T *dst = reinterpret_cast<T *>(a.out) + (int64_t)seq * a.o_stride_s +
-             (int64_t)qh * a.o_stride_h + c4 * 4;
-    uint2 pk;
-    pk.x = Elem<T>::pack(o.x * inv, o.y * inv);
-    pk.y = Elem<T>::pack(o.z * inv, o.w * inv);
-    *reinterpret_cast<uint2 *>(dst) = pk;
+  for (int p = threadIdx.x & 31; p < np; p += 32) mm = fmaxf(mm, a.part_max[base + p]);
+#pragma unroll
+  for (int off = 16; off; off >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, off));
+  float den = 0.f;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int p = g; p < np; p += groups) {
+    const float wgt = a.part_sum[base + p] * fast_exp2(a.part_max[base + p] - mm);
+    den += wgt;
+    const float4 v = *reinterpret_cast<const float4 *>(a.part_out + (base + p) * D + c4 * 4);
+    o.x += wgt * v.x, o.y += wgt * v.y, o.z += wgt * v.z, o.w += wgt * v.w;
   }
+  part_o[threadIdx.x] = o, part_den[threadIdx.x] = den;
+  __syncthreads();
+  if (g > 0) return;
+  for (int i = 1; i < min(groups, np); ++i) {
+    const float4 v = part_o[i * cols + c4];
+    den += part_den[i * cols + c4];
+    o.x += v.x, o.y += v.y, o.z += v.z, o.w += v.w;
+  }
+  const float inv = den > 0.f ? 1.f / den : 0.f;
+  T *dst = reinterpret_cast<T *>(a.out) + (int64_t)seq * a.o_stride_s + (int64_t)qh * a.o_stride_h + c4 * 4;
+  uint2 pk;
+  pk.x = Elem<T>::pack(o.x * inv, o.y * inv);
+  pk.y = Elem<T>::pack(o.z * inv, o.w * inv);
+  *reinterpret_cast<uint2 *>(dst) = pk;
 }
 
 template <typename IdxT>
@@ -507,11 +527,14 @@ static int decode(const fa_paged_args *a, const Sizing &z, cudaStream_t s) {
 
 static int reduce(const fa_paged_args *a, const Sizing &z, cudaStream_t s) {
   dim3 grid(a->num_seqs, a->num_q_heads);
-  const int threads = a->head_size / 4 < 32 ? 32 : a->head_size / 4;
-  if (a->dtype == FA_F16)
-    paged_reduce_kernel<__half><<<grid, threads, 0, s>>>(*a, z);
-  else
-    paged_reduce_kernel<__nv_bfloat16><<<grid, threads, 0, s>>>(*a, z);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3(kReduceThreads), cfg.stream = s, cfg.attrs = &attr, cfg.numAttrs = 1;
+  const cudaError_t st = a->dtype == FA_F16 ? cudaLaunchKernelEx(&cfg, paged_reduce_kernel<__half>, *a, z)
+                                            : cudaLaunchKernelEx(&cfg, paged_reduce_kernel<__nv_bfloat16>, *a, z);
+  if (st != cudaSuccess) return FA_ERR_LAUNCH;
   FA_CHECK_LAUNCH();
   return FA_OK;
 }
