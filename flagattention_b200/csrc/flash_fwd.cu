@@ -66,6 +66,8 @@ static FwdParams make_fwd_params(const fa_flash_shape *s, const fa_tensor4 *q, c
 namespace tc {
 int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                  const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream, void *bits);
+int flash_fwd_fine_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
+                      const fa_tensor4 *o, float *lse, cudaStream_t stream);
 }
 
 }  // namespace fa
@@ -95,6 +97,19 @@ extern "C" int fa_flash_fwd_keep(const fa_flash_shape *s, const fa_tensor4 *q, c
   if (need == 0) return FA_ERR_UNSUPPORTED;
   if (bits_bytes < need) return FA_ERR_WORKSPACE;
   const int tc_status = tc::flash_fwd_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream), bits);
+  return tc_status == 1 ? FA_ERR_UNSUPPORTED : tc_status;   // 1: nothing launched
+}
+
+extern "C" int fa_flash_fwd_few_rows(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
+                                     const fa_tensor4 *v, const fa_tensor4 *o, float *lse, void *stream) {
+  if (int st = validate_shape(s)) return st;
+  if (int st = validate_tensors({q, k, v, o})) return st;
+  if (!lse) return FA_ERR_BAD_ARG;
+  // A query tile here has 128 rows (and up to 8 CTAs), one of the split-KV kernels 16.  bf16, split-KV -> this, us:
+  // H=8 M=32 N=16384 D=128 43.7 -> 30.2, H=4 M=128 N=16384 79.8 -> 31.4, H=16 M=64 N=4096 43.6 -> 17.4, B=8 H=4 M=37
+  // N=346 D=64 8.0 -> 8.9, H=4 M=32 N=1000 9.1 -> 10.9 (and one launch and two allocations less).
+  if (s->M < 32) return FA_ERR_UNSUPPORTED;   // H=4 M=17 N=131072 157 -> 192
+  const int tc_status = tc::flash_fwd_fine_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream));
   return tc_status == 1 ? FA_ERR_UNSUPPORTED : tc_status;   // 1: nothing launched
 }
 

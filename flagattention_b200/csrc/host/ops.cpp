@@ -105,11 +105,19 @@ fa_flash_shape shape_of(const Tensor &q, const Tensor &k, bool causal, double sc
 }
 
 // ---- flash_attention -----------------------------------------------------------------------------------------------
-std::pair<Tensor, Tensor> flash_forward(const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale) {
+// `few_rows`: the form for calls that split their keys; undefined tensors where the split-KV kernels do it
+std::pair<Tensor, Tensor> flash_forward(const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale,
+                                        bool few_rows) {
   Tensor o = new_like(q), lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
   const fa_flash_shape s = shape_of(q, k, causal, scale);
   const fa_tensor4 tq = tensor4(q), tk = tensor4(k), tv = tensor4(v), to = tensor4(o);
-  check(fa_flash_fwd(&s, &tq, &tk, &tv, &to, lse.data_ptr<float>(), stream_of(q)), "fa_flash_fwd");
+  if (few_rows) {
+    const int st = fa_flash_fwd_few_rows(&s, &tq, &tk, &tv, &to, lse.data_ptr<float>(), stream_of(q));
+    if (st == FA_ERR_UNSUPPORTED) return {};
+    check(st, "fa_flash_fwd_few_rows");
+  } else {
+    check(fa_flash_fwd(&s, &tq, &tk, &tv, &to, lse.data_ptr<float>(), stream_of(q)), "fa_flash_fwd");
+  }
   return {o, lse};
 }
 
@@ -144,8 +152,10 @@ variable_list flash_backward(const Tensor &q, const Tensor &k, const Tensor &v, 
 }
 
 struct FlashAttention : torch::autograd::Function<FlashAttention> {
-  static Tensor forward(AutogradContext *ctx, const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale) {
-    auto out = flash_forward(q, k, v, causal, scale);
+  // o and lse: computed by the caller, who may find that the call is not for this form
+  static Tensor forward(AutogradContext *ctx, const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale,
+                        const std::pair<Tensor, Tensor> *computed) {
+    const auto &out = *computed;
     ctx->save_for_backward({q, k, v, out.first, out.second});
     ctx->saved_data["causal"] = causal;
     ctx->saved_data["scale"] = scale;
@@ -155,7 +165,7 @@ struct FlashAttention : torch::autograd::Function<FlashAttention> {
     const auto t = ctx->get_saved_variables();
     variable_list g = flash_backward(t[0], t[1], t[2], t[3], t[4], grads[0], ctx->saved_data["causal"].toBool(),
                                      ctx->saved_data["scale"].toDouble());
-    g.resize(5);
+    g.resize(6);
     return g;
   }
 };
@@ -166,37 +176,34 @@ int64_t coarsen_partition(int64_t size, int64_t pairs, int64_t context, int64_t 
   return size;
 }
 
-// flash._decode_covered() and what _decode_forward() passes on without a copy
-bool decode_covered(const Tensor &q, const Tensor &k, const Tensor &v, bool causal) {
-  const int64_t H = q.size(1), M = q.size(2), N = k.size(2), Hk = k.size(1);
-  if (N % 16 != 0 || H / Hk * M > 64 || (causal && M > 1 && N < M)) return false;
+// flash._decode_covered() for one query a head, and what _decode_forward() passes on without a copy
+bool decode_covered(const Tensor &q, const Tensor &k, const Tensor &v) {
+  if (k.size(2) % 16 != 0 || q.size(1) / k.size(1) > 64) return false;
   if (k.strides() != v.strides() || k.stride(3) != 1 || !aligned16(k) || !aligned16(v)) return false;
   const int64_t sl = k.stride(2);
   if (sl <= 0 || sl % 8 || k.stride(1) % 8 || k.stride(0) % (16 * sl)) return false;
-  return q.stride(3) == 1 && q.stride(0) % 8 == 0 && q.stride(1) % 8 == 0 && q.stride(2) % 8 == 0 &&
-         (M == 1 || q.stride(1) == M * q.stride(2));
+  return q.stride(3) == 1 && q.stride(0) % 8 == 0 && q.stride(1) % 8 == 0;
 }
 
 // flash._decode_forward()
-Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double scale, bool causal) {
-  const int64_t B = q.size(0), H = q.size(1), M = q.size(2), D = q.size(3), Hk = k.size(1), N = k.size(2);
+Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double scale) {
+  const int64_t B = q.size(0), H = q.size(1), D = q.size(3), Hk = k.size(1), N = k.size(2);
   const int64_t sb = k.stride(0), sl = k.stride(2);
   int64_t partition = coarsen_partition(256, B * Hk, N, sm_count(), 4096);
   if (N <= partition) partition = 0;
   Tensor o = new_like(q), ws;
   fa_paged_args a{};
   dtype_code(q, &a.dtype);
-  a.num_seqs = (int32_t)B, a.num_q_heads = (int32_t)(H * M), a.num_kv_heads = (int32_t)Hk, a.head_size = (int32_t)D;
+  a.num_seqs = (int32_t)B, a.num_q_heads = (int32_t)H, a.num_kv_heads = (int32_t)Hk, a.head_size = (int32_t)D;
   a.block_size = 16, a.max_context_len = (int32_t)N, a.block_table_is_i64 = FA_BLOCK_TABLE_IN_PLACE;
   a.partition_size = (int32_t)partition, a.attn_scale = (float)scale;
-  a.query = q.data_ptr(), a.q_stride_s = q.stride(0), a.q_stride_h = M == 1 ? q.stride(1) : q.stride(2);
+  a.query = q.data_ptr(), a.q_stride_s = q.stride(0), a.q_stride_h = q.stride(1);
   a.key_cache = k.data_ptr(), a.value_cache = v.data_ptr();
   a.kv_stride_b = 16 * sl, a.kv_stride_h = Hk > 1 ? k.stride(1) : 0, a.kv_stride_t = sl;
   a.bt_stride_s = sb / (16 * sl);
-  a.out = o.data_ptr(), a.o_stride_s = H * M * D, a.o_stride_h = D;
-  a.causal_rows = causal && M > 1 ? (int32_t)M : 0;
+  a.out = o.data_ptr(), a.o_stride_s = H * D, a.o_stride_h = D;
   if (partition) {
-    const int64_t rows = B * H * M, P = (N + partition - 1) / partition, stats = (rows * P + 63) / 64 * 64;
+    const int64_t rows = B * H, P = (N + partition - 1) / partition, stats = (rows * P + 63) / 64 * 64;
     ws = at::empty({rows * P * D + 2 * stats}, q.options().dtype(at::kFloat));
     a.part_out = ws.data_ptr<float>();
     a.part_max = a.part_out + rows * P * D;
@@ -224,11 +231,15 @@ Tensor flash(const Tensor &q, const Tensor &k, const Tensor &v, bool causal, boo
   if (default_scale) scale = 1.0 / std::sqrt((double)D);
   const bool grads = q.requires_grad() || k.requires_grad() || v.requires_grad();
   const bool split = fa_num_splits_heuristic((int32_t)B, (int32_t)H, (int32_t)M, (int32_t)N, 16, 128, sm_count(), 128) > 1;
-  if (M <= 16 && !grads && (M == 1 || split))
-    return decode_covered(q, k, v, causal) ? decode_forward(q, k, v, scale, causal) : Tensor();
-  if (split) return {};   // the split-KV kernels
-  if (!grads || !at::GradMode::is_enabled()) return flash_forward(q, k, v, causal, scale).first;
-  return FlashAttention::apply(q, k, v, causal, scale);
+  if (M <= 16 && !grads && (M == 1 || split))   // (several queries a head: the Python form)
+    return M == 1 && decode_covered(q, k, v) ? decode_forward(q, k, v, scale) : Tensor();
+  std::pair<Tensor, Tensor> out;
+  {
+    at::AutoGradMode no_graph(false);
+    out = flash_forward(q, k, v, causal, scale, split);
+  }
+  if (!out.first.defined() || !grads || !at::GradMode::is_enabled()) return out.first;
+  return FlashAttention::apply(q, k, v, causal, scale, &out);
 }
 
 // ---- piecewise_attention -------------------------------------------------------------------------------------------

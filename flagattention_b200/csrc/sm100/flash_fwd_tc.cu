@@ -207,6 +207,18 @@ static bool covered(const fa_flash_shape *s, bool piecewise = false) {
   return !generic_forced() && s->sm_scale > 0.f && s->N >= fewest_keys(s, piecewise);
 }
 
+// Calls of few rows, which went to the split-KV kernels: those follow the row maximum exactly, so P goes in with its
+// remainder here.  Return values as below.
+int flash_fwd_fine_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
+                      const fa_tensor4 *o, float *lse, cudaStream_t stream) {
+  if (!covered(s) || s->dropout_p > 0.f) return 1;
+  if (s->dtype == FA_F16)
+    return s->D == 128 ? launch_fwd_tc<__half, 128, false, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
+                       : launch_fwd_tc<__half, 64, false, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
+  return s->D == 128 ? launch_fwd_tc<__nv_bfloat16, 128, false, false, true>(s, 0, q, k, q, k, v, o, lse, stream)
+                     : launch_fwd_tc<__nv_bfloat16, 64, false, false, true>(s, 0, q, k, q, k, v, o, lse, stream);
+}
+
 // Return FA_OK / a negative status, or 1 when this path does not cover the call.
 int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                  const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream, void *bits) {

@@ -93,7 +93,7 @@ enum FwdBar { Q_FULL = 0, K_FULL = 1, K_FREE = 3, V_FULL = 5, V_FREE = 7, S_FULL
 // re-loaded once, at the switch from the far to the near entries.
 // DROP = dropout on the probabilities that enter P V (the row sums stay undropped).  The keep bits of a
 // tile do not depend on its scores: they are computed before the wait for them.
-// PAD = the head_dim of the tensors is below D.
+// PAD = the head_dim of the tensors may be below D.
 // Both also give P to P V as a 16-bit value and a 16-bit remainder, in the two halves of the S columns: these
 // calls once ran on kernels that follow the row maximum exactly, so that a row's largest weight is 1 and has no
 // rounding error; here the reference may lag it by 2^8.  B=2 H=8 L=777 D=32 causal, bf16, scores of deviation 4,

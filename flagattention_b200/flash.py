@@ -101,6 +101,21 @@ def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0, keep=Fa
     return (o, L, None) if keep else (o, L)
 
 
+def _few_rows_forward(q, k, v, causal, sm_scale):
+    """(o, log-normaliser) of a call that splits its keys, by clusters of CTAs; None where the split-KV kernels do it."""
+    B, H, M, D = q.shape
+    N, Hk = k.shape[2], k.shape[1]
+    o = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
+    L = torch.empty((B, H, M), device=q.device, dtype=torch.float32)
+    st = _C.call("fa_flash_fwd_few_rows")(
+        _C.pack_shape(q.dtype, B, H, Hk, M, N, D, causal, sm_scale), _C.pack4(q), _C.pack4(k), _C.pack4(v), _C.pack4(o),
+        L.data_ptr(), _C.raw_stream(q.device))
+    if st == _C.FA_ERR_UNSUPPORTED:
+        return None
+    _C.check(st, "fa_flash_fwd_few_rows")
+    return o, L
+
+
 def _identity_block_table(B, blocks_per_batch, id_stride, device):
     """(block_tables, context_lens) with block_tables[b, c] = b * id_stride + c: what FA_BLOCK_TABLE_IN_PLACE
     stands for, under which a (B, Hk, N, D) key tensor is a paged cache of 16-token blocks.  The kernel works
@@ -293,7 +308,7 @@ class FlashAttention(torch.autograd.Function):
             S = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], _C.sm_count(q.device), 128)
             if S > 1:
                 assert not is_dropout, "Cannot apply dropout with splitkv."
-                o, L = _splitkv_forward(q, k, v, causal, sm_scale, S)
+                o, L = _few_rows_forward(q, k, v, causal, sm_scale) or _splitkv_forward(q, k, v, causal, sm_scale, S)
             elif is_dropout and any(ctx.needs_input_grad[:3]) and use_one_pass_backward():
                 o, L, bits = _forward(q, k, v, causal, sm_scale, dropout_p, seed, offset, True)
             else:

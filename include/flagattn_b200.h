@@ -93,6 +93,10 @@ int fa_splitkv_fwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor
                    float *o_partial, float *lse_partial, void *stream);
 int fa_splitkv_combine(const fa_flash_shape *s, int32_t num_splits, const float *o_partial,
                        const float *lse_partial, const fa_tensor4 *o, float *lse, void *stream);
+/* The same result in one call and without a workspace, where a cluster of CTAs can share the walk of a query tile:
+ * calls of at least 32 queries on the tcgen05 kernels.  FA_ERR_UNSUPPORTED, before anything is launched, elsewhere. */
+int fa_flash_fwd_few_rows(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
+                          const fa_tensor4 *o, float *lse, void *stream);
 /* Bytes of o_partial + lse_partial for a given problem (host-only helper). */
 int64_t fa_splitkv_workspace_bytes(const fa_flash_shape *s, int32_t num_splits);
 

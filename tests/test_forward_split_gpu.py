@@ -20,7 +20,9 @@ pytestmark = pytest.mark.gpu
     (1, 9, 3, 700, 520, 64, True),        # the first 180 rows see no key, whole tiles among them
     (3, 16, 4, 130, 1217, 64, True),
     (1, 8, 8, 1030, 2100, 32, True), (1, 8, 8, 1030, 2100, 16, False),
-    (1, 4, 4, 512, 513, 64, True)])
+    (1, 4, 4, 512, 513, 64, True),
+    # calls that the split-KV kernels took: P with its remainder
+    (1, 8, 8, 32, 2000, 128, True), (1, 4, 2, 300, 1000, 64, True), (2, 2, 1, 45, 40, 128, False), (1, 3, 3, 250, 77, 64, True)])
 def test_split_walks(B, H, Hk, M, N, D, causal, dtype):
     q, k, v, _ = make_qkv(B, H, Hk, M, N, D, dtype, "cuda", 2.0, seed=M + N)
     junk = torch.full_like(q, float("nan"))   # the outputs come from this memory
@@ -57,3 +59,18 @@ def test_values_at_the_edges_of_the_range():
         one = fa.flash_attention(q, k, v, True)
     assert torch.equal(torch.isnan(o), torch.isnan(one)) and torch.equal(torch.isinf(o), torch.isinf(one))
     assert not torch.isfinite(o).all() and torch.isfinite(o[0, 3]).all()
+
+
+@pytest.mark.parametrize("B,H,M,N,D,std", [(1, 8, 32, 3000, 128, 1.0), (1, 4, 200, 1500, 64, 2.0), (1, 4, 64, 400, 128, 2.0)])
+def test_few_rows_are_no_less_precise_than_the_split_kv_kernels(B, H, M, N, D, std):
+    from flagattention_b200 import flash, split_kv
+    q, k, v, _ = make_qkv(B, H, H, M, N, D, torch.bfloat16, "cuda", std, seed=M)
+    s = (q.double() @ k.double().transpose(2, 3)) * D ** -0.5
+    s.masked_fill_(torch.ones(M, N, dtype=torch.bool, device="cuda").triu(N - M + 1), float("-inf"))
+    want = torch.softmax(s, 3) @ v.double()
+    few = flash._few_rows_forward(q, k, v, True, D ** -0.5)
+    split = split_kv._splitkv_forward(q, k, v, True, D ** -0.5, 4)
+    errors = [((x[0].double() - want).norm() / want.norm()).item() for x in (few, split)]
+    assert errors[0] <= errors[1] * 1.02, errors     # (both end in the same rounding of o)
+    assert (few[1].double() - torch.logsumexp(s, 3)).abs().max() <= 2e-5
+    assert flash._few_rows_forward(q[:, :, :31], k, v, True, 0.1) is None
