@@ -1,4 +1,5 @@
 // Launcher and C entry points of the one-pass tcgen05 flash_attention backward.
+#include <algorithm>
 #include <cstdlib>
 #include <utility>
 #include <vector>
@@ -44,6 +45,11 @@ static int64_t fused_dq_acc_bytes(const fa_flash_shape *s) {
 static int64_t fused_workspace_bytes(const fa_flash_shape *s, int accumulators = 1) {
   return accumulators * fused_dq_acc_bytes(s) + 16;
 }
+// the shares of dK and dV where CTAs share the walk of a key block
+static int64_t share_bytes(const fa_flash_shape *s, int split) {
+  if (split <= 1) return 0;
+  return (int64_t)split * 2 * s->B * s->Hk * (((int64_t)s->N + 127) / 128 * 128) * fused_padded_dim(s) * 4;
+}
 
 // one persistent CTA per SM
 static int sm_count() {
@@ -52,6 +58,38 @@ static int sm_count() {
       cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
     return 0;
   return n;
+}
+
+// CTAs that share the walk of a key block (1, 2, 4 or 8): a call of a few kv heads with many query heads each is as slow as
+// its longest walk, whatever the other SMs do.  Estimated in tiles (2.2 us at head_dim 128): an item costs 2 beside its
+// walk, 6 where it leaves a share (128 KB of fp32), the combining launch 4 and its bytes; with more items than SMs a
+// longest one ends half of itself after the mean.  Taken where it saves a tenth and 4.  Backward, bf16 causal D=128, us at
+// 1 / 2 / 4 / 8 (items, longest walk):
+//   H=8 Hk=1 L=8192 (64, 512)          1126 /  609 /  450 /  363
+//   H=32 Hk=4 L=8192 (256, 512)        1689 / 1342 / 1331 / 1448
+//   H=32 Hk=8 L=8192 (512, 256)        1428 / 1465 / 1586 / 1884
+//   B=2 H=16 Hk=2 L=4096 (128, 256)     622 /  490 /  402 /  439
+//   H=8 Hk=2 L=2048 (32, 64)            206 /  135 /   94 /   95
+//   H=8 Hk=8 L=2048 (128, 16)            70 /   86 /  107 /  146
+//   H=4 Hk=1 L=512 D=64 (4, 16)          60 /   63 /   63 /   63
+static int walk_split(const fa_flash_shape *s) {
+  const int sms = sm_count();
+  const int64_t blocks = ((int64_t)s->N + 127) / 128, rows = ((int64_t)s->M + 127) / 128, items = blocks * s->B * s->Hk;
+  if (sms <= 0 || items > 2ll * sms) return 1;
+  const double longest = (double)rows * (s->H / s->Hk);
+  // (keys before the first query's see every query)
+  const double seen = s->causal && s->N <= s->M ? 0.5 * (1.0 + 1.0 / (double)rows) : 1.0;
+  auto estimate = [&](int c) {
+    const double walk = longest / c + (c > 1 ? 6 : 2);
+    const double mean = ((double)items * longest * seen + (c > 1 ? 6.0 : 2.0) * (double)(items * c)) / sms;
+    const double kernel = items * c > sms ? mean + 0.5 * walk : std::max(walk, mean);
+    return kernel + (c > 1 ? 4 + 0.01 * (double)(items * c) : 0);
+  };
+  int best = 1;
+  double least = 0.9 * estimate(1) - 4;
+  for (int c = 2; c <= 8; c *= 2)
+    if (estimate(c) < least) best = c, least = estimate(c);
+  return best;
 }
 
 // diff[i] holds +1 / -1 where coverage of unit i starts / ends; returns the maximal runs of
@@ -109,12 +147,13 @@ struct FarBranch {
 // key block is walked twice by the same CTA, near pairs with (q, k) -> (dq, dk), far pairs with
 // (q2, k2) -> (dq2, dk2); dV accumulates across the two walks and is rounded once).
 // Workspace: dq accumulator [| dq2 accumulator] | 16 bytes of work-item counter.
-template <typename T, int D, bool DROP = false>
+template <typename T, int D, bool DROP = false, bool SPLIT = false>
 static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                         const fa_tensor4 *v, const fa_tensor4 *d_o, const float *lse,
                         const float *delta, const fa_tensor4 *dq, const fa_tensor4 *dk,
                         const fa_tensor4 *dv, float *workspace, cudaStream_t stream,
-                        const FarBranch *far = nullptr, int stages = 7, const void *bits = nullptr) {
+                        const FarBranch *far = nullptr, int stages = 7, const void *bits = nullptr,
+                        int split = 1, void *shares = nullptr) {
   using C = FusedBwdCfg<D>;
   const fa_tensor4 *q2 = far ? far->q2 : q, *k2 = far ? far->k2 : k, *dk2 = far ? far->dk2 : dk;
   CUtensorMap mq, mdo, mk, mv, mdk, mdv, mq2, mk2, mdk2;
@@ -130,7 +169,7 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
               !make_map_bhld(&mk2, k2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN) ||
               !make_map_bhld(&mdk2, dk2, s->dtype, s->B, s->Hk, s->N, s->D, C::BN)))
     return FA_ERR_UNSUPPORTED;
-  auto kern = flash_bwd_fused_tc_kernel<T, D, DROP>;
+  auto kern = flash_bwd_fused_tc_kernel<T, D, DROP, SPLIT>;
   static unsigned long long done = 0;
   if (int st = ensure_dyn_smem(kern, C::kTotal, &done)) return st;
   FusedBwdParams fp{};
@@ -153,6 +192,9 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
   fp.dk2 = dk2->ptr;
   fp.Mpad = (s->M + 127) / 128 * 128;
   fp.sched = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(workspace) + n_acc * acc_bytes);
+  fp.split = split;
+  fp.dk_part = static_cast<float *>(shares);
+  fp.dv_part = split > 1 ? fp.dk_part + share_bytes(s, split) / 8 : nullptr;
   // stages: 1 = zero-fill of the workspace, 2 = the kernel, 4 = scale + convert the workspace to dq
   if ((stages & 1) &&
       cudaMemsetAsync(workspace, 0, (size_t)(n_acc * acc_bytes + 16), stream) != cudaSuccess)
@@ -160,11 +202,11 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
   if (stages & 2) {
     // the CTAs of a (batch, kv head) pair share its Q and dO tiles and its slice of the dq workspace
     p.num_blocks = (s->N + C::BN - 1) / C::BN;
-    const int64_t items = (int64_t)p.num_blocks * s->Hk * s->B;
+    const int64_t blocks = (int64_t)p.num_blocks * s->Hk * s->B, items = blocks * split;
     const int sms = sm_count();
     if (items > 0x3fffffff) return FA_ERR_TOO_LARGE;
     if (sms <= 0) return FA_ERR_LAUNCH;
-    p.group_size = backward_group_size((int64_t)(s->H / s->Hk) * s->M * D * 8 * n_acc, s->B * s->Hk, items, sms,
+    p.group_size = backward_group_size((int64_t)(s->H / s->Hk) * s->M * D * 8 * n_acc, s->B * s->Hk, blocks, sms,
                                        s->causal);
     fp.num_items = (int)items;
     // dk / dv rows of key blocks that walk no query tile (which the kernel skips) get their zeros
@@ -188,6 +230,13 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
     FA_CHECK_LAUNCH();
   }
   if (stages & 4) {
+    if constexpr (SPLIT) {
+      constexpr int kRows = 256 / (D / 8);
+      dim3 sgrid((s->N + kRows - 1) / kRows, s->B * s->Hk, 2);
+      dkdv_combine_kernel<T, D><<<sgrid, 256, 0, stream>>>(fp, dk->ptr, strides_of(dk), dv->ptr, strides_of(dv), s->sm_scale,
+                                                           DROP ? fp.drop.rp : 1.f, s->D);
+      FA_CHECK_LAUNCH();
+    }
     dim3 cgrid((s->M + 31) / 32, s->H, s->B);
     dq_convert_kernel<T, D><<<cgrid, 256, 0, stream>>>(fp.dq_acc, dq->ptr, strides_of(dq), s->H,
                                                        s->M, fp.Mpad, s->sm_scale, s->D);
@@ -298,10 +347,22 @@ extern "C" int fa_flash_bwd_fused_stages(const fa_flash_shape *s, const fa_tenso
 
 // ---- the whole backward in one call -----------------------------------------------------------
 
-// workspace: that of the one-pass kernel | delta (B, H, M) fp32
+// workspace: that of the one-pass kernel | delta (B, H, M) fp32 | shares of dK and dV
+struct WholeWorkspace {
+  int split;
+  int64_t shares, total;
+};
+static WholeWorkspace whole_workspace(const fa_flash_shape *s) {
+  WholeWorkspace w{};
+  w.split = tc::walk_split(s);
+  w.shares = tc::fused_workspace_bytes(s) + (int64_t)s->B * s->H * s->M * 4;
+  if (w.split > 1) w.shares = (w.shares + 15) / 16 * 16;
+  w.total = w.shares + tc::share_bytes(s, w.split);
+  return w;
+}
 extern "C" int64_t fa_flash_bwd_workspace_bytes(const fa_flash_shape *s) {
   if (!s || validate_shape(s) != FA_OK || !tc::one_pass_covered(s)) return 0;
-  return tc::fused_workspace_bytes(s) + (int64_t)s->B * s->H * s->M * 4;
+  return whole_workspace(s).total;
 }
 
 // Both directions on the tcgen05 kernels, whatever the layout turns out to be
@@ -318,9 +379,8 @@ static int whole_backward(const fa_flash_shape *s, const fa_tensor4 *q, const fa
   if (int st = validate_tensors({q, k, v, o, d_o, dq, dk, dv})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
   if (!tc::one_pass_covered(s)) return FA_ERR_UNSUPPORTED;
-  if (!workspace || workspace_bytes < fa_flash_bwd_workspace_bytes(s) ||
-      (reinterpret_cast<uintptr_t>(workspace) & 15))
-    return FA_ERR_WORKSPACE;
+  const WholeWorkspace w = whole_workspace(s);
+  if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 15)) return FA_ERR_WORKSPACE;
   // before the first launch: the caller's other path starts with delta again
   for (const fa_tensor4 *t : {q, d_o, dq})
     if (tc::is_broadcast(t, s->B, s->H, s->M)) return FA_ERR_UNSUPPORTED;
@@ -331,17 +391,23 @@ static int whole_backward(const fa_flash_shape *s, const fa_tensor4 *q, const fa
   const int64_t acc = tc::fused_workspace_bytes(s);
   float *delta = reinterpret_cast<float *>(static_cast<char *>(workspace) + acc);
   if (int rc = fa_flash_bwd_delta_zero(s, o, d_o, delta, workspace, acc, stream)) return rc;
-#define FA_BWD_ARGS s, q, k, v, d_o, lse, delta, dq, dk, dv, ws, st, nullptr, 6, bits
-#define FA_BWD_CASE(DROP)                                                        \
-  if (s->dtype == FA_F16)                                                        \
-    return s->D == 128 ? tc::launch_fused<__half, 128, DROP>(FA_BWD_ARGS)        \
-                       : tc::launch_fused<__half, 64, DROP>(FA_BWD_ARGS);        \
-  return s->D == 128 ? tc::launch_fused<__nv_bfloat16, 128, DROP>(FA_BWD_ARGS)   \
-                     : tc::launch_fused<__nv_bfloat16, 64, DROP>(FA_BWD_ARGS);
+#define FA_BWD_ARGS s, q, k, v, d_o, lse, delta, dq, dk, dv, ws, st, nullptr, 6, bits, w.split, static_cast<char *>(workspace) + w.shares
+#define FA_BWD_CASE(DROP, SPLIT)                                                        \
+  if (s->dtype == FA_F16)                                                               \
+    return s->D == 128 ? tc::launch_fused<__half, 128, DROP, SPLIT>(FA_BWD_ARGS)        \
+                       : tc::launch_fused<__half, 64, DROP, SPLIT>(FA_BWD_ARGS);        \
+  return s->D == 128 ? tc::launch_fused<__nv_bfloat16, 128, DROP, SPLIT>(FA_BWD_ARGS)   \
+                     : tc::launch_fused<__nv_bfloat16, 64, DROP, SPLIT>(FA_BWD_ARGS);
   if (s->dropout_p > 0.f) {
-    FA_BWD_CASE(true)
+    if (w.split > 1) {
+      FA_BWD_CASE(true, true)
+    }
+    FA_BWD_CASE(true, false)
   }
-  FA_BWD_CASE(false)
+  if (w.split > 1) {
+    FA_BWD_CASE(false, true)
+  }
+  FA_BWD_CASE(false, false)
 #undef FA_BWD_CASE
 #undef FA_BWD_ARGS
 }

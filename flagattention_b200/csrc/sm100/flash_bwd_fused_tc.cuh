@@ -90,7 +90,11 @@ struct FusedBwdParams {
   void *dk2;          // piecewise: dk of the far branch (base.dk: near branch), same strides
   int Mpad;           // M rounded up to a multiple of 128
   unsigned *sched;    // work-item counter; zero at launch and at exit (see the kernel)
-  int num_items;      // key blocks x (batch, kv head) pairs
+  int num_items;      // key blocks x (batch, kv head) pairs x split
+  // flash_attention: `split` CTAs share the walk of a key block (its tiles split_begin(T, c) .. split_begin(T, c + 1)) and
+  // leave their share of dK and dV unscaled, in fp32, for dkdv_combine_kernel: (split, B * Hk, N rounded up to 128, D) each
+  int split;
+  float *dk_part, *dv_part;
   DropoutRule drop;   // DROP kernels only
 };
 
@@ -154,7 +158,11 @@ constexpr int kFusedThreads = (kFusedEwWarp + kEwWarps) * 32;   // 768
 __device__ __forceinline__ void regs_keep_48() { asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n"); }
 __device__ __forceinline__ void regs_take_96() { asm volatile("setmaxnreg.inc.sync.aligned.u32 96;\n"); }
 
-// One work item = one block of 128 keys of one (batch, kv head) pair: its query-tile range.
+__host__ __device__ __forceinline__ int split_begin(int tiles, int c, int split) {
+  return (int)((int64_t)tiles * c / split);
+}
+
+// One work item = one block of 128 keys of one (batch, kv head) pair: its query-tile range, or a share of its walk.
 // Under piecewise_attention a block is walked twice, back to back by the same CTA: first the
 // tiles that hold a near pair (mode 1: q1, k1 -> dq1, dk1), then the tiles that hold a far pair
 // (mode 2: q2, k2 -> dq2, dk2).  V stays in shared memory and dV keeps accumulating in TMEM
@@ -162,6 +170,7 @@ __device__ __forceinline__ void regs_take_96() { asm volatile("setmaxnreg.inc.sy
 // once and V and dO of a straddling tile are not fetched by a second launch.
 struct FusedItem {
   int n0, hk, b, mt_lo, mt_hi, T_tiles;
+  int h0, mt0, chunk;   // query head and tile the walk starts at; which share of the key block's it is
   int mode;          // 0 flash, 1 near walk, 2 far walk
   bool first, last;  // of its key block's walks (those with tiles)
 };
@@ -184,7 +193,8 @@ struct FusedItem {
 // about 90 us of the 194 the first of them has come to since; read, the whole training call takes 363 -> 279 us.
 // The drawing does not fit the registers beside the rest: 76 and 180 bytes of spill stores and loads a thread at 64,
 // 32 and 32 at 128 (without dropout 48 and 188, and 12 and 92).
-template <typename T, int D, bool DROP>
+// SPLIT = fp.split CTAs share the walk of a key block.
+template <typename T, int D, bool DROP, bool SPLIT>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     flash_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                               const __grid_constant__ CUtensorMap map_do,
@@ -232,12 +242,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
   const int end_id = pw ? 2 * total : total;
   auto decode = [&](int id) -> FusedItem {
     const int unit = pw ? (id >> 1) : id;
-    const CtaCoord cta = grouped_cta((unsigned)unit, p.num_blocks, p.B * p.Hk, p.group_size);
     FusedItem it;
+    const int block = SPLIT ? unit / fp.split : unit;
+    it.chunk = SPLIT ? unit - block * fp.split : 0;
+    const CtaCoord cta = grouped_cta((unsigned)block, p.num_blocks, p.B * p.Hk, p.group_size);
     it.n0 = cta.blk * BN, it.hk = cta.pair % p.Hk, it.b = cta.pair / p.Hk;
     it.mode = pw ? 1 + (id & 1) : p.mode;
     tile_range(it.n0, it.mode, it.mt_lo, it.mt_hi);
     it.T_tiles = max(0, it.mt_hi - it.mt_lo) * G;
+    it.h0 = it.hk * G, it.mt0 = it.mt_lo;
+    if (SPLIT) {
+      const int per_head = max(it.mt_hi - it.mt_lo, 1), begin = split_begin(it.T_tiles, it.chunk, fp.split);
+      it.T_tiles = split_begin(it.T_tiles, it.chunk + 1, fp.split) - begin;
+      it.h0 += begin / per_head, it.mt0 += begin % per_head;
+    }
     it.first = it.last = true;
     if (pw) {
       int lo, hi;
@@ -321,7 +339,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     }
     if (w_first < end_id) {
       const FusedItem first = decode(w_first);
-      const int h0 = first.hk * G, m00 = first.mt_lo * BM;
+      const int h0 = first.h0, m00 = first.mt0 * BM;
       const CUtensorMap *mk = first.mode == 2 ? &map_k2 : &map_k, *mq = first.mode == 2 ? &map_q2 : &map_q;
       mbar_expect_tx(bar(FB_KV_FULL), C::kTile);
       for (int s = 0; s < KSUB; ++s)
@@ -376,10 +394,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           ++inflight_do;
         };
         // dV then dK of the previous item leave through the copy engine as soon as the element-wise
-        // warps have staged them; `between` runs after the dV store has been requested
+        // warps have staged them (shares are stored by those warps)
         auto store_dv = [&]() -> bool {
           if (!mbar_wait(bar(FB_DV_STAGED), (real - 1) & 1, actx, 721)) return false;
-          if (plast && !p.dv_accumulate) {   // a near walk that a far walk follows stages nothing
+          if (plast && !SPLIT) {   // a near walk that a far walk follows stages nothing
 #pragma unroll
             for (int s = 0; s < KSUB; ++s)
               tma_store_4d(&map_dv, smem + C::kV + s * BN * 128, s * 64, pn0, phk, pb);
@@ -389,6 +407,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         };
         auto store_dk = [&]() -> bool {
           if (!mbar_wait(bar(FB_DK_STAGED), (real - 1) & 1, actx, 722)) return false;
+          if (SPLIT) return true;
 #pragma unroll
           for (int s = 0; s < KSUB; ++s)
             tma_store_4d(pmode == 2 ? &map_dk2 : &map_dk, smem + C::kPD + s * BN * 128, s * 64, pn0, phk, pb);
@@ -405,7 +424,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
           const unsigned fetched = more ? 0u : atomicAdd(fp.sched, 1u);
           int w_next = end_id;
           {
-            int h = it.hk * G, mt = it.mt_lo;
+            int h = it.h0, mt = it.mt0;
             const bool preissued = (ic == 0);   // tile 0, K and V of the first item: see set-up
             if (preissued) {
               inflight_q = inflight_do = 1;
@@ -663,7 +682,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         const int w = ring_item(ic, 950);
         if (w < 0 || w >= end_id) break;
         const FusedItem it = decode(w);
-        int h = it.hk * G, mt = it.mt_lo;
+        int h = it.h0, mt = it.mt0;
         for (int t = 0; t < it.T_tiles; ++t, ++gt) {
           const int m = mt * BM + lane * 4;
           const int64_t li = ((int64_t)it.b * p.H + h) * p.M + m;
@@ -720,7 +739,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       }
       if (w >= end_id) break;
       const FusedItem it = decode(w);
-      int h = it.hk * G, mt = it.mt_lo;
+      int h = it.h0, mt = it.mt0;
       for (int t = 0; t < it.T_tiles; ++t, ++gt) {
         // the tile's block of the workspace: D / 4 runs of (128 queries x 4 columns), contiguous
         float *dst = (it.mode == 2 ? fp.dq_acc2 : fp.dq_acc) +
@@ -827,28 +846,17 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       ok = __all_sync(0xffffffffu, w >= 0);
       if (!ok || w >= end_id) break;
       const FusedItem it = decode(w);
-      const int n0 = it.n0, key = n0 + row;
-      const bool key_ok = key < p.N;
-      auto direct = [&](void *out, const Strides &so, uint32_t (&ov)[QC], float scale, bool add) {
-        if (!key_ok) return;
-        T *orow = row_ptr_mut<T>(out, so, it.b, it.hk, key) + col0;
+      const int n0 = it.n0;
+      // this thread's columns of a row of its share of dK or dV (rows of the last block past N, too)
+      auto store_share = [&](float *part, const uint32_t (&ov)[QC]) {
+        const int64_t Npad = (int64_t)p.num_blocks * BN;
+        uint4 *dst = reinterpret_cast<uint4 *>(
+            part + (((int64_t)it.chunk * p.B * p.Hk + (int64_t)it.b * p.Hk + it.hk) * Npad + n0 + row) * D + col0);
 #pragma unroll
-        for (int j = 0; j < QC / 8; ++j) {
-          if (add) {
-            const uint4 old = *reinterpret_cast<const uint4 *>(orow + j * 8);
-            const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
-#pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2) {
-              const float2 f = TcElem<T>::unpack(ow[e2]);
-              ov[8 * j + 2 * e2] = __float_as_uint(__uint_as_float(ov[8 * j + 2 * e2]) + f.x);
-              ov[8 * j + 2 * e2 + 1] = __float_as_uint(__uint_as_float(ov[8 * j + 2 * e2 + 1]) + f.y);
-            }
-          }
-          *reinterpret_cast<uint4 *>(orow + j * 8) = pack8(ov + 8 * j, scale);
-        }
+        for (int j = 0; j < QC / 4; ++j) dst[j] = make_uint4(ov[4 * j], ov[4 * j + 1], ov[4 * j + 2], ov[4 * j + 3]);
       };
-      int mt = it.mt_lo;   // query tile of the current tile
-      int h = it.hk * G;   // and its query head
+      int mt = it.mt0;     // query tile of the current tile
+      int h = it.h0;       // and its query head
 
       for (int t = 0; t < it.T_tiles; ++t, ++gt) {
         const int m0 = mt * BM;
@@ -996,8 +1004,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
       // dV is final once its last product has been committed, so it is converted and staged while dQ and dK of the last tile still run on the tensor
       // cores; dK follows after the last commit.  dV is staged in the shared memory of V and dK in
       // the P^T / dS^T tile (both dead by then) in the layout of an operand load, and the producer
-      // thread sends them off as bulk tensor stores, which also drop the rows past N.  A dV that is
-      // added to (the second launch of a piecewise backward) keeps per-thread global stores.
+      // thread sends them off as bulk tensor stores, which also drop the rows past N.  Shares of a key
+      // block go to the workspace from the registers, 128 bytes a thread and row (64 at head_dim 64).
       {
         uint32_t ov[QC];
         ok = mbar_wait(bar(FB_DV_DONE), real & 1, actx, 915);   // the last dV product
@@ -1006,11 +1014,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         tc_fence_after();
         if (it.last) {   // (a near walk that a far walk follows leaves dV in TMEM and V in place)
           load_cols(C::kColDV, ov);
-          if (!p.dv_accumulate) {
+          if (!SPLIT) {
             stage(C::kV, ov, DROP ? fp.drop.rp : 1.f);
             fence_proxy_async_smem();
           } else {
-            direct(p.dv, p.sdv, ov, 1.f, true);
+            store_share(fp.dv_part, ov);
           }
         }
         __syncwarp();
@@ -1020,8 +1028,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (!ok) break;
         tc_fence_after();
         load_cols(C::kColDK, ov);
-        stage(C::kPD, ov, p.sm_scale);
-        fence_proxy_async_smem();
+        if (!SPLIT) {
+          stage(C::kPD, ov, p.sm_scale);
+          fence_proxy_async_smem();
+        } else {
+          store_share(fp.dk_part, ov);
+        }
         // the accumulator columns are free for the next item once every warp has read them
         tc_fence_before();
         __syncwarp();
@@ -1037,6 +1049,41 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     tc_fence_after();
     tmem_dealloc(tmem, C::kTmemCols);
   }
+}
+
+// dk = sm_scale * the sum of the shares, dv = dv_scale * theirs, in the order of the shares, rounded once.  A thread owns 8
+// columns of a row; blockIdx.z: 0 dk, 1 dv.
+template <typename T, int D>
+__global__ void __launch_bounds__(256)
+    dkdv_combine_kernel(const FusedBwdParams fp, void *dk, Strides sdk, void *dv, Strides sdv, float dk_scale,
+                        float dv_scale, int d) {
+  const BwdTcParams &p = fp.base;
+  constexpr int kRows = 256 / (D / 8);
+  const int n = blockIdx.x * kRows + threadIdx.x / (D / 8), c = threadIdx.x % (D / 8) * 8;
+  if (n >= p.N || c >= d) return;
+  const int b = blockIdx.y / p.Hk, hk = blockIdx.y % p.Hk;
+  // shares without a tile have left nothing
+  const int n0 = n / 128 * 128;
+  const int mt_lo = p.causal ? max(0, n0 - (p.N - p.M)) / 128 : 0;
+  const int tiles = max(0, (p.M + 127) / 128 - mt_lo) * (p.H / p.Hk);
+  const float *part = blockIdx.z ? fp.dv_part : fp.dk_part;
+  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int i = 0; i < fp.split; ++i) {
+    if (split_begin(tiles, i, fp.split) == split_begin(tiles, i + 1, fp.split)) continue;
+    const float4 *src = reinterpret_cast<const float4 *>(
+        part + (((int64_t)i * p.B * p.Hk + blockIdx.y) * ((int64_t)p.num_blocks * 128) + n) * D + c);
+    const float4 x = src[0], y = src[1];
+    sum[0] += x.x, sum[1] += x.y, sum[2] += x.z, sum[3] += x.w;
+    sum[4] += y.x, sum[5] += y.y, sum[6] += y.z, sum[7] += y.w;
+  }
+  const float scale = blockIdx.z ? dv_scale : dk_scale;
+  uint4 v;
+  v.x = TcElem<T>::pack(sum[0] * scale, sum[1] * scale);
+  v.y = TcElem<T>::pack(sum[2] * scale, sum[3] * scale);
+  v.z = TcElem<T>::pack(sum[4] * scale, sum[5] * scale);
+  v.w = TcElem<T>::pack(sum[6] * scale, sum[7] * scale);
+  T *row = blockIdx.z ? row_ptr_mut<T>(dv, sdv, b, hk, n) : row_ptr_mut<T>(dk, sdk, b, hk, n);
+  *reinterpret_cast<uint4 *>(row + c) = v;
 }
 
 // dq = dq_acc * scale, converted to 16 bits.  Block = 32 queries x 8 warps; warp w converts the

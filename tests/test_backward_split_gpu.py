@@ -1,0 +1,44 @@
+"""Backward calls of a few kv heads with many query heads each: several CTAs share the walk of a key block and leave their
+shares of dK and dV in fp32.  Shares that begin inside a query head, empty ones, partial last blocks, dropout and padded
+head_dims, against the oracle and the pair of kernels; dk and dv stay bitwise reproducible."""
+import pytest
+import torch
+
+import flagattention_b200 as fa
+import oracle
+from flagattention_b200 import flash
+from helpers import assert_within_2x, make_qkv
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B,H,Hk,M,N,D,causal", [
+    (1, 8, 1, 1000, 1000, 128, True), (2, 16, 2, 700, 700, 64, True), (1, 24, 1, 300, 420, 128, True),
+    (1, 16, 1, 500, 333, 64, False), (1, 32, 2, 257, 129, 128, True), (1, 32, 1, 400, 400, 32, True)])
+def test_shared_walks(B, H, Hk, M, N, D, causal, dtype):
+    q, k, v, do = make_qkv(B, H, Hk, M, N, D, dtype, "cuda", seed=M + N)
+    for x in (q, k, v):
+        x.requires_grad_()
+    run = lambda: torch.autograd.grad(fa.flash_attention(q, k, v, causal), (q, k, v), do)
+    with flash.backward_mode("one_pass"):
+        got, again = run(), run()
+    assert torch.equal(got[1], again[1]) and torch.equal(got[2], again[2])
+    ref = torch.autograd.grad(oracle.flash_attention(q, k, v, causal, upcast=True), (q, k, v), do)
+    tor = torch.autograd.grad(oracle.flash_attention(q, k, v, causal, upcast=False), (q, k, v), do)
+    for name, x, r, t in zip(("dq", "dk", "dv"), got, ref, tor):
+        assert_within_2x(x, r, t, name)
+
+
+def test_shares_use_their_own_workspace_and_their_dropout():
+    from flagattention_b200 import _C
+    need = lambda Hk: _C.call("fa_flash_bwd_workspace_bytes")(_C.pack_shape(torch.float16, 1, 16, Hk, 1000, 1000, 64, True, 0.1))
+    plain = 16 * 1024 * 64 * 4 + 16 + 16 * 1000 * 4
+    assert need(16) == plain and (need(1) - plain) % (2 * 1024 * 64 * 4) == 0 and need(1) > plain
+    q, k, v, do = make_qkv(1, 16, 1, 1000, 1000, 64, torch.float16, "cuda", seed=3)
+    o, lse = flash._forward(q, k, v, True, 0.125, 0.25, 11, 7)
+    got = flash._backward(q, k, v, o, lse, do, True, 0.125, None, 0.25, 11, 7)
+    with flash.backward_mode("two_kernel"):
+        want = flash._backward(q, k, v, o, lse, do, True, 0.125, None, 0.25, 11, 7)
+    for a, b in zip(got, want):   # both round P, dS and the result to 16 bits
+        assert (a.float() - b.float()).norm() <= 4 * 2 ** -11 * b.float().norm()
