@@ -111,10 +111,10 @@ inline void keep_bits_in(DropoutRule &r, const fa_flash_shape *s, void *bits) {
 
 // Keep bits of the elements whose counters are ctr + at(0), ctr + at(1), .. ctr + at(31) (bit i: the i-th), none
 // larger than `most`.
-// What bounds a kernel with dropout is this: Philox costs 10 multiplications an element and only its
-// first output word is used.  While the counters share their upper 32 bits (all but one in 2^32 / most calls) one product of round 2 depends on nothing else and is taken out of the loop; words of
-// rounds 4 to 6 that do not reach the first output are not computed: 9 multiplications and 9 three-input
-// xors an element.
+// What bounds a kernel with dropout is this: Philox costs 10 multiplications an element and only its first output word
+// is used.  While the counters share their upper 32 bits (all but one in 2^32 / most calls) one product of round 2
+// depends on nothing else and is taken out of the loop; words of rounds 4 to 6 that do not reach the first output are
+// not computed: 9 multiplications and 9 three-input xors an element.
 template <typename At>
 __device__ __forceinline__ uint32_t dropout_keep_bits32(const DropoutRule &r, uint64_t ctr, uint64_t most, At at) {
   constexpr uint32_t A = 0xD2511F53u, B = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;

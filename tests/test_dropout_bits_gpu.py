@@ -45,11 +45,15 @@ def test_where_none_are_kept():
 
 def test_backward_kernels_chosen_later():
     """The mode in force when the gradients are asked for decides, whatever the forward kept."""
-    q, k, v, do = make_qkv(1, 8, 8, 400, 400, 64, torch.float16, "cuda", seed=9)
+    q, k, v, do = make_qkv(4, 16, 16, 768, 768, 64, torch.float16, "cuda", seed=9)   # 38 M elements: kept
     for x in (q, k, v):
         x.requires_grad_()
+    saved = []
     torch.cuda.manual_seed(5)
-    o = fa.flash_attention(q, k, v, True, dropout_p=0.2)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t) or t, lambda t: t):
+        o = fa.flash_attention(q, k, v, True, dropout_p=0.2)
+        fa.flash_attention(q[:, :, :256], k[:, :, :256], v[:, :, :256], True, dropout_p=0.2)   # 4 M: drawn again
+    assert len(saved) == 6 + 5
     one = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
     with flash.backward_mode("two_kernel"):
         two = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
