@@ -33,13 +33,15 @@
 // Element-wise order:         phase 1 (t) | phase 2 (t)
 //   phase 1: P^T = exp2(S^T * scale - L) -> TMEM     phase 2: dS^T = P^T * (dP^T - delta) -> PD
 //
-// What bounds it is the chain of an element-wise warp through a tile, not a unit (tensor pipe 35 % at
-// head_dim 64 and 56 % at 128, exponentials 28 and 23 %, issue 44 and 41 %): a wait costs such a warp 150 to
+// What bounds it is the chain of an element-wise warp through a tile, not a unit (before what follows: tensor pipe 35 %
+// at head_dim 64 and 56 % at 128, exponentials 28 and 23 %, issue 44 and 41 %): a wait costs such a warp 150 to
 // 300 clocks even where it is satisfied (cycle stamps), so it makes two a tile.  S_FULL is completed by
 // the product and by the statistics warp together, DP_FULL by the product, the statistics warp and (128) the
 // reduction warps, and since commits complete in issue order DP_FULL also says that dV(t-1) and dK have read
 // the P^T and dS^T that the tile is about to overwrite.  Seven waits -> two, with S^T and dP^T apart at 64,
-// backward call of B=2 H=16 L=4096 not causal, fp16: 478 -> 449 us at 64, 675 -> 655 us at 128.
+// backward call of B=2 H=16 L=4096 not causal, fp16: 478 -> 449 us at 64, 675 -> 655 us at 128; with the steps noted
+// below 380 and 640 (B=4 H=32 L=4096 causal at 128: 1.36 -> 1.25 ms, tensor pipe 54 -> 61 %, the reductions' path to
+// L2 64 -> 69 %).
 #pragma once
 
 #include "flash_bwd_tc.cuh"
