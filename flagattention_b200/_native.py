@@ -14,6 +14,14 @@ _module = None
 _backward_mode = 0
 
 
+def _check_release(module):
+    """Raises for an extension built against another torch or Python: its inlined layouts would be silently wrong."""
+    from . import build
+    if module.built_for != build.host_tag():
+        raise RuntimeError("flagattn_host.so was built for %s, this is %s. Run `python -m flagattention_b200.build`."
+                           % (module.built_for, build.host_tag()))
+
+
 def load():
     """The extension module, raising if it has not been built."""
     global _module
@@ -26,6 +34,7 @@ def load():
                 loader = importlib.machinery.ExtensionFileLoader("flagattn_host", PATH)
                 module = importlib.util.module_from_spec(importlib.util.spec_from_loader("flagattn_host", loader))
                 loader.exec_module(module)
+                _check_release(module)
                 module.set_backward_mode(_backward_mode)
                 _module = module
     return _module

@@ -20,6 +20,7 @@ OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libflagattn_b200.so")
 HOST_SRC = os.path.join(CSRC, "host", "ops.cpp")
 HOST_PATH = os.path.join(LIB_DIR, "flagattn_host.so")
+HOST_STAMP = os.path.join(OBJ_DIR, "flagattn_host.command")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -27,6 +28,10 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC",
     "-I", INCLUDE, "-I", CSRC,
 ]
+
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared"]
+HOST_LIBS = ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-lflagattn_b200",
+             "-Wl,-rpath,$ORIGIN"]
 
 
 def _nvcc():
@@ -100,28 +105,52 @@ def build(force=False, verbose=False):
     return LIB_PATH
 
 
-def _build_host(force, verbose):
-    """The operators' host side (csrc/host/ops.cpp), a Python extension on torch's C++ interface and the library."""
+def host_tag():
+    """What a build of the host extension is good for: it inlines torch's C++ headers, whose layouts hold for one release
+    and one way of compiling only, and Python's own interface."""
     import sysconfig
 
     import torch
-    header = os.path.join(INCLUDE, "flagattn_b200.h")
-    if not force and os.path.exists(HOST_PATH) and \
-            os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(HOST_SRC), os.path.getmtime(header)):
+    return "torch %s, %s, cxx11 abi %d" % (torch.__version__, sysconfig.get_config_var("SOABI"),
+                                           torch._C._GLIBCXX_USE_CXX11_ABI)
+
+
+def _host_stamp():
+    """What the extension on disk has to have been made for and with (no paths: a built tree may be moved)."""
+    return host_tag() + "\n" + " ".join(HOST_FLAGS + HOST_LIBS)
+
+
+def _host_current(header):
+    if not os.path.exists(HOST_PATH) or not os.path.exists(HOST_STAMP):
+        return False
+    with open(HOST_STAMP) as f:
+        if f.read() != _host_stamp():
+            return False
+    return os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(HOST_SRC), os.path.getmtime(header))
+
+
+def _build_host(force, verbose):
+    """The operators' host side (csrc/host/ops.cpp), a Python extension on torch's C++ interface and the library."""
+    if not force and _host_current(os.path.join(INCLUDE, "flagattn_b200.h")):
         return
+    import sysconfig
+
+    import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, "-I", INCLUDE,
-           "-isystem", os.path.join(root, "include"),
-           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           "-isystem", os.path.join(cuda, "include"), "-isystem", sysconfig.get_paths()["include"],
-           HOST_SRC, "-o", HOST_PATH, "-L", os.path.join(root, "lib"),
-           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
-           "-L", LIB_DIR, "-lflagattn_b200", "-Wl,-rpath,$ORIGIN"]
+    fresh = HOST_PATH + ".new"
+    cmd = (["g++"] + HOST_FLAGS
+           + ["-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI, '-DFA_HOST_TAG="%s"' % host_tag(), "-I", INCLUDE,
+              "-isystem", os.path.join(root, "include"),
+              "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+              "-isystem", os.path.join(cuda, "include"), "-isystem", sysconfig.get_paths()["include"],
+              HOST_SRC, "-o", fresh, "-L", os.path.join(root, "lib"), "-L", LIB_DIR] + HOST_LIBS)
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed for %s:\n%s\n%s" % (HOST_SRC, res.stdout, res.stderr))
+    os.replace(fresh, HOST_PATH)   # a process that has the old one loaded keeps it
+    with open(HOST_STAMP, "w") as f:
+        f.write(_host_stamp())
     if verbose:
         print("linked", HOST_PATH, flush=True)
 

@@ -597,4 +597,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "flagattn_host", nullptr, -1, metho
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_flagattn_host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit_flagattn_host(void) {
+  PyObject *m = PyModule_Create(&module);
+  // what build.host_tag() said when this was compiled; the loader compares
+  if (m && PyModule_AddStringConstant(m, "built_for", FA_HOST_TAG) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}
