@@ -98,9 +98,15 @@ def partition_workspace(rows, P, D, device):
     return ws, base, part_max, part_max + stats * 4
 
 
-@functools.lru_cache(maxsize=1024)
 def _plan(num_seqs, num_q_heads, num_kv_heads, kv_block_size, max_context_len, num_splits, num_sms):
     """(partition size, partitions of the workspace, sizing or None) of a call; partition size 0: one pass."""
+    # kept for plain numbers only: a tensor hashes by identity, and its value may change
+    plan = _kept_plan if type(num_splits) is int else _kept_plan.__wrapped__
+    return plan(num_seqs, num_q_heads, num_kv_heads, kv_block_size, max_context_len, num_splits, num_sms)
+
+
+@functools.lru_cache(maxsize=1024)
+def _kept_plan(num_seqs, num_q_heads, num_kv_heads, kv_block_size, max_context_len, num_splits, num_sms):
     free_choice = num_splits == 0
     num_splits, partition_size = plan_partitions(num_seqs, num_kv_heads, kv_block_size, max_context_len, num_splits,
                                                  num_sms)

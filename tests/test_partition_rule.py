@@ -55,6 +55,14 @@ def test_workspace_partitions(base, seqs, ctas, context):
         assert finest == base or seqs * ctas >= 2 * 148
 
 
+def test_a_split_count_that_changes_in_place_makes_another_plan():
+    plan = lambda n: paged._plan(2, 8, 8, 16, 5000, n, 148)
+    n = torch.tensor(4)
+    assert plan(n) == plan(4) == (2048, 3, None)
+    n.fill_(8)
+    assert plan(n) == plan(8) == (1024, 5, None)
+
+
 def _partitions(monkeypatch, lens, most, Hk, group, D=64, block=16):
     """Partitions each sequence was cut into: the slots of the NaN-filled workspace that the kernel wrote."""
     kept = []
