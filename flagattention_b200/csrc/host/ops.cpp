@@ -458,13 +458,13 @@ bool integer(PyObject *o, int64_t *out) {
   *out = PyLong_AsLongLongAndOverflow(o, &overflow);
   return overflow == 0;
 }
-// a float that a 32-bit one can hold (the Python form raises OverflowError for others), an int, or None for the default
+// a float, an int, or None for the default
 bool scale_of(PyObject *o, bool *is_default, double *out) {
   *is_default = o == Py_None;
   if (*is_default) return true;
   if (PyFloat_CheckExact(o)) {
     *out = PyFloat_AS_DOUBLE(o);
-    return std::isinf(*out) || !std::isinf((float)*out);
+    return true;
   }
   int64_t i;
   if (!integer(o, &i)) return false;
