@@ -7,6 +7,7 @@
 #include "flash_fwd_persist_tc.cuh"
 #include "tma_host.cuh"
 #include "../common.cuh"
+#include "../dense_host.cuh"
 
 namespace fa {
 int *device_status_word();
@@ -39,10 +40,13 @@ static int sm_count_fwd() {
   return v;
 }
 
-// CTAs that share the walk of a query tile (SPLIT): 1, 2, 4 or 8.  One CTA walks a 64-key tile in about 0.75 us and two
-// on an SM in 0.84 each, so an SM with a single CTA, or none, is idle for want of query tiles; combining costs about
-// five tiles.  Estimated in tiles, and taken where it saves a tenth; all CTAs have to be resident, except that two
-// may share a walk where the longest is about twice the mean load.  bf16, us at 1 / 2 / 4 / 8 CTAs a query tile:
+// CTAs that share the walk of a query tile (SPLIT): 1, 2, 4 or 8, and the estimated time in tiles.  One CTA walks a 64-key
+// tile in 0.62 us (0.66 at head_dim 128), so an SM with a single CTA, or none, is idle for want of query tiles.  Sharing
+// costs the set-up and the combining, 3.75 tiles (4.25).  The CTAs of a cluster take SMs of their own while there are
+// any: 74 clusters of 2, 33 of 4, 15 of 8.  Beyond that two share an SM, which costs a quarter of their walk and up to
+// 2.4 tiles (3.6: 64 KB of O a CTA; less where most walks are shorter), and beyond twice that (33 of 8) a cluster waits
+// for another.  Taken where it saves a tenth; two CTAs may also share a walk where the longest is about twice the mean
+// load.  us at 1 / 2 / 4 / 8 CTAs, bf16:
 //   H=32 Hk=8 M=512 N=7300 D=128 (128 query tiles of 107..115 key tiles)   83.4 / 62.2 / 70.6 / 86.6
 //   H=32 Hk=8 M=64 N=7300 D=128 (32 of 115)    82.1 / 47.7 / 28.4 / 25.4
 //   H=8 M=1024 N=16384 D=128 (64 of 256)       185 / 99 / 69 / 79
@@ -52,20 +56,36 @@ static int sm_count_fwd() {
 //   H=32 Hk=8 M=1024 N=4096 D=128 (256 of 50..64)  59.0 / 69.4 / 85.0 / 118
 //   H=4 L=8192 D=128 causal (256 of 2..128)    96.4 / 78.8 / 91.0 / 125
 //   H=12 L=4096 D=128 causal (384 of 2..64)    56.6 / 69.5 / 90.6 / 145
-static int key_split(const fa_flash_shape *s, int sms) {
+// and where clusters are too many to run at once or CTAs share SMs for short walks (1 / 2 / 4 / 8):
+//   H=8 Hk=1 L=1152 D=128 causal (72 of 2..18)     16.8 / 14.1 / 19.0
+//   H=3 B=2 L=1536 D=64 not causal (72 of 24)      19.0 / 14.3 / 20.3
+//   H=3 M=3072 N=3170 D=128 causal (72 of 4..50)   37.2 / 24.5 / 23.0
+//   H=3 L=1536 D=64 not causal (36 of 24)          19.2 / 13.9 / 13.0 / 16.6
+//   B=2 H=8 L=1115 D=128 not causal (144 of 18)    17.4 / 19.1
+struct KeySplit {
+  int ctas;
+  double tiles;
+};
+static KeySplit key_split(const fa_flash_shape *s, int sms) {
   const int64_t blocks = (s->M + 127) / 128, ctas = blocks * s->B * s->H;
-  if (sms <= 0 || ctas > 2ll * sms) return 1;
   const int64_t longest = (s->N + 63) / 64;
   // key tiles of the last query tile and, roughly, of the first
-  const int64_t shortest = s->causal ? std::max<int64_t>(0, (s->N - s->M + 128 + 63) / 64) : longest;
-  int best = 1;
-  double least = 0.9 * (double)longest * (ctas > sms ? 1.15 : 1.0);
-  for (int c = 2; c <= 8 && ctas * c <= 2ll * sms; c *= 2) {
-    const double tiles = (double)longest / c * (ctas * c > sms ? 1.15 : 1.0) + (c == 8 ? 7 : 5);
-    if (tiles < least) best = c, least = tiles;
+  const int64_t shortest = s->causal ? std::max<int64_t>(0, ((int64_t)s->N - s->M + 128 + 63) / 64) : longest;
+  const double mean = 0.5 * (double)(longest + std::min(shortest, longest)), pair = 1.0 + 0.25 * mean / (double)longest;
+  KeySplit best{1, (double)longest * (ctas > sms ? pair : 1.0)};
+  if (sms <= 0 || ctas > 2ll * sms) return best;
+  const bool wide = s->D == 128;
+  const int64_t alone[3] = {sms / 2, sms * 33 / 148, sms * 15 / 148};   // clusters of 2, 4 and 8 on SMs of their own
+  double least = 0.9 * best.tiles;
+  for (int i = 0, c = 2; c <= 8 && ctas * c <= 2ll * sms; ++i, c *= 2) {
+    const bool share = ctas > alone[i];
+    double tiles = (double)longest / c * (share ? pair : 1.0) + (wide ? 4.25 : 3.75) + (share ? (wide ? 3.6 : 2.4) * mean / (double)longest : 0.0);
+    if (c == 8 && ctas > alone[1]) break;                       // (two an SM: a cluster of 8 takes four SMs)
+    if (c < 8 && ctas > 2 * alone[i]) tiles += mean / c + 0.5;   // the last clusters follow others
+    if (tiles < least) best = KeySplit{c, tiles}, least = tiles;
   }
-  const double load = (double)ctas * 0.5 * (double)(longest + std::min(shortest, longest)) / (2.0 * sms);
-  if (best == 1 && longest >= 64 && load <= 0.55 * (double)longest) best = 2;
+  const double load = (double)ctas * mean / (2.0 * sms);
+  if (best.ctas == 1 && longest >= 64 && load <= 0.55 * (double)longest) best.ctas = 2;
   return best;
 }
 
@@ -97,7 +117,7 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal);
   const int64_t tiles = (int64_t)p.num_m_blocks * s->B * s->H;
-  p.split = DROP || one_cta_per_tile_forced() ? 1 : key_split(s, sm_count_fwd());
+  p.split = DROP || one_cta_per_tile_forced() ? 1 : key_split(s, sm_count_fwd()).ctas;
   if constexpr (!DROP) {
     if (p.split > 1) {
       auto kern = flash_fwd_tc_kernel<T, D, PW, DROP, PAD, true>;
@@ -282,5 +302,10 @@ int piecewise_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q1, const
 
 }  // namespace tc
 }  // namespace fa
+
+extern "C" int32_t fa_flash_key_split(const fa_flash_shape *s, int32_t num_sms) {
+  if (const int st = fa::validate_shape(s)) return st;
+  return s->dropout_p > 0.f ? 1 : fa::tc::key_split(s, num_sms).ctas;
+}
 
 extern "C" int32_t fa_set_kernel_family(int32_t family) { return fa::tc::set_kernel_family(family); }

@@ -80,6 +80,9 @@ typedef struct fa_flash_shape {
  * (src/flag_attn/flash.py:64-87; kernel :325-489). */
 int fa_flash_fwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                  const fa_tensor4 *v, const fa_tensor4 *o, float *lse, void *stream);
+/* CTAs (1, 2, 4 or 8) among which the tcgen05 forward shares the walk of a query tile on a GPU of num_sms SMs;
+ * host-only, no CUDA call. */
+int32_t fa_flash_key_split(const fa_flash_shape *s, int32_t num_sms);
 
 /* Split-KV forward for small M.  Stage 1 writes, per split, a normalised
  * fp32 partial output (B,H,S,M,D) and its fp32 log-normaliser (B,H,S,M);

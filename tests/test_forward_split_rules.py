@@ -1,0 +1,23 @@
+"""The rule that has a cluster of CTAs share the walk of a query tile, at calls whose forms were measured; no GPU needed."""
+import pytest
+import torch
+
+from flagattention_b200 import _C
+
+
+def _split(B, H, M, N, D, causal, dropout=0.0):
+    return _C.call("fa_flash_key_split")(_C.pack_shape(torch.float16, B, H, H, M, N, D, causal, 0.1, dropout), 148)
+
+
+@pytest.mark.parametrize("B,H,M,N,D,causal,best", [
+    # more clusters than run at once, or two CTAs of them an SM: slower than fewer CTAs a tile, or than one
+    (1, 8, 1152, 1152, 128, True, 2), (1, 12, 672, 672, 64, True, 2), (2, 3, 1536, 1536, 64, False, 2),
+    (1, 3, 1536, 1536, 64, False, 4), (2, 3, 668, 1729, 64, False, 4), (2, 8, 1115, 1115, 128, False, 1),
+    (1, 8, 1159, 1159, 128, False, 1), (1, 8, 1195, 1195, 128, True, 2), (1, 24, 254, 549, 128, True, 1),
+    # what the rule gained from
+    (1, 32, 512, 7300, 128, True, 2), (1, 32, 64, 7300, 128, True, 8), (1, 8, 1024, 16384, 128, True, 4),
+    (1, 4, 1024, 1024, 128, True, 4), (1, 4, 512, 512, 64, True, 4), (2, 4, 256, 256, 64, True, 1),
+    (1, 32, 1024, 4096, 128, True, 1), (1, 4, 8192, 8192, 128, True, 2), (1, 12, 4096, 4096, 128, True, 1),
+    (1, 3, 3072, 3170, 128, True, 4), (1, 16, 1052, 1052, 64, True, 2)])
+def test_walks_are_shared_where_it_was_faster(built_lib, B, H, M, N, D, causal, best):
+    assert _split(B, H, M, N, D, causal) == best
