@@ -3,9 +3,9 @@
 // 27 us of it for 8 us of kernels, a training step 150 us for 22), most of that in Python's autograd.Function, argument
 // packing and ctypes.
 //
-// Every function returns None for a call that it does not take: other dtypes, devices, layouts that need a copy,
-// options, transforms (functorch, forward mode, tracing, dispatch modes), and everything that is an error.  The caller
-// then goes through the Python form of the same operator, which words the errors and holds the general path.
+// Every function returns None for a call that it does not take: other dtypes, devices, options, transforms (functorch,
+// forward mode, tracing, dispatch modes), and everything that is an error.  The caller then goes through the Python form
+// of the same operator, which words the errors and holds the general path.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -105,7 +105,26 @@ fa_flash_shape shape_of(const Tensor &q, const Tensor &k, bool causal, double sc
 }
 
 // ---- flash_attention -----------------------------------------------------------------------------------------------
-// `few_rows`: the form for calls that split their keys; undefined tensors where the split-KV kernels do it
+// the split-KV kernels: split_kv._splitkv_forward()
+std::pair<Tensor, Tensor> splitkv_forward(const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale,
+                                          int64_t splits) {
+  const int64_t B = q.size(0), H = q.size(1), M = q.size(2), D = q.size(3), N = k.size(2), tile = 64;
+  const int64_t per_split = ((N + tile - 1) / tile + splits - 1) / splits * tile;
+  splits = (N + per_split - 1) / per_split;   // (none empty)
+  const auto f32 = q.options().dtype(at::kFloat);
+  Tensor o = new_like(q), lse = at::empty({B, H, M}, f32);
+  Tensor o_part = at::empty({B, H, splits, M, D}, f32), l_part = at::empty({B, H, splits, M}, f32);
+  const fa_flash_shape s = shape_of(q, k, causal, scale);
+  const fa_tensor4 tq = tensor4(q), tk = tensor4(k), tv = tensor4(v), to = tensor4(o);
+  void *stream = stream_of(q);
+  check(fa_splitkv_fwd(&s, &tq, &tk, &tv, (int32_t)splits, (int32_t)per_split, o_part.data_ptr<float>(),
+                       l_part.data_ptr<float>(), stream), "fa_splitkv_fwd");
+  check(fa_splitkv_combine(&s, (int32_t)splits, o_part.data_ptr<float>(), l_part.data_ptr<float>(), &to,
+                           lse.data_ptr<float>(), stream), "fa_splitkv_combine");
+  return {o, lse};
+}
+
+// `few_rows`: the form for calls that split their keys; undefined tensors for a layout that it does not take
 std::pair<Tensor, Tensor> flash_forward(const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale,
                                         bool few_rows) {
   Tensor o = new_like(q), lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
@@ -152,14 +171,17 @@ variable_list flash_backward(const Tensor &q, const Tensor &k, const Tensor &v, 
 }
 
 struct FlashAttention : torch::autograd::Function<FlashAttention> {
-  // o and lse: computed by the caller, who may find that the call is not for this form
-  static Tensor forward(AutogradContext *ctx, const Tensor &q, const Tensor &k, const Tensor &v, bool causal, double scale,
-                        const std::pair<Tensor, Tensor> *computed) {
-    const auto &out = *computed;
-    ctx->save_for_backward({q, k, v, out.first, out.second});
+  // q, k, v (or their copies in the kernels' layout), o and lse: made by the caller, who may find that the call is not
+  // for this form
+  struct Computed {
+    Tensor q, k, v, o, lse;
+  };
+  static Tensor forward(AutogradContext *ctx, const Tensor &, const Tensor &, const Tensor &, bool causal, double scale,
+                        const Computed *c) {
+    ctx->save_for_backward({c->q, c->k, c->v, c->o, c->lse});
     ctx->saved_data["causal"] = causal;
     ctx->saved_data["scale"] = scale;
-    return out.first;
+    return c->o;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const auto t = ctx->get_saved_variables();
@@ -176,37 +198,44 @@ int64_t coarsen_partition(int64_t size, int64_t pairs, int64_t context, int64_t 
   return size;
 }
 
-// flash._decode_covered() for one query a head, and what _decode_forward() passes on without a copy
-bool decode_covered(const Tensor &q, const Tensor &k, const Tensor &v) {
-  if (k.size(2) % 16 != 0 || q.size(1) / k.size(1) > 64) return false;
+// flash._decode_covered()
+bool decode_covered(const Tensor &q, const Tensor &k, const Tensor &v, bool causal) {
+  const int64_t M = q.size(2), N = k.size(2);
+  if (M < 1 || N % 16 != 0 || N == 0 || q.size(1) / k.size(1) * M > 64) return false;
+  if (causal && M > 1 && N < M) return false;   // rows that see no key at all
   if (k.strides() != v.strides() || k.stride(3) != 1 || !aligned16(k) || !aligned16(v)) return false;
   const int64_t sl = k.stride(2);
-  if (sl <= 0 || sl % 8 || k.stride(1) % 8 || k.stride(0) % (16 * sl)) return false;
-  return q.stride(3) == 1 && q.stride(0) % 8 == 0 && q.stride(1) % 8 == 0;
+  return sl > 0 && sl % 8 == 0 && k.stride(1) % 8 == 0 && k.stride(0) % (16 * sl) == 0;
 }
 
 // flash._decode_forward()
-Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double scale) {
-  const int64_t B = q.size(0), H = q.size(1), D = q.size(3), Hk = k.size(1), N = k.size(2);
+Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double scale, bool causal) {
+  const int64_t B = q.size(0), H = q.size(1), M = q.size(2), D = q.size(3), Hk = k.size(1), N = k.size(2);
   const int64_t sb = k.stride(0), sl = k.stride(2);
   int64_t partition = coarsen_partition(256, B * Hk, N, sm_count(), 4096);
   if (N <= partition) partition = 0;
+  // the M queries of a head go in as M "query heads" of its kv head: rows one stride apart
+  Tensor rows;
+  int64_t row_stride = M == 1 ? q.stride(1) : q.stride(2), seq_stride = q.stride(0);
+  if ((M > 1 && H > 1 && q.stride(1) != M * q.stride(2)) || row_stride % 8 || seq_stride % 8)
+    rows = q.contiguous(), row_stride = D, seq_stride = H * M * D;
   Tensor o = new_like(q), ws;
   fa_paged_args a{};
   dtype_code(q, &a.dtype);
-  a.num_seqs = (int32_t)B, a.num_q_heads = (int32_t)H, a.num_kv_heads = (int32_t)Hk, a.head_size = (int32_t)D;
+  a.num_seqs = (int32_t)B, a.num_q_heads = (int32_t)(H * M), a.num_kv_heads = (int32_t)Hk, a.head_size = (int32_t)D;
   a.block_size = 16, a.max_context_len = (int32_t)N, a.block_table_is_i64 = FA_BLOCK_TABLE_IN_PLACE;
   a.partition_size = (int32_t)partition, a.attn_scale = (float)scale;
-  a.query = q.data_ptr(), a.q_stride_s = q.stride(0), a.q_stride_h = q.stride(1);
+  a.query = (rows.defined() ? rows : q).data_ptr(), a.q_stride_s = seq_stride, a.q_stride_h = row_stride;
   a.key_cache = k.data_ptr(), a.value_cache = v.data_ptr();
   a.kv_stride_b = 16 * sl, a.kv_stride_h = Hk > 1 ? k.stride(1) : 0, a.kv_stride_t = sl;
   a.bt_stride_s = sb / (16 * sl);
-  a.out = o.data_ptr(), a.o_stride_s = H * D, a.o_stride_h = D;
+  a.out = o.data_ptr(), a.o_stride_s = H * M * D, a.o_stride_h = D;
+  a.causal_rows = causal && M > 1 ? (int32_t)M : 0;
   if (partition) {
-    const int64_t rows = B * H, P = (N + partition - 1) / partition, stats = (rows * P + 63) / 64 * 64;
-    ws = at::empty({rows * P * D + 2 * stats}, q.options().dtype(at::kFloat));
+    const int64_t n = B * H * M, P = (N + partition - 1) / partition, stats = (n * P + 63) / 64 * 64;
+    ws = at::empty({n * P * D + 2 * stats}, q.options().dtype(at::kFloat));
     a.part_out = ws.data_ptr<float>();
-    a.part_max = a.part_out + rows * P * D;
+    a.part_max = a.part_out + n * P * D;
     a.part_sum = a.part_max + stats;
   }
   void *stream = stream_of(q);
@@ -217,29 +246,45 @@ Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double 
 
 bool head_dim_built(int64_t D) { return D == 16 || D == 32 || D == 64 || D == 128; }
 
-// o, or an undefined tensor
-Tensor flash(const Tensor &q, const Tensor &k, const Tensor &v, bool causal, bool default_scale, double scale) {
-  if (!q.is_cuda() || !usual_surroundings()) return {};
+// o, or an undefined tensor.  `rest`: the calls that the usual form leaves, since their views need a copy or their keys
+// are for the split-KV kernels.  (Refused calls pay for both forms: a view or a split call took 58 us where the Python
+// form alone takes 38 and this one 12.)
+Tensor flash(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, bool causal, bool default_scale, double scale,
+             bool rest) {
+  if (!q_in.is_cuda() || !usual_surroundings()) return {};
   const int device = c10::cuda::current_device();
-  if (!plain(q, device) || !plain(k, device) || !plain(v, device)) return {};
-  if (q.dim() != 4 || k.dim() != 4 || k.sizes() != v.sizes() || !fits(q) || !fits(k)) return {};
+  if (!plain(q_in, device) || !plain(k_in, device) || !plain(v_in, device)) return {};
+  if (q_in.dim() != 4 || k_in.dim() != 4 || k_in.sizes() != v_in.sizes() || !fits(q_in) || !fits(k_in)) return {};
   int32_t code;
-  if (!dtype_code(q, &code) || q.scalar_type() != k.scalar_type() || q.scalar_type() != v.scalar_type()) return {};
-  const int64_t B = q.size(0), H = q.size(1), M = q.size(2), D = q.size(3), Hk = k.size(1), N = k.size(2);
-  if (!head_dim_built(D) || k.size(3) != D || k.size(0) != B || H % Hk != 0) return {};
-  if (!kernel_ready(q) || !kernel_ready(k) || !kernel_ready(v)) return {};
+  if (!dtype_code(q_in, &code) || q_in.scalar_type() != k_in.scalar_type() || q_in.scalar_type() != v_in.scalar_type())
+    return {};
+  const int64_t B = q_in.size(0), H = q_in.size(1), M = q_in.size(2), D = q_in.size(3), Hk = k_in.size(1), N = k_in.size(2);
+  if (!head_dim_built(D) || k_in.size(3) != D || k_in.size(0) != B || H % Hk != 0) return {};
+  Tensor copies[3];
+  const bool copy = !kernel_ready(q_in) || !kernel_ready(k_in) || !kernel_ready(v_in);
+  if (copy) {
+    if (!rest) return {};
+    at::AutoGradMode no_graph(false);
+    copies[0] = ready(q_in), copies[1] = ready(k_in), copies[2] = ready(v_in);
+    for (const Tensor &t : copies)
+      if (!kernel_ready(t)) return {};
+  }
+  const Tensor &q = copy ? copies[0] : q_in, &k = copy ? copies[1] : k_in, &v = copy ? copies[2] : v_in;
   if (default_scale) scale = 1.0 / std::sqrt((double)D);
-  const bool grads = q.requires_grad() || k.requires_grad() || v.requires_grad();
-  const bool split = fa_num_splits_heuristic((int32_t)B, (int32_t)H, (int32_t)M, (int32_t)N, 16, 128, sm_count(), 128) > 1;
-  if (M <= 16 && !grads && (M == 1 || split))   // (several queries a head: the Python form)
-    return M == 1 && decode_covered(q, k, v) ? decode_forward(q, k, v, scale) : Tensor();
+  const bool grads = q_in.requires_grad() || k_in.requires_grad() || v_in.requires_grad();
+  const int64_t splits =
+      fa_num_splits_heuristic((int32_t)B, (int32_t)H, (int32_t)M, (int32_t)N, 16, 128, sm_count(), 128);
+  if (M <= 16 && !grads && (M == 1 || splits > 1) && decode_covered(q, k, v, causal))
+    return decode_forward(q, k, v, scale, causal);
   std::pair<Tensor, Tensor> out;
   {
     at::AutoGradMode no_graph(false);
-    out = flash_forward(q, k, v, causal, scale, split);
+    if (splits <= 1 || M >= 32) out = flash_forward(q, k, v, causal, scale, splits > 1);
+    if (!out.first.defined() && rest) out = splitkv_forward(q, k, v, causal, scale, splits);
   }
   if (!out.first.defined() || !grads || !at::GradMode::is_enabled()) return out.first;
-  return FlashAttention::apply(q, k, v, causal, scale, &out);
+  const FlashAttention::Computed c{q, k, v, out.first, out.second};
+  return FlashAttention::apply(q_in, k_in, v_in, causal, scale, &c);
 }
 
 // ---- piecewise_attention -------------------------------------------------------------------------------------------
@@ -255,10 +300,11 @@ std::pair<Tensor, Tensor> piecewise_forward(const Tensor &q1, const Tensor &k1, 
 }
 
 struct PiecewiseAttention : torch::autograd::Function<PiecewiseAttention> {
-  static Tensor forward(AutogradContext *ctx, const Tensor &q1, const Tensor &k1, const Tensor &q2, const Tensor &k2,
-                        const Tensor &v, int64_t w, bool causal, double scale) {
-    auto out = piecewise_forward(q1, k1, q2, k2, v, w, causal, scale);
-    ctx->save_for_backward({q1, k1, q2, k2, v, out.first, out.second});
+  // x: q1, k1, q2, k2, v, or their copies in the kernels' layout
+  static Tensor forward(AutogradContext *ctx, const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &,
+                        int64_t w, bool causal, double scale, const Tensor *x) {
+    auto out = piecewise_forward(x[0], x[1], x[2], x[3], x[4], w, causal, scale);
+    ctx->save_for_backward({x[0], x[1], x[2], x[3], x[4], out.first, out.second});
     ctx->saved_data["w"] = w;
     ctx->saved_data["causal"] = causal;
     ctx->saved_data["scale"] = scale;
@@ -280,7 +326,7 @@ struct PiecewiseAttention : torch::autograd::Function<PiecewiseAttention> {
     void *stream = stream_of(q1);
     const float *l = lse.data_ptr<float>();
     float *d = delta.data_ptr<float>();
-    const variable_list out{dq1, dk1, dq2, dk2, dv, Tensor(), Tensor(), Tensor()};
+    const variable_list out{dq1, dk1, dq2, dk2, dv, Tensor(), Tensor(), Tensor(), Tensor()};
     check(fa_flash_bwd_delta(&s, &to, &tdo, d, stream), "fa_flash_bwd_delta");
     if (one_pass()) {
       const int64_t bytes = fa_piecewise_bwd_fused_workspace_bytes(&s);
@@ -308,7 +354,7 @@ Tensor piecewise(const Tensor &q1, const Tensor &k1, const Tensor &q2, const Ten
   int32_t code;
   bool grads = false;
   for (const Tensor *t : {&q1, &k1, &q2, &k2, &v}) {
-    if (!plain(*t, device) || !kernel_ready(*t) || !fits(*t) || t->scalar_type() != q1.scalar_type()) return {};
+    if (!plain(*t, device) || t->dim() != 4 || !fits(*t) || t->scalar_type() != q1.scalar_type()) return {};
     grads = grads || t->requires_grad();
   }
   if (!dtype_code(q1, &code) || w < INT_MIN || w > INT_MAX) return {};
@@ -316,8 +362,17 @@ Tensor piecewise(const Tensor &q1, const Tensor &k1, const Tensor &q2, const Ten
   if (!head_dim_built(q1.size(3)) || k1.size(3) != q1.size(3) || k1.size(1) != q1.size(1) || k1.size(0) != q1.size(0))
     return {};
   if (default_scale) scale = 1.0 / std::sqrt((double)q1.size(3));
-  if (!grads || !at::GradMode::is_enabled()) return piecewise_forward(q1, k1, q2, k2, v, w, causal, scale).first;
-  return PiecewiseAttention::apply(q1, k1, q2, k2, v, w, causal, scale);
+  Tensor x[5];
+  {
+    at::AutoGradMode no_graph(false);
+    int i = 0;
+    for (const Tensor *t : {&q1, &k1, &q2, &k2, &v}) {
+      x[i] = ready(*t);
+      if (!kernel_ready(x[i++])) return {};
+    }
+  }
+  if (!grads || !at::GradMode::is_enabled()) return piecewise_forward(x[0], x[1], x[2], x[3], x[4], w, causal, scale).first;
+  return PiecewiseAttention::apply(q1, k1, q2, k2, v, w, causal, scale, static_cast<const Tensor *>(x));
 }
 
 // ---- rotary_pair (no positions) ------------------------------------------------------------------------------------
@@ -380,6 +435,13 @@ bool caches_ready(const Tensor &kc, const Tensor &vc, const Tensor &like, int de
   return kc.stride(0) % 8 == 0 && kc.stride(1) % 8 == 0 && kc.stride(2) % 8 == 0;
 }
 
+// 32 or 64 bit integers
+bool integers(const Tensor &t) { return t.scalar_type() == at::kInt || t.scalar_type() == at::kLong; }
+// unit inner stride, 16-byte aligned rows
+bool rows_ready(const Tensor &t) {
+  return t.stride(2) == 1 && aligned16(t) && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0;
+}
+
 Tensor paged(const Tensor &query, const Tensor &kc, const Tensor &vc, const Tensor &lens, const Tensor &table,
              double scale, int64_t most, int64_t partition, const uintptr_t (&parts)[3], const int64_t (&sizing)[4]) {
   if (!query.is_cuda() || !usual_surroundings()) return {};
@@ -391,11 +453,14 @@ Tensor paged(const Tensor &query, const Tensor &kc, const Tensor &vc, const Tens
   const int64_t seqs = query.size(0), H = query.size(1), D = query.size(2), Hk = kc.size(1), block = kc.size(2);
   if (kc.size(3) != D || H % Hk != 0 || (H != Hk && block < 16)) return {};
   if (D != 16 && D != 32 && D != 64 && D != 128 && D != 256) return {};
-  if (query.stride(2) != 1 || !aligned16(query) || query.stride(0) % 8 || query.stride(1) % 8) return {};
-  if (!plain(lens, device) || lens.scalar_type() != at::kInt || !lens.is_contiguous()) return {};
-  if (!plain(table, device) || table.dim() != 2 || table.stride(1) != 1 ||
-      (table.scalar_type() != at::kInt && table.scalar_type() != at::kLong))
-    return {};
+  if (!plain(lens, device) || !integers(lens) || !plain(table, device) || table.dim() != 2 || !integers(table)) return {};
+  const bool table_ready = table.stride(1) == 1 || table.size(1) <= 1;
+  if (!rows_ready(query) || lens.scalar_type() != at::kInt || !lens.is_contiguous() || !table_ready) {
+    if (!rows_ready(query) && query.is_contiguous()) return {};   // off the alignment
+    at::AutoGradMode no_graph(false);
+    return paged(rows_ready(query) ? query : query.contiguous(), kc, vc, lens.to(at::kInt).contiguous(),
+                 table_ready ? table : table.contiguous(), scale, most, partition, parts, sizing);
+  }
   if (most > INT_MAX || (partition && (partition < block || partition % block || partition % 16))) return {};
   Tensor out = new_like(query);
   fa_paged_args a{};
@@ -429,11 +494,15 @@ bool append(const Tensor &key, const Tensor &value, const Tensor &kc, const Tens
   if (!plain(key, device) || !plain(value, device) || key.dim() != 3 || !fits(key) ||
       !dtype_code(key, &code) || value.scalar_type() != key.scalar_type() || !caches_ready(kc, vc, key, device))
     return false;
-  if (value.sizes() != key.sizes() || value.strides() != key.strides() || key.stride(2) != 1 || !aligned16(key) ||
-      !aligned16(value) || key.stride(0) % 8 || key.stride(1) % 8 || kc.size(1) != key.size(1) || kc.size(3) != key.size(2))
-    return false;
-  if (!plain(slots, device) || slots.scalar_type() != at::kLong || !slots.is_contiguous() || slots.numel() != key.size(0))
-    return false;
+  if (value.sizes() != key.sizes() || kc.size(1) != key.size(1) || kc.size(3) != key.size(2)) return false;
+  if (!plain(slots, device) || !integers(slots) || slots.numel() != key.size(0)) return false;
+  if (slots.scalar_type() != at::kLong || !slots.is_contiguous())
+    return append(key, value, kc, vc, slots.to(at::kLong).contiguous());
+  if (value.strides() != key.strides() || !rows_ready(key) || !rows_ready(value)) {
+    if (key.is_contiguous() && value.is_contiguous()) return false;   // off the alignment
+    at::AutoGradMode no_graph(false);
+    return append(key.contiguous(), value.contiguous(), kc, vc, slots);
+  }
   check(fa_paged_cache_append(code, (int32_t)key.size(0), (int32_t)key.size(1), (int32_t)key.size(2), (int32_t)kc.size(2),
                               key.data_ptr(), value.data_ptr(), key.stride(0), key.stride(1), kc.data_ptr(),
                               vc.data_ptr(), kc.stride(0), kc.stride(1), kc.stride(2), slots.data_ptr<int64_t>(),
@@ -481,6 +550,7 @@ PyObject *wrap_or_none(const Tensor &t) {
   return THPVariable_Wrap(t);
 }
 
+template <bool REST>
 PyObject *py_flash(PyObject *, PyObject *const *args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const Tensor *t[3];
@@ -490,7 +560,7 @@ PyObject *py_flash(PyObject *, PyObject *const *args, Py_ssize_t n) {
   Tensor o;
   {
     pybind11::gil_scoped_release release;
-    o = flash(*t[0], *t[1], *t[2], causal, is_default, scale);
+    o = flash(*t[0], *t[1], *t[2], causal, is_default, scale, REST);
   }
   return wrap_or_none(o);
   END_HANDLE_TH_ERRORS
@@ -584,13 +654,34 @@ PyObject *py_coarsen(PyObject *, PyObject *const *args, Py_ssize_t n) {
   return PyLong_FromLongLong(coarsen_partition(x[0], x[1], x[2], x[3], x[4]));
 }
 
+// (tensor): whether the kernels take it without a copy; (q, k, v, causal): the decode rule.  For comparison with the
+// Python form of the rules, on any device.
+PyObject *py_kernel_ready(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Tensor *t[1];
+  if (n != 1 || !tensors(args, 1, t)) Py_RETURN_NONE;
+  return PyBool_FromLong(kernel_ready(*t[0]));
+  END_HANDLE_TH_ERRORS
+}
+PyObject *py_decode_covered(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const Tensor *t[3];
+  bool causal;
+  if (n != 4 || !tensors(args, 3, t) || !truth(args[3], &causal)) Py_RETURN_NONE;
+  return PyBool_FromLong(decode_covered(*t[0], *t[1], *t[2], causal));
+  END_HANDLE_TH_ERRORS
+}
+
 #define FAST(f) (PyCFunction)(void *)f, METH_FASTCALL, nullptr
-PyMethodDef methods[] = {{"flash", FAST(py_flash)},
+PyMethodDef methods[] = {{"flash", FAST(py_flash<false>)},
+                         {"flash_rest", FAST(py_flash<true>)},
                          {"piecewise", FAST(py_piecewise)},
                          {"rotary_pair", FAST(py_rotary_pair)},
                          {"paged", FAST(py_paged)},
                          {"append", FAST(py_append)},
                          {"coarsen_partition", FAST(py_coarsen)},
+                         {"kernel_ready", FAST(py_kernel_ready)},
+                         {"decode_covered", FAST(py_decode_covered)},
                          {"set_backward_mode", py_backward_mode, METH_O, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "flagattn_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -363,7 +363,10 @@ def attention(q, k, v, causal=False, sm_scale=None, dropout_p=0.0,
     """
     if (dropout_p == 0 and not (return_log_normalizer or return_total_attention or return_seed_offset)
             and _native.usable(q)):
-        o = _native.load().flash(q, k, v, causal, sm_scale)
+        native = _native.load()
+        o = native.flash(q, k, v, causal, sm_scale)
+        if o is None:   # a view that needs a copy, or keys for the split-KV kernels; else the form below
+            o = native.flash_rest(q, k, v, causal, sm_scale)
         if o is not None:
             return o
     return FlashAttention.apply(q, k, v, causal, sm_scale, dropout_p, return_log_normalizer,

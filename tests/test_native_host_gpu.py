@@ -48,6 +48,87 @@ def test_flash_calls(python_form, B, H, Hk, M, N, D, causal, layout):
         _same([call(causal)], [python_form(lambda: call(causal))])
 
 
+@pytest.mark.parametrize("B,H,Hk,M,N,D,causal", [
+    (1, 8, 8, 4, 1024, 64, True), (2, 8, 2, 16, 2048, 128, True), (2, 8, 2, 3, 512, 32, False), (1, 4, 4, 16, 16, 64, True),
+    (1, 8, 8, 1, 1000, 64, False), (1, 4, 1, 5, 1001, 128, True), (1, 8, 8, 20, 1024, 64, True), (1, 2, 1, 31, 700, 128, True),
+    (1, 4, 4, 40, 300, 32, True), (2, 2, 2, 20, 10, 64, True), (1, 4, 2, 60, 90, 16, False)])
+@pytest.mark.parametrize("layout", ["BHTD", "BTHD"])
+def test_few_queries_and_split_keys(python_form, B, H, Hk, M, N, D, causal, layout):
+    """Decoding of several queries, and calls that the split-KV kernels take."""
+    q, k, v, do = make_qkv(B, H, Hk, M, N, D, torch.bfloat16, "cuda", layout=layout, seed=N + M)
+    call = lambda: fa.flash_attention(q, k, v, causal)
+    assert any(f(q, k, v, causal, None) is not None for f in (_native.load().flash, _native.load().flash_rest))
+    _same([call()], [python_form(call)])
+    for x in (q, k, v):
+        x.requires_grad_()
+    with flash.backward_mode("two_kernel"):
+        grads = lambda: (lambda o: (o,) + torch.autograd.grad(o, (q, k, v), do))(call())
+        _same(grads(), python_form(grads))
+
+
+def test_views_that_need_a_copy(python_form):
+    gen = torch.Generator().manual_seed(4)
+    mk = lambda *s: torch.randn(s, generator=gen).half().cuda()
+    inner = [mk(2, 4, 64, 200).transpose(2, 3).requires_grad_() for _ in range(5)]
+    rows = [mk(2, 4, 200, 68)[..., :64].requires_grad_() for _ in range(5)]     # rows 136 bytes apart
+    off = [mk(2, 4, 200, 72)[..., 4:68].requires_grad_() for _ in range(5)]     # rows that start off 16 bytes
+    do = mk(2, 4, 200, 64)
+    n = _native.load()
+    for x in (inner, rows, off):
+        assert n.flash(*x[:3], True, None) is None and n.flash_rest(*x[:3], True, None) is not None
+        with flash.backward_mode("two_kernel"):
+            one = lambda: (lambda o: (o,) + torch.autograd.grad(o, x[:3], do))(fa.flash_attention(*x[:3], True))
+            _same(one(), python_form(one))
+            five = lambda: (lambda o: (o,) + torch.autograd.grad(o, x, do))(fa.piecewise_attention(*x, 60, True))
+            _same(five(), python_form(five))
+        assert n.piecewise(*x, 60, True, None) is not None
+        with torch.no_grad():
+            _same([fa.flash_attention(x[0][:, :, :1], x[1], x[2])], [python_form(lambda: fa.flash_attention(x[0][:, :, :1], x[1], x[2]))])
+    # the copies are saved, not the views: what becomes of these afterwards does not matter, in either form
+    o = fa.flash_attention(*inner[:3], True)
+    with torch.no_grad():
+        inner[0].zero_()
+    torch.autograd.grad(o, inner[:3], do)
+    # a contiguous tensor off the alignment is refused as before
+    bad = mk(2 * 4 * 200 * 64 + 4)[4:].view(2, 4, 200, 64)
+    assert n.flash_rest(bad, bad, bad, True, None) is None and n.piecewise(bad, bad, bad, bad, bad, 3, True, None) is None
+    with pytest.raises(RuntimeError):
+        fa.flash_attention(bad, bad, bad, True)
+
+
+def test_paged_operands_that_are_converted(python_form):
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *s: torch.randn(s, generator=gen, device="cuda", dtype=torch.float16)
+    kc, vc, key, value = rnd(400, 2, 16, 128), rnd(400, 2, 16, 128), rnd(3, 128, 2), rnd(3, 2, 128)
+    most = 700
+    table = torch.randint(0, 400, (3, 44), generator=gen, device="cuda", dtype=torch.int32)
+    lens = torch.tensor([most, 1, 250], device="cuda")
+    wide = torch.stack([lens.int(), lens.int()], 1)
+    n = _native.load()
+    for q, l, t in ((rnd(3, 8, 128), lens, table), (rnd(3, 128, 8).transpose(1, 2), lens.int(), table),
+                    (rnd(3, 8, 132)[..., 4:], wide[:, 0], table.t().contiguous().t()), (rnd(8, 3, 128).transpose(0, 1), lens, table.long())):
+        assert n.paged(q, kc, vc, l, t, 0.1, most, 0, 0, 0, 0, 0, 0, 0, 0) is not None
+        call = lambda: fa.paged_attention(q, kc, vc, l, t, 0.1, most)
+        _same([call()], [python_form(call)])
+    q, column = rnd(3, 8, 128), table[:, 3:4]   # (contiguous, whatever its last stride)
+    assert n.paged(q, kc, vc, lens.clamp(max=16), column.t().contiguous().t(), 0.1, 16, 0, 0, 0, 0, 0, 0, 0, 0) is not None
+    call = lambda: fa.paged_attention(q, kc, vc, lens.clamp(max=16), torch.stack([column[:, 0]] * 2, 1)[:, ::2], 0.1, 16)
+    _same([call()], [python_form(call)])
+    # neither form can help a contiguous operand off the alignment
+    assert n.append(rnd(3 * 256 + 4)[4:].view(3, 2, 128), value, kc, vc, torch.zeros(3, dtype=torch.int64, device="cuda")) is False
+    assert n.paged(rnd(3 * 1024 + 4)[4:].view(3, 8, 128), kc, vc, lens, table, 0.1, most, 0, 0, 0, 0, 0, 0, 0, 0) is None
+    slots = torch.tensor([5, -1, 400 * 16 - 1], device="cuda")
+
+    def write(k, v, s):
+        caches = kc.clone(), vc.clone()
+        paged.reshape_and_cache(k, v, *caches, s)
+        return caches
+    for k, v, s in ((key.transpose(1, 2), value, slots), (value, value + 1, slots.int()),
+                    (value, value, torch.stack([slots, slots], 1)[:, 0]), (rnd(3, 2, 132)[..., 4:], rnd(3, 2, 132)[..., 4:], slots)):
+        assert n.append(k, v, kc.clone(), vc.clone(), s)
+        _same(write(k, v, s), python_form(lambda: write(k, v, s)))
+
+
 def test_piecewise_and_rotary_calls(python_form):
     B, H, L, D = 2, 4, 300, 64
     gen = torch.Generator().manual_seed(1)
