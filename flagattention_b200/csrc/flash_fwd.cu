@@ -68,6 +68,7 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
                  const fa_tensor4 *v, const fa_tensor4 *o, float *lse, cudaStream_t stream, void *bits);
 int flash_fwd_fine_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
                       const fa_tensor4 *o, float *lse, cudaStream_t stream);
+double fine_microseconds(const fa_flash_shape *s, int sms);
 }
 
 }  // namespace fa
@@ -105,12 +106,27 @@ extern "C" int fa_flash_fwd_few_rows(const fa_flash_shape *s, const fa_tensor4 *
   if (int st = validate_shape(s)) return st;
   if (int st = validate_tensors({q, k, v, o})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
-  // A query tile here has 128 rows (and up to 8 CTAs), one of the split-KV kernels 16.  bf16, split-KV -> this, us:
-  // H=8 M=32 N=16384 D=128 43.7 -> 30.2, H=4 M=128 N=16384 79.8 -> 31.4, H=16 M=64 N=4096 43.6 -> 17.4, B=8 H=4 M=37
-  // N=346 D=64 8.0 -> 8.9, H=4 M=32 N=1000 9.1 -> 10.9 (and one launch and two allocations less).
-  if (s->M < 32) return FA_ERR_UNSUPPORTED;   // H=4 M=17 N=131072 157 -> 192
+  if (s->M < 32) return FA_ERR_UNSUPPORTED;   // H=4 M=17 N=131072 157 -> 192 us
   const int tc_status = tc::flash_fwd_fine_tc(s, q, k, v, o, lse, static_cast<cudaStream_t>(stream));
   return tc_status == 1 ? FA_ERR_UNSUPPORTED : tc_status;   // 1: nothing launched
+}
+
+// The split-KV kernels give a query tile of 64 rows to as many CTAs as the heuristic says, at 0.67 / 0.81 / 1.17 us a tile
+// of 64 keys (head_dim up to 32 / 64 / 128), and then combine; the cluster form has tiles of 128 rows, at most 8 CTAs each and
+// one launch.  The rule is the smaller of two fits (260 calls of 32..400 queries, each 5 % off).  bf16, split-KV -> cluster, us:
+//   taken    H=8 M=32 N=16384 D=128 43.7 -> 30.2, H=4 M=128 N=16384 79.8 -> 31.4, H=16 M=64 N=4096 43.6 -> 17.4,
+//            H=12 M=88 N=11400 109 -> 24.4, H=2 M=45 N=180 D=128 8.2 -> 6.9
+//   refused  H=3 M=37 N=424 D=64 6.9 -> 9.0, H=1 M=41 N=8859 D=64 14.8 -> 19.0, H=1 M=222 N=921 D=64 8.1 -> 9.7,
+//            H=4 M=46 N=9570 D=32 16.7 -> 19.2, B=8 H=4 M=37 N=346 D=64 8.0 -> 8.9, H=4 M=32 N=1000 9.1 -> 10.9
+extern "C" int32_t fa_flash_few_rows_pays(const fa_flash_shape *s, int32_t num_sms) {
+  if (validate_shape(s) != FA_OK || s->M < 32 || s->dropout_p > 0.f || num_sms <= 0) return 0;
+  const double cluster = tc::fine_microseconds(s, num_sms);
+  if (cluster <= 0.0) return 0;
+  const int splits = fa_num_splits_heuristic(s->B, s->H, s->M, s->N, 16, 128, num_sms, 128);
+  const int tiles = (s->N + SplitTile::BN - 1) / SplitTile::BN, per_split = (tiles + splits - 1) / splits;
+  const double used = (tiles + per_split - 1) / per_split;
+  const double fixed = s->D == 128 ? 5.65 : (s->D == 64 ? 4.9 : 4.65), a_tile = s->D == 128 ? 1.17 : (s->D == 64 ? 0.81 : 0.67);
+  return cluster < fixed + a_tile * per_split + 0.166 * used;
 }
 
 extern "C" int fa_splitkv_fwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,

@@ -112,15 +112,14 @@ std::pair<Tensor, Tensor> splitkv_forward(const Tensor &q, const Tensor &k, cons
   const int64_t per_split = ((N + tile - 1) / tile + splits - 1) / splits * tile;
   splits = (N + per_split - 1) / per_split;   // (none empty)
   const auto f32 = q.options().dtype(at::kFloat);
-  Tensor o = new_like(q), lse = at::empty({B, H, M}, f32);
-  Tensor o_part = at::empty({B, H, splits, M, D}, f32), l_part = at::empty({B, H, splits, M}, f32);
+  const int64_t rows = B * H * splits * M;
+  Tensor parts = at::empty({rows * (D + 1)}, f32), o = new_like(q), lse = at::empty({B, H, M}, f32);
+  float *o_part = parts.data_ptr<float>(), *l_part = o_part + rows * D;   // (B, H, splits, M, D) and (B, H, splits, M)
   const fa_flash_shape s = shape_of(q, k, causal, scale);
   const fa_tensor4 tq = tensor4(q), tk = tensor4(k), tv = tensor4(v), to = tensor4(o);
   void *stream = stream_of(q);
-  check(fa_splitkv_fwd(&s, &tq, &tk, &tv, (int32_t)splits, (int32_t)per_split, o_part.data_ptr<float>(),
-                       l_part.data_ptr<float>(), stream), "fa_splitkv_fwd");
-  check(fa_splitkv_combine(&s, (int32_t)splits, o_part.data_ptr<float>(), l_part.data_ptr<float>(), &to,
-                           lse.data_ptr<float>(), stream), "fa_splitkv_combine");
+  check(fa_splitkv_fwd(&s, &tq, &tk, &tv, (int32_t)splits, (int32_t)per_split, o_part, l_part, stream), "fa_splitkv_fwd");
+  check(fa_splitkv_combine(&s, (int32_t)splits, o_part, l_part, &to, lse.data_ptr<float>(), stream), "fa_splitkv_combine");
   return {o, lse};
 }
 
@@ -246,8 +245,8 @@ Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double 
 
 bool head_dim_built(int64_t D) { return D == 16 || D == 32 || D == 64 || D == 128; }
 
-// o, or an undefined tensor.  `rest`: the calls that the usual form leaves, since their views need a copy or their keys
-// are for the split-KV kernels.  (Refused calls pay for both forms: a view or a split call took 58 us where the Python
+// o, or an undefined tensor.  `rest`: the calls that the usual form leaves, since their views need a copy or their few
+// queries are for the split-KV kernels.  (Refused calls pay for both forms: a view or a split call took 58 us where the Python
 // form alone takes 38 and this one 12.)
 Tensor flash(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, bool causal, bool default_scale, double scale,
              bool rest) {
@@ -276,11 +275,16 @@ Tensor flash(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, bool ca
       fa_num_splits_heuristic((int32_t)B, (int32_t)H, (int32_t)M, (int32_t)N, 16, 128, sm_count(), 128);
   if (M <= 16 && !grads && (M == 1 || splits > 1) && decode_covered(q, k, v, causal))
     return decode_forward(q, k, v, scale, causal);
+  bool clusters = false;
+  if (splits > 1) {
+    const fa_flash_shape s = shape_of(q, k, causal, scale);
+    clusters = fa_flash_few_rows_pays(&s, sm_count());
+  }
   std::pair<Tensor, Tensor> out;
   {
     at::AutoGradMode no_graph(false);
-    if (splits <= 1 || M >= 32) out = flash_forward(q, k, v, causal, scale, splits > 1);
-    if (!out.first.defined() && rest) out = splitkv_forward(q, k, v, causal, scale, splits);
+    if (splits <= 1 || clusters) out = flash_forward(q, k, v, causal, scale, splits > 1);
+    if (!out.first.defined() && (rest || M >= 32)) out = splitkv_forward(q, k, v, causal, scale, splits);
   }
   if (!out.first.defined() || !grads || !at::GradMode::is_enabled()) return out.first;
   const FlashAttention::Computed c{q, k, v, out.first, out.second};

@@ -6,6 +6,7 @@ when any return_* flag is set), same AssertionErrors on bad shapes, autograd
 through q, k, v only.  The kernels run on the current CUDA stream of the
 inputs' device.
 """
+import functools
 import math
 
 import torch
@@ -101,8 +102,15 @@ def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0, keep=Fa
     return (o, L, None) if keep else (o, L)
 
 
+@functools.lru_cache(maxsize=1024)
+def _few_rows_pay(B, H, M, N, D, causal, num_sms):
+    """Whether a call that splits its keys is faster by clusters of CTAs than by the split-KV kernels."""
+    return bool(_C.call("fa_flash_few_rows_pays")(_C.pack_shape(torch.float16, B, H, H, M, N, D, causal, 1.0), num_sms))
+
+
 def _few_rows_forward(q, k, v, causal, sm_scale):
-    """(o, log-normaliser) of a call that splits its keys, by clusters of CTAs; None where the split-KV kernels do it."""
+    """(o, log-normaliser) of a call that splits its keys, by clusters of CTAs; None for what only the split-KV kernels
+    take."""
     B, H, M, D = q.shape
     N, Hk = k.shape[2], k.shape[1]
     o = torch.empty((B, H, M, D), dtype=q.dtype, device=q.device)
@@ -313,7 +321,9 @@ class FlashAttention(torch.autograd.Function):
             S = num_splits_herustic(B, H, M, N, cfg[0], cfg[1], _C.sm_count(q.device), 128)
             if S > 1:
                 assert not is_dropout, "Cannot apply dropout with splitkv."
-                o, L = _few_rows_forward(q, k, v, causal, sm_scale) or _splitkv_forward(q, k, v, causal, sm_scale, S)
+                pays = _few_rows_pay(B, H, M, N, D, bool(causal), _C.sm_count(q.device))
+                o, L = ((pays and _few_rows_forward(q, k, v, causal, sm_scale))
+                        or _splitkv_forward(q, k, v, causal, sm_scale, S))
             elif (is_dropout and B * H * M * N >= _KEEP_BITS_FROM and any(ctx.needs_input_grad[:3])
                   and use_one_pass_backward()):
                 o, L, bits = _forward(q, k, v, causal, sm_scale, dropout_p, seed, offset, True)

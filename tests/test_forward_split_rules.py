@@ -1,8 +1,9 @@
-"""The rule that has a cluster of CTAs share the walk of a query tile, at calls whose forms were measured; no GPU needed."""
+"""The rules that have a cluster of CTAs share the walk of a query tile, at calls whose forms were
+measured; no GPU needed."""
 import pytest
 import torch
 
-from flagattention_b200 import _C
+from flagattention_b200 import _C, flash
 
 
 def _split(B, H, M, N, D, causal, dropout=0.0):
@@ -21,3 +22,25 @@ def _split(B, H, M, N, D, causal, dropout=0.0):
     (1, 3, 3072, 3170, 128, True, 4), (1, 16, 1052, 1052, 64, True, 2)])
 def test_walks_are_shared_where_it_was_faster(built_lib, B, H, M, N, D, causal, best):
     assert _split(B, H, M, N, D, causal) == best
+
+
+@pytest.mark.parametrize("B,H,M,N,D,causal,pays", [
+    # split-KV kernels against clusters, us
+    (1, 3, 37, 424, 64, False, 0),      # 6.9, 9.0
+    (1, 1, 41, 8859, 64, True, 0),      # 14.8, 19.0
+    (8, 2, 91, 424, 64, True, 0),       # 7.4, 9.4
+    (1, 32, 33, 389, 64, True, 0),      # 7.4, 9.0
+    (1, 1, 222, 921, 64, True, 0),      # 8.1, 9.7
+    (2, 16, 44, 497, 32, True, 0),      # 6.7, 7.9
+    (1, 4, 46, 9570, 32, True, 0),      # 16.7, 19.2
+    (8, 4, 37, 346, 64, True, 0), (1, 4, 32, 1000, 128, True, 0),
+    (1, 4, 300, 300, 32, True, 0),      # fewer keys than the tcgen05 kernels take at head_dim 32
+    (1, 8, 31, 16384, 128, True, 0),
+    (1, 8, 32, 16384, 128, True, 1),    # 43.7, 30.2
+    (1, 4, 128, 16384, 128, True, 1),   # 79.8, 31.4
+    (1, 16, 64, 4096, 128, True, 1),    # 43.6, 17.4
+    (1, 12, 88, 11400, 128, True, 1),   # 109, 24.4
+    (1, 16, 57, 3500, 64, True, 1),     # 27.9, 14.1
+    (1, 1, 45, 180, 128, True, 1)])     # 8.2, 6.9
+def test_few_rows_go_to_the_faster_form(built_lib, B, H, M, N, D, causal, pays):
+    assert flash._few_rows_pay(B, H, M, N, D, causal, 148) == bool(pays)
