@@ -130,8 +130,11 @@ inline int cta_group_size(int64_t hot_bytes_per_pair, int npairs) {
 // B=2 H=32 M=1627 N=2855 142 -> 148 (94 MB), B=2 H=32 L=4096 278 -> 311 (134 MB); backward B=3 H=32 Hk=8 L=1867 381 -> 321 (360
 // blocks), H=32 Hk=8 L=8192 1871 -> 1383 (512), H=16 L=6144 493 -> 409 (768), B=2 H=32 Hk=16 L=4096 840 -> 762 (1024),
 // B=4 H=32 L=1024 197 -> 203 (1024, 128 pairs), H=24 L=8192 1099 -> 1079 (1536), B=2 H=32 L=4096 760 -> 845 (2048).
+inline bool one_group_in_l2(int64_t hot_bytes_per_pair, int npairs, bool causal) {
+  return causal && hot_bytes_per_pair * npairs <= 88ll << 20;
+}
 inline int forward_group_size(int64_t hot_bytes_per_pair, int npairs, bool causal) {
-  if (causal && hot_bytes_per_pair * npairs <= 88ll << 20) return npairs > 0 ? npairs : 1;
+  if (one_group_in_l2(hot_bytes_per_pair, npairs, causal)) return npairs > 0 ? npairs : 1;
   return cta_group_size(hot_bytes_per_pair, npairs);
 }
 inline int backward_group_size(int64_t hot_bytes_per_pair, int npairs, int64_t blocks, int sms, bool causal) {
