@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "flagattn_b200.h"
@@ -206,6 +207,19 @@ inline int ensure_dyn_smem(K kernel, int bytes, unsigned long long *done_mask) {
     *done_mask |= bit;
   }
   return FA_OK;
+}
+
+// SMs of the current device, 0 where there is none
+inline int sm_count_of_device() {
+  static std::atomic<int> n[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int v = n[dev].load(std::memory_order_relaxed);
+  if (!v) {
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n[dev].store(v, std::memory_order_relaxed);
+  }
+  return v;
 }
 
 #define FA_CHECK_LAUNCH()                                   \

@@ -387,19 +387,33 @@ __global__ void __launch_bounds__(PagedCfg<D>::kWarps * 32) paged_decode_kernel(
   }
 }
 
-// One CTA per (seq, query head): its 256 threads are 1024 / D groups of D / 4, a thread owning 4 output columns of every
-// (1024 / D)-th partition.  What bounds it is latency, two round trips to L2 (statistics, then rows): a CTA that went
+// One CTA per (seq, query head): its threads are 4 blockDim / D groups of D / 4, a thread owning 4 output columns of every
+// so many partitions.  What bounds it is latency, two round trips to L2 (statistics, then rows): a CTA that went
 // through the partitions one after another with the threads of one row took 13.4 us for 32 partitions of 32 rows (dense
 // decoding, B=2 H=16 N=131072, beside 299 us of decoding) and 8.9 us for 64 sequences of 32 heads up to 32768 tokens:
 // the first of these calls 317 -> 307 us.  It is launched while the decode kernel's last CTAs run (programmatic stream
 // serialization) and waits for that grid: 307 -> 305 us, H=16 N=512 7.9 -> 6.8 us, 4 sequences up to 1500 10.0 -> 8.4.
+//
+// Threads a row: up to 256 while all rows find room beside the decode kernel's CTAs, which still hold about half of every
+// SM (1024 threads); more rows with fewer threads run at once.  fp16, rows and us at 32 / 64 / 128 / 256 threads a row:
+//   128 sequences up to 1562 tokens, 16 heads over 2, D=128 (2048)   27.9 / 28.0 / 30.3 / 33.6
+//   64 up to 3029, 16 over 2, D=64 (1024)    26.7 / 26.7 / 27.0 / 29.7      64 up to 3125, D=128 24.4 / 23.9 / 23.9 / 26.1
+//   128 up to 1488, 8 over 1, D=256 (1024)     -  / 40.5 / 40.2 / 42.7      100 up to 2000, 8 over 1, D=128 (800)
+//   12 up to 13860, 32 over 8, D=128 (384)   75.6 / 74.8 / 73.8 / 74.1      19.5 / 19.2 / 19.5 / 20.0
+//   10 up to 19849, 32 over 8, D=128 (320)   89.3 / 85.5 / 83.8 / 83.1      1 up to 28326, 8 over 8, D=256 (8)
+//   7 up to 19563, 8 over 1, D=128 (56)      23.3 / 18.1 / 15.6 / 14.4        -  / 47.3 / 44.1 / 42.5
 constexpr int kReduceThreads = 256;
+static int reduce_threads(int64_t rows, int head_size, int sms) {
+  int threads = kReduceThreads;
+  while (threads > 32 && threads > head_size / 4 && rows * threads > 1024ll * sms) threads /= 2;
+  return threads;
+}
 template <typename T>
 __global__ void __launch_bounds__(kReduceThreads) paged_reduce_kernel(const fa_paged_args a, const Sizing z) {
   __shared__ float4 part_o[kReduceThreads];
   __shared__ float part_den[kReduceThreads];
   const int seq = blockIdx.x, qh = blockIdx.y;
-  const int D = a.head_size, cols = D / 4, groups = kReduceThreads / cols;
+  const int D = a.head_size, cols = D / 4, groups = blockDim.x / cols;
   const int g = threadIdx.x / cols, c4 = threadIdx.x % cols;
   const int P = (a.max_context_len + a.partition_size - 1) / a.partition_size;
   const int ctx = context_len(a, seq);
@@ -531,7 +545,8 @@ static int reduce(const fa_paged_args *a, const Sizing &z, cudaStream_t s) {
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid, cfg.blockDim = dim3(kReduceThreads), cfg.stream = s, cfg.attrs = &attr, cfg.numAttrs = 1;
+  cfg.gridDim = grid, cfg.stream = s, cfg.attrs = &attr, cfg.numAttrs = 1;
+  cfg.blockDim = dim3(reduce_threads((int64_t)a->num_seqs * a->num_q_heads, a->head_size, sm_count_of_device()));
   const cudaError_t st = a->dtype == FA_F16 ? cudaLaunchKernelEx(&cfg, paged_reduce_kernel<__half>, *a, z)
                                             : cudaLaunchKernelEx(&cfg, paged_reduce_kernel<__nv_bfloat16>, *a, z);
   if (st != cudaSuccess) return FA_ERR_LAUNCH;

@@ -28,18 +28,6 @@ int set_kernel_family(int family) {
   return g_kernel_family.exchange(family == 1 ? 1 : (family == 2 ? 2 : 0));
 }
 
-static int sm_count_fwd() {
-  static std::atomic<int> n[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  int v = n[dev].load(std::memory_order_relaxed);
-  if (!v) {
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    n[dev].store(v, std::memory_order_relaxed);
-  }
-  return v;
-}
-
 // CTAs that share the walk of a query tile (SPLIT): 1, 2, 4 or 8, and the estimated time in tiles.  One CTA walks a 64-key
 // tile in 0.62 us (0.66 at head_dim 128), so an SM with a single CTA, or none, is idle for want of query tiles.  Sharing
 // costs the set-up and the combining, 3.75 tiles (4.25).  The CTAs of a cluster take SMs of their own while there are
@@ -117,7 +105,7 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal);
   const int64_t tiles = (int64_t)p.num_m_blocks * s->B * s->H;
-  p.split = DROP || one_cta_per_tile_forced() ? 1 : key_split(s, sm_count_fwd()).ctas;
+  p.split = DROP || one_cta_per_tile_forced() ? 1 : key_split(s, sm_count_of_device()).ctas;
   if constexpr (!DROP) {
     if (p.split > 1) {
       auto kern = flash_fwd_tc_kernel<T, D, PW, DROP, PAD, true>;
@@ -197,7 +185,7 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
   p.group_size = forward_group_size((int64_t)s->N * D * 2 * 2 * s->Hk / s->H, s->B * s->H, s->causal);
   const int64_t items = (int64_t)p.num_m_blocks * s->B * s->H;
-  const int sms = sm_count_fwd();
+  const int sms = sm_count_of_device();
   fp.sched = fwd_sched_slot();
   if (items <= 0 || items > (1ll << 30) || sms <= 0 || !fp.sched) return 1;
   fp.num_items = (int)items;
@@ -265,7 +253,7 @@ int flash_fwd_tc(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 
   // in case the two walked in step, changed nothing).
   const bool short_walks = s->D <= 64 || s->N <= 1536;
   if (!one_cta_per_tile_forced() && short_walks &&
-      (int64_t)((s->M + 127) / 128) * s->B * s->H > 2 * (int64_t)sm_count_fwd()) {
+      (int64_t)((s->M + 127) / 128) * s->B * s->H > 2 * (int64_t)sm_count_of_device()) {
     int st;
     if (s->D < 64)
       st = s->dtype == FA_F16 ? launch_fwd_persist<__half, 64, true>(s, q, k, v, o, lse, stream)

@@ -20,6 +20,14 @@ def test_partitions_double_while_the_gpu_is_busy(start, pairs, context):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("seqs,Hk,group,hi,block", [(60, 1, 16, 1100, 16), (37, 2, 8, 1100, 16), (38, 2, 8, 1100, 16),
+                                                    (290, 1, 16, 1100, 16), (290, 1, 8, 1100, 16)])
+def test_rows_of_the_reduction(seqs, Hk, group, hi, block):
+    """Few and many rows: 256, 128, 64 and 32 threads reduce one."""
+    test_paged_against_one_pass(seqs, Hk, group, hi, block)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("seqs,Hk,group,hi,block", [(1, 1, 4, 40000, 16), (3, 4, 8, 32769, 32), (30, 8, 1, 4097, 16),
                                                     (80, 4, 4, 4096, 16), (2, 2, 1, 1025, 16)])
 def test_paged_against_one_pass(seqs, Hk, group, hi, block):
