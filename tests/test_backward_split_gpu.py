@@ -6,16 +6,55 @@ import torch
 
 import flagattention_b200 as fa
 import oracle
-from flagattention_b200 import flash
+from flagattention_b200 import _C, flash
 from helpers import assert_within_2x, make_qkv
 
 pytestmark = pytest.mark.gpu
 
+SHARED = [
+    (1, 8, 1, 1000, 1000, 128, True), (2, 16, 2, 700, 700, 64, True), (1, 24, 1, 300, 420, 128, True),
+    (1, 16, 1, 500, 333, 64, False), (1, 32, 2, 257, 129, 128, True), (1, 32, 1, 400, 400, 32, True)]
+
+
+def _workspace(B, H, Hk, M, N, D, causal):
+    """(bytes of the backward's workspace, CTAs that share a walk)"""
+    total = _C.call("fa_flash_bwd_workspace_bytes")(_C.pack_shape(torch.float16, B, H, Hk, M, N, D, causal, 0.1))
+    up, width = (lambda n: -(-n // 128) * 128), max(D, 64)
+    plain = B * H * up(M) * width * 4 + 16 + B * H * M * 4
+    return total, max(1, (total - plain) // (2 * B * Hk * up(N) * width * 4))
+
+
+@pytest.mark.parametrize("B,H,Hk,M,N,D,causal", SHARED)
+def test_these_walks_are_shared(B, H, Hk, M, N, D, causal):
+    assert _workspace(B, H, Hk, M, N, D, causal)[1] in (2, 4, 8)
+
+
+@pytest.mark.parametrize("B,H,Hk,M,N,D,split", [
+    (1, 4, 2, 4096, 4096, 128, 4),    # the last key block has 2 tiles: 2 of its 4 shares are empty
+    (1, 4, 1, 2100, 2100, 64, 8),
+    (1, 2, 1, 3000, 3333, 128, 4)])
+def test_shares_without_a_tile(B, H, Hk, M, N, D, split):
+    """They leave nothing behind, and what is in their memory reaches neither dk nor dv."""
+    bytes_, shares = _workspace(B, H, Hk, M, N, D, True)
+    blocks = [(-(-M // 128) - max(0, n0 - (N - M)) // 128) * (H // Hk) for n0 in range(0, N, 128)]
+    assert shares == split > min(blocks) > 0
+    q, k, v, do = make_qkv(B, H, Hk, M, N, D, torch.bfloat16, "cuda", seed=M)
+    for x in (q, k, v):
+        x.requires_grad_()
+    with flash.backward_mode("one_pass"):
+        o = fa.flash_attention(q, k, v, True)
+        torch.cuda.empty_cache()
+        junk = torch.full((bytes_,), 255, dtype=torch.uint8, device="cuda")   # NaN; the workspace comes from this memory
+        del junk
+        got = torch.autograd.grad(o, (q, k, v), do)
+    ref = torch.autograd.grad(oracle.flash_attention(q, k, v, True, upcast=True), (q, k, v), do)
+    tor = torch.autograd.grad(oracle.flash_attention(q, k, v, True, upcast=False), (q, k, v), do)
+    for name, x, r, t in zip(("dq", "dk", "dv"), got, ref, tor):
+        assert_within_2x(x, r, t, name)
+
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("B,H,Hk,M,N,D,causal", [
-    (1, 8, 1, 1000, 1000, 128, True), (2, 16, 2, 700, 700, 64, True), (1, 24, 1, 300, 420, 128, True),
-    (1, 16, 1, 500, 333, 64, False), (1, 32, 2, 257, 129, 128, True), (1, 32, 1, 400, 400, 32, True)])
+@pytest.mark.parametrize("B,H,Hk,M,N,D,causal", SHARED)
 def test_shared_walks(B, H, Hk, M, N, D, causal, dtype):
     q, k, v, do = make_qkv(B, H, Hk, M, N, D, dtype, "cuda", seed=M + N)
     for x in (q, k, v):
@@ -31,7 +70,6 @@ def test_shared_walks(B, H, Hk, M, N, D, causal, dtype):
 
 
 def test_shares_use_their_own_workspace_and_their_dropout():
-    from flagattention_b200 import _C
     need = lambda Hk: _C.call("fa_flash_bwd_workspace_bytes")(_C.pack_shape(torch.float16, 1, 16, Hk, 1000, 1000, 64, True, 0.1))
     plain = 16 * 1024 * 64 * 4 + 16 + 16 * 1000 * 4
     assert need(16) == plain and (need(1) - plain) % (2 * 1024 * 64 * 4) == 0 and need(1) > plain

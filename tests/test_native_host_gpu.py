@@ -267,3 +267,29 @@ def test_several_threads_and_streams():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not bad
+
+
+@pytest.mark.parametrize("B,H,Hk,L,D", [(2, 8, 8, 300, 64), (1, 16, 2, 500, 128)])   # the second: shared walks
+def test_gradients_from_several_threads_and_streams(B, H, Hk, L, D):
+    """Each call has its own workspace and work-item counter, and its backward runs on the stream of its forward."""
+    import threading
+    q, k, v, do = make_qkv(B, H, Hk, L, L, D, torch.float16, "cuda", seed=8)
+    for x in (q, k, v):
+        x.requires_grad_()
+    want = torch.autograd.grad(fa.flash_attention(q, k, v, True), (q, k, v), do)
+    torch.cuda.synchronize()
+    bad = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                got = torch.autograd.grad(fa.flash_attention(q, k, v, True), (q, k, v), do)
+                # dk, dv bitwise; dq is summed in any order: a rounding to 16 bits apart at most
+                if not (torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+                        and (got[0].float() - want[0].float()).abs().max() <= 2 ** -10 * want[0].float().abs().max()):
+                    bad.append(1)
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=work) for _ in range(3)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
