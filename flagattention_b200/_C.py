@@ -25,7 +25,7 @@ EXPORTED_SYMBOLS = (
     "fa_flash_bwd_dq", "fa_piecewise_fwd", "fa_piecewise_bwd_dkdv", "fa_piecewise_bwd_dq",
     "fa_paged_decode", "fa_paged_reduce", "fa_paged_workspace_bytes", "fa_paged_trace_blocks",
     "fa_paged_attention", "fa_paged_attention_noalloc", "fa_dropout_mask",
-    "fa_flash_bwd", "fa_flash_bwd_workspace_bytes", "fa_flash_keep_bits_bytes", "fa_flash_fwd_keep", "fa_flash_bwd_keep",
+    "fa_flash_bwd", "fa_flash_bwd_workspace_bytes", "fa_flash_bwd_least_workspace_bytes", "fa_flash_keep_bits_bytes", "fa_flash_fwd_keep", "fa_flash_bwd_keep",
     "fa_flash_fwd_few_rows", "fa_flash_few_rows_pays", "fa_flash_key_split",
     "fa_flash_bwd_fused", "fa_flash_bwd_fused_stages", "fa_flash_bwd_fused_workspace_bytes", "fa_piecewise_bwd_fused",
     "fa_piecewise_bwd_fused_workspace_bytes",
@@ -147,6 +147,7 @@ PAGED_ARGS = struct.Struct("@9ifP2q2P3q2PqP2q3Pi4x")                # PagedArgs
 _SIGNATURES = {
     "fa_flash_keep_bits_bytes": "p", "fa_flash_fwd_keep": "pppppp" + "plp", "fa_flash_bwd_keep": "p" * 11 + "lplp",
     "fa_flash_fwd": "ppppppp", "fa_flash_fwd_few_rows": "ppppppp", "fa_flash_key_split": "pi", "fa_flash_few_rows_pays": "pi", "fa_flash_bwd": "ppppppppppplp", "fa_flash_bwd_workspace_bytes": "p",
+    "fa_flash_bwd_least_workspace_bytes": "p",
     "fa_piecewise_fwd": "pipppppppp", "fa_paged_decode": "pp", "fa_paged_reduce": "pp", "fa_paged_attention": "piiiip",
     "fa_paged_cache_append": "iiiiippllpplllpp", "fa_splitkv_fwd": "ppppiippp", "fa_splitkv_combine": "pippppp",
     "fa_total_attention": "pppppp", "fa_flash_bwd_delta": "ppppp", "fa_piecewise_bwd_fused_workspace_bytes": "p",

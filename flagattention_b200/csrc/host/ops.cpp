@@ -151,9 +151,17 @@ variable_list flash_backward(const Tensor &q, const Tensor &k, const Tensor &v, 
   void *stream = stream_of(q);
   const float *l = lse.data_ptr<float>();
   if (one_pass()) {
-    const int64_t bytes = fa_flash_bwd_workspace_bytes(&s);
+    int64_t bytes = fa_flash_bwd_workspace_bytes(&s);
     if (bytes > 0) {
-      Tensor ws = at::empty({bytes}, q.options().dtype(at::kByte));
+      const auto u8 = q.options().dtype(at::kByte);
+      Tensor ws;
+      try {
+        ws = at::empty({bytes}, u8);
+      } catch (const c10::OutOfMemoryError &) {   // without room for shared walks, if that is less
+        const int64_t least = fa_flash_bwd_least_workspace_bytes(&s);
+        if (least >= bytes) throw;
+        ws = at::empty({bytes = least}, u8);
+      }
       const int st = fa_flash_bwd(&s, &tq, &tk, &tv, &to, &tdo, l, &tdq, &tdk, &tdv, ws.data_ptr(), bytes, stream);
       if (st != FA_ERR_UNSUPPORTED) {   // a layout the one-pass kernel cannot map goes to the pair below
         check(st, "fa_flash_bwd");

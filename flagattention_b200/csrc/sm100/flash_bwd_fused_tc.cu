@@ -347,15 +347,15 @@ extern "C" int fa_flash_bwd_fused_stages(const fa_flash_shape *s, const fa_tenso
 
 // ---- the whole backward in one call -----------------------------------------------------------
 
-// workspace: that of the one-pass kernel | delta (B, H, M) fp32 | shares of dK and dV
+// workspace: that of the one-pass kernel | delta (B, H, M) fp32 | shares of dK and dV, which a caller may do without
 struct WholeWorkspace {
   int split;
-  int64_t shares, total;
+  int64_t least, shares, total;
 };
 static WholeWorkspace whole_workspace(const fa_flash_shape *s) {
   WholeWorkspace w{};
   w.split = tc::walk_split(s);
-  w.shares = tc::fused_workspace_bytes(s) + (int64_t)s->B * s->H * s->M * 4;
+  w.least = w.shares = tc::fused_workspace_bytes(s) + (int64_t)s->B * s->H * s->M * 4;
   if (w.split > 1) w.shares = (w.shares + 15) / 16 * 16;
   w.total = w.shares + tc::share_bytes(s, w.split);
   return w;
@@ -363,6 +363,10 @@ static WholeWorkspace whole_workspace(const fa_flash_shape *s) {
 extern "C" int64_t fa_flash_bwd_workspace_bytes(const fa_flash_shape *s) {
   if (!s || validate_shape(s) != FA_OK || !tc::one_pass_covered(s)) return 0;
   return whole_workspace(s).total;
+}
+extern "C" int64_t fa_flash_bwd_least_workspace_bytes(const fa_flash_shape *s) {
+  if (!s || validate_shape(s) != FA_OK || !tc::one_pass_covered(s)) return 0;
+  return whole_workspace(s).least;
 }
 
 // Both directions on the tcgen05 kernels, whatever the layout turns out to be
@@ -379,8 +383,9 @@ static int whole_backward(const fa_flash_shape *s, const fa_tensor4 *q, const fa
   if (int st = validate_tensors({q, k, v, o, d_o, dq, dk, dv})) return st;
   if (!lse) return FA_ERR_BAD_ARG;
   if (!tc::one_pass_covered(s)) return FA_ERR_UNSUPPORTED;
-  const WholeWorkspace w = whole_workspace(s);
-  if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 15)) return FA_ERR_WORKSPACE;
+  WholeWorkspace w = whole_workspace(s);
+  if (!workspace || workspace_bytes < w.least || (reinterpret_cast<uintptr_t>(workspace) & 15)) return FA_ERR_WORKSPACE;
+  if (workspace_bytes < w.total) w.split = 1;   // no room for shares: one CTA a key block
   // before the first launch: the caller's other path starts with delta again
   for (const fa_tensor4 *t : {q, d_o, dq})
     if (tc::is_broadcast(t, s->B, s->H, s->M)) return FA_ERR_UNSUPPORTED;

@@ -90,8 +90,13 @@ def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0, keep=Fa
     args = (shape, _C.pack4(q), _C.pack4(k), _C.pack4(v), _C.pack4(o), L.data_ptr())
     stream = _C.raw_stream(q.device)
     bits_bytes = _C.call("fa_flash_keep_bits_bytes")(shape) if keep else 0
+    bits = None
     if bits_bytes:
-        bits = torch.empty(bits_bytes, dtype=torch.uint8, device=q.device)
+        try:
+            bits = torch.empty(bits_bytes, dtype=torch.uint8, device=q.device)
+        except torch.OutOfMemoryError:   # the backward draws them again
+            pass
+    if bits is not None:
         st = _C.call("fa_flash_fwd_keep")(*args, bits.data_ptr(), bits_bytes, stream)
         if st != _C.FA_ERR_UNSUPPORTED:   # a layout for the kernels below
             _C.check(st, "fa_flash_fwd_keep")
@@ -224,7 +229,14 @@ def _backward(q, k, v, o, L, do, causal, sm_scale, mark=None, dropout_p=0.0, see
             # everything in one call: one workspace, one trip through the binding
             ws_bytes = _C.call("fa_flash_bwd_workspace_bytes")(shape)
             if ws_bytes > 0:
-                ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+                try:
+                    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+                except torch.OutOfMemoryError:   # without room for shared walks, if that is less
+                    least = _C.call("fa_flash_bwd_least_workspace_bytes")(shape)
+                    if least >= ws_bytes:
+                        raise
+                    ws_bytes = least
+                    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
                 args = (shape, tq, tk, tv, to, tdo, L.data_ptr(), tdq, tdk, tdv)
                 if bits is None:
                     st = _C.call("fa_flash_bwd")(*args, ws.data_ptr(), ws_bytes, stream)

@@ -172,6 +172,9 @@ int fa_flash_bwd_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_te
  * 0: the shape is not covered, call fa_flash_bwd_delta, fa_flash_bwd_dkdv and fa_flash_bwd_dq).  Same
  * reproducibility, and the same FA_ERR_UNSUPPORTED for broadcast strides, as fa_flash_bwd_fused. */
 int64_t fa_flash_bwd_workspace_bytes(const fa_flash_shape *s);
+/* The least it does with: below the figure above, CTAs do not share the walk of a key block (slower where query heads are
+ * many and kv heads few). */
+int64_t fa_flash_bwd_least_workspace_bytes(const fa_flash_shape *s);
 int fa_flash_bwd(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k,
                  const fa_tensor4 *v, const fa_tensor4 *o, const fa_tensor4 *d_o, const float *lse,
                  const fa_tensor4 *dq, const fa_tensor4 *dk, const fa_tensor4 *dv, void *workspace,

@@ -6,7 +6,7 @@ import torch
 
 import flagattention_b200 as fa
 import oracle
-from flagattention_b200 import _C, flash
+from flagattention_b200 import _C, _native, flash
 from helpers import assert_within_2x, make_qkv
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +80,61 @@ def test_shares_use_their_own_workspace_and_their_dropout():
         want = flash._backward(q, k, v, o, lse, do, True, 0.125, None, 0.25, 11, 7)
     for a, b in zip(got, want):   # both round P, dS and the result to 16 bits
         assert (a.float() - b.float()).norm() <= 4 * 2 ** -11 * b.float().norm()
+
+
+class _memory_left:
+    """`with _memory_left(n)`: at most n bytes beside what is allocated."""
+
+    def __init__(self, n):
+        self.n = n
+
+    def __enter__(self):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + self.n) / total)
+
+    def __exit__(self, *exc):
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        return False
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_walks_are_not_shared_where_memory_is_short(monkeypatch, native):
+    B, H, Hk, L, D = 1, 16, 2, 8192, 128
+    bytes_, shares = _workspace(B, H, Hk, L, L, D, True)
+    least = _C.call("fa_flash_bwd_least_workspace_bytes")(_C.pack_shape(torch.float16, B, H, Hk, L, L, D, True, 0.1))
+    assert shares > 1 and bytes_ - least >= 64 << 20
+    if not native:
+        monkeypatch.setattr(_native, "usable", lambda x: False)
+    q, k, v, do = make_qkv(B, H, Hk, L, L, D, torch.bfloat16, "cuda", seed=1)
+    for x in (q, k, v):
+        x.requires_grad_()
+    run = lambda o: torch.autograd.grad(o, (q, k, v), do)
+    with flash.backward_mode("one_pass"):
+        want = run(fa.flash_attention(q, k, v, True))
+        o = fa.flash_attention(q, k, v, True)
+        grads = 2 * q.numel() + 4 * k.numel()
+        with _memory_left(least + grads + (40 << 20)):   # (the allocator's segments: 20 MB)
+            got = run(o)
+    for a, b in zip(got, want):   # other sums in fp32, each rounded to 16 bits once
+        assert (a.float() - b.float()).norm() <= 2 * 2 ** -8 * b.float().norm()
+
+
+def test_decisions_are_drawn_again_where_memory_is_short():
+    B, H, L, D = 1, 32, 4096, 128
+    q, k, v, do = make_qkv(B, H, H, L, L, D, torch.bfloat16, "cuda", seed=2)
+    for x in (q, k, v):
+        x.requires_grad_()
+    kept = _C.call("fa_flash_keep_bits_bytes")(_C.pack_shape(torch.bfloat16, B, H, H, L, L, D, True, 0.1, 0.2))
+    assert kept >= 64 << 20
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t.shape) or t, lambda t: t):
+        torch.cuda.manual_seed(4)
+        want = torch.autograd.grad(fa.flash_attention(q, k, v, True, dropout_p=0.2), (q, k, v), do)
+        with _memory_left(2 * q.numel() + (30 << 20)):
+            torch.cuda.manual_seed(4)
+            o = fa.flash_attention(q, k, v, True, dropout_p=0.2)
+    assert len(saved) == 6 + 5
+    got = torch.autograd.grad(o, (q, k, v), do)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
