@@ -100,7 +100,7 @@ int fa_splitkv_combine(const fa_flash_shape *s, int32_t num_splits, const float 
  * calls of at least 32 queries on the tcgen05 kernels.  FA_ERR_UNSUPPORTED, before anything is launched, elsewhere. */
 int fa_flash_fwd_few_rows(const fa_flash_shape *s, const fa_tensor4 *q, const fa_tensor4 *k, const fa_tensor4 *v,
                           const fa_tensor4 *o, float *lse, void *stream);
-/* Whether that is the faster form, by a rule on the shape, for a call whose keys fa_num_splits_heuristic() splits on a
+/* Whether that is the faster form, by a rule on the shape, for a call whose keys the split-count heuristic below splits on a
  * GPU of num_sms SMs; host-only, no CUDA call. */
 int32_t fa_flash_few_rows_pays(const fa_flash_shape *s, int32_t num_sms);
 /* Bytes of o_partial + lse_partial for a given problem (host-only helper). */
