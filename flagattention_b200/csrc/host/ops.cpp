@@ -215,31 +215,27 @@ bool decode_covered(const Tensor &q, const Tensor &k, const Tensor &v, bool caus
   return sl > 0 && sl % 8 == 0 && k.stride(1) % 8 == 0 && k.stride(0) % (16 * sl) == 0;
 }
 
-// flash._decode_forward()
-Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double scale, bool causal) {
-  const int64_t B = q.size(0), H = q.size(1), M = q.size(2), D = q.size(3), Hk = k.size(1), N = k.size(2);
+// flash._decode_forward() for one query a head
+Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double scale) {
+  const int64_t B = q.size(0), H = q.size(1), D = q.size(3), Hk = k.size(1), N = k.size(2);
   const int64_t sb = k.stride(0), sl = k.stride(2);
   int64_t partition = coarsen_partition(256, B * Hk, N, sm_count(), 4096);
   if (N <= partition) partition = 0;
-  // the M queries of a head go in as M "query heads" of its kv head: rows one stride apart
-  Tensor rows;
-  int64_t row_stride = M == 1 ? q.stride(1) : q.stride(2), seq_stride = q.stride(0);
-  if ((M > 1 && H > 1 && q.stride(1) != M * q.stride(2)) || row_stride % 8 || seq_stride % 8)
-    rows = q.contiguous(), row_stride = D, seq_stride = H * M * D;
-  Tensor o = new_like(q), ws;
+  Tensor rows, o = new_like(q), ws;
+  int64_t row_stride = q.stride(1), seq_stride = q.stride(0);
+  if (row_stride % 8 || seq_stride % 8) rows = q.contiguous(), row_stride = D, seq_stride = H * D;   // of a size of one
   fa_paged_args a{};
   dtype_code(q, &a.dtype);
-  a.num_seqs = (int32_t)B, a.num_q_heads = (int32_t)(H * M), a.num_kv_heads = (int32_t)Hk, a.head_size = (int32_t)D;
+  a.num_seqs = (int32_t)B, a.num_q_heads = (int32_t)H, a.num_kv_heads = (int32_t)Hk, a.head_size = (int32_t)D;
   a.block_size = 16, a.max_context_len = (int32_t)N, a.block_table_is_i64 = FA_BLOCK_TABLE_IN_PLACE;
   a.partition_size = (int32_t)partition, a.attn_scale = (float)scale;
   a.query = (rows.defined() ? rows : q).data_ptr(), a.q_stride_s = seq_stride, a.q_stride_h = row_stride;
   a.key_cache = k.data_ptr(), a.value_cache = v.data_ptr();
   a.kv_stride_b = 16 * sl, a.kv_stride_h = Hk > 1 ? k.stride(1) : 0, a.kv_stride_t = sl;
   a.bt_stride_s = sb / (16 * sl);
-  a.out = o.data_ptr(), a.o_stride_s = H * M * D, a.o_stride_h = D;
-  a.causal_rows = causal && M > 1 ? (int32_t)M : 0;
+  a.out = o.data_ptr(), a.o_stride_s = H * D, a.o_stride_h = D;
   if (partition) {
-    const int64_t n = B * H * M, P = (N + partition - 1) / partition, stats = (n * P + 63) / 64 * 64;
+    const int64_t n = B * H, P = (N + partition - 1) / partition, stats = (n * P + 63) / 64 * 64;
     ws = at::empty({n * P * D + 2 * stats}, q.options().dtype(at::kFloat));
     a.part_out = ws.data_ptr<float>();
     a.part_max = a.part_out + n * P * D;
@@ -254,10 +250,12 @@ Tensor decode_forward(const Tensor &q, const Tensor &k, const Tensor &v, double 
 bool head_dim_built(int64_t D) { return D == 16 || D == 32 || D == 64 || D == 128; }
 
 // o, or an undefined tensor.  `rest`: the calls that the usual form leaves, since their views need a copy or their few
-// queries are for the split-KV kernels.  (Refused calls pay for both forms: a view or a split call took 58 us where the Python
+// queries are for the split-KV kernels.  `few`: set, with no o, for a step of 2 to 16 queries a head that the decode kernels
+// take: flash._decode_forward() launches those.  (Refused calls pay for both forms: a view or a split call took 58 us where the Python
 // form alone takes 38 and this one 12.)
 Tensor flash(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, bool causal, bool default_scale, double scale,
-             bool rest) {
+             bool rest, bool *few) {
+  *few = false;
   if (!q_in.is_cuda() || !usual_surroundings()) return {};
   const int device = c10::cuda::current_device();
   if (!plain(q_in, device) || !plain(k_in, device) || !plain(v_in, device)) return {};
@@ -281,8 +279,10 @@ Tensor flash(const Tensor &q_in, const Tensor &k_in, const Tensor &v_in, bool ca
   const bool grads = q_in.requires_grad() || k_in.requires_grad() || v_in.requires_grad();
   const int64_t splits =
       fa_num_splits_heuristic((int32_t)B, (int32_t)H, (int32_t)M, (int32_t)N, 16, 128, sm_count(), 128);
-  if (M <= 16 && !grads && (M == 1 || splits > 1) && decode_covered(q, k, v, causal))
-    return decode_forward(q, k, v, scale, causal);
+  if (M <= 16 && !grads && (M == 1 || splits > 1) && decode_covered(q, k, v, causal)) {
+    *few = M > 1;
+    return *few ? Tensor() : decode_forward(q, k, v, scale);
+  }
   bool clusters = false;
   if (splits > 1) {
     const fa_flash_shape s = shape_of(q, k, causal, scale);
@@ -570,10 +570,12 @@ PyObject *py_flash(PyObject *, PyObject *const *args, Py_ssize_t n) {
   double scale = 0;
   if (n != 5 || !tensors(args, 3, t) || !truth(args[3], &causal) || !scale_of(args[4], &is_default, &scale)) Py_RETURN_NONE;
   Tensor o;
+  bool few;
   {
     pybind11::gil_scoped_release release;
-    o = flash(*t[0], *t[1], *t[2], causal, is_default, scale, REST);
+    o = flash(*t[0], *t[1], *t[2], causal, is_default, scale, REST, &few);
   }
+  if (few) Py_RETURN_FALSE;
   return wrap_or_none(o);
   END_HANDLE_TH_ERRORS
 }

@@ -389,6 +389,9 @@ def attention(q, k, v, causal=False, sm_scale=None, dropout_p=0.0,
         o = native.flash(q, k, v, causal, sm_scale)
         if o is None:   # a view that needs a copy, or keys for the split-KV kernels; else the form below
             o = native.flash_rest(q, k, v, causal, sm_scale)
+        if o is False:   # 2 to 16 queries a head, for the decode kernels
+            return _decode_forward(_C.kernel_ready(q), _C.kernel_ready(k), _C.kernel_ready(v),
+                                   1. / math.sqrt(q.shape[-1]) if sm_scale is None else sm_scale, causal)
         if o is not None:
             return o
     return FlashAttention.apply(q, k, v, causal, sm_scale, dropout_p, return_log_normalizer,
