@@ -103,7 +103,8 @@ static int launch_fwd_tc(const fa_flash_shape *s, int w, const fa_tensor4 *q, co
   }
   // the CTAs of a (batch, head) pair share its K and V (and K2 under piecewise), with those of its group's heads
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
-  p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal);
+  p.group_size = forward_group_size((int64_t)s->N * D * 2 * (PW ? 3 : 2) * s->Hk / s->H, s->B * s->H, s->causal,
+                                    p.num_m_blocks, D == 128);
   const int64_t tiles = (int64_t)p.num_m_blocks * s->B * s->H;
   p.split = DROP || one_cta_per_tile_forced() ? 1 : key_split(s, sm_count_of_device()).ctas;
   if constexpr (!DROP) {
@@ -183,7 +184,8 @@ static int launch_fwd_persist(const fa_flash_shape *s, const fa_tensor4 *q, cons
   p.status = device_status_word();
   p.d = s->D;
   p.num_m_blocks = (s->M + C::BM - 1) / C::BM;
-  p.group_size = forward_group_size((int64_t)s->N * D * 2 * 2 * s->Hk / s->H, s->B * s->H, s->causal);
+  p.group_size = forward_group_size((int64_t)s->N * D * 2 * 2 * s->Hk / s->H, s->B * s->H, s->causal,
+                                    p.num_m_blocks, D == 128);
   const int64_t items = (int64_t)p.num_m_blocks * s->B * s->H;
   const int sms = sm_count_of_device();
   fp.sched = fwd_sched_slot();

@@ -130,11 +130,17 @@ inline int cta_group_size(int64_t hot_bytes_per_pair, int npairs) {
 // B=2 H=32 M=1627 N=2855 142 -> 148 (94 MB), B=2 H=32 L=4096 278 -> 311 (134 MB); backward B=3 H=32 Hk=8 L=1867 381 -> 321 (360
 // blocks), H=32 Hk=8 L=8192 1871 -> 1383 (512), H=16 L=6144 493 -> 409 (768), B=2 H=32 Hk=16 L=4096 840 -> 762 (1024),
 // B=4 H=32 L=1024 197 -> 203 (1024, 128 pairs), H=24 L=8192 1099 -> 1079 (1536), B=2 H=32 L=4096 760 -> 845 (2048).
+// At D=64: forward B=2 H=20 L=4096 160 -> 135, B=3 H=32 Hk=8 L=1867 88 -> 82, B=4 H=32 L=1024 46.3 -> 43.5, H=24 L=8192
+// 346 -> 307, 500 pairs of 330 39.1 -> 36.9; backward H=16 L=6144 244 -> 218, H=32 Hk=8 L=8192 954 -> 752, B=2 H=32 Hk=16
+// L=4096 425 -> 416.
+// Walks of a few blocks at head_dim 128 (`wide`) have little tail to gain and bear 64 MB: forward, 250 pairs of 672 63.2 ->
+// 65.3, 512 of 300 48.2 -> 50.1, 500 of 330 50.3 -> 51.2; but 192 of 672 (63 MB) 52.1 -> 49.9, 70 of 672 28.1 -> 24.6.
 inline bool one_group_in_l2(int64_t hot_bytes_per_pair, int npairs, bool causal) {
   return causal && hot_bytes_per_pair * npairs <= 88ll << 20;
 }
-inline int forward_group_size(int64_t hot_bytes_per_pair, int npairs, bool causal) {
-  if (one_group_in_l2(hot_bytes_per_pair, npairs, causal)) return npairs > 0 ? npairs : 1;
+inline int forward_group_size(int64_t hot_bytes_per_pair, int npairs, bool causal, int blocks, bool wide) {
+  const bool too_much = wide && blocks <= 6 && hot_bytes_per_pair * npairs > 64ll << 20;
+  if (!too_much && one_group_in_l2(hot_bytes_per_pair, npairs, causal)) return npairs > 0 ? npairs : 1;
   return cta_group_size(hot_bytes_per_pair, npairs);
 }
 inline int backward_group_size(int64_t hot_bytes_per_pair, int npairs, int64_t blocks, int sms, bool causal) {

@@ -32,6 +32,18 @@ def test_every_block_is_visited_once(B, H, Hk, M, N, D, causal):
         assert_within_2x(x, r, t, name)
 
 
+@pytest.mark.parametrize("pairs,N", [(192, 672), (200, 672), (512, 300)])
+def test_forward_of_many_short_walks(pairs, N):
+    """Around 64 MB of keys and values in walks of at most 6 blocks: one group and groups, the same bits as a call for some
+    of the heads alone."""
+    q, k, v, _ = make_qkv(1, pairs, pairs, N, N, 128, torch.float16, "cuda", seed=pairs)
+    with _C.kernel_family("one_cta_per_tile"):
+        o = fa.flash_attention(q, k, v, True)
+        for h in (0, 33, pairs - 40):   # (40: fewer would go to the split-KV kernels)
+            some = slice(h, h + 40)
+            assert torch.equal(o[:, some], fa.flash_attention(q[:, some], k[:, some], v[:, some], True)), h
+
+
 @pytest.mark.parametrize("H,N", [(22, 8192), (23, 8192)])
 def test_forward_at_the_l2_line(H, N):
     """22 x 8192 keys at head_dim 128 are 88 MiB and one group, 23 heads go in groups of 8: the same bits as a call
