@@ -13,7 +13,7 @@
 //   warp 1       MMA issuer (one thread); every MMA is 128 x 128 x 16 (128 x 64 x 16 at D = 64)
 //   warp 2       stages lse / delta of every tile in shared memory (warp 3 idles)
 //   warps 4..7   dQ reduction: TMEM -> shared-memory staging -> cp.reduce.async.bulk
-//   warps 8..23  element-wise stage, one thread per (accumulator row, 32 columns)
+//   warps 8..23  element-wise stage, 32 keys x 32 queries a warp, held as matrix fragments (4 keys x 8 queries a thread)
 //
 // TMEM (512 columns):  S^T, then dP^T (128) | dQ (D), P^T over its first 64 columns | dK | dV.
 //   The two score products of a tile share one 128-column region: dP^T is issued as soon as the
@@ -195,7 +195,8 @@ struct FusedItem {
 // about 90 us of the 194 the first of them has come to since; read, the whole training call takes 363 -> 279 us.
 // The drawing does not fit the registers beside the rest: 76 and 180 bytes of spill stores and loads a thread at 64,
 // 32 and 32 at 128 (without dropout 48 and 188, and 12 and 92).
-// SPLIT = fp.split CTAs share the walk of a key block.
+// SPLIT = fp.split CTAs share the walk of a key block.  The item's divisions and the shares' 64-bit addresses add to the
+// spills: 64 and 240 bytes a thread at 64, 72 and 212 at 128, with dropout 84 and 264, and 88 and 232.
 template <typename T, int D, bool DROP, bool SPLIT>
 __global__ void __launch_bounds__(kFusedThreads, 1)
     flash_bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -375,7 +376,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         int sq = 0, phq = 1, sd = 0, phd = 1;   // ring slot and the "free" parity to wait for
         int inflight_q = 0, inflight_do = 0;    // loads requested (for the drain after an abort)
         int real = 0;                           // items with tiles handled so far
-        uint32_t gt = 0;                        // tiles of those items
         bool pending = false;                   // dV / dK of the previous such item not stored yet
         int pn0 = 0, phk = 0, pb = 0;           // its coordinates,
         int pmode = 0;                          // its walk
@@ -491,7 +491,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
               if (++mt == it.mt_hi) mt = it.mt_lo, ++h;
             }
             if (!ok) break;
-            gt += (uint32_t)it.T_tiles;
             // K and V of the next item are read by nobody else: start them towards L2 now, a couple
             // of tiles before this item ends (any earlier and they would be evicted again)
             if (w_next < end_id) {
@@ -718,7 +717,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     // dQ(t) = dS K is a complete 128 x D product per tile.  These four warps (one per TMEM lane
     // slice = 32 query rows) move it out of TMEM 32 columns at a time into a
     // shared-memory staging buffer, from where the copy engine adds it to the fp32 workspace
-    // (`cp.reduce.async.bulk`, 2 KB runs).  An SM retires fp32 reductions at about 26 bytes per
+    // (`cp.reduce.async.bulk`, one run of 16 KB a part).  An SM retires fp32 reductions at about 26 bytes per
     // clock whoever issues them, so the 64 KB of a tile take about as long as its GEMMs; issued
     // as `red` instructions they fill the load/store queue and stall every warp of the SM that
     // shuffles or touches shared memory.  Two staging buffers: one part drains while the next

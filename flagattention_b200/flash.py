@@ -75,8 +75,8 @@ def get_fwd_config(B, H, M, N, D, causal):
 
 
 def get_bwd_config(B, H, M, N, D, causal):
-    """Counterpart of src/flag_attn/flash.py:493-519; informational only."""
-    return (128, 128, 3, 18)
+    """Counterpart of src/flag_attn/flash.py:493-519, for the one-pass kernel; informational only."""
+    return (128, 128, 2 if D == 128 else 3, 24)
 
 
 def _forward(q, k, v, causal, sm_scale, dropout_p=0.0, seed=0, offset=0, keep=False):
@@ -138,9 +138,11 @@ def _identity_block_table(B, blocks_per_batch, id_stride, device):
     return tab, torch.full((B,), blocks_per_batch * 16, dtype=torch.int32, device=device)
 
 
-# Elements of the attention matrix from which the forward keeps its dropout decisions for the backward.  Drawing them again
-# takes about 1.4 us a million on the GPU, keeping them 15 us of host work, which bounds smaller calls: forward and backward
-# in all, p = 0.1, B=14 H=16 L=191 D=128 (8 M) 180 us drawn and 195 kept, B=16 H=16 L=512 D=64 (67 M) 363 and 279.
+# Elements of the attention matrix from which the forward keeps its dropout decisions for the backward.  On the GPU keeping
+# is the faster at every size (4 M 55 us kept and 70 drawn, 16.8 M 110 and 140, forward and backward at D=64, p = 0.1, not
+# causal), but it takes 5 to 8 us of host work, which bounds a call up to about 20 M, causal 40 M.  A call in a loop, us
+# kept / drawn: 8.4 M 187 / 179, 16.8 M 183 / 182, 25 M 185 / 209, 33.6 M 192 / 217, 67 M 281 / 370; causal at D=128
+# 16.8 M 186 / 182, 33.5 M 182 / 177, 67 M 207 / 263.  The line lies between the two crossings.
 _KEEP_BITS_FROM = 1 << 25
 
 _DECODE_MAX_ROWS = 64   # query rows (group x queries) per kv head the gather kernel is given
