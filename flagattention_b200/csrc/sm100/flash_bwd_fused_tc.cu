@@ -51,15 +51,6 @@ static int64_t share_bytes(const fa_flash_shape *s, int split) {
   return (int64_t)split * 2 * s->B * s->Hk * (((int64_t)s->N + 127) / 128 * 128) * fused_padded_dim(s) * 4;
 }
 
-// one persistent CTA per SM
-static int sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-    return 0;
-  return n;
-}
-
 // CTAs that share the walk of a key block (1, 2, 4 or 8): a call of a few kv heads with many query heads each is as slow as
 // its longest walk, whatever the other SMs do.  Estimated in tiles (2.2 us at head_dim 128): an item costs 2 beside its
 // walk, 6 where it leaves a share (128 KB of fp32), the combining launch 4 and its bytes; with more items than SMs a
@@ -73,7 +64,7 @@ static int sm_count() {
 //   H=8 Hk=8 L=2048 (128, 16)            70 /   86 /  107 /  146
 //   H=4 Hk=1 L=512 D=64 (4, 16)          60 /   63 /   63 /   63
 static int walk_split(const fa_flash_shape *s) {
-  const int sms = sm_count();
+  const int sms = sm_count_of_device();
   const int64_t blocks = ((int64_t)s->N + 127) / 128, rows = ((int64_t)s->M + 127) / 128, items = blocks * s->B * s->Hk;
   if (sms <= 0 || items > 2ll * sms) return 1;
   const double longest = (double)rows * (s->H / s->Hk);
@@ -203,7 +194,7 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
     // the CTAs of a (batch, kv head) pair share its Q and dO tiles and its slice of the dq workspace
     p.num_blocks = (s->N + C::BN - 1) / C::BN;
     const int64_t blocks = (int64_t)p.num_blocks * s->Hk * s->B, items = blocks * split;
-    const int sms = sm_count();
+    const int sms = sm_count_of_device();
     if (items > 0x3fffffff) return FA_ERR_TOO_LARGE;
     if (sms <= 0) return FA_ERR_LAUNCH;
     p.group_size = backward_group_size((int64_t)(s->H / s->Hk) * s->M * D * 8 * n_acc, s->B * s->Hk, blocks, sms,
@@ -224,7 +215,7 @@ static int launch_fused(const fa_flash_shape *s, const fa_tensor4 *q, const fa_t
     if (int st = zero_rows(dk, far ? 1 : 0)) return st;
     if (far)
       if (int st = zero_rows(dk2, 2)) return st;
-    // persistent: a CTA takes key block `blockIdx.x`, then blocks handed out by the counter
+    // persistent, one CTA per SM: a CTA takes key block `blockIdx.x`, then blocks handed out by the counter
     dim3 grid((unsigned)(items < sms ? items : sms), 1, 1);
     kern<<<grid, kFusedThreads, C::kTotal, stream>>>(mq, mdo, mk, mv, mdk, mdv, mq2, mk2, mdk2, fp);
     FA_CHECK_LAUNCH();
